@@ -359,8 +359,8 @@ def run_ours(args):
             tj = json.load(open(tp))
             if tj.get("grid") == list(W["grid"]):
                 trc = int(nb * tj["dram_bytes_per_kpoint"])
-        roof = {"bound": "hbm", "kernel": f"FP32 CG iteration = plane_inv<IN_CG> + pencil<PEN_QBQ_CG> + "
-                                          f"plane_fwd<EPI_CGR> + cg_decide over a batch of {nb} k-points",
+        roof = {"bound": "hbm", "kernel": f"FP32 CG iteration = plane_cg + cg_decide + pencil<PEN_QBQ_CG> over a "
+                                          f"batch of {nb} k-points",
                 "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s", "frac": round(ach / hbm, 4),
                 "peak_source": src, "traffic": trc, "algorithmic_bytes": algc, "batch": nb,
                 "ms_per_launch": round(msc, 5), "us_per_kpoint": round(msc * 1e3 / nb, 2),
@@ -441,18 +441,18 @@ def cg_iter_bytes(N):
     B_QBQ = (2M + 6N).s + 3N.r: the operator's vector in and out, the field out of Q_r
     and into Q_r^* (one read and one write of the 3-component field per 3-D transform),
     1/eps, and the CG vectors (read r, p, x, Ap; write x, r, p), s = 8, r = 4.  The
-    kernels move a different set: Ap never reaches memory, but the field makes one
-    more round trip between the plane and pencil stages (cg_stage_bytes)."""
+    kernels move a different set (cg_stage_bytes): r, r_old, x, x_old for r, p, x, Ap, two of
+    them written instead of three, and one more round trip of the field between the stages."""
     M = 2 * N
     return (2 * M + 6 * N) * 8 + 3 * N * 4 + 7 * M * 8
 
 
 def cg_stage_bytes(N):
-    """Bytes each fused FP32 CG kernel moves per k-point: plane_inv reads r, p, x and
-    writes p, x and the 3-component field; the pencil stage reads and writes the field
-    and reads 1/eps; plane_fwd reads the field and reads and writes r."""
+    """Bytes each FP32 CG kernel moves per k-point: plane_cg reads and writes the
+    3-component field, reads r, r_old, x, x_old and writes r' and x'; k_cg_decide moves the
+    partial sums (left out); the pencil stage reads and writes the field and reads 1/eps."""
     M = 2 * N
-    return [5 * M * 8 + 3 * N * 8, 6 * N * 8 + 3 * N * 4, 3 * N * 8 + 2 * M * 8]
+    return [6 * N * 8 + 6 * M * 8, 0, 6 * N * 8 + 3 * N * 4]
 
 
 def apply_options(ctx, args):

@@ -95,6 +95,13 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+// one real value
+__device__ __forceinline__ void cp_async_real(float* smem, const float* gmem) { cp_async4(smem, gmem); }
+__device__ __forceinline__ void cp_async_real(double* smem, const double* gmem) { cp_async8(smem, gmem); }
 // one element of 8 or 16 bytes
 template <typename T> __device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
   static_assert(sizeof(T) == 8 || sizeof(T) == 16, "8- or 16-byte elements");

@@ -13,9 +13,8 @@
 // A "tile" holds `nl` lines of length n; element m of line l sits at
 // buf[l*ls + m*es].  Every pass is register staged: each thread reads all inputs
 // of its butterflies, the block synchronises, then every thread writes, so the
-// transform runs in place in one shared buffer.  Radices 2,3,4,5,7,8 (and odd
-// 11, 13 through the symmetric-pair DFT) use butterflies; any other factor (a
-// large prime such as 23 or 107) uses a register-blocked symmetric-pair DFT pass
+// transform runs in place in one shared buffer.  Radices 2 to 13 use butterflies (5, 7, 11
+// and 13 through the symmetric-pair DFT); any other factor (a large prime such as 23 or 107) uses a register-blocked symmetric-pair DFT pass
 // (prime_pass), or an output-stationary pass where each thread forms its outputs
 // as length-R sums when a line needs more threads than the block has.
 #pragma once
@@ -251,6 +250,60 @@ template <typename R> struct Dft<R, 12> {
   }
 };
 
+// Radices 6 = 2 x 3 and 10 = 2 x 5, prime-factor DFTs like radix 12: input n = (N2 n1 + N1 n2)
+// mod N, output k by the Chinese remainder map (k = 3 k1 + 4 k2 mod 6, 5 k1 + 6 k2 mod 10).
+template <typename R, int H, int C> struct Dft2xH {
+  __device__ __forceinline__ static void run(cplx<R>* a, bool inv) {
+    cplx<R> y[2][H];
+#pragma unroll
+    for (int n1 = 0; n1 < 2; n1++) {
+#pragma unroll
+      for (int n2 = 0; n2 < H; n2++) y[n1][n2] = a[(H * n1 + 2 * n2) % (2 * H)];
+      Dft<R, H>::run(y[n1], inv);
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < H; k2++) {
+      cplx<R> z[2] = {y[0][k2], y[1][k2]};
+      Dft<R, 2>::run(z, inv);
+      a[(C * k2) % (2 * H)] = z[0];
+      a[(H + C * k2) % (2 * H)] = z[1];
+    }
+  }
+};
+template <typename R> struct Dft<R, 6> : Dft2xH<R, 3, 4> {};
+template <typename R> struct Dft<R, 10> : Dft2xH<R, 5, 6> {};
+
+// Radix 9 = 3 x 3 (Cooley-Tukey) with the inner twiddles e^{-/+ 2 pi i m / 9}, m = 1, 2, 4.
+template <typename R> struct Dft<R, 9> {
+  __device__ __forceinline__ static cplx<R> tw(cplx<R> a, R c, R s, bool inv) {
+    // a e^{-i phi} (forward) or a e^{+i phi} (inverse)
+    return inv ? mk<R>(a.x * c - a.y * s, a.x * s + a.y * c) : mk<R>(a.x * c + a.y * s, a.y * c - a.x * s);
+  }
+  __device__ __forceinline__ static void run(cplx<R>* a, bool inv) {
+    cplx<R> y[3][3];  // [n2][k1]
+#pragma unroll
+    for (int n2 = 0; n2 < 3; n2++) {
+#pragma unroll
+      for (int n1 = 0; n1 < 3; n1++) y[n2][n1] = a[3 * n1 + n2];
+      Dft<R, 3>::run(y[n2], inv);
+    }
+    const R c1 = (R)0.76604444311897803520, s1 = (R)0.64278760968653932632;   // 2 pi / 9
+    const R c2 = (R)0.17364817766693034885, s2 = (R)0.98480775301220805937;   // 4 pi / 9
+    const R c4 = (R)-0.93969262078590838405, s4 = (R)0.34202014332566873304;  // 8 pi / 9
+    y[1][1] = tw(y[1][1], c1, s1, inv);
+    y[1][2] = tw(y[1][2], c2, s2, inv);
+    y[2][1] = tw(y[2][1], c2, s2, inv);
+    y[2][2] = tw(y[2][2], c4, s4, inv);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; k1++) {
+      cplx<R> z[3] = {y[0][k1], y[1][k1], y[2][k1]};
+      Dft<R, 3>::run(z, inv);
+#pragma unroll
+      for (int k2 = 0; k2 < 3; k2++) a[k1 + 3 * k2] = z[k2];
+    }
+  }
+};
+
 // Odd radix via symmetric pairs: X_t = a0 + sum_s c(ts) (a_s + a_{R-s})
 //                                       -/+ i sum_s s(ts) (a_s - a_{R-s}).
 template <typename R, int RAD> struct DftOdd {
@@ -305,58 +358,67 @@ struct Div {
   __device__ __forceinline__ unsigned q(unsigned n) const { return d == 1 ? n : __umulhi(n, m); }
 };
 
-// One radix-RAD Stockham pass over all lines, in place.  Every round stages the
-// butterflies of G complete lines in registers (read all, barrier, write all,
-// barrier): a line's outputs overwrite positions other butterflies of the same
-// line still read, so a line never spans two rounds.  Thread t works on line
-// l0 + t mod G and butterflies j = t / G + jstep * q (q < MAXB), with jstep * MAXB
-// >= n / RAD; consecutive threads touch consecutive lines.
+// One radix-RAD Stockham pass over all lines, in place.  The butterflies of G complete
+// lines are one round (read all, barrier, write all, barrier): a line's outputs
+// overwrite positions other butterflies of the same line still read, so a line never
+// spans two rounds.  The round's G * n / RAD butterflies are dealt to the threads one by
+// one, lines fastest (thread t takes t, t + T, ...; at most MAXB each), so consecutive
+// threads touch consecutive lines and at most the last deal of a round has idle threads.
+// G is the largest line count that T * MAXB butterflies cover, evened out over the rounds.
 template <typename R, int RAD, int MAXB>
 __device__ __forceinline__ void stockham_pass(cplx<R>* buf, int n, int Ns, LineSet L, const cplx<R>* tw,
                                               bool inv) {
   const int T = blockDim.x;
   const int nb = n / RAD;
   const int stw = n / (Ns * RAD);
-  const int per_line = (nb + MAXB - 1) / MAXB;  // threads one line needs
-  const int G = min(L.nl, max(1, T / per_line));
+  const int gmax = max(1, (T * MAXB) / nb);
+  const int rounds = (L.nl + gmax - 1) / gmax;
+  const int G = (L.nl + rounds - 1) / rounds;
   const Div dg(G), dns(Ns);
+  const int items = G * nb;
   const int t = threadIdx.x;
-  const int j0 = (int)dg.q(t);
-  const int lt = t - j0 * G;
-  const int jstep = T / G;
   for (int l0 = 0; l0 < L.nl; l0 += G) {
-    const int l = l0 + lt;
-    const bool live = j0 < jstep && l < L.nl;
-    cplx<R>* base = buf + l * L.ls;
     cplx<R> v[MAXB][RAD];
     int dst[MAXB];
+    // (every value is defined on every path: left undefined for idle threads, the values of all
+    // twelve radices stayed live around the loop over the passes, 1.3 KB of spills per thread)
+#pragma unroll
+    for (int q = 0; q < MAXB; q++)
+#pragma unroll
+      for (int u = 0; u < RAD; u++) v[q][u] = mk<R>(0, 0);
 #pragma unroll
     for (int q = 0; q < MAXB; q++) {
-      const int j = j0 + jstep * q;
+      const int i = t + q * T;
+      const int j = (int)dg.q(i);
+      const int l = l0 + i - j * G;
       dst[q] = -1;
-      if (live && j < nb) {
+      if (i < items && l < L.nl) {
         const int jb = (int)dns.q(j);
         const int k = j - jb * Ns;
+        const cplx<R>* src = buf + l * L.ls + j * L.es;
+        const int step = nb * L.es;
 #pragma unroll
-        for (int u = 0; u < RAD; u++) {
-          cplx<R> a = base[(j + u * nb) * L.es];
-          if (u > 0 && k > 0) {
-            cplx<R> w = tw[u * k * stw];
+        for (int u = 0; u < RAD; u++) v[q][u] = src[u * step];
+        if (k > 0) {
+          const int kt = k * stw;
+#pragma unroll
+          for (int u = 1; u < RAD; u++) {
+            cplx<R> w = tw[u * kt];
             if (inv) w.y = -w.y;
-            a = cmul(a, w);
+            v[q][u] = cmul(v[q][u], w);
           }
-          v[q][u] = a;
         }
         Dft<R, RAD>::run(v[q], inv);
-        dst[q] = (jb * Ns * RAD + k) * L.es;
+        dst[q] = l * L.ls + (jb * Ns * RAD + k) * L.es;
       }
     }
     __syncthreads();
+    const int ostep = Ns * L.es;
 #pragma unroll
     for (int q = 0; q < MAXB; q++) {
       if (dst[q] >= 0) {
 #pragma unroll
-        for (int u = 0; u < RAD; u++) base[dst[q] + u * Ns * L.es] = v[q][u];
+        for (int u = 0; u < RAD; u++) buf[dst[q] + u * ostep] = v[q][u];
       }
     }
     __syncthreads();
@@ -388,6 +450,7 @@ __device__ __forceinline__ void generic_pass(cplx<R>* buf, int n, int r, int Ns,
     for (int q = 0; q < MAXE; q++) {
       const int o = o0 + ostep * q;
       dst[q] = -1;
+      v[q] = mk<R>(0, 0);
       if (live && o < n) {
         const int k = o % Ns;
         const int u = (o / Ns) % r;
@@ -552,54 +615,52 @@ __device__ __forceinline__ bool prime_pass(cplx<R>* buf, int n, int r, int Ns, L
   return true;
 }
 
+// outputs x lines a thread accumulates in the prime pass
 template <typename R> struct PrimeBlock;
 template <> struct PrimeBlock<float> { static constexpr int mu = 4, ml = 3; };
 template <> struct PrimeBlock<double> { static constexpr int mu = 2, ml = 2; };
 
-// Passes for radix 7, 11, 13 (LEVEL >= 1) and primes >= 17 (LEVEL 2).
-template <typename R, int EMAX, int LEVEL>
-__device__ __forceinline__ void rare_pass(cplx<R>* buf, int n, int r, int Ns, LineSet L, const cplx<R>* tw,
-                                       bool inv) {
-  switch (r) {
-    case 7: stockham_pass<R, 7, (EMAX / 7 > 0 ? EMAX / 7 : 1)>(buf, n, Ns, L, tw, inv); break;
-    case 11: stockham_pass<R, 11, 1>(buf, n, Ns, L, tw, inv); break;
-    case 13: stockham_pass<R, 13, 1>(buf, n, Ns, L, tw, inv); break;
-    default:
-      if constexpr (LEVEL >= 2) {
-        if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml>(buf, n, r, Ns, L, tw, inv))
-          generic_pass<R, EMAX>(buf, n, r, Ns, L, tw, inv);
-      }
-      break;
-  }
-}
+// Butterflies of radix r a thread stages per round when it holds at most emax elements.
+constexpr int pass_maxb(int emax, int r) { return emax / r > 0 ? emax / r : 1; }
 
-// Full transform of all lines along one axis.  RARE selects the passes compiled
-// in beyond radix 2, 3, 4, 5, 8: none (0), radix 7, 11, 13 (1), and also primes
-// >= 17 (2).  They are register hungry, so each grid runs the lowest level its
-// axis plans need (plan_level; the host picks the instantiation).  EMAX bounds
-// the elements a thread stages in registers per round.
+// Full transform of all lines along one axis.  RARE >= 2 compiles the passes for prime
+// factors >= 17 in; they are register hungry, so each stage kernel exists with and
+// without them and the host picks by its axes (plan_level).  EMAX bounds the elements
+// a thread stages in registers per round.
 template <typename R, int EMAX, int RARE>
-__device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPlan P, LineSet L, const cplx<R>* tw,
+__device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPlan& P, LineSet L, const cplx<R>* tw,
                                           bool inv) {
   const int n = P.n;
-  constexpr int MB5 = EMAX / 5 > 2 ? 2 : (EMAX / 5 > 0 ? EMAX / 5 : 1);
   int Ns = 1;
+#pragma unroll 1
   for (int p = 0; p < P.npass; p++) {
     const int r = P.radix[p];
     switch (r) {
-      case 2: stockham_pass<R, 2, EMAX / 2>(buf, n, Ns, L, tw, inv); break;
-      case 3: stockham_pass<R, 3, EMAX / 3>(buf, n, Ns, L, tw, inv); break;
-      case 4: stockham_pass<R, 4, EMAX / 4>(buf, n, Ns, L, tw, inv); break;
-      case 5: stockham_pass<R, 5, MB5>(buf, n, Ns, L, tw, inv); break;
-      case 8: stockham_pass<R, 8, EMAX / 8>(buf, n, Ns, L, tw, inv); break;
+#define FAME_PASS(r_) \
+  case r_: stockham_pass<R, r_, pass_maxb(EMAX, r_)>(buf, n, Ns, L, tw, inv); break;
+      FAME_PASS(2)
+      FAME_PASS(3)
+      FAME_PASS(4)
+      FAME_PASS(5)
+      FAME_PASS(6)
+      FAME_PASS(7)
+      FAME_PASS(8)
+      FAME_PASS(9)
+      FAME_PASS(10)
+      FAME_PASS(11)
+      FAME_PASS(12)
+      FAME_PASS(13)
+#undef FAME_PASS
       default:
-        if constexpr (RARE >= 1) rare_pass<R, EMAX, RARE>(buf, n, r, Ns, L, tw, inv);
+        if constexpr (RARE >= 2) {
+          if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml>(buf, n, r, Ns, L, tw, inv))
+            generic_pass<R, EMAX>(buf, n, r, Ns, L, tw, inv);
+        }
         break;
     }
     Ns *= r;
   }
 }
-
 
 // ---------------------------------------------------------------- compile-time plans
 // Static plans: a two-pass split n = r0 * r1 with both radices in {4, 8, 12}
@@ -662,6 +723,11 @@ __device__ __forceinline__ void spass(cplx<R>* buf, int ls, int es, const cplx<R
     cplx<R> v[MAXB][RAD];
     bool on[MAXB];
     int jbk[MAXB];
+    // (defined on every path, see stockham_pass)
+#pragma unroll
+    for (int q = 0; q < MAXB; q++)
+#pragma unroll
+      for (int u = 0; u < RAD; u++) v[q][u] = mk<R>(0, 0);
 #pragma unroll
     for (int q = 0; q < MAXB; q++) {
       const int j = j0 + jstep * q;
@@ -723,15 +789,28 @@ __device__ __forceinline__ void sfft(cplx<R>* buf, int ls, int es, const cplx<R>
   }
 }
 
-// The lowest fft_lines level (RARE) that has a pass for every radix of the plan.
+// Pass level of an axis plan: 2 if it has a prime factor >= 17, 1 if it has a factor 7, 11
+// or 13, else 0.
 inline int plan_level(const AxisPlan& P) {
   int lv = 0;
   for (int p = 0; p < P.npass; p++) {
     const int r = P.radix[p];
-    if (r == 2 || r == 3 || r == 4 || r == 5 || r == 8) continue;
-    lv = (r == 7 || r == 11 || r == 13) ? (lv > 1 ? lv : 1) : 2;
+    if (r > 13) return 2;
+    if (r == 7 || r == 11 || r == 13) lv = 1;
   }
   return lv;
+}
+
+// Threads a CTA needs so that every pass of the plan can stage one whole line.
+inline int plan_threads(const AxisPlan& P, int emax) {
+  int t = 1;
+  for (int p = 0; p < P.npass; p++) {
+    const int r = P.radix[p];
+    if (r > 13) continue;
+    const int nb = P.n / r, mb = pass_maxb(emax, r);
+    t = t > (nb + mb - 1) / mb ? t : (nb + mb - 1) / mb;
+  }
+  return t;
 }
 
 }  // namespace fame

@@ -10,20 +10,22 @@
 
 namespace fame {
 
-constexpr int kPlaneThreads = 512;      // most threads of a plane CTA (runtime geometry)
+constexpr int kPlaneThreads = 512;      // most threads of a plane CTA that an option can set
 constexpr int kStatPlaneThreads = 384;  // threads of a plane CTA with a static geometry
-constexpr int kPencilThreads = 256;     // threads of a pencil CTA
+constexpr int kPencilThreads = 256;     // threads of a pencil CTA (at most, with runtime plans)
 
 struct DynGeom {
   static constexpr bool kStatic = false;
-  static constexpr int kMaxPlaneThreads = kPlaneThreads;
-  // The stage kernels' register budgets (launch bounds in op_kernels.cuh) are
-  // sized for two resident plane CTAs per SM (64 registers at 512 threads) and
-  // three pencil CTAs (85 registers), except that plane kernels with the prime
-  // pass (RARE 2), whose MU x ML accumulator block needs more, take one.
+  // Launch bounds of the plane kernels: registers per thread.  FP32: 80 (768 threads per
+  // SM), so 24 warps are resident whether a CTA has 96 threads or 768.  FP64, and the kernels
+  // with the prime pass (RARE 2), whose MU x ML accumulator block needs more: 128 (512).
+  template <typename R, int RARE> static constexpr int max_plane_threads() {
+    return sizeof(R) == 4 && RARE < 2 ? 768 : 512;
+  }
   __device__ __forceinline__ static int plane_threads() { return blockDim.x; }
-  // plane CTAs per SM the register budget is sized for (launch bounds)
-  template <typename R, int RARE> static constexpr int plane_min_blocks() { return RARE >= 2 ? 1 : 2; }
+  __device__ __forceinline__ static int pencil_threads() { return blockDim.x; }
+  // plane CTAs of that size per SM the register budget is sized for (launch bounds)
+  template <typename R, int RARE> static constexpr int plane_min_blocks() { return 1; }
   __device__ __forceinline__ static int Lf(const Geom& g) { return g.Lf; }
   __device__ __forceinline__ static int Lm(const Geom& g) { return g.Lm; }
   __device__ __forceinline__ static int Ls(const Geom& g) { return g.Ls; }
@@ -76,6 +78,7 @@ template <> struct SlowEmax<double> { static constexpr int v = 4; };
 // instantiated in ops_slow_static.cu.
 template <int LSL>
 struct DynGeomSlow : DynGeom {
+  __device__ __forceinline__ static constexpr int pencil_threads() { return kPencilThreads; }
   template <typename R, int RARE>
   __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom&, const cplx<R>* tw, bool inv) {
     constexpr int TW = PencilTW<R>::v;
@@ -91,6 +94,7 @@ struct DynGeomSlow : DynGeom {
 template <int LF, int LM, int T, int MB>
 struct DynGeomPlane : DynGeom {
   static constexpr int kMaxPlaneThreads = T;
+  template <typename R, int RARE> static constexpr int max_plane_threads() { return T; }
   __device__ __forceinline__ static constexpr int plane_threads() { return T; }
   template <typename R, int RARE> static constexpr int plane_min_blocks() { return MB; }
   template <typename R, int RARE>
@@ -109,10 +113,11 @@ struct StatGeom {
   static constexpr int kS = LF | 1;
   // 384 = 4 threads per line of a 96 x 96 plane: every pass of the 8 x 12 plan
   // is one round with all threads busy
-  static constexpr int kMaxPlaneThreads = kStatPlaneThreads;
+  template <typename R, int RARE> static constexpr int max_plane_threads() { return kStatPlaneThreads; }
   // two FP32 plane CTAs per SM (80 registers), one FP64 plane CTA; three FP32 and
   // two FP64 pencil CTAs
   __device__ __forceinline__ static constexpr int plane_threads() { return kStatPlaneThreads; }
+  __device__ __forceinline__ static constexpr int pencil_threads() { return kPencilThreads; }
   template <typename R, int RARE> static constexpr int plane_min_blocks() { return sizeof(R) == 4 ? 2 : 1; }
   __device__ __forceinline__ static constexpr int Lf(const Geom&) { return LF; }
   __device__ __forceinline__ static constexpr int Lm(const Geom&) { return LM; }
@@ -145,9 +150,9 @@ struct StatGeom {
 
 using Stat96 = StatGeom<96, 96, 96>;
 // static plane plans of the general-lattice benchmark grids (fast, mid, threads, CTAs per SM)
-using PlaneFcc64 = DynGeomPlane<52, 55, 256, 2>;
-using PlaneBcc48 = DynGeomPlane<39, 45, 256, 2>;
-using PlaneHex128f = DynGeomPlane<92, 107, 256, 2>;
-using PlaneHex128d = DynGeomPlane<92, 107, 512, 1>;
+template <typename R> using PlaneFcc64 = DynGeomPlane<52, 55, 128, sizeof(R) == 4 ? 5 : 4>;
+template <typename R> using PlaneBcc48 = DynGeomPlane<39, 45, 128, sizeof(R) == 4 ? 5 : 4>;
+template <typename R>
+using PlaneHex128 = DynGeomPlane<92, 107, sizeof(R) == 4 ? 256 : 512, sizeof(R) == 4 ? 2 : 1>;
 
 }  // namespace fame

@@ -15,40 +15,77 @@
 
 namespace fame {
 
-// Radix order of a plan: the listed radices as often as they divide n, in order, then
-// the remaining prime factors from 17 up.  kRadixOrders[0] (largest power-of-two
-// radix first: fewest passes) is the default; the plan tuner tries the others.
-constexpr int kNumRadixOrder = 8;
+// Radix plan of an axis.  Radix order 0 (the default): the fewest passes out of the
+// butterflies 2..13, the smallest radix sum among those, largest radix first; every
+// length up to 144 without a prime factor >= 17 takes at most two passes but a few (75, 98, 105, ...),
+// where 8, 4, 2, 5, 3 in turn took three or four, each a round trip of the
+// whole plane through shared memory.  Order 1: the same radices, smallest first.  Orders
+// 2 and 3: the listed radices as often as they divide n, in turn.  Prime factors
+// from 17 up come last.  The plan tuner tries all four.
 constexpr int kNumRadixOrders = 4;
-constexpr int kRadixOrders[kNumRadixOrders][kNumRadixOrder] = {
+constexpr int kNumListed = 8;
+constexpr int kListedRadices[2][kNumListed] = {
     {8, 4, 2, 5, 3, 7, 11, 13},  // 64 = 8 8, 96 = 8 4 3
-    {4, 2, 8, 3, 5, 7, 11, 13},  // 64 = 4 4 4, 96 = 4 4 2 3
-    {8, 2, 4, 3, 5, 7, 11, 13},  // 64 = 8 8, 32 = 8 2 2
     {3, 5, 7, 11, 13, 4, 8, 2},  // odd radices first: 96 = 3 4 4 2
 };
-constexpr const int* kRadixOrder = kRadixOrders[0];
 
-inline bool factor_axis(int n, AxisPlan& p, const int* order = kRadixOrder, int norder = kNumRadixOrder) {
-  p.n = n;
-  p.npass = 0;
-  int m = n;
-  for (int i = 0; i < norder; i++) {
-    const int r = order[i];
-    while (m % r == 0) {
-      if (p.npass >= kMaxPasses) return false;
-      p.radix[p.npass++] = r;
-      m /= r;
+// Fewest radices <= hi whose product is m (smallest sum among equals), non-increasing;
+// returns their number or kMaxPasses + 1.
+inline int fewest_radices(int m, int hi, int* out) {
+  if (m == 1) return 0;
+  int best = kMaxPasses + 1, best_sum = 0;
+  for (int r = std::min(hi, m); r >= 2; r--) {
+    if (m % r) continue;
+    int rest[kMaxPasses + 1] = {};
+    const int c = 1 + fewest_radices(m / r, r, rest);
+    if (c > kMaxPasses) continue;
+    int sum = r;
+    for (int i = 0; i < c - 1; i++) sum += rest[i];
+    if (c < best || (c == best && sum < best_sum)) {
+      best = c;
+      best_sum = sum;
+      out[0] = r;
+      for (int i = 0; i < c - 1; i++) out[i + 1] = rest[i];
     }
   }
-  for (int q = 17; m > 1 && q <= m; q++) {
-    while (m % q == 0) {
-      if (p.npass >= kMaxPasses) return false;
-      p.radix[p.npass++] = q;
+  return best;
+}
+
+inline bool factor_axis(int n, AxisPlan& p, int order = 0) {
+  p.n = n;
+  p.npass = 0;
+  int m = n;  // n without its prime factors >= 17
+  for (int q = 17; q <= m; q++) {
+    int k = m;
+    while (k % 2 == 0) k /= 2;
+    for (int r : {3, 5, 7, 11, 13})
+      while (k % r == 0) k /= r;
+    if (k == 1) break;
+    while (k % q == 0) {
+      k /= q;
       m /= q;
     }
   }
-  if (n == 1) p.npass = 0;
-  return m == 1;
+  const int big = n / m;
+  if (order <= 1) {
+    int rad[kMaxPasses + 1] = {};
+    const int c = fewest_radices(m, 13, rad);
+    if (c > kMaxPasses) return false;
+    for (int i = 0; i < c; i++) p.radix[p.npass++] = rad[order == 0 ? i : c - 1 - i];
+  } else {
+    for (int r : kListedRadices[order - 2])
+      for (; m % r == 0; m /= r) {
+        if (p.npass >= kMaxPasses) return false;
+        p.radix[p.npass++] = r;
+      }
+  }
+  int rest = big;
+  for (int q = 17; rest > 1 && q <= rest; q++)
+    for (; rest % q == 0; rest /= q) {
+      if (p.npass >= kMaxPasses) return false;
+      p.radix[p.npass++] = q;
+    }
+  return true;
 }
 
 // Lengths, plans, table and twiddle offsets of lattice L.  Simple lattices walk
@@ -81,8 +118,8 @@ inline int layout_geom(const fame_lattice& L, Geom& g, long max_points, std::str
   g.Lf = g.general ? g.Nz : g.Nx;
   g.P = g.Lm * g.Lf;
   g.S = g.Lf | 1;  // odd row pitch: bank-conflict-free passes along both plane axes
-  const int* ord = kRadixOrders[radix_order];
-  if (!factor_axis(g.Lf, g.pf, ord) || !factor_axis(g.Lm, g.pm, ord) || !factor_axis(g.Ls, g.ps, ord)) {
+  if (!factor_axis(g.Lf, g.pf, radix_order) || !factor_axis(g.Lm, g.pm, radix_order) ||
+      !factor_axis(g.Ls, g.ps, radix_order)) {
     err = "axis length needs more than 10 FFT passes";
     return FAME_ERR_UNSUPPORTED;
   }
@@ -115,27 +152,69 @@ inline int layout_geom(const fame_lattice& L, Geom& g, long max_points, std::str
   return FAME_OK;
 }
 
-// fft_lines level (kernel instantiation) the three axis plans need.
+// Pass level of the three axis plans.
 inline int geom_level(const Geom& g) {
   return std::max(plan_level(g.pf), std::max(plan_level(g.pm), plan_level(g.ps)));
 }
 // ... the plane stages' axes (fast, mid) and the pencil stage's axis (slow) alone: each
-// stage kernel runs the lowest level its own axes need (fewer registers, no spills
-// from passes it never runs)
+// stage kernel carries the prime passes only when its own axes need them (fewer
+// registers, no spills from passes it never runs)
 inline int plane_level(const Geom& g) { return std::max(plan_level(g.pf), plan_level(g.pm)); }
 inline int pencil_level(const Geom& g) { return plan_level(g.ps); }
 
-// Threads of a runtime-geometry plane CTA: about 8 plane elements per thread, at most
-// 512; at most 256 when two planes of precision R fit one SM's shared memory (more,
-// smaller CTAs per SM hide the latency of the staged passes better), except FP64
-// planes with the prime pass (level 2), whose 128-register budget admits one CTA per SM.
+// Threads a plane CTA of precision R must have: every pass stages whole lines.
+template <typename R> inline int plane_threads_min(const Geom& g) {
+  return (std::max(plan_threads(g.pf, Emax<R>::v), plan_threads(g.pm, Emax<R>::v)) + 31) / 32 * 32;
+}
+
+// Threads of a runtime-plan CTA that works on `work` elements, for a launch of `ctas` CTAs with
+// `smem` bytes each, from `lo` up to `hi` in steps of 32; `sm_threads` is what the register
+// budget leaves resident per SM.  A CTA's time hardly falls with its threads (barriers and
+// global latency make up most of it: about 35 + 1.25 work / threads, in microseconds at 3,000
+// elements), so what counts is how many run at once: the choice minimises waves times that
+// time, a partly filled last wave counted half beyond the first.  The clusters of three fill
+// about 0.94 of the CTA places.  Measured on launches of 4 to 6 k-points against about 12 elements per thread
+// (FP32 CG plane stage, us per k-point): 45x66x50 23.6 -> 17.8, 50x63x45 23.1 -> 15.9, 36x30x26
+// 14.7 -> 14.0, 92x80x75 63.5 -> 57.7.
+inline int stage_threads(long work, long ctas, size_t smem, int sm_threads, int lo, int hi) {
+  constexpr int kSMs = 148;
+  constexpr size_t kSmemSM = 228 * 1024, kSmemCta = 1024;
+  lo = std::max(64, (lo + 31) / 32 * 32);
+  hi = (int)std::max<long>(lo, std::min<long>(hi, (work / 8 + 31) / 32 * 32));
+  int best = lo;
+  double best_cost = 1e300;
+  for (int t = lo; t <= hi; t += 32) {
+    const int per_sm = std::min<int>({sm_threads / t, (int)(kSmemSM / (smem + kSmemCta)), 32});
+    if (per_sm < 1) continue;
+    const double w = ctas / (0.94 * kSMs * per_sm), up = ceil(w);
+    const double cost = (w <= 1.0 ? 1.0 : w + 0.5 * (up - w)) * (35.0 + 1.25 * work / t);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = t;
+    }
+  }
+  return best;
+}
+
+// ... of a plane stage: `planes` planes (3 CTAs each) of precision R.
 template <typename R>
-inline int plane_threads_rule(const Geom& g, int level) {
-  const int pt = std::min(512, std::max(64, ((g.P + 7) / 8 + 31) / 32 * 32));
-  const size_t kSmemSM = 227 * 1024;
-  const bool two = 2 * plane_smem_bytes<R>(g.Lf, g.Lm, g.S) <= kSmemSM;
-  if (sizeof(R) == 8 && level >= 2) return pt;
-  return two ? std::min(pt, 256) : pt;
+inline int plane_threads_rule(const Geom& g, int level, long planes) {
+  // the kernels' launch bounds (DynGeom::max_plane_threads)
+  const int most = sizeof(R) == 4 && level < 2 ? 768 : 512;
+  return stage_threads(g.P, 3 * planes, plane_smem_bytes<R>(g.Lf, g.Lm, g.S), most, plane_threads_min<R>(g), 512);
+}
+// ... and of a pencil stage over `vecs` vectors: with a prime pass, enough that it is one round
+// (92 = 4 x 23 in FP64: 51.7 us per k-point with 256 threads, 81.6 with 64).
+template <typename R>
+inline int pencil_threads_rule(const Geom& g, int level, long vecs) {
+  constexpr int TW = PencilTW<R>::v, mu = PrimeBlock<R>::mu, ml = PrimeBlock<R>::ml;
+  int lo = plan_threads(g.ps, Emax<R>::v);
+  for (int p = 0; p < g.ps.npass; p++) {
+    const int r = g.ps.radix[p];
+    if (r > 13) lo = std::max(lo, g.ps.n / r * (((r - 1) / 2 + mu) / mu) * ((TW + ml - 1) / ml));
+  }
+  return stage_threads((long)g.Ls * TW, 3 * vecs * ((g.P + TW - 1) / TW), pencil_smem_bytes<R>(g.Ls),
+                       level < 2 ? 768 : 512, std::min(lo, kPencilThreads), kPencilThreads);
 }
 
 // theta_x, theta_y(xy), theta_z(xyz) of wave vector k (FAME_Main/FAME_Matrix_Lambdas.cu:43-70)

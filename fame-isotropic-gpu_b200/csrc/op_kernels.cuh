@@ -58,288 +58,504 @@ __device__ __forceinline__ bool plane_vec_range(int P, int s, int comp, const Sl
   return i1 > i0;
 }
 
+// ------------------------------------------------------------------ plane stages
 // One cluster = 3 CTAs = the 3 components of plane s.  grid = (3*Ls, vec_per_slot, nslots)
-template <typename R, bool GEN, int IN, bool PR, int RARE, class GP>
-__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::kMaxPlaneThreads, GP::template plane_min_blocks<R, RARE>())
-    k_plane_inv(PlaneInArgs<R> a) {
-  FAME_COUNT_LAUNCH();
-  if ((threadIdx.x | blockIdx.x | blockIdx.y | blockIdx.z) == 0) set_cond(a.reset, 0);
+struct PlanePos {
+  int s, comp, vec, slot;
+};
+// Read afresh from the special registers at every call (the empty asm hides the value from
+// the compiler): a kernel asks again after its transforms, so that nothing but the plane
+// lives across them.  Kept in registers instead, the two dozen values of the mixing
+// phase were spilled and reloaded around every one of the runtime plans' passes.
+__device__ __forceinline__ PlanePos plane_pos() {
+  unsigned x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
+  asm volatile("" : "+r"(x), "+r"(y), "+r"(z));
+  PlanePos p;
+  p.s = (int)(x / 3);
+  p.comp = (int)x - 3 * p.s;
+  p.vec = (int)y;
+  p.slot = (int)z;
+  return p;
+}
+
+// Dynamic shared memory of a plane CTA.  Plane rows have the odd pitch S >= Lf.  lx, ly hold
+// the Lambda tables of the plane's axes (Simple lattices) or, in ly, D_ky(s, .) (General).
+template <typename R> struct PlaneSmem {
+  cplx<R>*plane, *twf, *twm, *lx, *ly;
+};
+template <typename R, class GP> __device__ __forceinline__ PlaneSmem<R> plane_smem_of(const Geom& g) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const Geom& g = a.g;
-  const int Lf = GP::Lf(g), Lm = GP::Lm(g), S = GP::S(g), P = GP::P(g);
-  const Div dlf(Lf);  // row of plane element e: e / Lf (folds to a constant for static geometries)
-  cplx<R>* plane = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* twf = plane + Lm * S;  // plane rows have the odd pitch S >= Lf
-  cplx<R>* twm = twf + Lf;
-  cplx<R>* lx = twm + Lm;
-  cplx<R>* ly = lx + Lf;
-  cg::cluster_group cl = cg::this_cluster();
-  const int comp = (int)cl.block_rank();
-  const int s = blockIdx.x / 3;
-  const int vec = blockIdx.y;
-  const int slot = blockIdx.z;
-  const Slot sl = a.slots[slot];
-  if (!sl.active) return;  // uniform over the cluster
-  CgState* st = nullptr;
-  if constexpr (IN == IN_CG || IN == IN_REFINE) {
-    st = a.cg + slot;
-    if constexpr (IN == IN_CG) {
-      if (!st->active) return;
-    } else {
-      if (!st->outer_active) return;
-    }
-  }
-  if constexpr (IN == IN_CG) {
-    // this CTA's own r, p and x, all at once: the batched loads of the mix below then
-    // wait on one DRAM latency and find the rest in L2
-    long i0, i1;
-    if (a.self_pf && threadIdx.x < (st->iter == 1 ? 2 : 6) && plane_vec_range(P, s, comp, sl, i0, i1)) {
-      const cplx<R>* v = threadIdx.x < 2 ? a.r : threadIdx.x < 4 ? a.p : a.x;
-      const long base = (long)(slot * a.vec_per_slot + vec) * a.vstride + ((threadIdx.x & 1) ? sl.Nd : 0);
-      prefetch_l2(v + base + i0, (i1 - i0) * sizeof(cplx<R>));
-    }
-  }
-  if constexpr (IN == IN_CG) {
-    // r, p and x of the CTA one wave ahead (p and x once its k-point is past k = 1)
-    int x2, y2, z2;
-    if (a.pf_dist > 0 && threadIdx.x < 6 && cta_of(cta_linear() + a.pf_dist, x2, y2, z2)) {
-      const Slot s2 = a.slots[z2];
-      const CgState* c2 = a.cg + z2;
-      long i0, i1;
-      const int which = threadIdx.x >> 1;  // 0 r, 1 p, 2 x
-      if (s2.active && c2->active && (which == 0 || c2->iter > 1) &&
-          plane_vec_range(P, x2 / 3, x2 % 3, s2, i0, i1)) {
-        const cplx<R>* v = which == 0 ? a.r : which == 1 ? a.p : a.x;
-        const long base = (long)(z2 * a.vec_per_slot + y2) * a.vstride + ((threadIdx.x & 1) ? s2.Nd : 0);
-        prefetch_l2(v + base + i0, (i1 - i0) * sizeof(cplx<R>));
-      }
-    }
-  }
-  // Static geometries exchange the mixed components with st.async into the owner's
-  // plane, counted on the owner's barrier `xbar` (P values arrive per plane); the
-  // others use a cluster barrier after the exchange.
-  constexpr bool kAsyncMix = GP::kStatic;
-  __shared__ __align__(8) unsigned long long xbar;
-  const unsigned bar = smem_u32(&xbar);
-  // after a failed exchange (the fault marker), later launches skip their work: the
-  // cluster's rank-0 CTA reads the marker and all three CTAs act on its value
-  __shared__ int skip;
-  if (kAsyncMix && threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    mbar_init_fence_cluster();
-    skip = a.fault ? *(volatile int*)a.fault : 0;
-  }
-  const double2* tab = a.tabs + (size_t)slot * g.tab_stride;
+  PlaneSmem<R> m;
+  m.plane = reinterpret_cast<cplx<R>*>(smem_raw);
+  m.twf = m.plane + GP::Lm(g) * GP::S(g);
+  m.twm = m.twf + GP::Lf(g);
+  m.lx = m.twm + GP::Lm(g);
+  m.ly = m.lx + GP::Lf(g);
+  return m;
+}
+
+// Twiddle and Lambda (or D_ky) tables into shared memory; a barrier must follow.
+template <typename R, bool GEN, class GP>
+__device__ __forceinline__ void plane_tables(const Geom& g, const cplx<R>* tw, const double2* tab, int s,
+                                             const PlaneSmem<R>& m) {
+  const int Lf = GP::Lf(g), Lm = GP::Lm(g);
   for (int i = threadIdx.x; i < Lf; i += GP::plane_threads()) {
-    twf[i] = a.tw[g.twf + i];
-    if constexpr (!GEN) lx[i] = cvt<R>(tab[g.oLx + i]);
+    m.twf[i] = tw[g.twf + i];
+    if constexpr (!GEN) m.lx[i] = cvt<R>(tab[g.oLx + i]);
   }
   for (int i = threadIdx.x; i < Lm; i += GP::plane_threads()) {
-    twm[i] = a.tw[g.twm + i];
-    if constexpr (!GEN) ly[i] = cvt<R>(tab[g.oLy + i]);
+    m.twm[i] = tw[g.twm + i];
+    m.ly[i] = cvt<R>(GEN ? tab[g.oDky + s * g.Ny + i] : tab[g.oLy + i]);
   }
-  const cplx<R> lz = GEN ? mk<R>(0, 0) : cvt<R>(tab[g.oLz + s]);
-  cl.sync();  // every CTA of the cluster is running (and the tables and barriers are in place)
-  if constexpr (kAsyncMix) {
-    if (*cl.map_shared_rank(&skip, 0)) {
-      cl.sync();  // rank 0's marker stays readable until all three have read it
-      return;
-    }
-  }
-  if (kAsyncMix && threadIdx.x == 0) mbar_arrive_expect_tx(bar, (unsigned)(P * sizeof(cplx<R>)));
-  unsigned rplane[3], rbar[3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    rplane[c] = kAsyncMix ? mapa_u32(smem_u32(plane), c) : 0u;
-    rbar[c] = kAsyncMix ? mapa_u32(bar, c) : 0u;
-  }
+}
 
-  const long vb = (long)(slot * a.vec_per_slot + vec) * a.vstride;
-  const int Nd = sl.Nd, off = sl.off;
-  cplx<R>* dst[3] = {cl.map_shared_rank(plane, 0), cl.map_shared_rank(plane, 1),
-                     cl.map_shared_rank(plane, 2)};
-  const int per = (P + 2) / 3;
-  const int e0 = comp * per, e1 = min(P, e0 + per);
-  R beta = 0;
-  bool first = false;
-  R rscale = 0;
-  // CG step size a of the last update: the solution update x += a p is applied here
-  // (IN_CG: the previous iteration's, IN_REFINE: the inner solve's last) instead of
-  // in the vector update kernel, where it would cost another pass over p and x
-  R are = 0, aim = 0;
-  if constexpr (IN == IN_CG) {
-    first = st->iter == 1;
-    beta = (R)st->beta;
-    are = (R)st->a_re;
-    aim = (R)st->a_im;
-  }
-  float fre = 0.f, fim = 0.f;
-  bool pend = false;
-  if constexpr (IN == IN_REFINE) {
-    rscale = (R)(1.0 / st->scale);
-    pend = st->iter > 1;
-    fre = (float)st->a_re;
-    fim = (float)st->a_im;
-  }
-  // Input stage and the 2 -> 3 mix.  IN_CG: p = r + beta p (p = r at k = 1) and the
-  // deferred x += a p (CG.cu:39-51, :65-66).  IN_REFINE: y += x32 / scale with the
-  // inner solve's last update folded in.  The operands of KB points per thread are
-  // loaded up front, so one global-load latency covers KB points.
-  // (runtime geometries run at 64 registers: two points)
-  constexpr int KB = !GP::kStatic ? 2 : IN == IN_VEC ? 8 : 2;
-  const int NT = GP::plane_threads();
-  for (int eb = e0 + threadIdx.x; eb < e1; eb += KB * NT) {
-    cplx<R> A1[KB], A2[KB], B1[KB], B2[KB], C1[KB], C2[KB];
-    float2 F1[KB], F2[KB], G1[KB], G2[KB];
-#pragma unroll
-    for (int k = 0; k < KB; k++) {
-      const int e = eb + k * NT;
-      if (e < e1 && s * P + e >= off) {
-        const long i = s * P + e - off;
-        if constexpr (IN == IN_VEC) {
-          A1[k] = a.in[vb + i];
-          A2[k] = a.in[vb + Nd + i];
-        } else if constexpr (IN == IN_CG) {
-          A1[k] = a.r[vb + i];
-          A2[k] = a.r[vb + Nd + i];
-          if (!first) {
-            B1[k] = a.p[vb + i];
-            B2[k] = a.p[vb + Nd + i];
-            C1[k] = a.x[vb + i];
-            C2[k] = a.x[vb + Nd + i];
-          }
-        } else {  // IN_REFINE (R = double)
-          A1[k] = a.y64[vb + i];
-          A2[k] = a.y64[vb + Nd + i];
-          F1[k] = a.x32[vb + i];
-          F2[k] = a.x32[vb + Nd + i];
-          if (pend) {
-            G1[k] = a.p32[vb + i];
-            G2[k] = a.p32[vb + Nd + i];
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < KB; k++) {
-      const int e = eb + k * NT;
-      if (e >= e1) break;
-      const int fi = s * P + e;
-      const int m = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - m * Lf;
-      cplx<R> v[3] = {mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0)};
-      if (fi >= off) {
-        const long i = fi - off;
-        cplx<R> Lx, Ly, Lz;
-        lam_elem<R, GEN>(g, tab, lx, ly, lz, s, m, f, Lx, Ly, Lz);
-        cplx<R> x1 = A1[k], x2 = A2[k];
-        if constexpr (IN == IN_VEC) {
-          if (a.sigma) {
-            const R sc = sqrt(cabs2(Lx) + cabs2(Ly) + cabs2(Lz));
-            x1 = cscale(x1, sc);
-            x2 = cscale(x2, sc);
-          }
-        } else if constexpr (IN == IN_CG) {
-          if (!first) {
-            cplx<R> s1 = C1[k], s2 = C2[k];
-            const cplx<R> p1 = B1[k], p2 = B2[k];
-            if constexpr (sizeof(R) == 4) {
-              // the FP32 CG's step size is real (<p, Ap> from the pencil stage): packed pairs
-              s1 = pfma(p1, are, s1);
-              s2 = pfma(p2, are, s2);
-              x1 = pfma(p1, beta, x1);
-              x2 = pfma(p2, beta, x2);
-            } else {
-              s1.x += are * p1.x - aim * p1.y;
-              s1.y += are * p1.y + aim * p1.x;
-              s2.x += are * p2.x - aim * p2.y;
-              s2.y += are * p2.y + aim * p2.x;
-              x1 = mk<R>(x1.x + beta * p1.x, x1.y + beta * p1.y);
-              x2 = mk<R>(x2.x + beta * p2.x, x2.y + beta * p2.y);
-            }
-            a.x[vb + i] = s1;
-            a.x[vb + Nd + i] = s2;
-          }
-          a.p[vb + i] = x1;
-          a.p[vb + Nd + i] = x2;
-        } else {  // IN_REFINE
-          float2 c1 = F1[k], c2 = F2[k];
-          if (pend) {
-            const float2 q1 = G1[k], q2 = G2[k];
-            c1.x += fre * q1.x - fim * q1.y;
-            c1.y += fre * q1.y + fim * q1.x;
-            c2.x += fre * q2.x - fim * q2.y;
-            c2.y += fre * q2.y + fim * q2.x;
-          }
-          x1.x += (double)c1.x * rscale;
-          x1.y += (double)c1.y * rscale;
-          x2.x += (double)c2.x * rscale;
-          x2.y += (double)c2.y * rscale;
-          a.y64[vb + i] = x1;
-          a.y64[vb + Nd + i] = x2;
-        }
-        cplx<R> Pc[6];
-        pi_from<R>(GEN, PR, Lx, Ly, Lz, Pc);
-#pragma unroll
-        for (int c = 0; c < 3; c++) v[c] = cadd(cmul(Pc[c], x1), cmul(Pc[3 + c], x2));
-      }
-      if constexpr (kAsyncMix) {
-        const unsigned o = (unsigned)((m * S + f) * sizeof(cplx<R>));
-#pragma unroll
-        for (int c = 0; c < 3; c++) st_async(rplane[c] + o, v[c], rbar[c]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < 3; c++) dst[c][m * S + f] = v[c];
-      }
-    }
-  }
-  if constexpr (kAsyncMix) {
-    // this CTA's plane is complete once all P values have arrived.  A wait that runs out
-    // (about 0.1 s; it cannot unless the exchange is broken) records the fault and goes
-    // on, and later launches return at once (below), so the solve ends with an error.
-    if (!mbar_wait(bar, 0, 200000000LL) && a.fault) atomicExch(a.fault, 1);
-    __syncthreads();
-  } else {
-    cl.sync();
-  }
-
-  // inverse 2-D transform of this component's plane (unnormalised): fast axis,
-  // then mid axis.  One FFT call site per axis loop keeps the kernel within its
-  // register budget.
-  if constexpr (GP::kStatic && !GEN) {
-    GP::template fft_plane_c<R, true, true>(plane, twf);
-    GP::template fft_plane_c<R, false, true>(plane, twm);
-  }
-  for (int ax = 0; !(GP::kStatic && !GEN) && ax < 2; ax++) {
-    GP::template fft_plane<R, RARE>(plane, g, ax == 0, ax == 0 ? twf : twm, true);
-    if constexpr (GEN) {
-      // x D_kz(x,y,z) after the z (fast) pass (FAME_FFT_CUDA.cu:109, kernel :283-317),
-      // x D_ky(x,y) after the y (mid) pass (FAME_FFT_CUDA.cu:115, kernel :198-234)
-      for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
-        const int m = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - m * Lf;
-        const int q = m * S + f;
-        plane[q] = cmul(plane[q], ax == 0 ? dkz_at<R>(g, tab, s, m, f) : cvt<R>(tab[g.oDky + s * g.Ny + m]));
-      }
-      __syncthreads();
-    }
-  }
-  cplx<R>* T = a.T + (long)(slot * a.vec_per_slot + vec) * a.fstride + (long)comp * g.N + (long)s * P;
+// plane *= D_kz (inverse) or conj(D_kz) (forward), General lattices: from the table of the
+// k-point where there is one (coalesced; evaluated in place, the sincospi were a
+// quarter of the plane kernels' instructions), else evaluated.
+template <typename R, class GP>
+__device__ __forceinline__ void plane_times_dkz(const Geom& g, const double2* tabs, const cplx<R>* dkz, cplx<R>* plane,
+                                                bool inv) {
+  const PlanePos p = plane_pos();
+  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
+  const Div dlf(Lf);
+  const cplx<R>* d = dkz ? dkz + (size_t)p.slot * g.N + (size_t)p.s * P : nullptr;
+  const double2* tab = tabs + (size_t)p.slot * g.tab_stride;
+#pragma unroll 4
   for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
-    const int m = GP::kStatic ? e / Lf : (int)dlf.q(e);
-    T[e] = plane[e + m * (S - Lf)];
+    const int m = (int)dlf.q(e), q = e + m * (S - Lf);
+    cplx<R> w = d ? d[e] : dkz_at<R>(g, tab, p.s, m, e - m * Lf);
+    if (!inv) w = cconj(w);
+    plane[q] = cmul(plane[q], w);
   }
+  __syncthreads();
+}
+
+// Unnormalised inverse 2-D transform of the CTA's plane: fast axis, (x D_kz), mid axis; x D_ky
+// follows in plane_store (General lattices, FAME_FFT_CUDA.cu:104-117).
+template <typename R, bool GEN, int RARE, class GP>
+__device__ __forceinline__ void plane_inverse(const Geom& g, const double2* tabs, const cplx<R>* dkz) {
+  const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
+  if constexpr (GP::kStatic && !GEN) {
+    GP::template fft_plane_c<R, true, true>(m.plane, m.twf);
+    GP::template fft_plane_c<R, false, true>(m.plane, m.twm);
+  } else {
+    // one FFT call site per axis loop: the runtime plans' passes are long
+#pragma unroll 1
+    for (int ax = 0; ax < 2; ax++) {
+      GP::template fft_plane<R, RARE>(m.plane, g, ax == 0, ax == 0 ? m.twf : m.twm, true);
+      if (GEN && ax == 0) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane, true);
+    }
+  }
+}
+
+// Unnormalised forward 2-D transform.  General lattices (T*, FAME_FFT_CUDA.cu:128-150): x conj(D_ky)
+// (in plane_load), mid pass, x conj(D_kz), fast pass.  Simple lattices: fast then mid axis.
+template <typename R, bool GEN, int RARE, class GP>
+__device__ __forceinline__ void plane_forward(const Geom& g, const double2* tabs, const cplx<R>* dkz) {
+  const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
+  if constexpr (GP::kStatic && !GEN) {
+    GP::template fft_plane_c<R, true, false>(m.plane, m.twf);
+    GP::template fft_plane_c<R, false, false>(m.plane, m.twm);
+  } else {
+#pragma unroll 1
+    for (int ax = 0; ax < 2; ax++) {
+      const bool fast = GEN ? ax == 1 : ax == 0;
+      if (GEN && ax == 1) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane, false);
+      GP::template fft_plane<R, RARE>(m.plane, g, fast, fast ? m.twf : m.twm, false);
+    }
+  }
+}
+
+// This CTA's plane of the field in global memory.
+template <typename R, class GP>
+__device__ __forceinline__ long plane_base(const Geom& g, const PlanePos& p, int vec_per_slot, long fstride) {
+  return (long)(p.slot * vec_per_slot + p.vec) * fstride + (long)p.comp * g.N + (long)p.s * GP::P(g);
+}
+
+// The plane into shared memory (x conj(D_ky), General): the tables must be in place for
+// General lattices; Simple ones leave cp.async copies in flight (cp_async_wait_all).
+template <typename R, bool GEN, class GP>
+__device__ __forceinline__ void plane_load(const Geom& g, const cplx<R>* T, const PlaneSmem<R>& m) {
+  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g), NT = GP::plane_threads();
+  const Div dlf(Lf);
+  if constexpr (!GEN) {
+    for (int e = threadIdx.x; e < P; e += NT) {
+      const int r = GP::kStatic ? e / Lf : (int)dlf.q(e);
+      cp_async_elem(m.plane + e + r * (S - Lf), T + e);
+    }
+  } else {
+    constexpr int U = 32 / (int)sizeof(R);  // loads in flight per thread
+    for (int eb = threadIdx.x; eb < P; eb += U * NT) {
+      cplx<R> v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (eb + u * NT < P) v[u] = T[eb + u * NT];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int e = eb + u * NT;
+        if (e < P) {
+          const int r = (int)dlf.q(e);
+          m.plane[e + r * (S - Lf)] = cmulc(m.ly[r], v[u]);
+        }
+      }
+    }
+  }
+}
+
+// The plane out to global memory (x D_ky, General).
+template <typename R, bool GEN, class GP>
+__device__ __forceinline__ void plane_store(const Geom& g, cplx<R>* T) {
+  const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
+  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
+  const Div dlf(Lf);
+#pragma unroll 4
+  for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
+    const int r = GP::kStatic ? e / Lf : (int)dlf.q(e);
+    const cplx<R> v = m.plane[e + r * (S - Lf)];
+    T[e] = GEN ? cmul(v, m.ly[r]) : v;
+  }
+}
+
+// Exchange of mixed components between the three CTAs.  Static geometries send them with
+// st.async into the owner's plane, counted on the owner's barrier (P values arrive per
+// plane); the others store to distributed shared memory and use a cluster barrier.
+template <typename R, bool ASYNC> struct PlaneExchange {
+  cplx<R>* dst[3];
+  unsigned rplane[3], rbar[3];
+  __device__ __forceinline__ PlaneExchange(cplx<R>* plane, unsigned bar) {
+    cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      dst[c] = cl.map_shared_rank(plane, c);
+      rplane[c] = ASYNC ? mapa_u32(smem_u32(plane), c) : 0u;
+      rbar[c] = ASYNC ? mapa_u32(bar, c) : 0u;
+    }
+  }
+  __device__ __forceinline__ void put(int q, const cplx<R>* v) const {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if constexpr (ASYNC)
+        st_async(rplane[c] + (unsigned)(q * sizeof(cplx<R>)), v[c], rbar[c]);
+      else
+        dst[c][q] = v[c];
+    }
+  }
+};
+
+// Start of an exchange (thread 0 of each CTA): the barrier, and the fault marker of an earlier
+// exchange, after which launches skip their work (rank 0 reads it, all three act on it).
+__device__ __forceinline__ void exchange_init(unsigned bar, int* skip, int* fault) {
+  mbar_init(bar, 1);
+  mbar_init_fence_cluster();
+  *skip = fault ? *(volatile int*)fault : 0;
+}
+// End of it: the CTA's plane is complete once all P values have arrived.  A wait that runs out
+// (about 0.1 s; it cannot unless the exchange is broken) records the fault and goes on.
+__device__ __forceinline__ void exchange_wait(unsigned bar, int* fault) {
+  if (!mbar_wait(bar, 0, 200000000LL) && fault) atomicExch(fault, 1);
+  __syncthreads();
+}
+
+template <typename R, bool GEN, int IN, bool PR, int RARE, class GP>
+__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
+    k_plane_inv(PlaneInArgs<R> a) {
+  FAME_COUNT_LAUNCH();
+  const Geom& g = a.g;
+  constexpr bool kAsyncMix = GP::kStatic;
+  __shared__ __align__(8) unsigned long long xbar;
+  __shared__ int skip;
+  const unsigned bar = smem_u32(&xbar);
+  {
+    const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
+    const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
+    const Div dlf(Lf);  // row of plane element e: e / Lf (folds to a constant for static geometries)
+    cg::cluster_group cl = cg::this_cluster();
+    const PlanePos p = plane_pos();
+    const Slot sl = a.slots[p.slot];
+    if (!sl.active) return;  // uniform over the cluster
+    const CgState* st = nullptr;
+    if constexpr (IN == IN_CG || IN == IN_REFINE) {
+      st = a.cg + p.slot;
+      if (IN == IN_CG ? !st->active : !st->outer_active) return;
+    }
+    if (kAsyncMix && threadIdx.x == 0) exchange_init(bar, &skip, a.fault);
+    const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
+    plane_tables<R, GEN, GP>(g, a.tw, tab, p.s, m);
+    const cplx<R> lz = GEN ? mk<R>(0, 0) : cvt<R>(tab[g.oLz + p.s]);
+    cl.sync();  // every CTA of the cluster is running (and the tables and barriers are in place)
+    if constexpr (kAsyncMix) {
+      if (*cl.map_shared_rank(&skip, 0)) {
+        cl.sync();  // rank 0's marker stays readable until all three have read it
+        return;
+      }
+      if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, (unsigned)(P * sizeof(cplx<R>)));
+    }
+    const PlaneExchange<R, kAsyncMix> ex(m.plane, bar);
+    const long vb = (long)(p.slot * a.vec_per_slot + p.vec) * a.vstride;
+    const int Nd = sl.Nd, off = sl.off;
+    const int per = (P + 2) / 3;
+    const int e0 = p.comp * per, e1 = min(P, e0 + per);
+    R rscale = 0;
+    const float2* x32 = nullptr;
+    if constexpr (IN == IN_REFINE) {
+      // the FP32 correction (none if the inner solve did no product), and its scale
+      rscale = (R)(1.0 / st->scale);
+      x32 = st->iter > 1 ? a.x32[st->iter & 1] : nullptr;
+    }
+    // Input stage and the 2 -> 3 mix.  IN_CG: the start residual r.  IN_REFINE: y += x32 / scale.
+    // The operands of KB points per thread are loaded up front, so one global-load latency
+    // covers KB points.
+    constexpr int KB = !GP::kStatic ? 2 : IN == IN_REFINE ? 2 : 8;
+    const int NT = GP::plane_threads();
+    for (int eb = e0 + threadIdx.x; eb < e1; eb += KB * NT) {
+      cplx<R> A1[KB], A2[KB];
+      float2 F1[KB], F2[KB];
+#pragma unroll
+      for (int k = 0; k < KB; k++) {
+        const int e = eb + k * NT;
+        A1[k] = A2[k] = mk<R>(0, 0);
+        F1[k] = F2[k] = make_float2(0.f, 0.f);
+        if (e < e1 && p.s * P + e >= off) {
+          const long i = p.s * P + e - off;
+          if constexpr (IN == IN_REFINE) {
+            A1[k] = a.y64[vb + i];
+            A2[k] = a.y64[vb + Nd + i];
+            F1[k] = x32 ? x32[vb + i] : make_float2(0.f, 0.f);
+            F2[k] = x32 ? x32[vb + Nd + i] : make_float2(0.f, 0.f);
+          } else {
+            A1[k] = a.in[vb + i];
+            A2[k] = a.in[vb + Nd + i];
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < KB; k++) {
+        const int e = eb + k * NT;
+        if (e >= e1) break;
+        const int fi = p.s * P + e;
+        const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - r * Lf;
+        cplx<R> v[3] = {mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0)};
+        if (fi >= off) {
+          const long i = fi - off;
+          cplx<R> Lx, Ly, Lz;
+          lam_elem<R, GEN>(g, tab, m.lx, m.ly, lz, p.s, r, f, Lx, Ly, Lz);
+          cplx<R> x1 = A1[k], x2 = A2[k];
+          if constexpr (IN == IN_VEC) {
+            if (a.sigma) {
+              const R sc = sqrt(cabs2(Lx) + cabs2(Ly) + cabs2(Lz));
+              x1 = cscale(x1, sc);
+              x2 = cscale(x2, sc);
+            }
+          } else if constexpr (IN == IN_REFINE) {
+            x1.x += (double)F1[k].x * rscale;
+            x1.y += (double)F1[k].y * rscale;
+            x2.x += (double)F2[k].x * rscale;
+            x2.y += (double)F2[k].y * rscale;
+            a.y64[vb + i] = x1;
+            a.y64[vb + Nd + i] = x2;
+          }
+          cplx<R> Pc[6];
+          pi_from<R>(GEN, PR, Lx, Ly, Lz, Pc);
+#pragma unroll
+          for (int c = 0; c < 3; c++) v[c] = cadd(cmul(Pc[c], x1), cmul(Pc[3 + c], x2));
+        }
+        ex.put(r * S + f, v);
+      }
+    }
+    if constexpr (kAsyncMix)
+      exchange_wait(bar, a.fault);
+    else
+      cl.sync();
+  }
+  plane_inverse<R, GEN, RARE, GP>(g, a.tabs, a.dkz);
+  plane_store<R, GEN, GP>(g, a.T + plane_base<R, GP>(g, plane_pos(), a.vec_per_slot, a.fstride));
+}
+
+// ------------------------------------------------------------------ CG plane stage
+// The middle of a CG iteration in one kernel: the forward plane transforms of A r's field,
+// the 3 -> 2 unmix (w = A r), the three-term recurrences
+//   r' = rho (r - gamma w) + (1 - rho) r_old,   x' = rho (x + gamma r) + (1 - rho) x_old,
+//   gamma = ||r||^2 / <r, A r>,   rho = 1 / (1 - gamma ||r||^2 / (gamma_old ||r_old||^2 rho_old))
+// (CG in the form without search directions: Hageman and Young, "Applied Iterative Methods",
+// 1981, section 7.3; the reference's CG.cu:36-77 takes the same steps through p), the
+// 2 -> 3 mix of r' and its inverse plane transforms.  The form with p needs ||r'||^2 of all
+// planes before it can mix p' = r' + beta p, so it splits here into two kernels, each of which
+// waits for its own loads and evaluates Pi; this one mixes r' itself, reads r, r_old, x and
+// x_old once, and evaluates Pi once for both directions.  In exchange the kernel's second half is idle work in
+// the last iteration of a solve.  r' and x' overwrite r_old and x_old: the current buffers are
+// those of the iteration's parity.
+// w and r' pass through the planes in place: element e of all three is read and written by
+// its owner alone, between the two exchanges.
+template <typename R, bool GEN, int RARE, class GP>
+__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
+    k_plane_cg(PlaneCgArgs<R> a) {
+  FAME_COUNT_LAUNCH();
+  if ((threadIdx.x | blockIdx.x | blockIdx.y | blockIdx.z) == 0) set_cond(a.reset, 0);
+  const Geom& g = a.g;
+  constexpr bool kAsyncMix = GP::kStatic;
+  __shared__ __align__(8) unsigned long long xbar;
+  __shared__ int skip;
+  __shared__ double s_coef[2];
+  const unsigned bar = smem_u32(&xbar);
+  {
+    const PlanePos p = plane_pos();
+    const Slot sl = a.slots[p.slot];
+    const CgState* st = a.cg + p.slot;
+    if (!sl.active || !st->active) return;  // uniform over the cluster
+    const int cur = st->iter & 1;
+    // this CTA's own part of r, r_old, x and x_old: it streams into L2 during the transforms
+    long i0, i1;
+    if (a.self_pf && threadIdx.x < (st->iter == 1 ? 2 : st->iter == 2 ? 6 : 8) &&
+        plane_vec_range(GP::P(g), p.s, p.comp, sl, i0, i1)) {
+      const int which = threadIdx.x >> 1;
+      const cplx<R>* v = which == 0 ? a.r[cur] : which == 1 ? a.r[cur ^ 1] : which == 2 ? a.x[cur] : a.x[cur ^ 1];
+      prefetch_l2(v + (long)p.slot * a.vstride + ((threadIdx.x & 1) ? sl.Nd : 0) + i0, (i1 - i0) * sizeof(cplx<R>));
+    }
+    if (kAsyncMix && threadIdx.x == 0) exchange_init(bar, &skip, a.fault);
+    const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
+    const cplx<R>* T = a.T + plane_base<R, GP>(g, p, 1, a.fstride);
+    if constexpr (!GEN) plane_load<R, GEN, GP>(g, T, m);
+    plane_tables<R, GEN, GP>(g, a.tw, a.tabs + (size_t)p.slot * g.tab_stride, p.s, m);
+    if constexpr (GEN) {
+      __syncthreads();  // D_ky is in place
+      plane_load<R, GEN, GP>(g, T, m);
+    }
+    // gamma and rho from the pencil stage's partial sums of <r, A r>, summed in order by one warp
+    // while the plane streams in (k_cg_decide forms the same numbers for the CG state)
+    if (threadIdx.x < 32) {
+      const double rAr = warp_sum_partials(a.partials + (size_t)p.slot * a.pstride, a.pen_parts) / g.N;
+      double gm, rho;
+      cg_coefficients(*st, rAr, gm, rho);
+      if (threadIdx.x == 0) {
+        s_coef[0] = gm;
+        s_coef[1] = rho;
+      }
+    }
+    if constexpr (!GEN) cp_async_wait_all();
+    __syncthreads();
+  }
+  plane_forward<R, GEN, RARE, GP>(g, a.tabs, a.dkz);
+  double acc[1] = {0.0};
+  {
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();  // all three component planes transformed (and the barriers in place)
+    if constexpr (kAsyncMix) {
+      if (*cl.map_shared_rank(&skip, 0)) {
+        cl.sync();  // rank 0's marker stays readable until all three have read it
+        return;
+      }
+      if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, (unsigned)(GP::P(g) * sizeof(cplx<R>)));
+    }
+    const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
+    const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
+    const Div dlf(Lf);
+    const PlanePos p = plane_pos();
+    const Slot sl = a.slots[p.slot];
+    const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
+    const cplx<R> lz = GEN ? mk<R>(0, 0) : cvt<R>(tab[g.oLz + p.s]);
+    const PlaneExchange<R, kAsyncMix> ex(m.plane, bar);
+    const int iter = a.cg[p.slot].iter, cur = iter & 1;
+    const bool have_r = iter > 1, have_x = iter > 2;  // r_old = 0 at k = 1; x = 0 at k = 1, x_old = 0 at k = 2
+    const long vb = (long)p.slot * a.vstride;
+    const cplx<R>*rc = a.r[cur] + vb, *xc = a.x[cur] + vb;
+    cplx<R>*ro = a.r[cur ^ 1] + vb, *xo = a.x[cur ^ 1] + vb;
+    // rho gamma and rho - 1 (rho = 1 at k = 1)
+    const R rg = (R)(s_coef[0] * s_coef[1]), rm = (R)(s_coef[1] - 1.0);
+    const int Nd = sl.Nd, off = sl.off;
+    const int per = (P + 2) / 3;
+    const int e0 = p.comp * per, e1 = min(P, e0 + per);
+    constexpr int KB = 2;
+    const int NT = GP::plane_threads();
+    for (int eb = e0 + threadIdx.x; eb < e1; eb += KB * NT) {
+      cplx<R> t[KB][3], R1[KB], R2[KB], O1[KB], O2[KB], X1[KB], X2[KB], Y1[KB], Y2[KB];
+#pragma unroll
+      for (int k = 0; k < KB; k++) {
+        const int e = eb + k * NT;
+        const int fi = p.s * P + e;
+        R1[k] = R2[k] = O1[k] = O2[k] = X1[k] = X2[k] = Y1[k] = Y2[k] = mk<R>(0, 0);
+        t[k][0] = t[k][1] = t[k][2] = mk<R>(0, 0);
+        if (e < e1 && fi >= off) {
+          const long i = fi - off;
+          R1[k] = rc[i];
+          R2[k] = rc[Nd + i];
+          if (have_r) {
+            O1[k] = ro[i];
+            O2[k] = ro[Nd + i];
+            X1[k] = xc[i];
+            X2[k] = xc[Nd + i];
+          }
+          if (have_x) {
+            Y1[k] = xo[i];
+            Y2[k] = xo[Nd + i];
+          }
+          const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), q = r * S + (e - r * Lf);
+#pragma unroll
+          for (int c = 0; c < 3; c++) t[k][c] = ex.dst[c][q];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < KB; k++) {
+        const int e = eb + k * NT;
+        if (e >= e1) break;
+        const int fi = p.s * P + e;
+        const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - r * Lf;
+        cplx<R> v[3] = {mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0)};
+        if (fi >= off) {
+          const long i = fi - off;
+          cplx<R> Lx, Ly, Lz;
+          lam_elem<R, GEN>(g, tab, m.lx, m.ly, lz, p.s, r, f, Lx, Ly, Lz);
+          cplx<R> Pc[6];
+          pi_from<R>(GEN, false, Lx, Ly, Lz, Pc);
+          const cplx<R> w1 = cadd(cadd(cmulc(Pc[0], t[k][0]), cmulc(Pc[1], t[k][1])), cmulc(Pc[2], t[k][2]));
+          const cplx<R> w2 = cadd(cadd(cmulc(Pc[3], t[k][0]), cmulc(Pc[4], t[k][1])), cmulc(Pc[5], t[k][2]));
+          // x' = x + rho gamma r + (rho - 1)(x - x_old), r' the same with -w: the corrections added to x and r
+          const cplx<R> n1 = cfma_r(csub(R1[k], O1[k]), rm, cfma_r(w1, -rg, R1[k]));
+          const cplx<R> n2 = cfma_r(csub(R2[k], O2[k]), rm, cfma_r(w2, -rg, R2[k]));
+          ro[i] = n1;
+          ro[Nd + i] = n2;
+          xo[i] = cfma_r(csub(X1[k], Y1[k]), rm, cfma_r(R1[k], rg, X1[k]));
+          xo[Nd + i] = cfma_r(csub(X2[k], Y2[k]), rm, cfma_r(R2[k], rg, X2[k]));
+          acc[0] += (double)(cabs2(n1) + cabs2(n2));
+#pragma unroll
+          for (int c = 0; c < 3; c++) v[c] = cadd(cmul(Pc[c], n1), cmul(Pc[3 + c], n2));
+        }
+        ex.put(r * S + f, v);
+      }
+    }
+    // All P values have arrived: every CTA has read its elements of this plane too, since an
+    // owner sends an element after reading it.
+    if constexpr (kAsyncMix)
+      exchange_wait(bar, a.fault);
+    else
+      cl.sync();
+  }
+  plane_inverse<R, GEN, RARE, GP>(g, a.tabs, a.dkz);
+  plane_store<R, GEN, GP>(g, a.T + plane_base<R, GP>(g, plane_pos(), 1, a.fstride));
+  // this CTA's part of ||r'||^2; k_cg_decide sums the slot's parts in order
+  __shared__ double sred[32];
+  block_reduce<1>(acc, sred);
+  if (threadIdx.x == 0) a.partials[(size_t)blockIdx.z * a.pstride + a.pen_parts + blockIdx.x] = acc[0];
 }
 
 // ------------------------------------------------------------------ pencil stage
 
-// grid = (Lm * ceil(Lf/TW), 3 * vec_per_slot, nslots), kPencilThreads threads
+// Pencil CTAs per SM the register budget is sized for: the prime passes (RARE 2) and the static
+// FP64 plans need 128 registers.
+template <typename R, int RARE, class GP> constexpr int pencil_min_blocks() {
+  return RARE >= 2 || (GP::kStatic && sizeof(R) == 8) ? 2 : 3;
+}
+
+// One CTA transforms TW consecutive positions e = m * Lf + f of the plane (a tile may span
+// rows, so only the last tile of a plane has idle lines).
+// grid = (ceil(P / TW), 3 * vec_per_slot, nslots), GP::pencil_threads() threads
 template <typename R, bool GEN, int MODE, int RARE, class GP>
-__global__ void __launch_bounds__(kPencilThreads, GP::kStatic ? (sizeof(R) == 4 ? 3 : 2) : 3)
+__global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>())
     k_pencil(PencilArgs<R> a) {
   FAME_COUNT_LAUNCH();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Geom& g = a.g;
   constexpr int TW = PencilTW<R>::v;
-  const int Lf = GP::Lf(g), Ls = GP::Ls(g), P = GP::P(g);
+  const int Lf = GP::Lf(g), Ls = GP::Ls(g), P = GP::P(g), NT = GP::pencil_threads();
   // shared memory: tile [Ls][TW] | 1/eps tile [Ls][TW] (PEN_QBQ) | slow-axis twiddles [Ls]
   cplx<R>* tile = reinterpret_cast<cplx<R>*>(smem_raw);
   R* ibt = reinterpret_cast<R*>(tile + Ls * TW);
@@ -351,85 +567,105 @@ __global__ void __launch_bounds__(kPencilThreads, GP::kStatic ? (sizeof(R) == 4 
   if (a.gate == 1 && !a.cg[slot].active) return;
   if (a.gate == 2 && !a.cg[slot].outer_active) return;
   const int comp = blockIdx.y % 3, vec = blockIdx.y / 3;
-  const int nft = (Lf + TW - 1) / TW;
-  const int m = blockIdx.x / nft;
-  const int f0 = (blockIdx.x - m * nft) * TW;
-  const int tw_n = min(TW, Lf - f0);
+  const int e0 = blockIdx.x * TW;
+  const int tw_n = min(TW, P - e0);
   if constexpr (MODE == PEN_QBQ_CG) {
     // the field rows and 1/eps rows of the tile of the CTA one wave ahead
     int x2, y2, z2;
-    if (a.pf_dist > 0 && threadIdx.x < 2 * Ls && cta_of(cta_linear() + a.pf_dist, x2, y2, z2) &&
-        a.slots[z2].active && a.cg[z2].active) {
-      const int m2 = x2 / nft, f2 = (x2 - m2 * nft) * TW, c2 = y2 % 3, v2 = y2 / 3;
-      const int n2 = min(TW, Lf - f2);
-      const int srow = threadIdx.x < Ls ? threadIdx.x : threadIdx.x - Ls;
-      const long off = (long)c2 * g.N + (long)srow * P + m2 * Lf + f2;
-      if (threadIdx.x < Ls)
-        prefetch_l2(a.T + (long)(z2 * a.vec_per_slot + v2) * a.fstride + off, n2 * sizeof(cplx<R>));
-      else
-        prefetch_l2(a.invB + off, n2 * sizeof(R));
+    if (a.pf_dist > 0 && cta_of(cta_linear() + a.pf_dist, x2, y2, z2) && a.slots[z2].active && a.cg[z2].active) {
+      const int f2 = x2 * TW, c2 = y2 % 3, v2 = y2 / 3;
+      const int n2 = min(TW, P - f2);
+      for (int i = threadIdx.x; i < 2 * Ls; i += NT) {
+        const long off = (long)c2 * g.N + (long)(i < Ls ? i : i - Ls) * P + f2;
+        if (i < Ls)
+          prefetch_l2(a.T + (long)(z2 * a.vec_per_slot + v2) * a.fstride + off, n2 * sizeof(cplx<R>));
+        else
+          prefetch_l2(a.invB + off, n2 * sizeof(R));
+      }
     }
   }
   const double2* tab = a.tabs + (size_t)slot * g.tab_stride;
-  for (int i = threadIdx.x; i < Ls; i += kPencilThreads) tws[i] = a.tw[g.tws + i];
+  for (int i = threadIdx.x; i < Ls; i += NT) tws[i] = a.tw[g.tws + i];
   const long fb = (long)(slot * a.vec_per_slot + vec) * a.fstride + (long)comp * g.N;
-  // ---- load.  Full tiles of the QBQ stream the field rows (TW contiguous
-  // elements at stride P) and the 1/eps rows (1/eps in the field layout) straight
-  // into shared memory with 16-byte cp.async copies.
+  const Div dlf(Lf);
+  // spatial index of slow position s at plane position e (QR_OUT, QRS_IN, 1/eps in the
+  // spatial layout)
+  auto spatial = [&](int s, int e) -> long {
+    if (!GEN) return (long)s * P + e;
+    const int m = (int)dlf.q(e);
+    return ((long)(e - m * Lf) * g.Ny + m) * g.Nx + s;
+  };
+  auto dk_at = [&](int s, int e) -> double2 {  // D_k (Simple) or D_kx
+    if (GEN) return tab[g.oDkx + s];
+    const int m = (int)dlf.q(e);
+    return cmul(cmul(tab[g.oDz + s], tab[g.oDy + m]), tab[g.oDx + (e - m * Lf)]);
+  };
+  // ---- load.  The QBQ streams the field rows (TW contiguous elements at stride P) and
+  // the 1/eps rows (1/eps in the field layout) straight into shared memory with
+  // cp.async: 16 bytes a copy when every row starts on a 16-byte boundary (P a
+  // multiple of the copy's elements, the base aligned), else one element.
   constexpr int CH = 16 / sizeof(cplx<R>);    // elements per 16-byte copy
   constexpr int CHB = 16 / sizeof(R);         // 1/eps values per 16-byte copy
-  const bool ib_field = !GEN || a.ib_field;  // 1/eps rows contiguous along the tile's fast positions
-  const bool async_tile = QBQ && ib_field && tw_n == TW && Lf % CHB == 0;
-  if (async_tile) {
-    for (int q = threadIdx.x; q < Ls * (TW / CH); q += kPencilThreads) {
-      const int s = q / (TW / CH), c = q - s * (TW / CH);
-      cp_async16(tile + s * TW + c * CH, a.T + fb + (long)s * P + m * Lf + f0 + c * CH);
-    }
-    for (int q = threadIdx.x; q < Ls * (TW / CHB); q += kPencilThreads) {
-      const int s = q / (TW / CHB), c = q - s * (TW / CHB);
-      cp_async16(ibt + s * TW + c * CHB, a.invB + (long)comp * g.N + (long)s * P + m * Lf + f0 + c * CHB);
-    }
-  } else {
-  for (int q = threadIdx.x; q < Ls * TW; q += kPencilThreads) {
-    const int s = q / TW, f = q - s * TW;
-    cplx<R> v = mk<R>(0, 0);
-    if (f < tw_n) {
-      if constexpr (MODE == PEN_QRS_IN) {
-        // spatial input, x conj(D) before the forward transform
-        long sp;
-        cplx<R> d;
-        if (!GEN) {
-          sp = (long)s * P + m * Lf + f0 + f;
-          const double2 dd = cmul(cmul(tab[g.oDz + s], tab[g.oDy + m]), tab[g.oDx + f0 + f]);
-          d = cvt<R>(cconj(dd));
-        } else {
-          sp = ((long)(f0 + f) * g.Ny + m) * g.Nx + s;
-          d = cvt<R>(cconj(tab[g.oDkx + s]));
-        }
-        v = cmul(a.in[(long)(slot * a.vec_per_slot + vec) * a.fstride + (long)comp * g.N + sp], d);
-      } else {
-        v = a.T[fb + (long)s * P + m * Lf + f0 + f];
+  const bool ib_field = !GEN || a.ib_field;  // 1/eps rows contiguous along the tile's positions
+  if constexpr (QBQ) {
+    const cplx<R>* src = a.T + fb + e0;
+    if (CH == 1 || P % CH == 0) {
+      for (int q = threadIdx.x; q < Ls * (TW / CH); q += NT) {
+        const int s = q / (TW / CH), c = (q - s * (TW / CH)) * CH;
+        if (c < tw_n) cp_async16(tile + s * TW + c, src + (long)s * P + c);
+      }
+    } else {
+      for (int q = threadIdx.x; q < Ls * TW; q += NT) {
+        const int s = q / TW, c = q - s * TW;
+        if (c < tw_n) cp_async_elem(tile + q, src + (long)s * P + c);
       }
     }
-    tile[q] = v;
+    if (ib_field) {
+      const R* ib = a.invB + (long)comp * g.N + e0;
+      if (P % CHB == 0 && ((uintptr_t)a.invB & 15) == 0) {
+        for (int q = threadIdx.x; q < Ls * (TW / CHB); q += NT) {
+          const int s = q / (TW / CHB), c = (q - s * (TW / CHB)) * CHB;
+          if (c < tw_n) cp_async16(ibt + s * TW + c, ib + (long)s * P + c);
+        }
+      } else {
+        for (int q = threadIdx.x; q < Ls * TW; q += NT) {
+          const int s = q / TW, c = q - s * TW;
+          if (c < tw_n) cp_async_real(ibt + q, ib + (long)s * P + c);
+        }
+      }
+    }
+    cp_async_wait_all();
+  } else {
+    for (int q = threadIdx.x; q < Ls * TW; q += NT) {
+      const int s = q / TW, f = q - s * TW;
+      cplx<R> v = mk<R>(0, 0);
+      if (f < tw_n) {
+        if constexpr (MODE == PEN_QRS_IN) {
+          // spatial input, x conj(D) before the forward transform
+          v = cmul(a.in[(long)(slot * a.vec_per_slot + vec) * a.fstride + (long)comp * g.N + spatial(s, e0 + f)],
+                   cvt<R>(cconj(dk_at(s, e0 + f))));
+        } else {
+          v = a.T[fb + (long)s * P + e0 + f];
+        }
+      }
+      tile[q] = v;
+    }
   }
-  }
-  if (async_tile) cp_async_wait_all();
   __syncthreads();
   // QBQ: inverse, x B^{-1}/N, forward.  QR_OUT: inverse, x D/N (and B^{-1}), store.
   // QRS_IN: forward only.  One FFT call site (dir loop) for the register budget.
   constexpr int ndir = QBQ ? 2 : 1;
   // PEN_QBQ_CG: sum of |v|^2 / eps over the tile after the inverse transform
-  float dot = 0.f;
+  R dot = 0;
   constexpr bool kStatQBQ = GP::kStatic && QBQ;  // whole tiles, 1/eps staged in shared memory
   if constexpr (kStatQBQ) {
     GP::template fft_slow_c<R, true>(tile, tws);
     const R invN = (R)(1.0 / g.N);
 #pragma unroll 4
-    for (int q = threadIdx.x; q < Ls * TW; q += kPencilThreads) {
+    for (int q = threadIdx.x; q < Ls * TW; q += NT) {
       const R ib = ibt[q];
       const cplx<R> v = tile[q];
-      if constexpr (MODE == PEN_QBQ_CG) dot += (float)(ib * cabs2(v));
+      if constexpr (MODE == PEN_QBQ_CG) dot += ib * cabs2(v);
       if constexpr (sizeof(R) == 4)
         tile[q] = pscale(v, ib * invN);
       else
@@ -443,25 +679,16 @@ __global__ void __launch_bounds__(kPencilThreads, GP::kStatic ? (sizeof(R) == 4 
     GP::template fft_slow<R, RARE>(tile, g, tws, inv);
     if (MODE != PEN_QRS_IN && dir == 0) {
       const R invN = (R)(1.0 / g.N);
-      for (int q = threadIdx.x; q < Ls * TW; q += kPencilThreads) {
+      for (int q = threadIdx.x; q < Ls * TW; q += NT) {
         const int s = q / TW, f = q - s * TW;
         if (f < tw_n) {
-          long sp;
-          if (!GEN)
-            sp = (long)s * P + m * Lf + f0 + f;
-          else
-            sp = ((long)(f0 + f) * g.Ny + m) * g.Nx + s;
           if constexpr (QBQ) {
-            const long ii = ib_field ? (long)s * P + m * Lf + f0 + f : sp;
-            const R ib = async_tile ? ibt[q] : a.invB[(long)comp * g.N + ii];
-            if constexpr (MODE == PEN_QBQ_CG) dot += (float)(ib * cabs2(tile[q]));
+            const R ib = ib_field ? ibt[q] : a.invB[(long)comp * g.N + spatial(s, e0 + f)];
+            if constexpr (MODE == PEN_QBQ_CG) dot += ib * cabs2(tile[q]);
             tile[q] = cscale(tile[q], ib * invN);
           } else {
-            cplx<R> d;
-            if (!GEN)
-              d = cvt<R>(cmul(cmul(tab[g.oDz + s], tab[g.oDy + m]), tab[g.oDx + f0 + f]));
-            else
-              d = cvt<R>(tab[g.oDkx + s]);
+            const long sp = spatial(s, e0 + f);
+            const cplx<R> d = cvt<R>(dk_at(s, e0 + f));
             cplx<R> v = cscale(cmul(tile[q], d), invN);
             if (a.invB) v = cscale(v, a.invB[(long)comp * g.N + sp]);
             a.out[(long)(slot * a.vec_per_slot + vec) * a.fstride + (long)comp * g.N + sp] = v;
@@ -472,17 +699,17 @@ __global__ void __launch_bounds__(kPencilThreads, GP::kStatic ? (sizeof(R) == 4 
     }
   }
   if constexpr (QBQ || MODE == PEN_QRS_IN) {
-    for (int q = threadIdx.x; q < Ls * TW; q += kPencilThreads) {
+    for (int q = threadIdx.x; q < Ls * TW; q += NT) {
       const int s = q / TW, f = q - s * TW;
-      if (f < tw_n) a.T[fb + (long)s * P + m * Lf + f0 + f] = tile[q];
+      if (f < tw_n) a.T[fb + (long)s * P + e0 + f] = tile[q];
     }
   }
   if constexpr (MODE == PEN_QBQ_CG) {
-    // <p, Ap> for A = Q_r^* B^-1 Q_r: Q_r^* is N times the adjoint of Q_r (unnormalised
-    // forward DFT against the 1/N-scaled inverse), so <p, Ap> = N ||B^-1/2 Q_r p||^2 =
-    // (1/N) sum_e |IDFT(Pi p)_e|^2 / eps_e, real and positive (CG.cu:57-63, with
-    // Zdotc(p, Ap) formed in the field domain).  This CTA writes its partial sum; the
-    // forward plane stage sums the slot's partials in order and forms a = ||r||^2 / <p, Ap>.
+    // <v, Av> for A = Q_r^* B^-1 Q_r: Q_r^* is N times the adjoint of Q_r (unnormalised
+    // forward DFT against the 1/N-scaled inverse), so <v, Av> = N ||B^-1/2 Q_r v||^2 =
+    // (1/N) sum_e |IDFT(Pi v)_e|^2 / eps_e, real and positive (CG.cu:57-63, with Zdotc
+    // formed in the field domain).  This CTA writes its partial sum; the CG plane stage
+    // sums the slot's partials in order.
     double acc[1] = {(double)dot};
     __shared__ double sred[32];
     block_reduce<1>(acc, sred);
@@ -541,7 +768,8 @@ __device__ __forceinline__ void pencil_pipe_issue(const PencilArgs<R>& a, int t,
   }
 }
 
-template <typename R>
+// DOT: also the partial sum of <v, Av> of every tile (PEN_QBQ_CG).
+template <typename R, bool DOT>
 __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_pencil_pipe(PencilArgs<R> a) {
   FAME_COUNT_LAUNCH();
   using GP = Stat96;
@@ -556,6 +784,7 @@ __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_penc
   cplx<R>* tiles = reinterpret_cast<cplx<R>*>(smem_raw);     // [2][TILE]
   R* ibts = reinterpret_cast<R*>(tiles + 2 * TILE);            // [2][TILE]
   cplx<R>* tws = reinterpret_cast<cplx<R>*>(ibts + 2 * TILE);  // [Ls]
+  __shared__ double sred[32];
   for (int i = threadIdx.x; i < Ls; i += kPencilThreads) tws[i] = a.tw[g.tws + i];
   const int total = a.nslots * 3 * a.vec_per_slot * Lm * nft;
   int t = blockIdx.x;
@@ -569,13 +798,17 @@ __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_penc
     __syncthreads();
     if (pencil_pipe_live(a, t)) {  // uniform over the CTA
       cplx<R>* tile = tiles + b * TILE;
+      double dot[1] = {0.0};
       // inverse, x B^{-1}/N, forward; one FFT call site for the register budget
       for (int dir = 0; dir < 2; dir++) {
         GP::template fft_slow<R, 0>(tile, g, tws, dir == 0);
         if (dir == 0) {
           const R invN = (R)(1.0 / g.N);
           const R* ibt = ibts + b * TILE;
-          for (int q = threadIdx.x; q < TILE; q += kPencilThreads) tile[q] = cscale(tile[q], ibt[q] * invN);
+          for (int q = threadIdx.x; q < TILE; q += kPencilThreads) {
+            if constexpr (DOT) dot[0] += (double)(ibt[q] * cabs2(tile[q]));
+            tile[q] = cscale(tile[q], ibt[q] * invN);
+          }
           __syncthreads();
         }
       }
@@ -586,6 +819,11 @@ __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_penc
         const int s = q / TW, f = q - s * TW;
         a.T[fb + (long)s * P + off + f] = tile[q];
       }
+      if constexpr (DOT) {
+        const int per_slot = 3 * Lm * nft, slot = t / per_slot;
+        block_reduce<1>(dot, sred);
+        if (threadIdx.x == 0) a.partials[(size_t)slot * a.pstride + (t - slot * per_slot)] = dot[0];
+      }
     }
     __syncthreads();  // every thread is done with buffer b before it is refilled
   }
@@ -593,171 +831,93 @@ __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_penc
 }
 
 // ------------------------------------------------------------------ plane stage (forward)
-
-// End of a loop body in the forward plane stage: the last CTA of the grid decides
-// whether the loop (EPI_RESID: outer refinement, EPI_CGR: CG) runs again.  Every CTA,
-// live or not, arrives here once.
-template <int EPI, typename R>
-__device__ __forceinline__ void plane_fwd_decide(const PlaneOutArgs<R>& a) {
+// The last CTA of the grid decides whether the refinement loop runs again.  Every CTA, live or
+// not, arrives here once.
+template <typename R> __device__ __forceinline__ void plane_fwd_decide(const PlaneOutArgs<R>& a) {
   if (grid_last(a.counters + a.nslots, gridDim.x * gridDim.y * gridDim.z)) {
     if (threadIdx.x == 0) {
       int any = 0;
-      for (int q = 0; q < a.nslots; q++)
-        any |= a.slots[q].active && (EPI == EPI_RESID ? a.cg[q].outer_active : a.cg[q].active);
+      for (int q = 0; q < a.nslots; q++) any |= a.slots[q].active && a.cg[q].outer_active;
       decide_cond(a.cond, any);
     }
   }
 }
 
 template <typename R, bool GEN, int EPI, bool PR, int RARE, class GP>
-__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::kMaxPlaneThreads, GP::template plane_min_blocks<R, RARE>())
+__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
     k_plane_fwd(PlaneOutArgs<R> a) {
   FAME_COUNT_LAUNCH();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
   const Geom& g = a.g;
-  const int Lf = GP::Lf(g), Lm = GP::Lm(g), S = GP::S(g), P = GP::P(g);
-  const Div dlf(Lf);  // row of plane element e: e / Lf (folds to a constant for static geometries)
-  cplx<R>* plane = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* twf = plane + Lm * S;  // plane rows have the odd pitch S >= Lf
-  cplx<R>* twm = twf + Lf;
-  cplx<R>* lx = twm + Lm;
-  cplx<R>* ly = lx + Lf;
-  cg::cluster_group cl = cg::this_cluster();
-  const int comp = (int)cl.block_rank();
-  const int s = blockIdx.x / 3;
-  const int vec = blockIdx.y;
-  const int slot = blockIdx.z;
-  const Slot sl = a.slots[slot];
-  bool live = sl.active;
-  if constexpr (EPI == EPI_CG || EPI == EPI_CGR) live = live && a.cg[slot].active;
-  if constexpr (EPI == EPI_RESID) live = live && a.cg[slot].outer_active;
-  if (!live) {
-    if constexpr (EPI == EPI_RESID) plane_fwd_decide<EPI>(a);
-    return;
-  }
-  if constexpr (EPI == EPI_CGR) {
-    // this CTA's own residual, read in the epilogue: it streams into L2 during the transforms
-    long i0, i1;
-    if (a.self_pf && threadIdx.x < 2 && plane_vec_range(P, s, comp, sl, i0, i1))
-      prefetch_l2(a.r + (long)(slot * a.vec_per_slot + vec) * a.vstride + (threadIdx.x ? sl.Nd : 0) + i0,
-                  (i1 - i0) * sizeof(cplx<R>));
-  }
-  if constexpr (EPI == EPI_CGR) {
-    // the field plane (4 pieces) and the residual of the CTA one wave ahead
-    int x2, y2, z2;
-    if (a.pf_dist > 0 && threadIdx.x < 6 && cta_of(cta_linear() + a.pf_dist, x2, y2, z2)) {
-      const Slot s2 = a.slots[z2];
-      if (s2.active && a.cg[z2].active) {
-        const int s2p = x2 / 3, c2 = x2 % 3;
-        if (threadIdx.x < 4) {
-          const long piece = (P + 3) / 4;
-          const long lo = threadIdx.x * piece, hi = min((long)P, lo + piece);
-          prefetch_l2(a.T + (long)(z2 * a.vec_per_slot + y2) * a.fstride + (long)c2 * g.N + (long)s2p * P + lo,
-                      (hi - lo) * sizeof(cplx<R>));
-        } else {
-          long i0, i1;
-          if (plane_vec_range(P, s2p, c2, s2, i0, i1))
-            prefetch_l2(a.r + (long)(z2 * a.vec_per_slot + y2) * a.vstride + ((threadIdx.x & 1) ? s2.Nd : 0) + i0,
-                        (i1 - i0) * sizeof(cplx<R>));
-        }
-      }
+  {
+    const PlanePos p = plane_pos();
+    bool live = a.slots[p.slot].active;
+    if constexpr (EPI == EPI_RESID) live = live && a.cg[p.slot].outer_active;
+    if (!live) {
+      if constexpr (EPI == EPI_RESID) plane_fwd_decide(a);
+      return;
     }
-  }
-  const double2* tab = a.tabs + (size_t)slot * g.tab_stride;
-  for (int i = threadIdx.x; i < Lf; i += GP::plane_threads()) {
-    twf[i] = a.tw[g.twf + i];
-    if constexpr (!GEN) lx[i] = cvt<R>(tab[g.oLx + i]);
-  }
-  for (int i = threadIdx.x; i < Lm; i += GP::plane_threads()) {
-    twm[i] = a.tw[g.twm + i];
-    if constexpr (!GEN) ly[i] = cvt<R>(tab[g.oLy + i]);
-  }
-  const cplx<R> lz = GEN ? mk<R>(0, 0) : cvt<R>(tab[g.oLz + s]);
-  const cplx<R>* T = a.T + (long)(slot * a.vec_per_slot + vec) * a.fstride + (long)comp * g.N + (long)s * P;
-  for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
-    const int m = GP::kStatic ? e / Lf : (int)dlf.q(e);
-    cp_async_elem(plane + e + m * (S - Lf), T + e);
-  }
-  __shared__ R s_step;
-  if constexpr (EPI == EPI_CGR) {
-    // the CG step a = ||r||^2 / <p, Ap> from the pencil stage's partial sums of this
-    // k-point, summed in order by one warp while the plane streams in (k_cg_decide forms
-    // the same sum for the solution update and the CG state)
-    if (threadIdx.x < 32) {
-      const double pAp = warp_sum_partials(a.partials + (size_t)slot * a.pstride, a.pen_parts) / g.N;
-      if (threadIdx.x == 0) s_step = (R)(pAp > 0 ? a.cg[slot].r1 / pAp : 0.0);
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  // forward 2-D transform.  General lattices (T*, FAME_FFT_CUDA.cu:128-150):
-  // x conj(D_ky), y (mid) pass, x conj(D_kz), z (fast) pass.  Simple lattices:
-  // fast then mid axis, no twiddles.
-  if constexpr (GP::kStatic && !GEN) {
-    GP::template fft_plane_c<R, true, false>(plane, twf);
-    GP::template fft_plane_c<R, false, false>(plane, twm);
-  }
-  for (int ax = 0; !(GP::kStatic && !GEN) && ax < 2; ax++) {
-    const bool fast = GEN ? ax == 1 : ax == 0;
+    const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
+    const cplx<R>* T = a.T + plane_base<R, GP>(g, p, a.vec_per_slot, a.fstride);
+    if constexpr (!GEN) plane_load<R, GEN, GP>(g, T, m);
+    plane_tables<R, GEN, GP>(g, a.tw, a.tabs + (size_t)p.slot * g.tab_stride, p.s, m);
     if constexpr (GEN) {
-      for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
-        const int m = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - m * Lf;
-        const int q = m * S + f;
-        plane[q] = cmul(plane[q], ax == 0 ? cvt<R>(cconj(tab[g.oDky + s * g.Ny + m]))
-                                          : cconj(dkz_at<R>(g, tab, s, m, f)));
-      }
-      __syncthreads();
+      __syncthreads();  // D_ky is in place
+      plane_load<R, GEN, GP>(g, T, m);
+    } else {
+      cp_async_wait_all();
     }
-    GP::template fft_plane<R, RARE>(plane, g, fast, fast ? twf : twm, false);
+    __syncthreads();
   }
+  plane_forward<R, GEN, RARE, GP>(g, a.tabs, a.dkz);
+  cg::cluster_group cl = cg::this_cluster();
   cl.sync();  // all three component planes transformed
 
-  const cplx<R>* src[3] = {cl.map_shared_rank(plane, 0), cl.map_shared_rank(plane, 1),
-                           cl.map_shared_rank(plane, 2)};
+  const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
+  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
+  const Div dlf(Lf);
+  const PlanePos p = plane_pos();
+  const Slot sl = a.slots[p.slot];
+  const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
+  const cplx<R> lz = GEN ? mk<R>(0, 0) : cvt<R>(tab[g.oLz + p.s]);
+  const cplx<R>* src[3] = {cl.map_shared_rank(m.plane, 0), cl.map_shared_rank(m.plane, 1),
+                           cl.map_shared_rank(m.plane, 2)};
   const int per = (P + 2) / 3;
-  const int e0 = comp * per, e1 = min(P, e0 + per);
+  const int e0 = p.comp * per, e1 = min(P, e0 + per);
   const int Nd = sl.Nd, off = sl.off;
-  const long vb = (long)(slot * a.vec_per_slot + vec) * a.vstride;
-  double acc[2] = {0.0, 0.0};
+  const long vb = (long)(p.slot * a.vec_per_slot + p.vec) * a.vstride;
+  double acc[1] = {0.0};
   // 3 -> 2 unmix and the epilogue.  The three components (remote shared memory) and
   // the vector operand of KB points per thread are read up front, so one latency of
   // each kind covers KB points.
   constexpr int KB = GP::kStatic ? 4 : 2;
   const int NT = GP::plane_threads();
-  R are = 0, aim = 0;
-  if constexpr (EPI == EPI_CGR) are = s_step;  // real: <p, Ap> > 0
   for (int eb = e0 + threadIdx.x; eb < e1; eb += KB * NT) {
     cplx<R> t[KB][3], va[KB], vb2[KB];
 #pragma unroll
     for (int k = 0; k < KB; k++) {
       const int e = eb + k * NT;
-      const int fi = s * P + e;
+      const int fi = p.s * P + e;
+      va[k] = vb2[k] = t[k][0] = t[k][1] = t[k][2] = mk<R>(0, 0);
       if (e < e1 && fi >= off) {
         const long i = fi - off;
-        const int m = GP::kStatic ? e / Lf : (int)dlf.q(e), q = m * S + (e - m * Lf);
+        const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), q = r * S + (e - r * Lf);
 #pragma unroll
         for (int c = 0; c < 3; c++) t[k][c] = src[c][q];
-        if constexpr (EPI == EPI_CG) {
-          va[k] = a.p[vb + i];
-          vb2[k] = a.p[vb + Nd + i];
-        } else if constexpr (EPI == EPI_RESID) {
+        if constexpr (EPI == EPI_RESID) {
           va[k] = a.b[vb + i];
           vb2[k] = a.b[vb + Nd + i];
-        } else if constexpr (EPI == EPI_CGR) {
-          va[k] = a.r[vb + i];
-          vb2[k] = a.r[vb + Nd + i];
         }
       }
     }
 #pragma unroll
     for (int k = 0; k < KB; k++) {
       const int e = eb + k * NT;
-      const int fi = s * P + e;
+      const int fi = p.s * P + e;
       if (e >= e1 || fi < off) continue;
       const long i = fi - off;
-      const int m = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - m * Lf;
+      const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - r * Lf;
       cplx<R> Lx, Ly, Lz;
-      lam_elem<R, GEN>(g, tab, lx, ly, lz, s, m, f, Lx, Ly, Lz);
+      lam_elem<R, GEN>(g, tab, m.lx, m.ly, lz, p.s, r, f, Lx, Ly, Lz);
       cplx<R> Pc[6];
       pi_from<R>(GEN, PR, Lx, Ly, Lz, Pc);
       const cplx<R> t0 = t[k][0], t1 = t[k][1], t2 = t[k][2];
@@ -766,30 +926,10 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::kMaxPlaneThreads
       if constexpr (EPI == EPI_OUT) {
         a.out[vb + i] = o1;
         a.out[vb + Nd + i] = o2;
-      } else if constexpr (EPI == EPI_CG) {
-        a.out[vb + i] = o1;
-        a.out[vb + Nd + i] = o2;
-        const cplx<R> d = cadd(cmulc(va[k], o1), cmulc(vb2[k], o2));  // conj(p) Ap
-        acc[0] += (double)d.x;
-        acc[1] += (double)d.y;
-      } else if constexpr (EPI == EPI_RESID) {
+      } else {  // EPI_RESID
         const cplx<R> r1 = csub(va[k], o1), r2 = csub(vb2[k], o2);
         a.out[vb + i] = r1;
         a.out[vb + Nd + i] = r2;
-        acc[0] += (double)(cabs2(r1) + cabs2(r2));
-      } else {  // EPI_CGR: r -= a Ap and ||r||^2 (CG.cu:71-76); Ap is never stored
-        cplx<R> r1 = va[k], r2 = vb2[k];
-        if constexpr (sizeof(R) == 4) {  // real step size: packed pairs
-          r1 = pfma(o1, -are, r1);
-          r2 = pfma(o2, -are, r2);
-        } else {
-          r1.x -= are * o1.x - aim * o1.y;
-          r1.y -= are * o1.y + aim * o1.x;
-          r2.x -= are * o2.x - aim * o2.y;
-          r2.y -= are * o2.y + aim * o2.x;
-        }
-        a.r[vb + i] = r1;
-        a.r[vb + Nd + i] = r2;
         acc[0] += (double)(cabs2(r1) + cabs2(r2));
       }
     }
@@ -799,38 +939,23 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::kMaxPlaneThreads
   // until all three CTAs have read it.
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
 
-  if constexpr (EPI == EPI_CGR) {
-    // this CTA's part of ||r||^2; k_cg_decide sums the slot's parts in order
+  if constexpr (EPI == EPI_RESID) {
     __shared__ double sred[32];
-    double acc1[1] = {acc[0]};
-    block_reduce<1>(acc1, sred);
-    if (threadIdx.x == 0) a.partials[(size_t)slot * a.pstride + a.pen_parts + blockIdx.x] = acc1[0];
-  }
-  if constexpr (EPI == EPI_CG || EPI == EPI_RESID) {
-    __shared__ double sred[2 * 32];
-    block_reduce<2>(acc, sred);
+    block_reduce<1>(acc, sred);
     const int nblk = gridDim.x;  // CTAs of this slot (vec_per_slot == 1 in solves)
-    double tot[2];
-    if (slot_reduce<2>(acc, a.partials + (size_t)slot * nblk * 2, a.counters + slot, blockIdx.x, nblk,
-                       tot)) {
+    double tot[1];
+    if (slot_reduce<1>(acc, a.partials + (size_t)p.slot * nblk, a.counters + p.slot, blockIdx.x, nblk, tot)) {
       if (threadIdx.x == 0) {
-        CgState* st = a.cg + slot;
-        if constexpr (EPI == EPI_CG) {
-          // a = r1 / dot  (CG.cu:60-63)
-          const double den = tot[0] * tot[0] + tot[1] * tot[1];
-          st->a_re = st->r1 * tot[0] / den;
-          st->a_im = -st->r1 * tot[1] / den;
-        } else {
-          st->rr = tot[0];
-          st->outer++;
-          st->outer_total++;
-          st->outer_active = (tot[0] > a.tol2) && (st->outer < st->outer_max);
-          st->scale = 1.0 / sqrt(tot[0] > 0 ? tot[0] : 1.0);
-        }
+        CgState* st = a.cg + p.slot;
+        st->rr = tot[0];
+        st->outer++;
+        st->outer_total++;
+        st->outer_active = (tot[0] > a.tol2) && (st->outer < st->outer_max);
+        st->scale = 1.0 / sqrt(tot[0] > 0 ? tot[0] : 1.0);
         __threadfence();
       }
     }
-    if constexpr (EPI == EPI_RESID) plane_fwd_decide<EPI>(a);
+    plane_fwd_decide(a);
   }
   asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");  // every CTA has read this plane
 }

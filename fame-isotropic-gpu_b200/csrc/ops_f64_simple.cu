@@ -1,4 +1,4 @@
-// Operator stage kernels, FP64, Simple lattices, radices 2, 3, 4, 5, 8.
+// Operator stage kernels, FP64, Simple lattices, radices 2 to 13.
 #include "op_kernels.cuh"
 
 namespace fame {
@@ -6,10 +6,11 @@ template __global__ void k_plane_inv<double, false, IN_CG, false, 0, DynGeom>(Pl
 template __global__ void k_plane_inv<double, false, IN_VEC, false, 0, DynGeom>(PlaneInArgs<double>);
 template __global__ void k_plane_inv<double, false, IN_VEC, true, 0, DynGeom>(PlaneInArgs<double>);
 template __global__ void k_plane_inv<double, false, IN_REFINE, false, 0, DynGeom>(PlaneInArgs<double>);
+template __global__ void k_plane_cg<double, false, 0, DynGeom>(PlaneCgArgs<double>);
 template __global__ void k_pencil<double, false, PEN_QBQ, 0, DynGeom>(PencilArgs<double>);
+template __global__ void k_pencil<double, false, PEN_QBQ_CG, 0, DynGeom>(PencilArgs<double>);
 template __global__ void k_pencil<double, false, PEN_QR_OUT, 0, DynGeom>(PencilArgs<double>);
 template __global__ void k_pencil<double, false, PEN_QRS_IN, 0, DynGeom>(PencilArgs<double>);
-template __global__ void k_plane_fwd<double, false, EPI_CG, false, 0, DynGeom>(PlaneOutArgs<double>);
 template __global__ void k_plane_fwd<double, false, EPI_OUT, false, 0, DynGeom>(PlaneOutArgs<double>);
 template __global__ void k_plane_fwd<double, false, EPI_OUT, true, 0, DynGeom>(PlaneOutArgs<double>);
 template __global__ void k_plane_fwd<double, false, EPI_RESID, false, 0, DynGeom>(PlaneOutArgs<double>);

@@ -6,10 +6,11 @@ template __global__ void k_plane_inv<double, false, IN_CG, false, 2, DynGeom>(Pl
 template __global__ void k_plane_inv<double, false, IN_VEC, false, 2, DynGeom>(PlaneInArgs<double>);
 template __global__ void k_plane_inv<double, false, IN_VEC, true, 2, DynGeom>(PlaneInArgs<double>);
 template __global__ void k_plane_inv<double, false, IN_REFINE, false, 2, DynGeom>(PlaneInArgs<double>);
+template __global__ void k_plane_cg<double, false, 2, DynGeom>(PlaneCgArgs<double>);
 template __global__ void k_pencil<double, false, PEN_QBQ, 2, DynGeom>(PencilArgs<double>);
+template __global__ void k_pencil<double, false, PEN_QBQ_CG, 2, DynGeom>(PencilArgs<double>);
 template __global__ void k_pencil<double, false, PEN_QR_OUT, 2, DynGeom>(PencilArgs<double>);
 template __global__ void k_pencil<double, false, PEN_QRS_IN, 2, DynGeom>(PencilArgs<double>);
-template __global__ void k_plane_fwd<double, false, EPI_CG, false, 2, DynGeom>(PlaneOutArgs<double>);
 template __global__ void k_plane_fwd<double, false, EPI_OUT, false, 2, DynGeom>(PlaneOutArgs<double>);
 template __global__ void k_plane_fwd<double, false, EPI_OUT, true, 2, DynGeom>(PlaneOutArgs<double>);
 template __global__ void k_plane_fwd<double, false, EPI_RESID, false, 2, DynGeom>(PlaneOutArgs<double>);

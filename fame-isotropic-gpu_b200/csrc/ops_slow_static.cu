@@ -9,6 +9,7 @@ namespace fame {
   template __global__ void k_pencil<float, true, PEN_QR_OUT, 0, DynGeomSlow<LS>>(PencilArgs<float>);   \
   template __global__ void k_pencil<float, true, PEN_QRS_IN, 0, DynGeomSlow<LS>>(PencilArgs<float>);   \
   template __global__ void k_pencil<double, true, PEN_QBQ, 0, DynGeomSlow<LS>>(PencilArgs<double>);    \
+  template __global__ void k_pencil<double, true, PEN_QBQ_CG, 0, DynGeomSlow<LS>>(PencilArgs<double>); \
   template __global__ void k_pencil<double, true, PEN_QR_OUT, 0, DynGeomSlow<LS>>(PencilArgs<double>); \
   template __global__ void k_pencil<double, true, PEN_QRS_IN, 0, DynGeomSlow<LS>>(PencilArgs<double>);
 FAME_SLOW_PENCILS(48)

@@ -45,7 +45,8 @@
 namespace fame {
 
 // defined with the solver (solver_kernels.cuh, solver.cu)
-__global__ void k_tables(Geom g, const Slot* slots, double2* tabs, double m1, double m2, double m3);
+__global__ void k_tables(Geom g, const Slot* slots, double2* tabs, double m1, double m2, double m3, double2* dkz64,
+                         float2* dkz32);
 void set_last_error(const std::string& s);
 
 namespace {
@@ -77,7 +78,8 @@ __global__ void k_static_prep(Slot sl, Geom g, Slot* slot, double2* tw) {
 }
 
 template <typename K> cudaError_t raise_smem(K* k, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
+  // (the 48 KB that need no opt-in hold the kernel's static shared memory too)
+  if (bytes <= 40 * 1024) return cudaSuccess;
   return cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
@@ -123,8 +125,7 @@ cudaError_t launch_qbq(const Geom& g, int threads, const Slot* slot, const doubl
   ap.ib_field = 0;  // the caller's 1/eps is in the spatial layout
   ap.nslots = 1;
   ap.TW = TW;
-  const int nft = (g.Lf + TW - 1) / TW;
-  kpen<<<dim3(g.Lm * nft, 3, 1), dim3(kPencilThreads), sm_pen, st>>>(ap);
+  kpen<<<dim3((g.P + TW - 1) / TW, 3, 1), dim3(pencil_threads_rule<double>(g, pencil_level(g), 1)), sm_pen, st>>>(ap);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
 
   PlaneOutArgs<double> ao;
@@ -164,7 +165,7 @@ int fame_qbq_static(const fame_lattice* lat, const double* k, const double* inv_
     return rc;
   }
   const int rare = geom_level(g);
-  const int threads = plane_threads_rule<double>(g, rare);
+  const int threads = plane_threads_rule<double>(g, rare, g.Ls);
   const size_t off_tw = align256(sizeof(Slot));
   const size_t off_tab = off_tw + align256(sizeof(double2) * (size_t)(g.Lf + g.Lm + g.Ls));
   const size_t off_T = off_tab + align256(sizeof(double2) * (size_t)g.tab_stride);
@@ -209,7 +210,7 @@ int fame_qbq_static(const fame_lattice* lat, const double* k, const double* inv_
   }
   const int tmax = std::max({g.Nx * g.Ny, g.Nx, g.Ny, g.Nz});
   k_tables<<<dim3((tmax + 255) / 256, 1), dim3(256), 0, st>>>(g, slot, tabs, (double)lat->m[0], (double)lat->m[1],
-                                                              (double)lat->m[2]);
+                                                              (double)lat->m[2], nullptr, nullptr);
   if ((e = cudaGetLastError()) != cudaSuccess) {
     set_last_error(std::string("table launch: ") + cudaGetErrorString(e));
     return FAME_ERR_CUDA;
@@ -217,13 +218,11 @@ int fame_qbq_static(const fame_lattice* lat, const double* k, const double* inv_
   const double2* xd = (const double2*)x;
   double2* yd = (double2*)y;
   if (g.general)
-    e = rare == 2   ? launch_qbq<true, 2>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st)
-        : rare == 1 ? launch_qbq<true, 1>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st)
-                    : launch_qbq<true, 0>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st);
+    e = rare == 2 ? launch_qbq<true, 2>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st)
+                  : launch_qbq<true, 0>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st);
   else
-    e = rare == 2   ? launch_qbq<false, 2>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st)
-        : rare == 1 ? launch_qbq<false, 1>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st)
-                    : launch_qbq<false, 0>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st);
+    e = rare == 2 ? launch_qbq<false, 2>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st)
+                  : launch_qbq<false, 0>(g, threads, slot, tabs, tw, xd, inv_b, T, yd, st);
   if (e != cudaSuccess) {
     set_last_error(std::string("QBQ launch: ") + cudaGetErrorString(e));
     return FAME_ERR_CUDA;

@@ -33,10 +33,6 @@ unsigned long long launches_ops_f32_simple();
 unsigned long long launches_ops_f32_general();
 unsigned long long launches_ops_f64_simple();
 unsigned long long launches_ops_f64_general();
-unsigned long long launches_ops_f32_simple_rare();
-unsigned long long launches_ops_f32_general_rare();
-unsigned long long launches_ops_f64_simple_rare();
-unsigned long long launches_ops_f64_general_rare();
 unsigned long long launches_ops_f32_simple_prime();
 unsigned long long launches_ops_f32_general_prime();
 unsigned long long launches_ops_f64_simple_prime();
@@ -81,16 +77,19 @@ struct fame_ctx {
   fame_lattice lat;
   Geom g;
   cudaStream_t stream = nullptr;
-  int plane_threads = 512;    // threads of a runtime-geometry plane CTA
-  int plane_threads32 = 512;  // the same for FP32 kernels
-  template <typename R> int plane_nt() const { return sizeof(R) == 4 ? plane_threads32 : plane_threads; }
   int pipe_ctas64 = 0;  // resident k_pencil_pipe<double> CTAs on the device
   int prefetch = 0;     // L2 prefetch one wave ahead in the CG stage kernels (fame_set_option; measured slower)
   int self_prefetch = 1;  // CG plane stages: L2 prefetch of the CTA's own operands at its start
   int radix_order = 0;  // kRadixOrders index of the runtime-geometry axis plans
   int threads32_opt = 0, threads64_opt = 0;  // plane CTA sizes set by fame_set_option (0: rule)
+  // threads of a runtime-geometry plane CTA in a launch of `planes` planes (an option below what
+  // the axis plans need is raised to it)
+  template <typename R> int plane_nt(long planes) const {
+    const int opt = sizeof(R) == 4 ? threads32_opt : threads64_opt;
+    return opt ? std::max(opt, plane_threads_min<R>(g)) : plane_threads_rule<R>(g, rare, planes);
+  }
   std::map<const void*, int> waves;  // resident CTAs of a stage kernel on the device
-  int rare = 0;      // fft_lines level the plane axes need: 0 radix 2-8, 1 + 7/11/13, 2 + primes >= 17
+  int rare = 0;      // pass level of the plane axes: 2 with prime factors >= 17, 1 with 7, 11 or 13
   int rare_pen = 0;  // the same for the pencil (slow) axis
   int static_planes = 1;  // static plane plans where instantiated (option "static_planes")
   // An automatic batch of at least 4 k-points per lane is split into `lanes` contiguous
@@ -127,8 +126,11 @@ struct fame_ctx {
   DBuf<double> partials, T0, T1, hcoef, theta, Z, G, stats;
   DBuf<unsigned> counters, tri_ctr;
   DBuf<int> map, prof, status, flags;
-  DBuf<double2> U, r64, x64, b64, p64, Ap64, T64, EV, AV, Tb, E;
-  DBuf<float2> r32, x32, p32, T32;
+  // CG vectors r and x come in pairs, the buffer of odd iterations first (r64, r64b ...)
+  DBuf<double2> U, r64, x64, b64, r64b, x64b, T64, EV, AV, Tb, E;
+  DBuf<float2> r32, x32, r32b, x32b, T32;
+  DBuf<double2> dkz64;  // General lattices: D_kz of every slot
+  DBuf<float2> dkz32;
   int* hflag = nullptr;  // pinned
   // eigenvectors kept on the device by the last solve (evec_out NULL): its k-points,
   // whether each is the Gamma point (Gamma keeps nwant - 2 restored bands), nwant
@@ -156,30 +158,20 @@ template <typename R> static int pencil_tw() { return PencilTW<R>::v; }
 template <typename R> static size_t pencil_smem(const Geom& g) { return pencil_smem_bytes<R>(g.Ls); }
 
 template <typename K> static void allow_smem(K* k, size_t bytes) {
-  if (bytes > 48 * 1024) FAME_CK(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  // (the 48 KB that need no opt-in hold the kernel's static shared memory too)
+  if (bytes > 40 * 1024) FAME_CK(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
-// CTAs of a stage kernel resident on the whole device at once (one wave): clusters of
-// three CTAs for the plane kernels (cluster = 3), single CTAs for the pencil kernels.
-// Cached per kernel in the context; 0 if the occupancy query fails.
-template <typename K> static int wave_ctas(fame_ctx* c, K* k, int threads, size_t smem, int cluster) {
+// CTAs of a pencil kernel resident on the whole device at once (one wave).  Cached per kernel in the
+// context; 0 if the occupancy query fails.
+template <typename K> static int wave_ctas(fame_ctx* c, K* k, int threads, size_t smem) {
   auto it = c->waves.find((const void*)k);
   if (it != c->waves.end()) return it->second;
-  int n = 0, dev = 0, sms = 0;
-  if (cluster > 1) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cluster * 64, 1, 1);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    int ncl = 0;
-    if (cudaOccupancyMaxActiveClusters(&ncl, (const void*)k, &cfg) == cudaSuccess) n = ncl * cluster;
-  } else {
-    int per = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) ==
-                                                   cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k, threads, smem) == cudaSuccess)
-      n = per * sms;
-  }
+  int n = 0, dev = 0, sms = 0, per = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k, threads, smem) == cudaSuccess)
+    n = per * sms;
   cudaGetLastError();  // a failed query only disables the prefetch
   c->waves[(const void*)k] = n;
   return n;
@@ -237,19 +229,30 @@ struct Ops {
     return 0;
   }
 
-  // partial sums per slot of the fused FP32 CG kernels: the pencil stage's <p, Ap>
-  // (one per CTA of a slot), then the forward plane stage's ||r||^2
-  int cg_pen_parts() const { return 3 * g().Lm * ((g().Lf + pencil_tw<float>() - 1) / pencil_tw<float>()); }
+  // partial sums per slot of the CG kernels: the pencil stage's <r, A r> (one per tile of a
+  // slot), then the plane stage's ||r||^2
+  template <typename R> int cg_pen_parts() const { return 3 * ((g().P + pencil_tw<R>() - 1) / pencil_tw<R>()); }
   int cg_fwd_parts() const { return 3 * g().Ls; }
 
-  // end of a fused FP32 CG iteration: step size, r1, beta, counters, loop decision
-  void cg_decide(Cond cond) {
+  // per-slot tables, with D_kz in the precisions that are allocated (General lattices)
+  void tables(bool d64, bool d32) {
+    const Geom& q = g();
+    int n = std::max({q.Nx * q.Ny, q.Nx, q.Ny, q.Nz});
+    if (q.general && (d64 || d32)) n = std::max(n, q.N);
+    P.launch(k_tables, dim3((n + 255) / 256, nslots), dim3(256), 0, q, (const Slot*)c->slots.p, c->tabs.p,
+             (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2],
+             q.general && d64 ? c->dkz64.p : (double2*)nullptr, q.general && d32 ? c->dkz32.p : (float2*)nullptr);
+  }
+  template <typename R> const cplx<R>* dkz() const;
+
+  // CG coefficients kept, counters, loop decision
+  template <typename R> void cg_decide(Cond cond) {
     CgDecideArgs d;
     d.slots = c->slots.p;
     d.cg = c->cg.p;
     d.partials = c->partials.p;
     d.pstride = c->part_stride;
-    d.pen_parts = cg_pen_parts();
+    d.pen_parts = cg_pen_parts<R>();
     d.fwd_parts = cg_fwd_parts();
     d.N = g().N;
     d.counters = c->counters.p;
@@ -258,69 +261,102 @@ struct Ops {
     P.launch(k_cg_decide, dim3(nslots), dim3(32), 0, d);
   }
 
-  // plane inverse stage
-  template <typename R, int IN, bool PR>
-  void plane_inv(const cplx<R>* in, cplx<R>* T, int nvec, long vstride, long fstride, int sigma,
-                 cplx<R>* p = nullptr, const cplx<R>* r = nullptr, double2* y64 = nullptr,
-                 const float2* x32 = nullptr, Cond reset = Cond{}, cplx<R>* x = nullptr,
-                 const float2* p32 = nullptr) {
-    PlaneInArgs<R> a;
-    a.reset = reset;
+  // What the plane kernels share: geometry, tables, twiddles; then the launch of kernel k
+  // (static plane plans: `pick` swaps in the kernel and its thread count).
+  template <typename R, typename A> A plane_args() const {
+    A a;
+    memset(&a, 0, sizeof(a));
     a.g = g();
     a.slots = c->slots.p;
     a.tabs = c->tabs.p;
+    a.dkz = g().general ? dkz<R>() : nullptr;
     a.tw = tw<R>();
-    a.vstride = vstride;
-    a.fstride = fstride;
+    a.vstride = 2L * g().N;
+    a.fstride = 3L * g().N;
+    return a;
+  }
+  template <typename R, typename A> void plane_launch(void (*k)(A), int nt, int nvec, const A& a) {
+    const size_t sm = plane_smem<R>(g());
+    allow_smem(k, sm);
+    P.launch(k, dim3(3 * g().Ls, nvec, nslots), dim3(nt), sm, a);
+  }
+
+  // plane inverse stage (the arguments of the input mode are set by the callers below)
+  template <typename R, int IN, bool PR> void plane_inv(PlaneInArgs<R> a, cplx<R>* T, int nvec) {
     a.vec_per_slot = nvec;
-    a.in = in;
-    a.p = p;
-    a.r = r;
     a.cg = c->cg.p;
-    a.y64 = y64;
-    a.x32 = x32;
-    a.x = x;
-    a.p32 = p32;
-    a.sigma = sigma;
     a.T = T;
     a.fault = c->flags.p ? c->flags.p + kFaultFlag : nullptr;
-    const size_t sm = plane_smem<R>(g());
-    dim3 grid(3 * g().Ls, nvec, nslots);
+    int nt = c->template plane_nt<R>((long)g().Ls * nvec * nslots);
     if (g().general) {
-      auto k = c->rare == 2   ? k_plane_inv<R, true, IN, PR, 2, DynGeom>
-               : c->rare == 1 ? k_plane_inv<R, true, IN, PR, 1, DynGeom>
-                              : k_plane_inv<R, true, IN, PR, 0, DynGeom>;
-      int nt = c->template plane_nt<R>();
+      auto k = c->rare == 2 ? k_plane_inv<R, true, IN, PR, 2, DynGeom> : k_plane_inv<R, true, IN, PR, 0, DynGeom>;
       if constexpr (kPlanInv<R, IN, PR>) {
         const int pp = plane_plan();
-        if (pp == 1) k = k_plane_inv<R, true, IN, PR, 0, PlaneFcc64>, nt = PlaneFcc64::kMaxPlaneThreads;
-        if (pp == 2) k = k_plane_inv<R, true, IN, PR, 0, PlaneBcc48>, nt = PlaneBcc48::kMaxPlaneThreads;
-        if (pp == 3) {
-          if constexpr (sizeof(R) == 4)
-            k = k_plane_inv<R, true, IN, PR, 0, PlaneHex128f>, nt = PlaneHex128f::kMaxPlaneThreads;
-          else
-            k = k_plane_inv<R, true, IN, PR, 0, PlaneHex128d>, nt = PlaneHex128d::kMaxPlaneThreads;
-        }
+        if (pp == 1) k = k_plane_inv<R, true, IN, PR, 0, PlaneFcc64<R>>, nt = PlaneFcc64<R>::kMaxPlaneThreads;
+        if (pp == 2) k = k_plane_inv<R, true, IN, PR, 0, PlaneBcc48<R>>, nt = PlaneBcc48<R>::kMaxPlaneThreads;
+        if (pp == 3) k = k_plane_inv<R, true, IN, PR, 0, PlaneHex128<R>>, nt = PlaneHex128<R>::kMaxPlaneThreads;
       }
-      allow_smem(k, sm);
-      a.pf_dist = IN == IN_CG && c->prefetch ? wave_ctas(c, k, nt, sm, 3) : 0;
-      a.self_pf = c->self_prefetch;
-      P.launch(k, grid, dim3(nt), sm, a);
+      plane_launch<R>(k, nt, nvec, a);
     } else {
-      auto k = c->rare == 2   ? k_plane_inv<R, false, IN, PR, 2, DynGeom>
-               : c->rare == 1 ? k_plane_inv<R, false, IN, PR, 1, DynGeom>
-                              : k_plane_inv<R, false, IN, PR, 0, DynGeom>;
-      int nt = c->template plane_nt<R>();
+      auto k = c->rare == 2 ? k_plane_inv<R, false, IN, PR, 2, DynGeom> : k_plane_inv<R, false, IN, PR, 0, DynGeom>;
       if constexpr (kStatInv<R, IN, PR>)
-        if (c->stat96) {
-          k = k_plane_inv<R, false, IN, PR, 0, Stat96>;
-          nt = kStatPlaneThreads;
-        }
-      allow_smem(k, sm);
-      a.pf_dist = IN == IN_CG && c->prefetch ? wave_ctas(c, k, nt, sm, 3) : 0;
-      a.self_pf = c->self_prefetch;
-      P.launch(k, grid, dim3(nt), sm, a);
+        if (c->stat96) k = k_plane_inv<R, false, IN, PR, 0, Stat96>, nt = kStatPlaneThreads;
+      plane_launch<R>(k, nt, nvec, a);
     }
+  }
+  template <typename R, bool PR> void plane_inv_vec(const cplx<R>* in, cplx<R>* T, int nvec, int sigma) {
+    auto a = plane_args<R, PlaneInArgs<R>>();
+    a.in = in;
+    a.sigma = sigma;
+    plane_inv<R, IN_VEC, PR>(a, T, nvec);
+  }
+
+  // CG plane stage and what starts a CG solve: the field of the start residual r[1]
+  template <typename R> void cg_start(cplx<R>* const (&r)[2], cplx<R>* T, const R* invB) {
+    auto a = plane_args<R, PlaneInArgs<R>>();
+    a.in = r[1];
+    plane_inv<R, IN_CG, false>(a, T, 1);
+    pencil<R, PEN_QBQ_CG>(T, 1, 3L * g().N, invB, 1);
+  }
+  template <typename R>
+  void plane_cg(cplx<R>* const (&r)[2], cplx<R>* const (&x)[2], cplx<R>* T, Cond reset) {
+    auto a = plane_args<R, PlaneCgArgs<R>>();
+    for (int i = 0; i < 2; i++) {
+      a.r[i] = r[i];
+      a.x[i] = x[i];
+    }
+    a.cg = c->cg.p;
+    a.T = T;
+    a.partials = c->partials.p;
+    a.pstride = c->part_stride;
+    a.pen_parts = cg_pen_parts<R>();
+    a.reset = reset;
+    a.self_pf = c->self_prefetch;
+    a.fault = c->flags.p ? c->flags.p + kFaultFlag : nullptr;
+    int nt = c->template plane_nt<R>((long)g().Ls * nslots);
+    if (g().general) {
+      auto k = c->rare == 2 ? k_plane_cg<R, true, 2, DynGeom> : k_plane_cg<R, true, 0, DynGeom>;
+      const int pp = plane_plan();
+      if (pp == 1) k = k_plane_cg<R, true, 0, PlaneFcc64<R>>, nt = PlaneFcc64<R>::kMaxPlaneThreads;
+      if (pp == 2) k = k_plane_cg<R, true, 0, PlaneBcc48<R>>, nt = PlaneBcc48<R>::kMaxPlaneThreads;
+      if (pp == 3) k = k_plane_cg<R, true, 0, PlaneHex128<R>>, nt = PlaneHex128<R>::kMaxPlaneThreads;
+      plane_launch<R>(k, nt, 1, a);
+    } else {
+      auto k = c->rare == 2 ? k_plane_cg<R, false, 2, DynGeom> : k_plane_cg<R, false, 0, DynGeom>;
+      if (c->stat96) k = k_plane_cg<R, false, 0, Stat96>, nt = kStatPlaneThreads;
+      plane_launch<R>(k, nt, 1, a);
+    }
+  }
+  // A CG solve from the start residual r[1]: while active, plane stage (with the vector
+  // updates), decision, pencil stage.  r[1] and the CG state are set before.
+  template <typename R>
+  void cg_solve(cplx<R>* const (&r)[2], cplx<R>* const (&x)[2], cplx<R>* T, const R* invB, Cond cond) {
+    cg_start<R>(r, T, invB);
+    P.while_loop(cond, [&] {
+      plane_cg<R>(r, x, T, cond);
+      cg_decide<R>(cond);
+      pencil<R, PEN_QBQ_CG>(T, 1, 3L * g().N, invB, 1);
+    });
   }
 
   template <typename R, int MODE>
@@ -341,38 +377,31 @@ struct Ops {
     a.cg = c->cg.p;
     a.gate = gate;
     a.partials = c->partials.p;
-    a.counters = c->counters.p;
     a.pstride = c->part_stride;
     a.TW = pencil_tw<R>();
     a.nslots = nslots;
     const size_t sm = pencil_smem<R>(g());
-    const int nft = (g().Lf + a.TW - 1) / a.TW;
-    dim3 grid(g().Lm * nft, 3 * nvec, nslots);
+    dim3 grid((g().P + a.TW - 1) / a.TW, 3 * nvec, nslots);
     a.pf_dist = 0;
+    int nt = pencil_threads_rule<R>(g(), c->rare_pen, (long)nvec * nslots);
     if (g().general) {
-      auto k = c->rare_pen == 2   ? k_pencil<R, true, MODE, 2, DynGeom>
-               : c->rare_pen == 1 ? k_pencil<R, true, MODE, 1, DynGeom>
-                              : k_pencil<R, true, MODE, 0, DynGeom>;
-      if constexpr (!(sizeof(R) == 8 && MODE == PEN_QBQ_CG))
-        if (c->rare_pen == 0) {  // static slow-axis plans (ops_slow_static.cu)
-          if (g().Ls == 48) k = k_pencil<R, true, MODE, 0, DynGeomSlow<48>>;
-          if (g().Ls == 64) k = k_pencil<R, true, MODE, 0, DynGeomSlow<64>>;
-          if (g().Ls == 128) k = k_pencil<R, true, MODE, 0, DynGeomSlow<128>>;
-        }
+      auto k = c->rare_pen == 2 ? k_pencil<R, true, MODE, 2, DynGeom> : k_pencil<R, true, MODE, 0, DynGeom>;
+      // static slow-axis plans (ops_slow_static.cu)
+      if (g().Ls == 48) k = k_pencil<R, true, MODE, 0, DynGeomSlow<48>>, nt = kPencilThreads;
+      if (g().Ls == 64) k = k_pencil<R, true, MODE, 0, DynGeomSlow<64>>, nt = kPencilThreads;
+      if (g().Ls == 128) k = k_pencil<R, true, MODE, 0, DynGeomSlow<128>>, nt = kPencilThreads;
       allow_smem(k, sm);
-      if (MODE == PEN_QBQ_CG && c->prefetch) a.pf_dist = wave_ctas(c, k, kPencilThreads, sm, 1);
-      P.launch(k, grid, dim3(kPencilThreads), sm, a);
+      if (MODE == PEN_QBQ_CG && c->prefetch) a.pf_dist = wave_ctas(c, k, nt, sm);
+      P.launch(k, grid, dim3(nt), sm, a);
     } else {
-      auto k = c->rare_pen == 2   ? k_pencil<R, false, MODE, 2, DynGeom>
-               : c->rare_pen == 1 ? k_pencil<R, false, MODE, 1, DynGeom>
-                              : k_pencil<R, false, MODE, 0, DynGeom>;
+      auto k = c->rare_pen == 2 ? k_pencil<R, false, MODE, 2, DynGeom> : k_pencil<R, false, MODE, 0, DynGeom>;
       if constexpr (kStatPen<R, MODE> && sizeof(R) == 4)
-        if (c->stat96) k = k_pencil<R, false, MODE, 0, Stat96>;
+        if (c->stat96) k = k_pencil<R, false, MODE, 0, Stat96>, nt = kPencilThreads;
       if constexpr (kStatPen<R, MODE> && sizeof(R) == 8)
         if (c->stat96) {
           // FP64: pipelined, as many CTAs as are resident, each walking tiles (the FP32
           // stage measured no faster this way: 13.5 against 13.1 us per k-point)
-          auto kp = k_pencil_pipe<R>;
+          auto kp = k_pencil_pipe<R, MODE == PEN_QBQ_CG>;
           const size_t smp = pencil_pipe_smem_bytes<R>(g().Ls);
           allow_smem(kp, smp);
           const int total = (int)(grid.x * grid.y * grid.z);
@@ -380,27 +409,18 @@ struct Ops {
           return;
         }
       allow_smem(k, sm);
-      if (MODE == PEN_QBQ_CG && c->prefetch) a.pf_dist = wave_ctas(c, k, kPencilThreads, sm, 1);
-      P.launch(k, grid, dim3(kPencilThreads), sm, a);
+      if (MODE == PEN_QBQ_CG && c->prefetch) a.pf_dist = wave_ctas(c, k, nt, sm);
+      P.launch(k, grid, dim3(nt), sm, a);
     }
   }
 
   template <typename R, int EPI, bool PR>
-  void plane_fwd(const cplx<R>* T, cplx<R>* out, int nvec, long vstride, long fstride,
-                 const cplx<R>* p = nullptr, const cplx<R>* b = nullptr, Cond cond = Cond{},
-                 double tol2 = 0, cplx<R>* r = nullptr) {
-    PlaneOutArgs<R> a;
-    a.r = r;
-    a.g = g();
-    a.slots = c->slots.p;
-    a.tabs = c->tabs.p;
-    a.tw = tw<R>();
-    a.vstride = vstride;
-    a.fstride = fstride;
+  void plane_fwd(const cplx<R>* T, cplx<R>* out, int nvec, const cplx<R>* b = nullptr, Cond cond = Cond{},
+                 double tol2 = 0) {
+    auto a = plane_args<R, PlaneOutArgs<R>>();
     a.vec_per_slot = nvec;
     a.T = T;
     a.out = out;
-    a.p = p;
     a.b = b;
     a.cg = c->cg.p;
     a.partials = c->partials.p;
@@ -408,49 +428,28 @@ struct Ops {
     a.cond = cond;
     a.nslots = nslots;
     a.tol2 = tol2;
-    a.pstride = c->part_stride;
-    a.pen_parts = cg_pen_parts();
-    const size_t sm = plane_smem<R>(g());
-    dim3 grid(3 * g().Ls, nvec, nslots);
+    int nt = c->template plane_nt<R>((long)g().Ls * nvec * nslots);
     if (g().general) {
-      auto k = c->rare == 2   ? k_plane_fwd<R, true, EPI, PR, 2, DynGeom>
-               : c->rare == 1 ? k_plane_fwd<R, true, EPI, PR, 1, DynGeom>
-                              : k_plane_fwd<R, true, EPI, PR, 0, DynGeom>;
-      int nt = c->template plane_nt<R>();
+      auto k = c->rare == 2 ? k_plane_fwd<R, true, EPI, PR, 2, DynGeom> : k_plane_fwd<R, true, EPI, PR, 0, DynGeom>;
       if constexpr (kPlanFwd<R, EPI, PR>) {
         const int pp = plane_plan();
-        if (pp == 1) k = k_plane_fwd<R, true, EPI, PR, 0, PlaneFcc64>, nt = PlaneFcc64::kMaxPlaneThreads;
-        if (pp == 2) k = k_plane_fwd<R, true, EPI, PR, 0, PlaneBcc48>, nt = PlaneBcc48::kMaxPlaneThreads;
-        if (pp == 3) {
-          if constexpr (sizeof(R) == 4)
-            k = k_plane_fwd<R, true, EPI, PR, 0, PlaneHex128f>, nt = PlaneHex128f::kMaxPlaneThreads;
-          else
-            k = k_plane_fwd<R, true, EPI, PR, 0, PlaneHex128d>, nt = PlaneHex128d::kMaxPlaneThreads;
-        }
+        if (pp == 1) k = k_plane_fwd<R, true, EPI, PR, 0, PlaneFcc64<R>>, nt = PlaneFcc64<R>::kMaxPlaneThreads;
+        if (pp == 2) k = k_plane_fwd<R, true, EPI, PR, 0, PlaneBcc48<R>>, nt = PlaneBcc48<R>::kMaxPlaneThreads;
+        if (pp == 3) k = k_plane_fwd<R, true, EPI, PR, 0, PlaneHex128<R>>, nt = PlaneHex128<R>::kMaxPlaneThreads;
       }
-      allow_smem(k, sm);
-      a.pf_dist = EPI == EPI_CGR && c->prefetch ? wave_ctas(c, k, nt, sm, 3) : 0;
-      a.self_pf = c->self_prefetch;
-      P.launch(k, grid, dim3(nt), sm, a);
+      plane_launch<R>(k, nt, nvec, a);
     } else {
-      auto k = c->rare == 2   ? k_plane_fwd<R, false, EPI, PR, 2, DynGeom>
-               : c->rare == 1 ? k_plane_fwd<R, false, EPI, PR, 1, DynGeom>
-                              : k_plane_fwd<R, false, EPI, PR, 0, DynGeom>;
-      int nt = c->template plane_nt<R>();
+      auto k = c->rare == 2 ? k_plane_fwd<R, false, EPI, PR, 2, DynGeom> : k_plane_fwd<R, false, EPI, PR, 0, DynGeom>;
       if constexpr (kStatFwd<R, EPI, PR>)
-        if (c->stat96) {
-          k = k_plane_fwd<R, false, EPI, PR, 0, Stat96>;
-          nt = kStatPlaneThreads;
-        }
-      allow_smem(k, sm);
-      a.pf_dist = EPI == EPI_CGR && c->prefetch ? wave_ctas(c, k, nt, sm, 3) : 0;
-      a.self_pf = c->self_prefetch;
-      P.launch(k, grid, dim3(nt), sm, a);
+        if (c->stat96) k = k_plane_fwd<R, false, EPI, PR, 0, Stat96>, nt = kStatPlaneThreads;
+      plane_launch<R>(k, nt, nvec, a);
     }
   }
 };
 template <> const double2* Ops::tw<double>() const { return c->tw64.p; }
 template <> const float2* Ops::tw<float>() const { return c->tw32.p; }
+template <> const double2* Ops::dkz<double>() const { return c->dkz64.p; }
+template <> const float2* Ops::dkz<float>() const { return c->dkz32.p; }
 
 // ------------------------------------------------------------------ geometry
 static int setup_geom(fame_ctx* c) {
@@ -475,10 +474,8 @@ static int setup_geom(fame_ctx* c) {
   }
   c->rare = plane_level(g);
   c->rare_pen = pencil_level(g);
-  c->plane_threads32 = plane_threads_rule<float>(g, c->rare);
-  c->plane_threads = plane_threads_rule<double>(g, c->rare);
   c->stat96 = !g.general && g.Nx == 96 && g.Ny == 96 && g.Nz == 96;
-  if (c->stat96) c->pipe_ctas64 = resident_ctas(k_pencil_pipe<double>, pencil_pipe_smem_bytes<double>(g.Ls));
+  if (c->stat96) c->pipe_ctas64 = resident_ctas(k_pencil_pipe<double, true>, pencil_pipe_smem_bytes<double>(g.Ls));
   // twiddles e^{-2 pi i m / n} for the fast, mid and slow axes
   std::vector<double2> tw;
   for (int n : {g.Lf, g.Lm, g.Ls})  // at g.twf, g.twm, g.tws
@@ -490,6 +487,18 @@ static int setup_geom(fame_ctx* c) {
   FAME_CK(cudaMemcpy(c->tw64.p, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice));
   FAME_CK(cudaMemcpy(c->tw32.p, tw32.data(), tw32.size() * sizeof(float2), cudaMemcpyHostToDevice));
   return FAME_OK;
+}
+
+// Lanczos vectors a restart after the first one keeps.  Plain FP64: nwant, as the reference does.
+// Mixed precision: three fifths of the way from nwant to nstep (thick restarts: Wu and Simon, SIAM
+// J. Matrix Anal. Appl. 22, 2000).  The first restart keeps nwant in both, and most k-points need
+// no other; one that does needs fewer steps this way (the 20-point 96^3 path: 100 -> 82 applies
+// where the second restart converges).  It also ends what could go on for a hundred restarts:
+// the FP32 rounding in A_r^-1 feeds every copy of a degenerate eigenvalue into the basis at about
+// the level of es_tol, and a restart that cuts a multiplet purges a copy, which grows back in
+// the next cycle (SC 16^3 at Gamma, nwant 4 of 3 + 3, nstep 20: 1460 applies, or none enough).
+static int keep_vectors(int nstep, int nwant, bool mixed) {
+  return mixed ? nwant + (nstep - nwant) * 3 / 5 : nwant;
 }
 
 static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool mixed, bool vec) {
@@ -522,13 +531,13 @@ static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool
   c->hcoef.ensure((size_t)nslots * 2 * (nstep + 2));
   c->theta.ensure((size_t)nslots * nstep);
   c->Z.ensure((size_t)nslots * nstep * nstep);
-  c->G.ensure((size_t)nslots * (nstep + 1) * (nwant + 1));
+  c->G.ensure((size_t)nslots * (nstep + 1) * (keep_vectors(nstep, nwant, mixed) + 1));
   c->stats.ensure((size_t)nslots * nwant * 8);
-  c->map.ensure((size_t)nslots * (nstep + 1) + (size_t)nslots * (nwant + 1));
+  c->map.ensure((size_t)nslots * (nstep + 1) + (size_t)nslots * (keep_vectors(nstep, nwant, mixed) + 1));
   c->prof.ensure((size_t)nslots * 3);
   c->status.ensure(nslots);
   c->flags.ensure(64);
-  const int nphys = nstep + 1 + nwant + 1;
+  const int nphys = nstep + 1 + keep_vectors(nstep, nwant, mixed) + 1;
   c->U.ensure((size_t)nslots * nphys * M);
   c->r64.ensure((size_t)nslots * M);
   c->x64.ensure((size_t)nslots * M);
@@ -540,13 +549,16 @@ static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool
     c->b64.ensure((size_t)nslots * M);
     c->r32.ensure((size_t)nslots * M);
     c->x32.ensure((size_t)nslots * M);
-    c->p32.ensure((size_t)nslots * M);
+    c->r32b.ensure((size_t)nslots * M);
+    c->x32b.ensure((size_t)nslots * M);
+    if (g.general) c->dkz32.ensure((size_t)nslots * N);
     c->T32.ensure((size_t)nslots * 3 * N);
   }
   // FP64 CG vectors: every context may run FP64 solves and A_r^-1 applies, whatever
   // precision it started with, so they grow with the slot count in both modes
-  c->p64.ensure((size_t)nslots * M);
-  c->Ap64.ensure((size_t)nslots * M);
+  c->r64b.ensure((size_t)nslots * M);
+  c->x64b.ensure((size_t)nslots * M);
+  if (g.general) c->dkz64.ensure((size_t)nslots * N);
   if (vec) c->E.ensure((size_t)nslots * nwant * 3 * N);
   c->bpart.ensure((size_t)nslots * nwant * kBandSplit * 4);
   c->cap_slots = nslots;
@@ -766,16 +778,9 @@ static void emit_step(Ops& o, const SolveCfg& s, LzArgs L, int j, int* flag_base
     Cond cc = loop_cond(P, flag_base, kLoopCG, s.ls_maxit + 2, s.loop_cap);
     P.launch(k_invar_pro<false>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(cc), L, j, c->r64.p, c->x64.p,
              (double2*)nullptr, tol2, s.ls_maxit);
-    P.while_loop(cc, [&] {
-      o.plane_inv<double, IN_CG, false>(nullptr, c->T64.p, 1, M, F, 0, c->p64.p, c->r64.p, nullptr, nullptr, cc,
-                                        c->x64.p);
-      o.pencil<double, PEN_QBQ>(c->T64.p, 1, F, c->ibq64(), 1);
-      o.plane_fwd<double, EPI_CG, false>(c->T64.p, c->Ap64.p, 1, M, F, c->p64.p);
-      P.launch(k_cg_update<double>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(cc), c->r64.p,
-               (const double2*)c->Ap64.p);
-    });
+    o.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
     P.launch(k_invar_epi<false>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L, j,
-             (const double2*)c->x64.p, (const double2*)c->p64.p);
+             (const double2*)c->x64.p, (const double2*)c->x64b.p);
   } else {
     Cond outer = loop_cond(P, flag_base, kLoopOuter, 42, s.loop_cap);
     Cond inner = loop_cond(P, flag_base, kLoopInner, s.inner_maxit + 2, s.loop_cap);
@@ -783,22 +788,15 @@ static void emit_step(Ops& o, const SolveCfg& s, LzArgs L, int j, int* flag_base
              c->b64.p, tol2, s.ls_maxit);
     P.while_loop(outer, [&] {
       P.launch(k_cg32_init, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(inner), (const double2*)c->r64.p,
-               c->r32.p, c->x32.p, s.inner_tol * s.inner_tol, s.inner_maxit, tol2, outer);
-      // FP32 CG per iteration: p and the deferred x update with the 2 -> 3 mix; the
-      // slow-axis transforms with the partial sums of <p, Ap>; the 3 -> 2 unmix with
-      // r -= a Ap and the partial sums of ||r||^2 (Ap is never stored); a one-warp-per-slot
-      // kernel that ends the iteration (step size, beta, loop decision)
-      P.while_loop(inner, [&] {
-        o.plane_inv<float, IN_CG, false>(nullptr, c->T32.p, 1, M, F, 0, c->p32.p, c->r32.p, nullptr, nullptr,
-                                         inner, c->x32.p);
-        o.pencil<float, PEN_QBQ_CG>(c->T32.p, 1, F, c->ibq32(), 1);
-        o.plane_fwd<float, EPI_CGR, false>(c->T32.p, nullptr, 1, M, F, nullptr, nullptr, inner, 0.0, c->r32.p);
-        o.cg_decide(inner);
-      });
-      o.plane_inv<double, IN_REFINE, false>(nullptr, c->T64.p, 1, M, F, 0, nullptr, nullptr, c->x64.p,
-                                            c->x32.p, Cond{}, nullptr, c->p32.p);
+               c->r32.p, s.inner_tol * s.inner_tol, s.inner_maxit, tol2, outer);
+      o.cg_solve<float>({c->r32b.p, c->r32.p}, {c->x32b.p, c->x32.p}, c->T32.p, c->ibq32(), inner);
+      auto a = o.plane_args<double, PlaneInArgs<double>>();
+      a.y64 = c->x64.p;
+      a.x32[0] = c->x32b.p;
+      a.x32[1] = c->x32.p;
+      o.plane_inv<double, IN_REFINE, false>(a, c->T64.p, 1);
       o.pencil<double, PEN_QBQ>(c->T64.p, 1, F, c->ibq64(), 2);
-      o.plane_fwd<double, EPI_RESID, false>(c->T64.p, c->r64.p, 1, M, F, nullptr, c->b64.p, outer, tol2);
+      o.plane_fwd<double, EPI_RESID, false>(c->T64.p, c->r64.p, 1, c->b64.p, outer, tol2);
     });
     P.launch(k_invar_epi<true>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L, j,
              (const double2*)c->x64.p, (const double2*)nullptr);
@@ -814,7 +812,8 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   const long M = 2L * g.N;
   const long F = 3L * g.N;
   const int nvb = vec_blocks(c, s.nslots);
-  const int nphys = s.nstep + 1 + s.nwant + 1;
+  const int nkeep = keep_vectors(s.nstep, s.nwant, s.mixed);
+  const int nphys = s.nstep + 1 + nkeep + 1;
   LzArgs L;
   L.U = c->U.p;
   L.ustride = M;
@@ -822,6 +821,7 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   L.map = c->map.p;
   L.nstep = s.nstep;
   L.nwant = s.nwant;
+  L.nkeep = nkeep;
   L.T0 = c->T0.p;
   L.T1 = c->T1.p;
   L.h = c->hcoef.p;
@@ -829,9 +829,7 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   L.prof = c->prof.p;
   L.status = c->status.p;
   int* flags = c->flags.p;
-  const int tmax = std::max({g.Nx * g.Ny, g.Nx, g.Ny, g.Nz});
-  P.launch(k_tables, dim3((tmax + 255) / 256, s.nslots), dim3(256), 0, g, (const Slot*)c->slots.p, c->tabs.p,
-           (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2]);
+  o.tables(true, s.mixed);
   P.launch(k_lz_init, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L);
   for (int j = 0; j < s.nstep; j++) emit_step(o, s, L, j, flags);
   Cond restart = loop_cond(P, flags, kLoopRestart, s.es_maxit + 2, s.loop_cap);
@@ -853,9 +851,9 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   P.launch(k_tridiag, dim3(s.nslots), dim3(32), tsm, ta);
   ta.first = 0;
   P.while_loop(restart, [&] {
-    for (int c0 = 0; c0 <= s.nwant; c0 += 8)
+    for (int c0 = 0; c0 <= nkeep; c0 += 8)
       P.launch(k_ugemm<8>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(restart), L, (const double*)c->G.p,
-               s.nstep + 1, s.nstep + 1, s.nwant + 1, 0, (double2*)nullptr, c0);
+               s.nstep + 1, s.nstep + 1, nkeep + 1, 0, (double2*)nullptr, c0);
     P.launch(k_remap, dim3(s.nslots), dim3(32), 0, L, (const Slot*)c->slots.p, s.nslots);
     for (int j = s.nwant; j < s.nstep; j++) emit_step(o, s, L, j, flags);
     P.launch(k_tridiag, dim3(s.nslots), dim3(32), tsm, ta);
@@ -865,9 +863,9 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
     P.launch(k_ugemm<8>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L, (const double*)c->Z.p,
              s.nstep, s.nstep, s.nwant, 1, c->EV.p, c0);
   // FP64 residual and Rayleigh quotient per band: v = QBQ(Sigma y)
-  o.plane_inv<double, IN_VEC, false>(c->EV.p, c->Tb.p, s.nwant, M, F, 1);
+  o.plane_inv_vec<double, false>(c->EV.p, c->Tb.p, s.nwant, 1);
   o.pencil<double, PEN_QBQ>(c->Tb.p, s.nwant, F, c->ibq64(), 0);
-  o.plane_fwd<double, EPI_OUT, false>(c->Tb.p, c->AV.p, s.nwant, M, F);
+  o.plane_fwd<double, EPI_OUT, false>(c->Tb.p, c->AV.p, s.nwant);
   P.launch(k_band_stats, dim3(kBandSplit, s.nwant, s.nslots), dim3(256), 0, o.va(Cond{}),
            (const double2*)c->EV.p, (const double2*)c->AV.p, M, s.nwant, (const double*)c->theta.p, s.nstep,
            c->bpart.p);
@@ -876,7 +874,7 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   if (s.vec || s.enorm) {
     // E = B^{-1} Q_r (Sigma ev), scaled by its norm (FAME_Fast_Algorithms_Isotropic.cu:107-122);
     // the norms go after the band statistics
-    o.plane_inv<double, IN_VEC, false>(c->EV.p, c->Tb.p, s.nwant, M, F, 1);
+    o.plane_inv_vec<double, false>(c->EV.p, c->Tb.p, s.nwant, 1);
     o.pencil<double, PEN_QR_OUT>(c->Tb.p, s.nwant, F, c->invB64.p, 0, c->E.p);
     P.launch(k_band_norm_part, dim3(kBandSplit, s.nwant, s.nslots), dim3(256), 0, (const Slot*)c->slots.p,
              (const double2*)c->E.p, F, s.nwant, F, c->bpart.p);
@@ -888,11 +886,12 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
 // Device bytes of one slot's workspace (the per-slot buffers of ensure_workspace).
 static double slot_bytes(const fame_ctx* c, int nstep, int nwant, bool mixed, bool vec) {
   const double N = c->g.N, M = 2.0 * N, z = 16.0;
-  double b = (nstep + 1 + nwant + 1) * M * z   // Lanczos basis U
+  double b = (nstep + 1 + keep_vectors(nstep, nwant, mixed) + 1) * M * z   // Lanczos basis U
              + 2 * M * z + 3 * N * z           // r64, x64, T64
              + 2 * nwant * M * z + nwant * 3 * N * z  // EV, AV, Tb
-             + 2 * M * z;                      // p64, Ap64
-  if (mixed) b += M * z + 3 * M * 8 + 3 * N * 8;  // b64, r32, x32, p32, T32
+             + 2 * M * z;                      // r64b, x64b
+  if (mixed) b += M * z + 4 * M * 8 + 3 * N * 8;  // b64, r32, x32, r32b, x32b, T32
+  if (c->g.general) b += N * (mixed ? 24 : 16);   // D_kz
   if (vec) b += nwant * 3 * N * z;               // E
   return b;
 }
@@ -979,10 +978,10 @@ void fame_ctx_destroy(fame_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->progs.clear();
-  for (auto* b : {&c->tw64, &c->tabs, &c->U, &c->r64, &c->x64, &c->b64, &c->p64, &c->Ap64, &c->T64, &c->EV,
-                  &c->AV, &c->Tb, &c->E})
+  for (auto* b : {&c->tw64, &c->tabs, &c->U, &c->r64, &c->x64, &c->b64, &c->r64b, &c->x64b, &c->T64, &c->EV,
+                  &c->AV, &c->Tb, &c->E, &c->dkz64})
     b->release();
-  for (auto* b : {&c->r32, &c->x32, &c->p32, &c->T32, &c->tw32}) b->release();
+  for (auto* b : {&c->r32, &c->x32, &c->r32b, &c->x32b, &c->T32, &c->tw32, &c->dkz32}) b->release();
   for (auto* b : {&c->invB64, &c->invB64q, &c->B64, &c->partials, &c->T0, &c->T1, &c->hcoef, &c->theta, &c->Z, &c->G,
                   &c->stats, &c->adj, &c->bpart, &c->adj_part})
     b->release();
@@ -1407,9 +1406,7 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
     Ops o{c, P, 1};
     const Geom& g = c->g;
     const long M = 2L * g.N, F = 3L * g.N;
-    const int tmax = std::max({g.Nx * g.Ny, g.Nx, g.Ny, g.Nz});
-    P.launch(k_tables, dim3((tmax + 255) / 256, 1), dim3(256), 0, g, (const Slot*)c->slots.p, c->tabs.p,
-             (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2]);
+    o.tables(precision == FAME_FP64, precision == FAME_MIXED);
     if (precision == FAME_FP64) {
       const double2* x = (const double2*)in;
       double2* y = (double2*)out;
@@ -1417,23 +1414,23 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
         case FAME_OP_QR:
         case FAME_OP_PR:
           if (op == FAME_OP_QR)
-            o.plane_inv<double, IN_VEC, false>(x, c->T64.p, 1, M, F, 0);
+            o.plane_inv_vec<double, false>(x, c->T64.p, 1, 0);
           else
-            o.plane_inv<double, IN_VEC, true>(x, c->T64.p, 1, M, F, 0);
+            o.plane_inv_vec<double, true>(x, c->T64.p, 1, 0);
           o.pencil<double, PEN_QR_OUT>(c->T64.p, 1, F, (const double*)nullptr, 0, y);
           break;
         case FAME_OP_QRS:
         case FAME_OP_PRS:
           o.pencil<double, PEN_QRS_IN>(c->T64.p, 1, F, (const double*)nullptr, 0, nullptr, x);
           if (op == FAME_OP_QRS)
-            o.plane_fwd<double, EPI_OUT, false>(c->T64.p, y, 1, M, F);
+            o.plane_fwd<double, EPI_OUT, false>(c->T64.p, y, 1);
           else
-            o.plane_fwd<double, EPI_OUT, true>(c->T64.p, y, 1, M, F);
+            o.plane_fwd<double, EPI_OUT, true>(c->T64.p, y, 1);
           break;
         case FAME_OP_QBQ:
-          o.plane_inv<double, IN_VEC, false>(x, c->T64.p, 1, M, F, 0);
+          o.plane_inv_vec<double, false>(x, c->T64.p, 1, 0);
           o.pencil<double, PEN_QBQ>(c->T64.p, 1, F, c->ibq64(), 0);
-          o.plane_fwd<double, EPI_OUT, false>(c->T64.p, y, 1, M, F);
+          o.plane_fwd<double, EPI_OUT, false>(c->T64.p, y, 1);
           break;
         case FAME_OP_INVAR: {
           // one A_r^{-1} apply through the solver's own invAr kernels (U column 0 -> 1)
@@ -1445,7 +1442,7 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
           L.nphys = nstep + 1 + nwant + 1;
           L.map = c->map.p;
           L.nstep = nstep;
-          L.nwant = nwant;
+          L.nwant = L.nkeep = nwant;
           L.T0 = c->T0.p;
           L.T1 = c->T1.p;
           L.h = c->hcoef.p;
@@ -1464,16 +1461,9 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
           Cond cc = loop_cond(P, c->flags.p, kLoopCG, s.ls_maxit + 2);
           P.launch(k_invar_pro<false>, dim3(nvb, 1, 1), dim3(256), 0, o.va(cc), L, 0, c->r64.p, c->x64.p,
                    (double2*)nullptr, s.ls_tol * s.ls_tol, s.ls_maxit);
-          P.while_loop(cc, [&] {
-            o.plane_inv<double, IN_CG, false>(nullptr, c->T64.p, 1, M, F, 0, c->p64.p, c->r64.p, nullptr, nullptr,
-                                              cc, c->x64.p);
-            o.pencil<double, PEN_QBQ>(c->T64.p, 1, F, c->ibq64(), 1);
-            o.plane_fwd<double, EPI_CG, false>(c->T64.p, c->Ap64.p, 1, M, F, c->p64.p);
-            P.launch(k_cg_update<double>, dim3(nvb, 1, 1), dim3(256), 0, o.va(cc), c->r64.p,
-                     (const double2*)c->Ap64.p);
-          });
+          o.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
           P.launch(k_invar_epi<false>, dim3(nvb, 1, 1), dim3(256), 0, o.va(Cond{}), L, 0,
-                   (const double2*)c->x64.p, (const double2*)c->p64.p);
+                   (const double2*)c->x64.p, (const double2*)c->x64b.p);
           FAME_CK(cudaMemcpyAsync(y, c->U.p + M, 2L * sl.Nd * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
           break;
         }
@@ -1485,23 +1475,23 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
         case FAME_OP_QR:
         case FAME_OP_PR:
           if (op == FAME_OP_QR)
-            o.plane_inv<float, IN_VEC, false>(x, c->T32.p, 1, M, F, 0);
+            o.plane_inv_vec<float, false>(x, c->T32.p, 1, 0);
           else
-            o.plane_inv<float, IN_VEC, true>(x, c->T32.p, 1, M, F, 0);
+            o.plane_inv_vec<float, true>(x, c->T32.p, 1, 0);
           o.pencil<float, PEN_QR_OUT>(c->T32.p, 1, F, (const float*)nullptr, 0, y);
           break;
         case FAME_OP_QRS:
         case FAME_OP_PRS:
           o.pencil<float, PEN_QRS_IN>(c->T32.p, 1, F, (const float*)nullptr, 0, nullptr, x);
           if (op == FAME_OP_QRS)
-            o.plane_fwd<float, EPI_OUT, false>(c->T32.p, y, 1, M, F);
+            o.plane_fwd<float, EPI_OUT, false>(c->T32.p, y, 1);
           else
-            o.plane_fwd<float, EPI_OUT, true>(c->T32.p, y, 1, M, F);
+            o.plane_fwd<float, EPI_OUT, true>(c->T32.p, y, 1);
           break;
         case FAME_OP_QBQ:
-          o.plane_inv<float, IN_VEC, false>(x, c->T32.p, 1, M, F, 0);
+          o.plane_inv_vec<float, false>(x, c->T32.p, 1, 0);
           o.pencil<float, PEN_QBQ>(c->T32.p, 1, F, c->ibq32(), 0);
-          o.plane_fwd<float, EPI_OUT, false>(c->T32.p, y, 1, M, F);
+          o.plane_fwd<float, EPI_OUT, false>(c->T32.p, y, 1);
           break;
       }
     }
@@ -1554,10 +1544,8 @@ int fame_set_option(fame_ctx* c, const char* name, int value) {
     c->g.ps = g.ps;
   } else if (n == "plane_threads32" && threads_ok) {
     c->threads32_opt = value;
-    c->plane_threads32 = value ? value : plane_threads_rule<float>(c->g, c->rare);
   } else if (n == "plane_threads64" && threads_ok) {
     c->threads64_opt = value;
-    c->plane_threads = value ? value : plane_threads_rule<double>(c->g, c->rare);
   } else {
     set_err("unknown option or value: " + n + " = " + std::to_string(value));
     return FAME_ERR_BAD_INPUT;
@@ -1584,9 +1572,11 @@ int fame_get_option(fame_ctx* c, const char* name, int* value) {
   } else if (n == "radix_order") {
     *value = c->radix_order;
   } else if (n == "plane_threads32") {
-    *value = c->plane_threads32;
+    *value = c->plane_nt<float>(c->g.Ls);
   } else if (n == "plane_threads64") {
-    *value = c->plane_threads;
+    *value = c->plane_nt<double>(c->g.Ls);
+  } else if (n == "plane_threads32_set" || n == "plane_threads64_set") {
+    *value = n == "plane_threads32_set" ? c->threads32_opt : c->threads64_opt;  // 0: by the rule
   } else if (n == "static96") {
     *value = c->stat96 ? 1 : 0;
   } else if (n == "general") {
@@ -1626,8 +1616,7 @@ int fame_launch_count(fame_ctx* c, unsigned long long* out) {
     FAME_CK(cudaSetDevice(c->device));
     FAME_CK(cudaStreamSynchronize(c->stream));
     *out = launches_solver() + launches_ops_f32_simple() + launches_ops_f32_general() + launches_ops_f64_simple() +
-           launches_ops_f64_general() + launches_ops_f32_simple_rare() + launches_ops_f32_general_rare() +
-           launches_ops_f64_simple_rare() + launches_ops_f64_general_rare() + launches_ops_f32_simple_prime() +
+           launches_ops_f64_general() + launches_ops_f32_simple_prime() +
            launches_ops_f32_general_prime() + launches_ops_f64_simple_prime() + launches_ops_f64_general_prime() +
            launches_ops_stat96_f32() +
            launches_ops_stat96_f64() + launches_ops_slow_static() + launches_ops_plane_static() +
@@ -1661,9 +1650,7 @@ int fame_bench_qbq(fame_ctx* c, const double* k, int precision, int reps, int nb
     Ops o{c, P, nbatch};
     const Geom& g = c->g;
     const long M = 2L * g.N, F = 3L * g.N;
-    const int tmax = std::max({g.Nx * g.Ny, g.Nx, g.Ny, g.Nz});
-    P.launch(k_tables, dim3((tmax + 255) / 256, nbatch), dim3(256), 0, g, (const Slot*)c->slots.p, c->tabs.p,
-             (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2]);
+    o.tables(precision == FAME_FP64, precision == FAME_MIXED);
     DBuf<unsigned char> flush;
     const size_t fl = 256ull << 20;
     flush.ensure(fl);
@@ -1679,17 +1666,17 @@ int fame_bench_qbq(fame_ctx* c, const double* k, int precision, int reps, int nb
       FAME_CK(cudaMemsetAsync(flush.p, it & 0xff, fl, c->stream));
       FAME_CK(cudaEventRecord(ev[0], c->stream));
       if (precision == FAME_FP64) {
-        o.plane_inv<double, IN_VEC, false>(c->r64.p, c->T64.p, 1, M, F, 0);
+        o.plane_inv_vec<double, false>(c->r64.p, c->T64.p, 1, 0);
         FAME_CK(cudaEventRecord(ev[1], c->stream));
         o.pencil<double, PEN_QBQ>(c->T64.p, 1, F, c->ibq64(), 0);
         FAME_CK(cudaEventRecord(ev[2], c->stream));
-        o.plane_fwd<double, EPI_OUT, false>(c->T64.p, c->x64.p, 1, M, F);
+        o.plane_fwd<double, EPI_OUT, false>(c->T64.p, c->x64.p, 1);
       } else {
-        o.plane_inv<float, IN_VEC, false>(c->r32.p, c->T32.p, 1, M, F, 0);
+        o.plane_inv_vec<float, false>(c->r32.p, c->T32.p, 1, 0);
         FAME_CK(cudaEventRecord(ev[1], c->stream));
         o.pencil<float, PEN_QBQ>(c->T32.p, 1, F, c->ibq32(), 0);
         FAME_CK(cudaEventRecord(ev[2], c->stream));
-        o.plane_fwd<float, EPI_OUT, false>(c->T32.p, c->x32.p, 1, M, F);
+        o.plane_fwd<float, EPI_OUT, false>(c->T32.p, c->x32.p, 1);
       }
       FAME_CK(cudaEventRecord(ev[3], c->stream));
       FAME_CK(cudaEventSynchronize(ev[3]));
@@ -1729,7 +1716,8 @@ int fame_bench_cg(fame_ctx* c, const double* k, int reps, int nbatch, double* ms
     FAME_CK(cudaMemcpyAsync(c->slots.p, hs.data(), nbatch * sizeof(Slot), cudaMemcpyHostToDevice, c->stream));
     const Geom& g = c->g;
     const long M = 2L * g.N, F = 3L * g.N;
-    // r: a fixed pseudo-random residual; p = x = 0; the first iteration takes p = r
+    float2 *const rb[2] = {c->r32b.p, c->r32.p}, *const xb[2] = {c->x32b.p, c->x32.p};
+    // r: a fixed pseudo-random residual
     std::vector<float2> hr((size_t)nbatch * M);
     unsigned long long z = 0x9e3779b97f4a7c15ull;
     for (auto& v : hr) {
@@ -1739,8 +1727,6 @@ int fame_bench_cg(fame_ctx* c, const double* k, int reps, int nbatch, double* ms
       v.y = (float)((double)(z >> 11) / 9007199254740992.0 - 0.5);
     }
     FAME_CK(cudaMemcpyAsync(c->r32.p, hr.data(), hr.size() * sizeof(float2), cudaMemcpyHostToDevice, c->stream));
-    FAME_CK(cudaMemsetAsync(c->x32.p, 0, (size_t)nbatch * M * sizeof(float2), c->stream));
-    FAME_CK(cudaMemsetAsync(c->p32.p, 0, (size_t)nbatch * M * sizeof(float2), c->stream));
     std::vector<CgState> cs(nbatch);
     for (auto& s : cs) {
       memset(&s, 0, sizeof(s));
@@ -1753,28 +1739,25 @@ int fame_bench_cg(fame_ctx* c, const double* k, int reps, int nbatch, double* ms
     FAME_CK(cudaMemcpyAsync(c->cg.p, cs.data(), nbatch * sizeof(CgState), cudaMemcpyHostToDevice, c->stream));
     Program P(c->stream, false, c->hflag, 1);
     Ops o{c, P, nbatch};
-    const int tmax = std::max({g.Nx * g.Ny, g.Nx, g.Ny, g.Nz});
-    P.launch(k_tables, dim3((tmax + 255) / 256, nbatch), dim3(256), 0, g, (const Slot*)c->slots.p, c->tabs.p,
-             (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2]);
+    o.tables(false, true);
     DBuf<unsigned char> flush;
     const size_t fl = 256ull << 20;
     flush.ensure(fl);
     cudaEvent_t ev[4];
     for (auto& e : ev) FAME_CK(cudaEventCreate(&e));
     double tot[3] = {0, 0, 0};
+    o.cg_start<float>(rb, c->T32.p, c->ibq32());
     for (int it = 0; it < reps + 1; it++) {
       FAME_CK(cudaMemsetAsync(flush.p, it & 0xff, fl, c->stream));
       FAME_CK(cudaEventRecord(ev[0], c->stream));
-      o.plane_inv<float, IN_CG, false>(nullptr, c->T32.p, 1, M, F, 0, c->p32.p, c->r32.p, nullptr, nullptr, Cond{},
-                                       c->x32.p);
+      o.plane_cg<float>(rb, xb, c->T32.p, Cond{});
       FAME_CK(cudaEventRecord(ev[1], c->stream));
-      o.pencil<float, PEN_QBQ_CG>(c->T32.p, 1, F, c->ibq32(), 1);
+      o.cg_decide<float>(Cond{});
       FAME_CK(cudaEventRecord(ev[2], c->stream));
-      o.plane_fwd<float, EPI_CGR, false>(c->T32.p, nullptr, 1, M, F, nullptr, nullptr, Cond{}, 0.0, c->r32.p);
-      o.cg_decide(Cond{});
+      o.pencil<float, PEN_QBQ_CG>(c->T32.p, 1, F, c->ibq32(), 1);
       FAME_CK(cudaEventRecord(ev[3], c->stream));
       FAME_CK(cudaEventSynchronize(ev[3]));
-      if (it == 0) continue;  // warm-up (the p = r iteration)
+      if (it == 0) continue;  // warm-up (the first iteration reads no r_old, x)
       for (int q = 0; q < 3; q++) {
         float ms = 0;
         FAME_CK(cudaEventElapsedTime(&ms, ev[q], ev[q + 1]));

@@ -6,8 +6,12 @@ namespace fame {
 
 // ------------------------------------------------------------------ tables
 // Per-k tables (FAME_Main/FAME_Matrix_Lambdas.cu:77-244 Simple, :288-489 General)
-// computed on the device: one thread per table entry, FP64 sincospi.
-__global__ void k_tables(Geom g, const Slot* slots, double2* tabs, double m1, double m2, double m3) {
+// computed on the device: one thread per table entry, FP64 sincospi.  General lattices:
+// also D_kz (…Lambdas.cu:389-400) of every point in the precisions asked for (dkz64, dkz32; N
+// values per slot), which the plane stages read instead of evaluating it six times per CG
+// iteration.
+__global__ void k_tables(Geom g, const Slot* slots, double2* tabs, double m1, double m2, double m3, double2* dkz64,
+                         float2* dkz32) {
   FAME_COUNT_LAUNCH();
   const int slot = blockIdx.y;
   const Slot sl = slots[slot];
@@ -53,6 +57,15 @@ __global__ void k_tables(Geom g, const Slot* slots, double2* tabs, double m1, do
       t[g.oPhi + i] = make_double2(ph, 0.0);
     }
     if (i < Nz) t[g.oWz + i] = expipi(2.0 * i / Nz);
+    if (dkz64 || dkz32) {
+      for (int e = i; e < g.N; e += gridDim.x * blockDim.x) {
+        const int xy = (int)((unsigned)e / (unsigned)Nz), z = e - xy * Nz;
+        const int x = (int)((unsigned)xy / (unsigned)Ny), y = xy - x * Ny;
+        const double2 d = expipi((sl.th[2] + c1 * x + c2 * y) * z * g.tnz);
+        if (dkz64) dkz64[(size_t)slot * g.N + e] = d;
+        if (dkz32) dkz32[(size_t)slot * g.N + e] = to_f(d);
+      }
+    }
   }
 }
 
@@ -72,59 +85,10 @@ struct VecArgs {
   int nslots;
 };
 
-// ---------------------------------------------------------------- CG update
-// x += a p ; r -= a Ap ; r1 = <r, r>  (FAME_Main/CG.cu:65-76); then beta, the
-// iteration counter and the loop test r1 > tol^2 && k <= maxit (:37, :77).
-template <typename R>
-__global__ void __launch_bounds__(256) k_cg_update(VecArgs va, cplx<R>* r, const cplx<R>* Ap) {
-  FAME_COUNT_LAUNCH();
-  const int slot = blockIdx.z;
-  const Slot sl = va.slots[slot];
-  CgState* st = va.cg + slot;
-  const bool live = sl.active && st->active;
-  if (live) {
-    const long b = (long)slot * va.vstride;
-    const int n = 2 * sl.Nd;
-    const R are = (R)st->a_re, aim = (R)st->a_im;
-    double acc[1] = {0.0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-      const cplx<R> ap = Ap[b + i];
-      cplx<R> rr = r[b + i];
-      rr.x -= are * ap.x - aim * ap.y;
-      rr.y -= are * ap.y + aim * ap.x;
-      r[b + i] = rr;
-      acc[0] += (double)cabs2(rr);
-    }
-    __shared__ double sred[32];
-    block_reduce<1>(acc, sred);
-    double tot[1];
-    if (slot_reduce<1>(acc, va.partials + (size_t)slot * gridDim.x, va.counters + slot, blockIdx.x,
-                       gridDim.x, tot)) {
-      if (threadIdx.x == 0) {
-        st->r0 = st->r1;
-        st->r1 = tot[0];
-        st->beta = st->r1 / st->r0;
-        st->iter++;
-        st->total++;
-        st->active = (st->r1 > st->tol2) && (st->iter <= st->maxit);
-        __threadfence();
-      }
-    }
-  }
-  if (grid_last(va.counters + va.nslots, gridDim.x * gridDim.y * gridDim.z)) {
-    if (threadIdx.x == 0) {
-      int any = 0;
-      for (int q = 0; q < va.nslots; q++) any |= va.slots[q].active && va.cg[q].active;
-      decide_cond(va.cond, any);
-    }
-  }
-}
-
-// ---------------------------------------------------------------- fused FP32 CG: end of an iteration
-// One CTA per slot.  From the partial sums the iteration's kernels wrote (the pencil
-// stage's <p, Ap> parts, then the forward plane stage's ||r||^2 parts): the step size
-// a = r1 / <p, Ap> (the same ordered sum as the forward plane stage formed), r0 = r1,
-// r1 = ||r||^2, beta = r1 / r0, k++ and the loop test r1 > tol^2 && k <= maxit
+// ---------------------------------------------------------------- CG: end of an iteration
+// One CTA per slot, between the CG plane stage and the pencil stage.  From the partial sums of
+// <r, A r> (pencil stage) and of the new ||r||^2 (plane stage): the coefficients the plane stage
+// used, kept for the next iteration's, k++ and the loop test r1 > tol^2 && k <= maxit
 // (CG.cu:37, :57-77); the last CTA of the grid sets the WHILE condition.
 struct CgDecideArgs {
   const Slot* slots;
@@ -144,14 +108,15 @@ __global__ void __launch_bounds__(32) k_cg_decide(CgDecideArgs d) {
   CgState* st = d.cg + slot;
   if (d.slots[slot].active && st->active) {
     const double* p = d.partials + (size_t)slot * d.pstride;
-    const double pAp = warp_sum_partials(p, d.pen_parts) / d.N;
+    const double rAr = warp_sum_partials(p, d.pen_parts) / d.N;
     const double rr = warp_sum_partials(p + d.pen_parts, d.fwd_parts);
     if (threadIdx.x == 0) {
-      st->a_re = pAp > 0 ? st->r1 / pAp : 0.0;
-      st->a_im = 0.0;
-      st->r0 = st->r1;
+      double gm, rho;
+      cg_coefficients(*st, rAr, gm, rho);
+      st->gm = gm;
+      st->rho = rho;
+      st->r1p = st->r1;
       st->r1 = rr;
-      st->beta = st->r1 / st->r0;
       st->iter++;
       st->total++;
       st->active = (st->r1 > st->tol2) && (st->iter <= st->maxit);
@@ -168,14 +133,16 @@ __global__ void __launch_bounds__(32) k_cg_decide(CgDecideArgs d) {
 
 // ---------------------------------------------------------------- invAr prologue
 // rhs = u / sqrt(Lambda_q) (…invAr.cu:26), CG start x = 0, r = rhs (CG.cu:30-33).
-// Plain FP64 (MIXED = false): r, x are the FP64 CG vectors.  Mixed: b = rhs, y = 0,
-// r64 = b, and the outer refinement loop state is initialised.
+// Plain FP64 (MIXED = false): r64 is the CG's residual (k_plane_cg takes x = 0 at k = 1 as
+// read).  Mixed: b = rhs, y = x64 = 0, r64 = b, and the outer refinement loop state is
+// initialised.
 struct LzArgs {
   double2* U;              // [nslots][nphys][ustride]
   long ustride;            // column stride (elements)
   int nphys;
   int* map;                // [nslots][nstep+1] logical -> physical column
   int nstep, nwant;
+  int nkeep;               // Lanczos vectors a restart after the first keeps (keep_vectors, >= nwant)
   double* T0;              // [nslots][nstep]
   double* T1;              // [nslots][nstep]
   double* h;               // [nslots][nstep+2] reorthogonalisation coefficients
@@ -190,6 +157,11 @@ struct LzArgs {
 // prints this case).  The host reports any of them as FAME_ERR_NO_CONVERGENCE.
 constexpr int kStatusQL = 1, kStatusLanczos = 2, kStatusCG = 4;
 
+// whether Lanczos step j is one of this slot's
+__device__ __forceinline__ bool lz_live(const LzArgs& L, int slot, int j) {
+  return !L.lz[slot].converged && j >= L.lz[slot].keep;
+}
+
 __device__ __forceinline__ double2* ucol(const LzArgs& L, int slot, int logical) {
   const int ph = L.map[slot * (L.nstep + 1) + logical];
   return L.U + ((size_t)slot * L.nphys + ph) * L.ustride;
@@ -202,7 +174,7 @@ __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, 
   const int slot = blockIdx.z;
   const Slot sl = va.slots[slot];
   CgState* st = va.cg + slot;
-  const bool live = sl.active && !L.lz[slot].converged;
+  const bool live = sl.active && lz_live(L, slot, j);
   if (live) {
     const long b = (long)slot * va.vstride;
     const double2* tab = va.tabs + (size_t)slot * va.g.tab_stride;
@@ -213,8 +185,10 @@ __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, 
       const double s = lq_sqrt_at(va.g, tab, full_index(i, Nd, sl.off));
       const double2 v = make_double2(u[i].x / s, u[i].y / s);
       r64[b + i] = v;
-      x64[b + i] = make_double2(0.0, 0.0);
-      if (MIXED) b64[b + i] = v;
+      if (MIXED) {
+        x64[b + i] = make_double2(0.0, 0.0);
+        b64[b + i] = v;
+      }
       acc[0] += cabs2(v);
     }
     __shared__ double sred[32];
@@ -225,7 +199,6 @@ __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, 
       if (threadIdx.x == 0) {
         if (!MIXED) {
           st->r1 = tot[0];
-          st->r0 = tot[0];
           st->r1_0 = tot[0];
           st->tol2 = tol2;
           st->iter = 1;
@@ -260,12 +233,11 @@ __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, 
   }
 }
 
-// Start of one FP32 inner solve: r32 = (float)(r64 * scale), x32 = 0; stop when
+// Start of one FP32 inner solve: r32 = (float)(r64 * scale) (x32 = 0 is implied); stop when
 // ||r32|| <= tau' ||r32_0|| or after `maxit` products, where tau' = max(tau,
 // ls_tol / (2 ||r64||)): a refinement step never reduces the residual further than
 // the outer tolerance needs (outer_tol2 = ls_tol^2).
-__global__ void __launch_bounds__(256) k_cg32_init(VecArgs va, const double2* r64, float2* r32,
-                                                   float2* x32, double tau2, int maxit, double outer_tol2,
+__global__ void __launch_bounds__(256) k_cg32_init(VecArgs va, const double2* r64, float2* r32, double tau2, int maxit, double outer_tol2,
                                                    Cond outer_reset) {
   FAME_COUNT_LAUNCH();
   if ((threadIdx.x | blockIdx.x | blockIdx.y | blockIdx.z) == 0) set_cond(outer_reset, 0);
@@ -281,7 +253,6 @@ __global__ void __launch_bounds__(256) k_cg32_init(VecArgs va, const double2* r6
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
       const float2 v = make_float2((float)(r64[b + i].x * sc), (float)(r64[b + i].y * sc));
       r32[b + i] = v;
-      x32[b + i] = make_float2(0.f, 0.f);
       acc[0] += (double)cabs2(v);
     }
     __shared__ double sred[32];
@@ -292,7 +263,6 @@ __global__ void __launch_bounds__(256) k_cg32_init(VecArgs va, const double2* r6
       if (threadIdx.x == 0) {
         const double need = st->rr > 0 ? 0.25 * outer_tol2 / st->rr : 0.0;
         st->r1 = tot[0];
-        st->r0 = tot[0];
         st->r1_0 = tot[0];
         st->tol2 = (need > tau2 ? need : tau2) * tot[0];
         st->iter = 1;
@@ -318,30 +288,25 @@ __global__ void __launch_bounds__(256) k_cg32_init(VecArgs va, const double2* r6
 // (…invAr.cu:41-43: ls_iter += k, es_iter++).
 template <bool MIXED>
 __global__ void __launch_bounds__(256) k_invar_epi(VecArgs va, LzArgs L, int j, const double2* x64,
-                                                   const double2* p64) {
+                                                   const double2* x64b) {
   FAME_COUNT_LAUNCH();
   const int slot = blockIdx.z;
   const Slot sl = va.slots[slot];
-  if (!sl.active || L.lz[slot].converged) return;
+  if (!sl.active || !lz_live(L, slot, j)) return;
   const long b = (long)slot * va.vstride;
   const double2* tab = va.tabs + (size_t)slot * va.g.tab_stride;
   const double2* u = ucol(L, slot, j);
   double2* w = ucol(L, slot, j + 1);
   const int Nd = sl.Nd, n = 2 * Nd;
-  // plain FP64: the CG's last solution update x += a p (applied by the next
-  // iteration's plane stage, which this solve does not run)
-  const CgState* cs = va.cg + slot;
-  const bool pend = !MIXED && cs->iter > 1;
-  const double are = cs->a_re, aim = cs->a_im;
+  // plain FP64: the solution is in the buffer of the last iteration's parity (x64 odd, x64b
+  // even), and zero if the CG did no product; mixed: the refinement's sum, in x64
+  const int iter = va.cg[slot].iter;
+  const double2* xs = MIXED || (iter & 1) ? x64 : x64b;
+  const bool none = !MIXED && iter == 1;
   double acc[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double s = lq_sqrt_at(va.g, tab, full_index(i, Nd, sl.off));
-    double2 xx = x64[b + i];
-    if (pend) {
-      const double2 pp = p64[b + i];
-      xx.x += are * pp.x - aim * pp.y;
-      xx.y += are * pp.y + aim * pp.x;
-    }
+    const double2 xx = none ? make_double2(0.0, 0.0) : xs[b + i];
     const double2 v = make_double2(xx.x / s, xx.y / s);
     w[i] = v;
     acc[0] += v.x * u[i].x + v.y * u[i].y;
@@ -376,7 +341,7 @@ __global__ void __launch_bounds__(256) k_lz_dots(VecArgs va, LzArgs L, int j) {
   __shared__ double red[(2 * 64 + 1) * 8];  // [value][warp]
   const int slot = blockIdx.z;
   const Slot sl = va.slots[slot];
-  if (!sl.active || L.lz[slot].converged) return;
+  if (!sl.active || !lz_live(L, slot, j)) return;
   const int n = 2 * sl.Nd;
   const int r0 = blockIdx.x * kLzRows;
   const int rows = min(kLzRows, n - r0);
@@ -457,7 +422,7 @@ __global__ void __launch_bounds__(256) k_lz_update(VecArgs va, LzArgs L, int j) 
   __shared__ double2 hs[64];
   const int slot = blockIdx.z;
   const Slot sl = va.slots[slot];
-  if (!sl.active || L.lz[slot].converged) return;
+  if (!sl.active || !lz_live(L, slot, j)) return;
   const int n = 2 * sl.Nd;
   const double beta = L.T1[slot * L.nstep + j];
   const double inv = 1.0 / beta;
@@ -506,12 +471,13 @@ __global__ void k_lz_init(VecArgs va, LzArgs L) {
   const int slot = blockIdx.z;
   const Slot sl = va.slots[slot];
   if (blockIdx.x == 0 && threadIdx.x <= L.nstep) L.map[slot * (L.nstep + 1) + threadIdx.x] = threadIdx.x;
-  if (blockIdx.x == 0 && threadIdx.x <= L.nwant)
-    L.map[va.nslots * (L.nstep + 1) + slot * (L.nwant + 1) + threadIdx.x] = L.nstep + 1 + threadIdx.x;
+  if (blockIdx.x == 0 && threadIdx.x <= L.nkeep)
+    L.map[va.nslots * (L.nstep + 1) + slot * (L.nkeep + 1) + threadIdx.x] = L.nstep + 1 + threadIdx.x;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     L.lz[slot].converged = 0;
     L.lz[slot].restarts = 0;
     L.lz[slot].nconv = 0;
+    L.lz[slot].keep = 0;
     L.prof[slot * 3] = 0;
     L.prof[slot * 3 + 1] = 0;
     L.prof[slot * 3 + 2] = 0;
@@ -533,7 +499,7 @@ __global__ void k_lz_init(VecArgs va, LzArgs L) {
 // (3) If not converged: the lock/purge restart of Lanczos_LockPurge_gpu.cu:7-48
 // (exact shifts = unwanted Ritz values, GVqrrq_g steps, :95-190), applied to an
 // identity matrix G of order nstep+1 instead of to U, so that U is updated later by
-// one product U*G[:, 0..nwant].
+// one product U*G[:, 0..nkeep].
 constexpr int kMaxStep = 64;
 
 struct TriArgs {
@@ -541,7 +507,7 @@ struct TriArgs {
   const Slot* slots;
   double* theta;   // [nslots][nstep] Ritz values (descending)
   double* Z;       // [nslots][nstep*nstep] eigenvectors, column-major (z[r + c*nstep])
-  double* G;       // [nslots][(nstep+1)*(nwant+1)] restart transform, column-major
+  double* G;       // [nslots][(nstep+1)*(nkeep+1)] restart transform, column-major
   double tol;
   int maxit;
   Cond cond;       // "some slot needs another restart"
@@ -711,12 +677,13 @@ __global__ void __launch_bounds__(32) k_tridiag(TriArgs a) {
       }
     } else {
       // ---- lock & purge on G (order nstep+1)
+      const int nk = lz->restarts == 0 ? nw : L.nkeep;
       const int n1 = n + 1;
       for (int q = lane; q < n1 * n1; q += 32) Gs[q] = (q % (n1 + 1)) == 0 ? 1.0 : 0.0;
       __syncwarp();
-      for (int jj0 = 0; jj0 < n - nw; jj0++) {
+      for (int jj0 = 0; jj0 < n - nk; jj0++) {
         const int nn = n - jj0;
-        const double shift = d[order[nw + jj0]];
+        const double shift = d[order[nk + jj0]];
         if (lane == 0) {
           // GVqrrq_g(T0, T1, T2, T3, c, s, shift, nn)
           for (int i = 0; i < nn - 1; i++) T3[i] = T1[i];
@@ -786,13 +753,17 @@ __global__ void __launch_bounds__(32) k_tridiag(TriArgs a) {
         }
         __syncwarp();
       }
-      double* Gg = a.G + (size_t)slot * n1 * (nw + 1);
-      for (int q = lane; q < n1 * (nw + 1); q += 32) Gg[q] = Gs[q];
+      double* Gg = a.G + (size_t)slot * n1 * (L.nkeep + 1);
+      for (int q = lane; q < n1 * (nk + 1); q += 32) Gg[q] = Gs[q];
       for (int i = lane; i < n; i += 32) {
         L.T0[slot * n + i] = T0[i];
         L.T1[slot * n + i] = T1[i];
       }
-      if (lane == 0) lz->restarts++;
+      __syncwarp();  // every lane has read lz->restarts
+      if (lane == 0) {
+        lz->restarts++;
+        lz->keep = nk;
+      }
     }
   }
   __syncwarp();
@@ -827,10 +798,14 @@ __global__ void __launch_bounds__(256) k_ugemm(VecArgs va, LzArgs L, const doubl
   const int slot = blockIdx.z;
   const Slot sl = va.slots[slot];
   if (!sl.active) return;
-  if (mode == 0 && L.lz[slot].converged) return;
+  if (mode == 0) {
+    if (L.lz[slot].converged) return;
+    ncols = L.lz[slot].keep + 1;
+    if (c0 >= ncols) return;
+  }
   __shared__ double Gs[(kMaxStep + 1) * CH];
   __shared__ int cols[kMaxStep + 1];
-  const double* Gg = G + (size_t)slot * ldg * (mode == 0 ? (L.nwant + 1) : L.nstep);
+  const double* Gg = G + (size_t)slot * ldg * (mode == 0 ? (L.nkeep + 1) : L.nstep);
   const int nc = min(CH, ncols - c0);
   for (int q = threadIdx.x; q < nrows * nc; q += blockDim.x) {
     const int r = q % nrows, c = q / nrows;
@@ -859,7 +834,7 @@ __global__ void __launch_bounds__(256) k_ugemm(VecArgs va, LzArgs L, const doubl
         double2* dst;
         if (mode == 0) {
           // free physical column: the pool entries after the logical map
-          const int ph = L.map[va.nslots * (L.nstep + 1) + slot * (L.nwant + 1) + c0 + c];
+          const int ph = L.map[va.nslots * (L.nstep + 1) + slot * (L.nkeep + 1) + c0 + c];
           dst = L.U + ((size_t)slot * L.nphys + ph) * L.ustride;
         } else {
           dst = out + ((size_t)slot * ncols + c0 + c) * L.ustride;
@@ -870,21 +845,23 @@ __global__ void __launch_bounds__(256) k_ugemm(VecArgs va, LzArgs L, const doubl
   }
 }
 
-// After the restart product: logical 0..nwant -> the former free columns; the old
-// columns become the new pool (first nstep-nwant reused as logical nwant+1..nstep).
+// After the restart product: logical 0..keep -> the first free columns; the first
+// nstep - keep old columns become logical keep+1..nstep, the others take the freed places
+// of the pool (nkeep + 1 columns).
 __global__ void k_remap(LzArgs L, const Slot* slots, int nslots) {
   FAME_COUNT_LAUNCH();
   const int slot = blockIdx.x;
   if (threadIdx.x != 0 || !slots[slot].active || L.lz[slot].converged) return;
   int* mp = L.map + slot * (L.nstep + 1);
-  int* pool = L.map + nslots * (L.nstep + 1) + slot * (L.nwant + 1);
+  const int keep = L.lz[slot].keep;
+  int* pool = L.map + nslots * (L.nstep + 1) + slot * (L.nkeep + 1);
   int old[kMaxStep + 1], fr[kMaxStep + 1];
   for (int c = 0; c <= L.nstep; c++) old[c] = mp[c];
-  for (int c = 0; c <= L.nwant; c++) fr[c] = pool[c];
-  for (int c = 0; c <= L.nwant; c++) mp[c] = fr[c];
-  const int rest = L.nstep - L.nwant;
-  for (int c = 0; c < rest; c++) mp[L.nwant + 1 + c] = old[c];
-  for (int c = 0; c <= L.nwant; c++) pool[c] = old[rest + c];
+  for (int c = 0; c <= keep; c++) fr[c] = pool[c];
+  for (int c = 0; c <= keep; c++) mp[c] = fr[c];
+  const int rest = L.nstep - keep;
+  for (int c = 0; c < rest; c++) mp[keep + 1 + c] = old[c];
+  for (int c = 0; c <= keep; c++) pool[c] = old[rest + c];
 }
 
 }  // namespace fame

@@ -5,20 +5,18 @@
 
 namespace fame {
 
-// complex elements a thread holds in registers during one FFT pass of the runtime
-// plans (per precision).  FP32 stages 8: the runtime plane kernels run at 64
-// registers, and 16 elements spilled twice as much (FP32 CG iteration on the
-// runtime plans of FCC 64x55x52: 38.6 -> 36.3 us per k-point, hex 36x30x26: 14.8 -> 13.6)
+// complex elements a thread stages in registers during one round of a runtime-plan
+// pass (per precision; a radix above it stages one butterfly)
 template <typename R> struct Emax;
-template <> struct Emax<float> { static constexpr int v = 8; };
+template <> struct Emax<float> { static constexpr int v = 16; };
 template <> struct Emax<double> { static constexpr int v = 8; };
-// fast-axis positions per pencil CTA: 256-byte rows
+// plane positions per pencil CTA: 256-byte rows
 template <typename R> struct PencilTW { static constexpr int v = 256 / (int)sizeof(cplx<R>); };
 
 // ------------------------------------------------------------------ state
 struct CgState {
-  double r1, r0, beta;       // ||r||^2 now / before, r1/r0
-  double a_re, a_im;         // CG step a = r1 / <p, Ap>
+  double r1, r1p;            // ||r||^2 now / one iteration before
+  double gm, rho;            // the last iteration's gamma and rho (cg_coefficients)
   double r1_0, tol2;         // initial ||r||^2, stop threshold on ||r||^2
   int iter;                  // the reference's counter k (starts at 1, CG.cu:36)
   int active;
@@ -30,11 +28,18 @@ struct CgState {
   int outer, outer_active, outer_max, outer_total;
 };
 
+// gamma = ||r||^2 / <r, A r> and rho of the three-term CG recurrences (k_plane_cg) from the state
+// before the iteration and <r, A r>.  <r, A r> <= 0 (a residual of zero): no step.
+__device__ __forceinline__ void cg_coefficients(const CgState& st, double rAr, double& gm, double& rho) {
+  gm = rAr > 0 ? st.r1 / rAr : 0.0;
+  rho = st.iter == 1 ? 1.0 : 1.0 / (1.0 - (gm / st.gm) * (st.r1 / st.r1p) / st.rho);
+}
+
 struct LzState {
   int converged;
   int restarts;
   int nconv;
-  int pad;
+  int keep;  // Lanczos vectors the last restart kept: steps j < keep are not this slot's (0 before)
 };
 
 // Condition of one CUDA-graph WHILE node (in host-driven mode only `flag` is used).
@@ -104,11 +109,10 @@ __device__ __forceinline__ cplx<R> dkz_at(const Geom& g, const double2* tab, int
 }
 
 // ------------------------------------------------------------------ plane stage
+// IN_CG: the start residual of a CG solve (gated on the solve being active)
 enum InMode { IN_VEC = 0, IN_CG = 1, IN_REFINE = 2 };
-// EPI_CG writes Ap and forms <p, Ap>; EPI_CGR (fused CG) keeps Ap in registers and
-// applies r -= a Ap with ||r||^2, the step size a coming from the PEN_QBQ_CG pencil.
-enum EpiMode { EPI_OUT = 0, EPI_CG = 1, EPI_RESID = 2, EPI_CGR = 3 };
-// PEN_QBQ_CG: PEN_QBQ that also reduces <p, Ap> = (1/N) sum_e |(IDFT v)_e|^2 / eps_e
+enum EpiMode { EPI_OUT = 0, EPI_RESID = 2 };
+// PEN_QBQ_CG: PEN_QBQ that also reduces <v, Av> = (1/N) sum_e |(IDFT Pi v)_e|^2 / eps_e
 enum PencilMode { PEN_QBQ = 0, PEN_QR_OUT = 1, PEN_QRS_IN = 2, PEN_QBQ_CG = 3 };
 
 template <typename R>
@@ -116,25 +120,38 @@ struct PlaneInArgs {
   Geom g;
   const Slot* slots;
   const double2* tabs;
+  const cplx<R>* dkz;     // General: D_kz of every slot (N values each), or NULL
   const cplx<R>* tw;      // forward twiddle tables, R precision
   long vstride;           // per-slot stride of reduced vectors (elements)
   long fstride;           // per-slot stride of 3N fields (elements)
   int vec_per_slot;       // number of vectors per slot (batched Qr over bands)
-  const cplx<R>* in;      // IN_VEC: reduced input
-  cplx<R>* p;             // IN_CG: search direction (updated in place)
-  const cplx<R>* r;       // IN_CG: residual
-  cplx<R>* x;             // IN_CG: solution; takes the previous iteration's a * p here
-  CgState* cg;            // IN_CG / IN_REFINE
+  const cplx<R>* in;      // IN_VEC, IN_CG: reduced input
+  const CgState* cg;      // IN_CG / IN_REFINE
   double2* y64;           // IN_REFINE: FP64 accumulated solution (updated)
-  const float2* x32;      // IN_REFINE: FP32 correction
-  const float2* p32;      // IN_REFINE: the FP32 search direction of the inner solve's last update
+  const float2* x32[2];   // IN_REFINE: FP32 correction, the buffer of the last iteration's parity
   int sigma;              // IN_VEC: multiply the input by sqrt(Lambda_q) first (Sigma, …_Isotropic.cu:109)
   cplx<R>* T;             // output field (3 components)
-  Cond reset;             // loop condition cleared by this kernel when it starts a loop body
-  int pf_dist;            // > 0: each CTA prefetches into L2 the operands of the CTA this
-                          // many places later in launch order (about one wave ahead)
-  int self_pf;            // IN_CG: L2 prefetch of this CTA's own r, p and x at its start
   int* fault;             // set to 1 if a bounded wait of the component exchange ran out (or NULL)
+};
+
+template <typename R>
+struct PlaneCgArgs {
+  Geom g;
+  const Slot* slots;
+  const double2* tabs;
+  const cplx<R>* dkz;
+  const cplx<R>* tw;
+  long vstride, fstride;
+  cplx<R>* r[2];          // residual: buffer iter & 1 is the current one, the other r_old / r'
+  cplx<R>* x[2];          // solution, the same way
+  CgState* cg;
+  cplx<R>* T;             // field of A r before the forward plane transforms in, of r' out
+  double* partials;       // per slot: the pencil's <r, A r> parts, then this kernel's ||r'||^2 parts
+  long pstride;           // per-slot stride of `partials`
+  int pen_parts;
+  Cond reset;             // loop condition cleared by this kernel, the first of the loop body
+  int self_pf;            // L2 prefetch of this CTA's own vectors at its start
+  int* fault;
 };
 
 template <typename R>
@@ -150,12 +167,11 @@ struct PencilArgs {
   int ib_field;            // invB in the field layout (else the spatial layout; same for Simple lattices)
   cplx<R>* out;            // PEN_QR_OUT: spatial field out (3N per vector)
   const cplx<R>* in;       // PEN_QRS_IN: spatial field in
-  CgState* cg;             // optional activity gate; PEN_QBQ_CG writes the step size a
+  const CgState* cg;       // optional activity gate
   int gate;                // 0 none, 1 CG active, 2 outer refinement active
-  double* partials;        // PEN_QBQ_CG: partial sums of <p, Ap>, [slot * pstride + CTA of the slot]
-  unsigned* counters;      // (unused by PEN_QBQ_CG)
+  double* partials;        // PEN_QBQ_CG: partial sums of <v, Av>, [slot * pstride + CTA (or tile) of the slot]
   long pstride;            // per-slot stride of `partials`
-  int TW;                  // fast positions per CTA
+  int TW;                  // plane positions per CTA
   int nslots;              // k-points of the launch (k_pencil_pipe walks all their tiles)
   int pf_dist;             // > 0: L2 prefetch of the tile of the CTA this many places later
 };
@@ -165,25 +181,19 @@ struct PlaneOutArgs {
   Geom g;
   const Slot* slots;
   const double2* tabs;
+  const cplx<R>* dkz;
   const cplx<R>* tw;
   long vstride, fstride;
   int vec_per_slot;
   const cplx<R>* T;        // field after the slow-axis forward pass
-  cplx<R>* out;            // EPI_OUT: reduced output; EPI_CG: Ap; EPI_RESID: r (FP64)
-  const cplx<R>* p;        // EPI_CG: p for <p, Ap>
-  cplx<R>* r;              // EPI_CGR: CG residual, updated in place
+  cplx<R>* out;            // EPI_OUT: reduced output; EPI_RESID: r (FP64)
   const cplx<R>* b;        // EPI_RESID: right-hand side
   CgState* cg;
-  double* partials;        // [nslots][blocks per slot][NV]
+  double* partials;        // EPI_RESID: [nslots][blocks per slot]
   unsigned* counters;      // [nslots] ticket counters, plus [nslots] = grid counter
-  Cond cond;               // EPI_RESID: outer WHILE condition; EPI_CGR: CG WHILE condition
+  Cond cond;               // EPI_RESID: outer WHILE condition
   int nslots;
   double tol2;             // EPI_RESID: absolute tolerance^2 on ||b - A y||
-  int pf_dist;             // > 0: L2 prefetch of the operands of the CTA this many places later
-  int self_pf;             // EPI_CGR: L2 prefetch of this CTA's own residual at its start
-  long pstride;            // EPI_CGR: per-slot stride of `partials`
-  int pen_parts;           // EPI_CGR: the pencil's <p, Ap> partials per slot (at the slot's start);
-                           // this kernel's ||r||^2 partials follow them
 };
 
 // Ordered sum of p[0], p[stride], ..., p[(n - 1) stride] by one warp (lane-strided,

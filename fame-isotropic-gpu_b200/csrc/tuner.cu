@@ -112,8 +112,8 @@ extern "C" int fame_tune(fame_ctx* c, const double* k, int precision, int batch,
     const int reps = 5;
     Plan cur;  // the context's current choices (the built-in ones unless tuned before)
     cur.radix_order = get(c, "radix_order");
-    cur.threads32 = get(c, "plane_threads32");
-    cur.threads64 = get(c, "plane_threads64");
+    cur.threads32 = get(c, "plane_threads32_set");  // 0: the built-in rule
+    cur.threads64 = get(c, "plane_threads64_set");
     cur.prefetch = get(c, "prefetch");
     double t_best = time_plan(c, cur, k, precision, batch, reps);
     if (t_best < 0) return t_best == -1 ? FAME_ERR_BAD_INPUT : FAME_ERR_CUDA;

@@ -192,14 +192,15 @@ int fame_set_loop_cap(fame_ctx* ctx, int max_trips);
 
 /* Execution options of a context, used by later solves and operator applies (they
  * change how the kernels run; the results agree to rounding):
- *   "prefetch"         1: each CTA of the mixed-precision CG's stage kernels issues L2
- *                      prefetches of the operands of the CTA one wave later; 0 (default): none.
+ *   "prefetch"         1: each CTA of the CG's pencil stage issues L2 prefetches of the tile of
+ *                      the CTA one wave later; 0 (default): none.
  *   "radix_order"      0..3: radix order of the FFT plans of runtime-geometry grids
  *                      (every grid but the compile-time 96^3 one); 0 is the default.
  *   "plane_threads32", "plane_threads64": threads of a runtime-geometry plane CTA in the
  *                      FP32 / FP64 kernels, a multiple of 32 in 64..512, or 0 for the
- *                      built-in rule.
- *   "self_prefetch"    1 (default): the CG plane stages prefetch their own operands into L2
+ *                      built-in rule (which goes by the launch's size; fame_get_option then gives
+ *                      its choice for one k-point).
+ *   "self_prefetch"    1 (default): the CG plane stage prefetches its own vectors into L2
  *                      at the CTA's start; 0: off.
  *   "static_planes"    1 (default): the plane stages of the FCC 64x55x52, BCC 48x45x39 and
  *                      hexagonal 128x107x92 grids run compile-time FFT plans (fixed CTA
@@ -213,7 +214,8 @@ int fame_set_loop_cap(fame_ctx* ctx, int max_trips);
  *                      it no longer needs; a call whose lane contexts cannot be created
  *                      runs as one batch.
  * Read-only (fame_get_option): "static96", "general", "grid_x", "grid_y", "grid_z",
- * "level" (the FFT pass level the grid needs).  fame_tune picks the first four by timing.
+ * "level" (the FFT pass level the grid needs), "plane_threads32_set", "plane_threads64_set"
+ * (the options above, 0 when the rule decides).  fame_tune picks the first four by timing.
  * Unknown names or values are FAME_ERR_BAD_INPUT.  No counterpart in the reference. */
 int fame_set_option(fame_ctx* ctx, const char* name, int value);
 int fame_get_option(fame_ctx* ctx, const char* name, int* value);
@@ -241,13 +243,12 @@ int fame_bench_qbq(fame_ctx* ctx, const double* k, int precision, int reps, int 
                    double* stage_ms_out);
 
 /* CG-iteration benchmark: `reps` iterations of the mixed-precision solve's FP32 CG
- * (the three kernels of one iteration: search direction and solution update with
- * the 2 -> 3 mix and the inverse plane transforms; slow-axis transforms with <p, Ap>;
- * forward plane transforms with the 3 -> 2 unmix, r -= a Ap and ||r||^2) on `nbatch`
- * k-points (1..64, the k-point repeated), from a fixed pseudo-random residual, each
- * iteration preceded by an L2 flush outside the timed span.  stage_ms_out[3]
- * (optional) receives the mean time of the three kernels over the batch, ms_out
- * their sum.  The CG iteration of FAME_Main/CG.cu:36-77 on QBQ. */
+ * (its three kernels: the plane stage, with the forward plane transforms, the 3 -> 2 unmix, the
+ * vector updates, ||r||^2, the 2 -> 3 mix and the inverse plane transforms; the decision; the
+ * slow-axis transforms with <r, A r>) on `nbatch` k-points (1..64, the k-point repeated), from
+ * a fixed pseudo-random residual, each iteration preceded by an L2 flush outside the timed
+ * span.  stage_ms_out[3] (optional) receives the mean time of the three kernels over the
+ * batch, ms_out their sum.  The CG iteration of FAME_Main/CG.cu:36-77 on QBQ. */
 int fame_bench_cg(fame_ctx* ctx, const double* k, int reps, int nbatch, double* ms_out, double* stage_ms_out);
 
 /* Grid size N and maximum reduced size 2N of the context, for buffer sizing. */
