@@ -8,7 +8,7 @@
 // writes output t to (j/Ns)*Ns*R + (j mod Ns) + t*Ns.  The result is in natural
 // order after the last pass.  Forward transforms use e^{-i...} (cuFFT
 // CUFFT_FORWARD, which the reference's FFT_CUDA uses, FAME_Main/FAME_FFT_CUDA.cu:31)
-// and inverse transforms e^{+i...}, both unnormalised.
+// and inverse transforms e^{+i...}, both unnormalised; the runtime plans only run forward (DynGeom).
 //
 // A "tile" holds `nl` lines of length n; element m of line l sits at
 // buf[l*ls + m*es].  Every pass is register staged: each thread reads all inputs
@@ -366,8 +366,7 @@ struct Div {
 // threads touch consecutive lines and at most the last deal of a round has idle threads.
 // G is the largest line count that T * MAXB butterflies cover, evened out over the rounds.
 template <typename R, int RAD, int MAXB>
-__device__ __forceinline__ void stockham_pass(cplx<R>* buf, int n, int Ns, LineSet L, const cplx<R>* tw,
-                                              bool inv) {
+__device__ __forceinline__ void stockham_pass(cplx<R>* buf, int n, int Ns, LineSet L, const cplx<R>* tw) {
   const int T = blockDim.x;
   const int nb = n / RAD;
   const int stw = n / (Ns * RAD);
@@ -402,13 +401,9 @@ __device__ __forceinline__ void stockham_pass(cplx<R>* buf, int n, int Ns, LineS
         if (k > 0) {
           const int kt = k * stw;
 #pragma unroll
-          for (int u = 1; u < RAD; u++) {
-            cplx<R> w = tw[u * kt];
-            if (inv) w.y = -w.y;
-            v[q][u] = cmul(v[q][u], w);
-          }
+          for (int u = 1; u < RAD; u++) v[q][u] = cmul(v[q][u], tw[u * kt]);
         }
-        Dft<R, RAD>::run(v[q], inv);
+        Dft<R, RAD>::run(v[q], false);
         dst[q] = l * L.ls + (jb * Ns * RAD + k) * L.es;
       }
     }
@@ -429,8 +424,7 @@ __device__ __forceinline__ void stockham_pass(cplx<R>* buf, int n, int Ns, LineS
 // rounds of G complete lines, thread t owns line l0 + t mod G and outputs
 // o = t / G + ostep * q.
 template <typename R, int MAXE>
-__device__ __forceinline__ void generic_pass(cplx<R>* buf, int n, int r, int Ns, LineSet L, const cplx<R>* tw,
-                                             bool inv) {
+__device__ __forceinline__ void generic_pass(cplx<R>* buf, int n, int r, int Ns, LineSet L, const cplx<R>* tw) {
   const int T = blockDim.x;
   const int stw = n / (Ns * r);
   const int nr = n / r;
@@ -460,9 +454,7 @@ __device__ __forceinline__ void generic_pass(cplx<R>* buf, int n, int r, int Ns,
         const cplx<R>* src = base + j * L.es;
         cplx<R> acc = mk<R>(0, 0);
         for (int s = 0; s < r; s++) {
-          cplx<R> w = tw[idx];
-          if (inv) w.y = -w.y;
-          acc = cadd(acc, cmul(src[s * nr * L.es], w));
+          acc = cadd(acc, cmul(src[s * nr * L.es], tw[idx]));
           idx += step;
           if (idx >= n) idx -= n;
         }
@@ -483,7 +475,7 @@ __device__ __forceinline__ void generic_pass(cplx<R>* buf, int n, int r, int Ns,
 // Stockham twiddle w^(s*k*stw) (k = j mod Ns) and are replaced in place by
 // P_s = a_s + a_{r-s} at s and Q_s = a_s - a_{r-s} at r - s (1 <= s <= H).
 // Phase B, in rounds of complete lines:
-//   X_u = a_0 + sum_s cos(2 pi us/r) P_s -/+ i sum_s sin(2 pi us/r) Q_s,
+//   X_u = a_0 + sum_s cos(2 pi us/r) P_s - i sum_s sin(2 pi us/r) Q_s,
 //   X_{r-u} the same with the sign of the second sum flipped (u = 0..H).
 // A thread owns one butterfly j, MU consecutive u and up to ML lines (Gt apart), so
 // each loaded P_s, Q_s feeds MU outputs and each cos/sin feeds ML lines: 4*MU*ML
@@ -494,8 +486,7 @@ __device__ __forceinline__ void generic_pass(cplx<R>* buf, int n, int r, int Ns,
 // whose kernels launch exactly TC threads), so that the cell and line split, the
 // rounds and the shared-memory offsets fold to constants; 0: blockDim.x.
 template <typename R, int MU, int ML, int TC = 0>
-__device__ __forceinline__ bool prime_pass(cplx<R>* buf, int n, int r, int Ns, LineSet L, const cplx<R>* tw,
-                                           bool inv) {
+__device__ __forceinline__ bool prime_pass(cplx<R>* buf, int n, int r, int Ns, LineSet L, const cplx<R>* tw) {
   const int T = TC > 0 ? TC : (int)blockDim.x;
   const int nb = n / r;
   const int stw = n / (Ns * r);
@@ -519,13 +510,8 @@ __device__ __forceinline__ bool prime_pass(cplx<R>* buf, int n, int r, int Ns, L
       cplx<R>* pb = base + (j + (r - s) * nb) * L.es;
       cplx<R> a = *pa, b = *pb;
       if (k > 0) {
-        cplx<R> wa = tw[s * k * stw], wb = tw[(r - s) * k * stw];
-        if (inv) {
-          wa.y = -wa.y;
-          wb.y = -wb.y;
-        }
-        a = cmul(a, wa);
-        b = cmul(b, wb);
+        a = cmul(a, tw[s * k * stw]);
+        b = cmul(b, tw[(r - s) * k * stw]);
       }
       *pa = cadd(a, b);
       *pb = csub(a, b);
@@ -605,7 +591,7 @@ __device__ __forceinline__ bool prime_pass(cplx<R>* buf, int n, int r, int Ns, L
       for (int m = 0; m < MU; m++) {
         const int u = u0 + m;
         if (u > H) break;
-        const cplx<R> rr = rot_mi(im[i][m], inv);
+        const cplx<R> rr = rot_mi(im[i][m], false);
         base[u * ostep] = cadd(re[i][m], rr);
         if (u > 0) base[(r - u) * ostep] = csub(re[i][m], rr);
       }
@@ -623,13 +609,12 @@ template <> struct PrimeBlock<double> { static constexpr int mu = 2, ml = 2; };
 // Butterflies of radix r a thread stages per round when it holds at most emax elements.
 constexpr int pass_maxb(int emax, int r) { return emax / r > 0 ? emax / r : 1; }
 
-// Full transform of all lines along one axis.  RARE >= 2 compiles the passes for prime
+// Full forward transform of all lines along one axis.  RARE >= 2 compiles the passes for prime
 // factors >= 17 in; they are register hungry, so each stage kernel exists with and
 // without them and the host picks by its axes (plan_level).  EMAX bounds the elements
 // a thread stages in registers per round.
 template <typename R, int EMAX, int RARE>
-__device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPlan& P, LineSet L, const cplx<R>* tw,
-                                          bool inv) {
+__device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPlan& P, LineSet L, const cplx<R>* tw) {
   const int n = P.n;
   int Ns = 1;
 #pragma unroll 1
@@ -637,7 +622,7 @@ __device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPlan& P, LineS
     const int r = P.radix[p];
     switch (r) {
 #define FAME_PASS(r_) \
-  case r_: stockham_pass<R, r_, pass_maxb(EMAX, r_)>(buf, n, Ns, L, tw, inv); break;
+  case r_: stockham_pass<R, r_, pass_maxb(EMAX, r_)>(buf, n, Ns, L, tw); break;
       FAME_PASS(2)
       FAME_PASS(3)
       FAME_PASS(4)
@@ -653,8 +638,8 @@ __device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPlan& P, LineS
 #undef FAME_PASS
       default:
         if constexpr (RARE >= 2) {
-          if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml>(buf, n, r, Ns, L, tw, inv))
-            generic_pass<R, EMAX>(buf, n, r, Ns, L, tw, inv);
+          if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml>(buf, n, r, Ns, L, tw))
+            generic_pass<R, EMAX>(buf, n, r, Ns, L, tw);
         }
         break;
     }
@@ -779,8 +764,9 @@ __device__ __forceinline__ void sfft(cplx<R>* buf, int ls, int es, const cplx<R>
     if constexpr (RAD >= 17) {
       // a prime factor >= 17: the symmetric-pair pass, its sizes compile-time constants
       const LineSet L{NL, ls, es};
-      if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml, T>(buf, N, RAD, NS, L, tw, inv))
-        generic_pass<R, EMAX>(buf, N, RAD, NS, L, tw, inv);
+      // (forward only, as all plans with primes run)
+      if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml, T>(buf, N, RAD, NS, L, tw))
+        generic_pass<R, EMAX>(buf, N, RAD, NS, L, tw);
     } else {
       constexpr int MB = smaxb(N, NL, T, EMAX, RAD);
       spass<R, N, NL, T, NS, RAD, MB>(buf, ls, es, tw, inv);

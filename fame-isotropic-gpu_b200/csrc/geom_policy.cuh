@@ -11,7 +11,6 @@
 namespace fame {
 
 constexpr int kPlaneThreads = 512;      // most threads of a plane CTA that an option can set
-constexpr int kStatPlaneThreads = 384;  // threads of a plane CTA with a static geometry
 constexpr int kPencilThreads = 256;     // threads of a pencil CTA (at most, with runtime plans)
 
 struct DynGeom {
@@ -33,17 +32,19 @@ struct DynGeom {
   __device__ __forceinline__ static int P(const Geom& g) { return g.P; }
   // lines of a plane (pitch S) along its fast axis (fast = true) or mid axis, and
   // the TW lines of a pencil tile.  One FFT call site per kernel keeps the kernel
-  // within its register budget, so the plane axis is a runtime argument.
+  // within its register budget, so the plane axis is a runtime argument.  Forward transforms
+  // only: the inverse ones run on values with swapped parts (plane stages) or come out in
+  // reversed order (pencil stage), which takes the conjugations and sign choices of a runtime
+  // direction out of every pass.
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const Geom& g, bool fast, const cplx<R>* tw,
-                                                   bool inv) {
+  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const Geom& g, bool fast, const cplx<R>* tw) {
     fft_lines<R, Emax<R>::v, RARE>(b, fast ? g.pf : g.pm, fast ? LineSet{g.Lm, g.S, 1} : LineSet{g.Lf, 1, g.S},
-                                   tw, inv);
+                                   tw);
   }
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom& g, const cplx<R>* tw, bool inv) {
+  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom& g, const cplx<R>* tw) {
     constexpr int TW = PencilTW<R>::v;
-    fft_lines<R, Emax<R>::v, RARE>(b, g.ps, LineSet{TW, 1, TW}, tw, inv);
+    fft_lines<R, Emax<R>::v, RARE>(b, g.ps, LineSet{TW, 1, TW}, tw);
   }
 };
 
@@ -80,9 +81,9 @@ template <int LSL>
 struct DynGeomSlow : DynGeom {
   __device__ __forceinline__ static constexpr int pencil_threads() { return kPencilThreads; }
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom&, const cplx<R>* tw, bool inv) {
+  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom&, const cplx<R>* tw) {
     constexpr int TW = PencilTW<R>::v;
-    sfft<R, LSL, TW, kPencilThreads, SlowEmax<R>::v>(b, 1, TW, tw, inv);
+    sfft<R, LSL, TW, kPencilThreads, SlowEmax<R>::v>(b, 1, TW, tw, false);
   }
 };
 
@@ -98,27 +99,26 @@ struct DynGeomPlane : DynGeom {
   __device__ __forceinline__ static constexpr int plane_threads() { return T; }
   template <typename R, int RARE> static constexpr int plane_min_blocks() { return MB; }
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const Geom&, bool fast, const cplx<R>* tw,
-                                                   bool inv) {
+  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const Geom&, bool fast, const cplx<R>* tw) {
     if (fast)
-      sfft<R, LF, LM, T, PlaneEmax<R>::v>(b, LF | 1, 1, tw, inv);
+      sfft<R, LF, LM, T, PlaneEmax<R>::v>(b, LF | 1, 1, tw, false);
     else
-      sfft<R, LM, LF, T, PlaneEmax<R>::v>(b, 1, LF | 1, tw, inv);
+      sfft<R, LM, LF, T, PlaneEmax<R>::v>(b, 1, LF | 1, tw, false);
   }
 };
 
-template <int LF, int LM, int LSL>
+template <int LF, int LM, int LSL, int T, int MB>
 struct StatGeom {
   static constexpr bool kStatic = true;
-  static constexpr int kS = LF | 1;
+  static constexpr int kS = LF | 1, kLf = LF, kLm = LM, kThreads = T;
   // 384 = 4 threads per line of a 96 x 96 plane: every pass of the 8 x 12 plan
   // is one round with all threads busy
-  template <typename R, int RARE> static constexpr int max_plane_threads() { return kStatPlaneThreads; }
+  template <typename R, int RARE> static constexpr int max_plane_threads() { return T; }
   // two FP32 plane CTAs per SM (80 registers), one FP64 plane CTA; three FP32 and
   // two FP64 pencil CTAs
-  __device__ __forceinline__ static constexpr int plane_threads() { return kStatPlaneThreads; }
+  __device__ __forceinline__ static constexpr int plane_threads() { return T; }
   __device__ __forceinline__ static constexpr int pencil_threads() { return kPencilThreads; }
-  template <typename R, int RARE> static constexpr int plane_min_blocks() { return sizeof(R) == 4 ? 2 : 1; }
+  template <typename R, int RARE> static constexpr int plane_min_blocks() { return MB; }
   __device__ __forceinline__ static constexpr int Lf(const Geom&) { return LF; }
   __device__ __forceinline__ static constexpr int Lm(const Geom&) { return LM; }
   __device__ __forceinline__ static constexpr int Ls(const Geom&) { return LSL; }
@@ -126,20 +126,14 @@ struct StatGeom {
   __device__ __forceinline__ static constexpr int P(const Geom&) { return LF * LM; }
   static_assert(LF == LM, "a static plane geometry has equal fast and mid lengths");
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const Geom&, bool fast, const cplx<R>* tw,
-                                                   bool inv) {
-    sfft<R, LF, LM, kStatPlaneThreads, SEmax<R>::v>(b, fast ? kS : 1, fast ? 1 : kS, tw, inv);
+  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom&, const cplx<R>* tw) {
+    fft_slow_c<R, false>(b, tw);
   }
-  template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom&, const cplx<R>* tw, bool inv) {
-    constexpr int TW = PencilTW<R>::v;
-    sfft<R, LSL, TW, kPencilThreads, SPenEmax<R>::v>(b, 1, TW, tw, inv);
-  }
-  // The same passes with the axis and the direction fixed at compile time: every
+  // Passes with the axis and the direction fixed at compile time: every
   // stride, twiddle sign and rotation folds to a constant (one call site each).
   template <typename R, bool FAST, bool INV>
   __device__ __forceinline__ static void fft_plane_c(cplx<R>* b, const cplx<R>* tw) {
-    sfft<R, LF, LM, kStatPlaneThreads, SEmax<R>::v>(b, FAST ? kS : 1, FAST ? 1 : kS, tw, INV);
+    sfft<R, LF, LM, T, SEmax<R>::v>(b, FAST ? kS : 1, FAST ? 1 : kS, tw, INV);
   }
   template <typename R, bool INV>
   __device__ __forceinline__ static void fft_slow_c(cplx<R>* b, const cplx<R>* tw) {
@@ -148,7 +142,7 @@ struct StatGeom {
   }
 };
 
-using Stat96 = StatGeom<96, 96, 96>;
+template <typename R> using Stat96 = StatGeom<96, 96, 96, sizeof(R) == 4 ? 192 : 384, sizeof(R) == 4 ? 3 : 1>;
 // static plane plans of the general-lattice benchmark grids (fast, mid, threads, CTAs per SM)
 template <typename R> using PlaneFcc64 = DynGeomPlane<52, 55, 128, sizeof(R) == 4 ? 5 : 4>;
 template <typename R> using PlaneBcc48 = DynGeomPlane<39, 45, 128, sizeof(R) == 4 ? 5 : 4>;

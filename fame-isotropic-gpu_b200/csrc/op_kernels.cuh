@@ -11,12 +11,12 @@ namespace fame {
 // Lambda_x, Lambda_y, Lambda_z at plane element (m, f) of plane s, in precision R.
 // Simple lattices read the per-CTA shared tables lx[f], ly[m] and the plane's lz.
 template <typename R, bool GEN>
-__device__ __forceinline__ void lam_elem(const Geom& g, const double2* tab, const cplx<R>* lx, const cplx<R>* ly,
+__device__ __forceinline__ void lam_elem(const Geom& g, const double2* tab, const cplx<R>* lx, const cplx<R>* ly, int lys,
                                          cplx<R> lz, int s, int m, int f, cplx<R>& Lx, cplx<R>& Ly,
                                          cplx<R>& Lz) {
   if constexpr (!GEN) {
     Lx = lx[f];
-    Ly = ly[m];
+    Ly = ly[m * lys];
     Lz = lz;
   } else {
     double2 a, b, c;
@@ -79,18 +79,22 @@ __device__ __forceinline__ PlanePos plane_pos() {
 }
 
 // Dynamic shared memory of a plane CTA.  Plane rows have the odd pitch S >= Lf.  lx, ly hold
-// the Lambda tables of the plane's axes (Simple lattices) or, in ly, D_ky(s, .) (General).
+// the Lambda tables of the plane's axes (Simple lattices) or, in ly, D_ky(s, .) (General);
+// element m of ly is ly[m * lys].  Static geometries have one twiddle table (equal axes) and
+// keep ly in the column that pads the rows.
 template <typename R> struct PlaneSmem {
   cplx<R>*plane, *twf, *twm, *lx, *ly;
+  int lys;
 };
 template <typename R, class GP> __device__ __forceinline__ PlaneSmem<R> plane_smem_of(const Geom& g) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PlaneSmem<R> m;
   m.plane = reinterpret_cast<cplx<R>*>(smem_raw);
   m.twf = m.plane + GP::Lm(g) * GP::S(g);
-  m.twm = m.twf + GP::Lf(g);
+  m.twm = GP::kStatic ? m.twf : m.twf + GP::Lf(g);
   m.lx = m.twm + GP::Lm(g);
-  m.ly = m.lx + GP::Lf(g);
+  m.ly = GP::kStatic ? m.plane + GP::Lf(g) : m.lx + GP::Lf(g);
+  m.lys = GP::kStatic ? GP::S(g) : 1;
   return m;
 }
 
@@ -104,17 +108,17 @@ __device__ __forceinline__ void plane_tables(const Geom& g, const cplx<R>* tw, c
     if constexpr (!GEN) m.lx[i] = cvt<R>(tab[g.oLx + i]);
   }
   for (int i = threadIdx.x; i < Lm; i += GP::plane_threads()) {
-    m.twm[i] = tw[g.twm + i];
-    m.ly[i] = cvt<R>(GEN ? tab[g.oDky + s * g.Ny + i] : tab[g.oLy + i]);
+    if constexpr (!GP::kStatic) m.twm[i] = tw[g.twm + i];
+    m.ly[i * m.lys] = cvt<R>(GEN ? tab[g.oDky + s * g.Ny + i] : tab[g.oLy + i]);
   }
 }
 
-// plane *= D_kz (inverse) or conj(D_kz) (forward), General lattices: from the table of the
-// k-point where there is one (coalesced; evaluated in place, the sincospi were a
-// quarter of the plane kernels' instructions), else evaluated.
+// plane *= conj(D_kz), General lattices: from the table of the k-point where there is one
+// (coalesced; evaluated in place, the sincospi were a quarter of the plane kernels'
+// instructions), else evaluated.  In the inverse direction the values have their parts swapped,
+// and multiplying by the conjugate is what multiplies the value by D_kz.
 template <typename R, class GP>
-__device__ __forceinline__ void plane_times_dkz(const Geom& g, const double2* tabs, const cplx<R>* dkz, cplx<R>* plane,
-                                                bool inv) {
+__device__ __forceinline__ void plane_times_dkz(const Geom& g, const double2* tabs, const cplx<R>* dkz, cplx<R>* plane) {
   const PlanePos p = plane_pos();
   const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
   const Div dlf(Lf);
@@ -123,11 +127,24 @@ __device__ __forceinline__ void plane_times_dkz(const Geom& g, const double2* ta
 #pragma unroll 4
   for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
     const int m = (int)dlf.q(e), q = e + m * (S - Lf);
-    cplx<R> w = d ? d[e] : dkz_at<R>(g, tab, p.s, m, e - m * Lf);
-    if (!inv) w = cconj(w);
-    plane[q] = cmul(plane[q], w);
+    plane[q] = cmulc(d ? d[e] : dkz_at<R>(g, tab, p.s, m, e - m * Lf), plane[q]);
   }
   __syncthreads();
+}
+
+// Whether the inverse transforms of a plane run as forward ones on values with swapped real and
+// imaginary parts, swap(z) = i conj(z): swap(IDFT z) = DFT swap(z).  The mix writes them so and
+// plane_store swaps them back.  (Static Simple geometries have the direction at compile time.)
+template <bool GEN, class GP> constexpr bool kSwapInv = !(GP::kStatic && !GEN);
+template <bool SWAP, typename T> __device__ __forceinline__ T maybe_swap(T z) {
+  if constexpr (SWAP) {
+    T y;
+    y.x = z.y;
+    y.y = z.x;
+    return y;
+  } else {
+    return z;
+  }
 }
 
 // Unnormalised inverse 2-D transform of the CTA's plane: fast axis, (x D_kz), mid axis; x D_ky
@@ -142,8 +159,8 @@ __device__ __forceinline__ void plane_inverse(const Geom& g, const double2* tabs
     // one FFT call site per axis loop: the runtime plans' passes are long
 #pragma unroll 1
     for (int ax = 0; ax < 2; ax++) {
-      GP::template fft_plane<R, RARE>(m.plane, g, ax == 0, ax == 0 ? m.twf : m.twm, true);
-      if (GEN && ax == 0) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane, true);
+      GP::template fft_plane<R, RARE>(m.plane, g, ax == 0, ax == 0 ? m.twf : m.twm);
+      if (GEN && ax == 0) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane);
     }
   }
 }
@@ -160,8 +177,8 @@ __device__ __forceinline__ void plane_forward(const Geom& g, const double2* tabs
 #pragma unroll 1
     for (int ax = 0; ax < 2; ax++) {
       const bool fast = GEN ? ax == 1 : ax == 0;
-      if (GEN && ax == 1) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane, false);
-      GP::template fft_plane<R, RARE>(m.plane, g, fast, fast ? m.twf : m.twm, false);
+      if (GEN && ax == 1) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane);
+      GP::template fft_plane<R, RARE>(m.plane, g, fast, fast ? m.twf : m.twm);
     }
   }
 }
@@ -211,7 +228,7 @@ __device__ __forceinline__ void plane_store(const Geom& g, cplx<R>* T) {
 #pragma unroll 4
   for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
     const int r = GP::kStatic ? e / Lf : (int)dlf.q(e);
-    const cplx<R> v = m.plane[e + r * (S - Lf)];
+    const cplx<R> v = maybe_swap<kSwapInv<GEN, GP>>(m.plane[e + r * (S - Lf)]);
     T[e] = GEN ? cmul(v, m.ly[r]) : v;
   }
 }
@@ -219,7 +236,8 @@ __device__ __forceinline__ void plane_store(const Geom& g, cplx<R>* T) {
 // Exchange of mixed components between the three CTAs.  Static geometries send them with
 // st.async into the owner's plane, counted on the owner's barrier (P values arrive per
 // plane); the others store to distributed shared memory and use a cluster barrier.
-template <typename R, bool ASYNC> struct PlaneExchange {
+// SWAP: the values are written with swapped parts (kSwapInv).
+template <typename R, bool ASYNC, bool SWAP> struct PlaneExchange {
   cplx<R>* dst[3];
   unsigned rplane[3], rbar[3];
   __device__ __forceinline__ PlaneExchange(cplx<R>* plane, unsigned bar) {
@@ -235,9 +253,9 @@ template <typename R, bool ASYNC> struct PlaneExchange {
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       if constexpr (ASYNC)
-        st_async(rplane[c] + (unsigned)(q * sizeof(cplx<R>)), v[c], rbar[c]);
+        st_async(rplane[c] + (unsigned)(q * sizeof(cplx<R>)), maybe_swap<SWAP>(v[c]), rbar[c]);
       else
-        dst[c][q] = v[c];
+        dst[c][q] = maybe_swap<SWAP>(v[c]);
     }
   }
 };
@@ -290,7 +308,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       }
       if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, (unsigned)(P * sizeof(cplx<R>)));
     }
-    const PlaneExchange<R, kAsyncMix> ex(m.plane, bar);
+    const PlaneExchange<R, kAsyncMix, kSwapInv<GEN, GP>> ex(m.plane, bar);
     const long vb = (long)(p.slot * a.vec_per_slot + p.vec) * a.vstride;
     const int Nd = sl.Nd, off = sl.off;
     const int per = (P + 2) / 3;
@@ -338,7 +356,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
         if (fi >= off) {
           const long i = fi - off;
           cplx<R> Lx, Ly, Lz;
-          lam_elem<R, GEN>(g, tab, m.lx, m.ly, lz, p.s, r, f, Lx, Ly, Lz);
+          lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lz, p.s, r, f, Lx, Ly, Lz);
           cplx<R> x1 = A1[k], x2 = A2[k];
           if constexpr (IN == IN_VEC) {
             if (a.sigma) {
@@ -401,7 +419,10 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     const PlanePos p = plane_pos();
     const Slot sl = a.slots[p.slot];
     const CgState* st = a.cg + p.slot;
-    if (!sl.active || !st->active) return;  // uniform over the cluster
+    if (!sl.active || !st->active) {  // uniform over the cluster
+      if (blockIdx.x == 0 && threadIdx.x == 0) a.cg_copy[p.slot].active = 0;
+      return;
+    }
     const int cur = st->iter & 1;
     // this CTA's own part of r, r_old, x and x_old: it streams into L2 during the transforms
     long i0, i1;
@@ -421,7 +442,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       plane_load<R, GEN, GP>(g, T, m);
     }
     // gamma and rho from the pencil stage's partial sums of <r, A r>, summed in order by one warp
-    // while the plane streams in (k_cg_decide forms the same numbers for the CG state)
+    // while the plane streams in
     if (threadIdx.x < 32) {
       const double rAr = warp_sum_partials(a.partials + (size_t)p.slot * a.pstride, a.pen_parts) / g.N;
       double gm, rho;
@@ -429,6 +450,12 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       if (threadIdx.x == 0) {
         s_coef[0] = gm;
         s_coef[1] = rho;
+        if (blockIdx.x == 0) {
+          CgState c = *st;
+          c.gm = gm;
+          c.rho = rho;
+          a.cg_copy[p.slot] = c;
+        }
       }
     }
     if constexpr (!GEN) cp_async_wait_all();
@@ -453,7 +480,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     const Slot sl = a.slots[p.slot];
     const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
     const cplx<R> lz = GEN ? mk<R>(0, 0) : cvt<R>(tab[g.oLz + p.s]);
-    const PlaneExchange<R, kAsyncMix> ex(m.plane, bar);
+    const PlaneExchange<R, kAsyncMix, kSwapInv<GEN, GP>> ex(m.plane, bar);
     const int iter = a.cg[p.slot].iter, cur = iter & 1;
     const bool have_r = iter > 1, have_x = iter > 2;  // r_old = 0 at k = 1; x = 0 at k = 1, x_old = 0 at k = 2
     const long vb = (long)p.slot * a.vstride;
@@ -503,7 +530,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
         if (fi >= off) {
           const long i = fi - off;
           cplx<R> Lx, Ly, Lz;
-          lam_elem<R, GEN>(g, tab, m.lx, m.ly, lz, p.s, r, f, Lx, Ly, Lz);
+          lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lz, p.s, r, f, Lx, Ly, Lz);
           cplx<R> Pc[6];
           pi_from<R>(GEN, false, Lx, Ly, Lz, Pc);
           const cplx<R> w1 = cadd(cadd(cmulc(Pc[0], t[k][0]), cmulc(Pc[1], t[k][1])), cmulc(Pc[2], t[k][2]));
@@ -531,18 +558,56 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
   }
   plane_inverse<R, GEN, RARE, GP>(g, a.tabs, a.dkz);
   plane_store<R, GEN, GP>(g, a.T + plane_base<R, GP>(g, plane_pos(), 1, a.fstride));
-  // this CTA's part of ||r'||^2; k_cg_decide sums the slot's parts in order
+  // this CTA's part of ||r'||^2; the pencil stage sums the slot's parts in order
   __shared__ double sred[32];
   block_reduce<1>(acc, sred);
   if (threadIdx.x == 0) a.partials[(size_t)blockIdx.z * a.pstride + a.pen_parts + blockIdx.x] = acc[0];
 }
 
+// ------------------------------------------------------------------ end of a CG iteration
+// The first CTA of a k-point in the pencil stage ends the CG iteration on the side (a kernel of its
+// own took 6 us of the 47 us of an iteration on a small grid): from the plane stage's ||r'||^2
+// parts it tells whether the solve goes on (CG.cu:37, :77) and steps the state.  The other CTAs
+// do not wait for that: the transforms after a solve's last iteration are work for nothing, but
+// a decision in every CTA cost the 96^3 pencil stage 17%.  The state before the step is read from
+// cg_in, the copy that the plane stage made (with the coefficients it used: the sums they came
+// from are this launch's to overwrite); the new one goes to cg.
+// One warp; returns (in all lanes) whether slot q goes on.
+template <typename R> __device__ __forceinline__ int cg_advance(const PencilArgs<R>& a, int q, bool write) {
+  const CgState* in = a.cg_in + q;
+  const double rr = warp_sum_partials<4>(a.partials + (size_t)q * a.pstride + a.pen_parts, a.fwd_parts);
+  const int go = rr > in->tol2 && in->iter + 1 <= in->maxit;
+  if (write && (threadIdx.x & 31) == 0) {
+    CgState* st = a.cg + q;
+    st->gm = in->gm;
+    st->rho = in->rho;
+    st->r1p = in->r1;
+    st->r1 = rr;
+    st->iter = in->iter + 1;
+    st->total = in->total + 1;
+    st->active = go;
+  }
+  return go;
+}
+
+// The WHILE condition of the CG loop, by one CTA of `nt` threads: whether any k-point goes on.
+template <typename R> __device__ __forceinline__ void cg_loop_decide(const PencilArgs<R>& a, int nt) {
+  __shared__ int any;
+  if (threadIdx.x == 0) any = 0;
+  __syncthreads();
+  for (int q = threadIdx.x >> 5; q < a.nslots; q += nt / 32)
+    if (a.slots[q].active && a.cg_in[q].active && cg_advance(a, q, false) && (threadIdx.x & 31) == 0) any = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) decide_cond(a.cond, any);
+}
+
 // ------------------------------------------------------------------ pencil stage
 
 // Pencil CTAs per SM the register budget is sized for: the prime passes (RARE 2) and the static
-// FP64 plans need 128 registers.
+// FP64 plans need 128 registers; the static FP32 ones fit 64 (four CTAs: 96^3 CG pencil stage 13.3
+// us per k-point at 3, 11.4 at 4).
 template <typename R, int RARE, class GP> constexpr int pencil_min_blocks() {
-  return RARE >= 2 || (GP::kStatic && sizeof(R) == 8) ? 2 : 3;
+  return RARE >= 2 || (GP::kStatic && sizeof(R) == 8) ? 2 : GP::kStatic ? 4 : 3;
 }
 
 // One CTA transforms TW consecutive positions e = m * Lf + f of the plane (a tile may span
@@ -561,18 +626,25 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
   R* ibt = reinterpret_cast<R*>(tile + Ls * TW);
   cplx<R>* tws = reinterpret_cast<cplx<R>*>(ibt + Ls * TW);
   constexpr bool QBQ = MODE == PEN_QBQ || MODE == PEN_QBQ_CG;
-  const int slot = blockIdx.z;
+  // The CG walks the k-points backwards here and forwards in its plane stage, so that each
+  // stage starts on fields that the other left in L2 (96^3, FP32 CG iteration: 66.8 -> 65.3 us
+  // per k-point in a solve of 8).
+  const int slot = MODE == PEN_QBQ_CG ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
+  if constexpr (MODE == PEN_QBQ_CG)
+    if (a.cg_in && blockIdx.x == 0 && blockIdx.y == 0 && slot == 0) cg_loop_decide(a, NT);
   const Slot sl = a.slots[slot];
   if (!sl.active) return;
-  if (a.gate == 1 && !a.cg[slot].active) return;
-  if (a.gate == 2 && !a.cg[slot].outer_active) return;
+  const CgState* st = MODE == PEN_QBQ_CG && a.cg_in ? a.cg_in + slot : a.cg + slot;
+  if (a.gate == 1 && !st->active) return;
+  if (a.gate == 2 && !st->outer_active) return;
   const int comp = blockIdx.y % 3, vec = blockIdx.y / 3;
   const int e0 = blockIdx.x * TW;
   const int tw_n = min(TW, P - e0);
   if constexpr (MODE == PEN_QBQ_CG) {
     // the field rows and 1/eps rows of the tile of the CTA one wave ahead
     int x2, y2, z2;
-    if (a.pf_dist > 0 && cta_of(cta_linear() + a.pf_dist, x2, y2, z2) && a.slots[z2].active && a.cg[z2].active) {
+    if (a.pf_dist > 0 && cta_of(cta_linear() + a.pf_dist, x2, y2, z2)) {
+      z2 = gridDim.z - 1 - z2;
       const int f2 = x2 * TW, c2 = y2 % 3, v2 = y2 / 3;
       const int n2 = min(TW, P - f2);
       for (int i = threadIdx.x; i < 2 * Ls; i += NT) {
@@ -634,6 +706,8 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
         }
       }
     }
+    if constexpr (MODE == PEN_QBQ_CG)
+      if (a.cg_in && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 32) cg_advance(a, slot, true);
     cp_async_wait_all();
   } else {
     for (int q = threadIdx.x; q < Ls * TW; q += NT) {
@@ -653,7 +727,9 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
   }
   __syncthreads();
   // QBQ: inverse, x B^{-1}/N, forward.  QR_OUT: inverse, x D/N (and B^{-1}), store.
-  // QRS_IN: forward only.  One FFT call site (dir loop) for the register budget.
+  // QRS_IN: forward only.  One FFT call site (dir loop) for the register budget, and forward
+  // transforms only: DFT(x) holds IDFT(x)[-s] in row s, and the DFT of what is then in rows -s
+  // comes out in rows -k, so the rows are counted backwards in between and in the store.
   constexpr int ndir = QBQ ? 2 : 1;
   // PEN_QBQ_CG: sum of |v|^2 / eps over the tile after the inverse transform
   R dot = 0;
@@ -675,15 +751,14 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
     GP::template fft_slow_c<R, false>(tile, tws);
   }
   for (int dir = 0; !kStatQBQ && dir < ndir; dir++) {
-    const bool inv = MODE == PEN_QRS_IN ? false : dir == 0;
-    GP::template fft_slow<R, RARE>(tile, g, tws, inv);
+    GP::template fft_slow<R, RARE>(tile, g, tws);
     if (MODE != PEN_QRS_IN && dir == 0) {
       const R invN = (R)(1.0 / g.N);
       for (int q = threadIdx.x; q < Ls * TW; q += NT) {
-        const int s = q / TW, f = q - s * TW;
+        const int row = q / TW, f = q - row * TW, s = row == 0 ? 0 : Ls - row;
         if (f < tw_n) {
           if constexpr (QBQ) {
-            const R ib = ib_field ? ibt[q] : a.invB[(long)comp * g.N + spatial(s, e0 + f)];
+            const R ib = ib_field ? ibt[s * TW + f] : a.invB[(long)comp * g.N + spatial(s, e0 + f)];
             if constexpr (MODE == PEN_QBQ_CG) dot += ib * cabs2(tile[q]);
             tile[q] = cscale(tile[q], ib * invN);
           } else {
@@ -700,7 +775,8 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
   }
   if constexpr (QBQ || MODE == PEN_QRS_IN) {
     for (int q = threadIdx.x; q < Ls * TW; q += NT) {
-      const int s = q / TW, f = q - s * TW;
+      const int row = q / TW, f = q - row * TW;
+      const int s = QBQ && !kStatQBQ && row > 0 ? Ls - row : row;
       if (f < tw_n) a.T[fb + (long)s * P + e0 + f] = tile[q];
     }
   }
@@ -741,19 +817,17 @@ __device__ __forceinline__ int pencil_pipe_tile(const PencilArgs<R>& a, int t, l
   off = m * 96 + f0;
   return slot;
 }
-template <typename R> __device__ __forceinline__ bool pencil_pipe_live(const PencilArgs<R>& a, int t) {
+template <typename R> __device__ __forceinline__ bool pencil_pipe_live(const PencilArgs<R>& a, int t, const unsigned* on) {
   const int slot = t / (3 * a.vec_per_slot * 96 * (96 / PencilTW<R>::v));
-  if (!a.slots[slot].active) return false;
-  if (a.gate == 1 && !a.cg[slot].active) return false;
-  if (a.gate == 2 && !a.cg[slot].outer_active) return false;
-  return true;
+  return (on[slot >> 5] >> (slot & 31)) & 1;
 }
 // Starts the 16-byte copies of tile t's field rows and 1/eps rows into (tile, ibt).
 template <typename R>
-__device__ __forceinline__ void pencil_pipe_issue(const PencilArgs<R>& a, int t, int total, cplx<R>* tile, R* ibt) {
+__device__ __forceinline__ void pencil_pipe_issue(const PencilArgs<R>& a, int t, int total, const unsigned* on, cplx<R>* tile,
+                                                  R* ibt) {
   constexpr int TW = PencilTW<R>::v, P = 96 * 96;
   constexpr int CH = 16 / sizeof(cplx<R>), CHB = 16 / sizeof(R);
-  if (t >= total || !pencil_pipe_live(a, t)) return;
+  if (t >= total || !pencil_pipe_live(a, t, on)) return;
   long fb;
   int off, comp;
   pencil_pipe_tile<R>(a, t, fb, off, comp);
@@ -772,7 +846,7 @@ __device__ __forceinline__ void pencil_pipe_issue(const PencilArgs<R>& a, int t,
 template <typename R, bool DOT>
 __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_pencil_pipe(PencilArgs<R> a) {
   FAME_COUNT_LAUNCH();
-  using GP = Stat96;
+  using GP = Stat96<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Geom& g = a.g;
   constexpr int TW = PencilTW<R>::v;
@@ -787,27 +861,50 @@ __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_penc
   __shared__ double sred[32];
   for (int i = threadIdx.x; i < Ls; i += kPencilThreads) tws[i] = a.tw[g.tws + i];
   const int total = a.nslots * 3 * a.vec_per_slot * Lm * nft;
+  // the live k-points (a slot of this grid takes over 0.3 GB, so 1024 of them do not fit), and,
+  // in the first CTA of a CG's launch, the end of the iteration for each
+  __shared__ unsigned on[32];
+  __shared__ int goes_on;
+  if (threadIdx.x < 32) on[threadIdx.x] = 0;
+  if (threadIdx.x == 0) goes_on = 0;
+  __syncthreads();
+  for (int q = threadIdx.x >> 5; q < a.nslots; q += kPencilThreads / 32) {
+    int live = a.slots[q].active;
+    if (live && DOT && a.cg_in) {
+      live = a.cg_in[q].active;
+      if (live && blockIdx.x == 0 && cg_advance(a, q, true) && (threadIdx.x & 31) == 0) goes_on = 1;
+    } else if (live && a.gate == 1)
+      live = a.cg[q].active;
+    else if (live && a.gate == 2)
+      live = a.cg[q].outer_active;
+    if ((threadIdx.x & 31) == 0 && live) atomicOr(&on[q >> 5], 1u << (q & 31));
+  }
+  __syncthreads();
+  if (DOT && a.cg_in && blockIdx.x == 0 && threadIdx.x == 0) decide_cond(a.cond, goes_on);
   int t = blockIdx.x;
-  pencil_pipe_issue<R>(a, t, total, tiles, ibts);
+  pencil_pipe_issue<R>(a, t, total, on, tiles, ibts);
   cp_async_commit();
   for (int b = 0; t < total; b ^= 1, t += gridDim.x) {
     // buffer b ^ 1 was released at the end of the last iteration
-    pencil_pipe_issue<R>(a, t + gridDim.x, total, tiles + (b ^ 1) * TILE, ibts + (b ^ 1) * TILE);
+    pencil_pipe_issue<R>(a, t + gridDim.x, total, on, tiles + (b ^ 1) * TILE, ibts + (b ^ 1) * TILE);
     cp_async_commit();
     cp_async_wait_group<1>();  // this tile's group has landed
     __syncthreads();
-    if (pencil_pipe_live(a, t)) {  // uniform over the CTA
+    if (pencil_pipe_live(a, t, on)) {  // uniform over the CTA
       cplx<R>* tile = tiles + b * TILE;
       double dot[1] = {0.0};
-      // inverse, x B^{-1}/N, forward; one FFT call site for the register budget
+      // inverse, x B^{-1}/N, forward; one FFT call site for the register budget, both
+      // transforms forward with the rows counted backwards in between (see k_pencil)
       for (int dir = 0; dir < 2; dir++) {
-        GP::template fft_slow<R, 0>(tile, g, tws, dir == 0);
+        GP::template fft_slow<R, 0>(tile, g, tws);
         if (dir == 0) {
           const R invN = (R)(1.0 / g.N);
           const R* ibt = ibts + b * TILE;
           for (int q = threadIdx.x; q < TILE; q += kPencilThreads) {
-            if constexpr (DOT) dot[0] += (double)(ibt[q] * cabs2(tile[q]));
-            tile[q] = cscale(tile[q], ibt[q] * invN);
+            const int row = q / TW;
+            const R ib = ibt[row == 0 ? q : q + (Ls - 2 * row) * TW];
+            if constexpr (DOT) dot[0] += (double)(ib * cabs2(tile[q]));
+            tile[q] = cscale(tile[q], ib * invN);
           }
           __syncthreads();
         }
@@ -816,8 +913,8 @@ __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_penc
       int off, comp;
       pencil_pipe_tile<R>(a, t, fb, off, comp);
       for (int q = threadIdx.x; q < TILE; q += kPencilThreads) {
-        const int s = q / TW, f = q - s * TW;
-        a.T[fb + (long)s * P + off + f] = tile[q];
+        const int row = q / TW, f = q - row * TW;
+        a.T[fb + (long)(row == 0 ? 0 : Ls - row) * P + off + f] = tile[q];
       }
       if constexpr (DOT) {
         const int per_slot = 3 * Lm * nft, slot = t / per_slot;
@@ -917,7 +1014,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       const long i = fi - off;
       const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - r * Lf;
       cplx<R> Lx, Ly, Lz;
-      lam_elem<R, GEN>(g, tab, m.lx, m.ly, lz, p.s, r, f, Lx, Ly, Lz);
+      lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lz, p.s, r, f, Lx, Ly, Lz);
       cplx<R> Pc[6];
       pi_from<R>(GEN, PR, Lx, Ly, Lz, Pc);
       const cplx<R> t0 = t[k][0], t1 = t[k][1], t2 = t[k][2];

@@ -121,7 +121,7 @@ struct fame_ctx {
   bool cap_mixed = false, cap_vec = false;
   DBuf<Slot> slots;
   DBuf<double2> tabs;
-  DBuf<CgState> cg;
+  DBuf<CgState> cg, cg_copy;
   DBuf<LzState> lz;
   DBuf<double> partials, T0, T1, hcoef, theta, Z, G, stats;
   DBuf<unsigned> counters, tri_ctr;
@@ -245,22 +245,6 @@ struct Ops {
   }
   template <typename R> const cplx<R>* dkz() const;
 
-  // CG coefficients kept, counters, loop decision
-  template <typename R> void cg_decide(Cond cond) {
-    CgDecideArgs d;
-    d.slots = c->slots.p;
-    d.cg = c->cg.p;
-    d.partials = c->partials.p;
-    d.pstride = c->part_stride;
-    d.pen_parts = cg_pen_parts<R>();
-    d.fwd_parts = cg_fwd_parts();
-    d.N = g().N;
-    d.counters = c->counters.p;
-    d.cond = cond;
-    d.nslots = nslots;
-    P.launch(k_cg_decide, dim3(nslots), dim3(32), 0, d);
-  }
-
   // What the plane kernels share: geometry, tables, twiddles; then the launch of kernel k
   // (static plane plans: `pick` swaps in the kernel and its thread count).
   template <typename R, typename A> A plane_args() const {
@@ -275,8 +259,8 @@ struct Ops {
     a.fstride = 3L * g().N;
     return a;
   }
-  template <typename R, typename A> void plane_launch(void (*k)(A), int nt, int nvec, const A& a) {
-    const size_t sm = plane_smem<R>(g());
+  template <typename R, typename A> void plane_launch(void (*k)(A), int nt, int nvec, const A& a, bool stat = false) {
+    const size_t sm = stat ? stat_plane_smem_bytes<R, Stat96<R>>() : plane_smem<R>(g());
     allow_smem(k, sm);
     P.launch(k, dim3(3 * g().Ls, nvec, nslots), dim3(nt), sm, a);
   }
@@ -300,7 +284,7 @@ struct Ops {
     } else {
       auto k = c->rare == 2 ? k_plane_inv<R, false, IN, PR, 2, DynGeom> : k_plane_inv<R, false, IN, PR, 0, DynGeom>;
       if constexpr (kStatInv<R, IN, PR>)
-        if (c->stat96) k = k_plane_inv<R, false, IN, PR, 0, Stat96>, nt = kStatPlaneThreads;
+        if (c->stat96) return plane_launch<R>(k_plane_inv<R, false, IN, PR, 0, Stat96<R>>, Stat96<R>::kThreads, nvec, a, true);
       plane_launch<R>(k, nt, nvec, a);
     }
   }
@@ -326,6 +310,7 @@ struct Ops {
       a.x[i] = x[i];
     }
     a.cg = c->cg.p;
+    a.cg_copy = c->cg_copy.p;
     a.T = T;
     a.partials = c->partials.p;
     a.pstride = c->part_stride;
@@ -343,26 +328,36 @@ struct Ops {
       plane_launch<R>(k, nt, 1, a);
     } else {
       auto k = c->rare == 2 ? k_plane_cg<R, false, 2, DynGeom> : k_plane_cg<R, false, 0, DynGeom>;
-      if (c->stat96) k = k_plane_cg<R, false, 0, Stat96>, nt = kStatPlaneThreads;
+      if (c->stat96) return plane_launch<R>(k_plane_cg<R, false, 0, Stat96<R>>, Stat96<R>::kThreads, 1, a, true);
       plane_launch<R>(k, nt, 1, a);
     }
   }
-  // A CG solve from the start residual r[1]: while active, plane stage (with the vector
-  // updates), decision, pencil stage.  r[1] and the CG state are set before.
+  // One CG iteration: plane stage (with the vector updates), then the pencil stage, which first
+  // ends the iteration (state, WHILE condition).
+  template <typename R>
+  void cg_iteration(cplx<R>* const (&r)[2], cplx<R>* const (&x)[2], cplx<R>* T, const R* invB, Cond cond) {
+    plane_cg<R>(r, x, T, cond);
+    pencil<R, PEN_QBQ_CG>(T, 1, 3L * g().N, invB, 1, nullptr, nullptr, &cond);
+  }
+  // A CG solve from the start residual r[1]; r[1] and the CG state are set before.  Two iterations
+  // per turn of the loop (a turn of a WHILE node costs about 2 us, of the host's loop about
+  // 10); after the last one of a solve the other finds nothing to do.
   template <typename R>
   void cg_solve(cplx<R>* const (&r)[2], cplx<R>* const (&x)[2], cplx<R>* T, const R* invB, Cond cond) {
     cg_start<R>(r, T, invB);
     P.while_loop(cond, [&] {
-      plane_cg<R>(r, x, T, cond);
-      cg_decide<R>(cond);
-      pencil<R, PEN_QBQ_CG>(T, 1, 3L * g().N, invB, 1);
+      for (int i = 0; i < 2; i++) cg_iteration<R>(r, x, T, invB, cond);
     });
   }
 
   template <typename R, int MODE>
   void pencil(cplx<R>* T, int nvec, long fstride, const R* invB, int gate, cplx<R>* out = nullptr,
-              const cplx<R>* in = nullptr) {
+              const cplx<R>* in = nullptr, const Cond* cg_end = nullptr) {
     PencilArgs<R> a;
+    a.cg_in = cg_end ? c->cg_copy.p : nullptr;
+    a.pen_parts = cg_pen_parts<R>();
+    a.fwd_parts = cg_fwd_parts();
+    a.cond = cg_end ? *cg_end : Cond{};
     a.g = g();
     a.slots = c->slots.p;
     a.tabs = c->tabs.p;
@@ -396,7 +391,7 @@ struct Ops {
     } else {
       auto k = c->rare_pen == 2 ? k_pencil<R, false, MODE, 2, DynGeom> : k_pencil<R, false, MODE, 0, DynGeom>;
       if constexpr (kStatPen<R, MODE> && sizeof(R) == 4)
-        if (c->stat96) k = k_pencil<R, false, MODE, 0, Stat96>, nt = kPencilThreads;
+        if (c->stat96) k = k_pencil<R, false, MODE, 0, Stat96<R>>, nt = kPencilThreads;
       if constexpr (kStatPen<R, MODE> && sizeof(R) == 8)
         if (c->stat96) {
           // FP64: pipelined, as many CTAs as are resident, each walking tiles (the FP32
@@ -441,7 +436,7 @@ struct Ops {
     } else {
       auto k = c->rare == 2 ? k_plane_fwd<R, false, EPI, PR, 2, DynGeom> : k_plane_fwd<R, false, EPI, PR, 0, DynGeom>;
       if constexpr (kStatFwd<R, EPI, PR>)
-        if (c->stat96) k = k_plane_fwd<R, false, EPI, PR, 0, Stat96>, nt = kStatPlaneThreads;
+        if (c->stat96) return plane_launch<R>(k_plane_fwd<R, false, EPI, PR, 0, Stat96<R>>, Stat96<R>::kThreads, nvec, a, true);
       plane_launch<R>(k, nt, nvec, a);
     }
   }
@@ -516,6 +511,7 @@ static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool
   c->slots.ensure(nslots);
   c->tabs.ensure((size_t)nslots * g.tab_stride);
   c->cg.ensure(nslots);
+  c->cg_copy.ensure(nslots);
   c->lz.ensure(nslots);
   const size_t lzblk = (M + kLzRows - 1) / kLzRows;
   const size_t part = std::max({lzblk * (2 * 64 + 1), (size_t)3 * g.Ls * 2 * 16, (size_t)1184 * 4,
@@ -990,6 +986,7 @@ void fame_ctx_destroy(fame_ctx* c) {
   c->invB32q.release();
   c->slots.release();
   c->cg.release();
+  c->cg_copy.release();
   c->lz.release();
   c->counters.release();
   c->tri_ctr.release();
@@ -1752,9 +1749,9 @@ int fame_bench_cg(fame_ctx* c, const double* k, int reps, int nbatch, double* ms
       FAME_CK(cudaEventRecord(ev[0], c->stream));
       o.plane_cg<float>(rb, xb, c->T32.p, Cond{});
       FAME_CK(cudaEventRecord(ev[1], c->stream));
-      o.cg_decide<float>(Cond{});
+      const Cond none{};
+      o.pencil<float, PEN_QBQ_CG>(c->T32.p, 1, F, c->ibq32(), 1, nullptr, nullptr, &none);
       FAME_CK(cudaEventRecord(ev[2], c->stream));
-      o.pencil<float, PEN_QBQ_CG>(c->T32.p, 1, F, c->ibq32(), 1);
       FAME_CK(cudaEventRecord(ev[3], c->stream));
       FAME_CK(cudaEventSynchronize(ev[3]));
       if (it == 0) continue;  // warm-up (the first iteration reads no r_old, x)

@@ -85,52 +85,6 @@ struct VecArgs {
   int nslots;
 };
 
-// ---------------------------------------------------------------- CG: end of an iteration
-// One CTA per slot, between the CG plane stage and the pencil stage.  From the partial sums of
-// <r, A r> (pencil stage) and of the new ||r||^2 (plane stage): the coefficients the plane stage
-// used, kept for the next iteration's, k++ and the loop test r1 > tol^2 && k <= maxit
-// (CG.cu:37, :57-77); the last CTA of the grid sets the WHILE condition.
-struct CgDecideArgs {
-  const Slot* slots;
-  CgState* cg;
-  const double* partials;
-  long pstride;
-  int pen_parts, fwd_parts;
-  int N;
-  unsigned* counters;  // [nslots] unused here, [nslots] = grid ticket
-  Cond cond;
-  int nslots;
-};
-
-__global__ void __launch_bounds__(32) k_cg_decide(CgDecideArgs d) {
-  FAME_COUNT_LAUNCH();
-  const int slot = blockIdx.x;
-  CgState* st = d.cg + slot;
-  if (d.slots[slot].active && st->active) {
-    const double* p = d.partials + (size_t)slot * d.pstride;
-    const double rAr = warp_sum_partials(p, d.pen_parts) / d.N;
-    const double rr = warp_sum_partials(p + d.pen_parts, d.fwd_parts);
-    if (threadIdx.x == 0) {
-      double gm, rho;
-      cg_coefficients(*st, rAr, gm, rho);
-      st->gm = gm;
-      st->rho = rho;
-      st->r1p = st->r1;
-      st->r1 = rr;
-      st->iter++;
-      st->total++;
-      st->active = (st->r1 > st->tol2) && (st->iter <= st->maxit);
-    }
-  }
-  if (grid_last(d.counters + d.nslots, gridDim.x)) {
-    if (threadIdx.x == 0) {
-      int any = 0;
-      for (int q = 0; q < d.nslots; q++) any |= d.slots[q].active && d.cg[q].active;
-      decide_cond(d.cond, any);
-    }
-  }
-}
-
 // ---------------------------------------------------------------- invAr prologue
 // rhs = u / sqrt(Lambda_q) (…invAr.cu:26), CG start x = 0, r = rhs (CG.cu:30-33).
 // Plain FP64 (MIXED = false): r64 is the CG's residual (k_plane_cg takes x = 0 at k = 1 as

@@ -144,7 +144,8 @@ struct PlaneCgArgs {
   long vstride, fstride;
   cplx<R>* r[2];          // residual: buffer iter & 1 is the current one, the other r_old / r'
   cplx<R>* x[2];          // solution, the same way
-  CgState* cg;
+  const CgState* cg;
+  CgState* cg_copy;       // the state with this iteration's gamma and rho, for the pencil stage that ends it
   cplx<R>* T;             // field of A r before the forward plane transforms in, of r' out
   double* partials;       // per slot: the pencil's <r, A r> parts, then this kernel's ||r'||^2 parts
   long pstride;           // per-slot stride of `partials`
@@ -167,7 +168,10 @@ struct PencilArgs {
   int ib_field;            // invB in the field layout (else the spatial layout; same for Simple lattices)
   cplx<R>* out;            // PEN_QR_OUT: spatial field out (3N per vector)
   const cplx<R>* in;       // PEN_QRS_IN: spatial field in
-  const CgState* cg;       // optional activity gate
+  CgState* cg;             // optional activity gate; the new state of a CG iteration (cg_in set)
+  const CgState* cg_in;    // PEN_QBQ_CG at the end of a CG iteration: the plane stage's copy, else NULL
+  int pen_parts, fwd_parts;  // partial sums per slot: <r, A r> (at the slot's start), then ||r'||^2
+  Cond cond;               // CG WHILE condition (cg_in set)
   int gate;                // 0 none, 1 CG active, 2 outer refinement active
   double* partials;        // PEN_QBQ_CG: partial sums of <v, Av>, [slot * pstride + CTA (or tile) of the slot]
   long pstride;            // per-slot stride of `partials`
@@ -218,22 +222,21 @@ __device__ __forceinline__ double warp_sum_strided_cg(const double* p, int n, in
 }
 
 // Ordered sum of n partial sums by one warp (lane-strided, then a fixed shuffle tree):
-// every caller gets the same bits, so kernels that need the same CG scalar (the step
-// size) agree exactly.  Valid in all lanes.
-__device__ __forceinline__ double warp_sum_partials(const double* p, int n) {
+// every caller gets the same bits, so CTAs that need the same CG scalar agree exactly.  Valid in
+// all lanes.  U independent loads per lane are in flight per round (a few hundred partials take
+// one or two L2 round trips, not one per element); they take 2 U registers.
+template <int U = 16> __device__ __forceinline__ double warp_sum_partials(const double* p, int n) {
   const int lane = threadIdx.x & 31;
   double s = 0.0;
-  // 16 independent loads per lane in flight per round (a few hundred partials take
-  // one or two L2 round trips, not one per element)
-  for (int b = 0; b < n; b += 32 * 16) {
-    double v[16];
+  for (int b = 0; b < n; b += 32 * U) {
+    double v[U];
 #pragma unroll
-    for (int u = 0; u < 16; u++) {
+    for (int u = 0; u < U; u++) {
       const int i = b + u * 32 + lane;
       v[u] = i < n ? p[i] : 0.0;
     }
 #pragma unroll
-    for (int u = 0; u < 16; u++) s += v[u];
+    for (int u = 0; u < U; u++) s += v[u];
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
