@@ -359,7 +359,7 @@ def run_ours(args):
             tj = json.load(open(tp))
             if tj.get("grid") == list(W["grid"]):
                 trc = int(nb * tj["dram_bytes_per_kpoint"])
-        roof = {"bound": "hbm", "kernel": f"FP32 CG iteration = plane_cg + cg_decide + pencil<PEN_QBQ_CG> over a "
+        roof = {"bound": "hbm", "kernel": f"FP32 CG iteration = plane_cg + pencil<PEN_QBQ_CG> over a "
                                           f"batch of {nb} k-points",
                 "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s", "frac": round(ach / hbm, 4),
                 "peak_source": src, "traffic": trc, "algorithmic_bytes": algc, "batch": nb,
@@ -449,10 +449,10 @@ def cg_iter_bytes(N):
 
 def cg_stage_bytes(N):
     """Bytes each FP32 CG kernel moves per k-point: plane_cg reads and writes the
-    3-component field, reads r, r_old, x, x_old and writes r' and x'; k_cg_decide moves the
-    partial sums (left out); the pencil stage reads and writes the field and reads 1/eps."""
+    3-component field, reads r, r_old, x, x_old and writes r' and x'; the pencil stage reads
+    and writes the field and reads 1/eps; the third span is empty."""
     M = 2 * N
-    return [6 * N * 8 + 6 * M * 8, 0, 6 * N * 8 + 3 * N * 4]
+    return [6 * N * 8 + 6 * M * 8, 6 * N * 8 + 3 * N * 4, 0]
 
 
 def apply_options(ctx, args):

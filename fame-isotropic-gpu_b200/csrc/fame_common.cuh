@@ -184,6 +184,14 @@ __device__ __forceinline__ void st_async(unsigned addr, double2 v, unsigned bar)
                : "memory");
 }
 
+// Programmatic dependent launch (sm_90+): a kernel launched with a programmatic edge starts once
+// every CTA of the kernel before it has called pdl_trigger (or has ended), and pdl_wait returns
+// when that kernel has ended and its writes are visible (at once without such an edge).  Every
+// CTA waits before it triggers or ends, so when a kernel starts early, all kernels before its
+// predecessor have ended: what it reads or writes before its own pdl_wait has to be older than that.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // Kernels launched on the device, counted by each kernel's first thread.  Every
 // translation unit has its own counter; FAME_DEFINE_LAUNCH_GETTER exposes it.
 static __device__ unsigned long long g_launches;

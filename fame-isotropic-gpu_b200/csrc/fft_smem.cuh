@@ -358,6 +358,20 @@ struct Div {
   __device__ __forceinline__ unsigned q(unsigned n) const { return d == 1 ? n : __umulhi(n, m); }
 };
 
+// The passes of one axis as the host lays them out for a CTA's threads (axis_passes): the index
+// arithmetic of a pass takes five integer divisions, which were a good part of what a thread does
+// on small grids (32^3, one k-point: 42 -> 33 us per FP32 CG iteration).
+struct PassDesc {
+  int radix, nb, ns, stw;  // n / radix, span, twiddle step
+  int G, items;            // lines and butterflies of a round
+  unsigned mG, mNs;        // ceil(2^32 / G), ceil(2^32 / ns): exact quotients, see Div (0 for a divisor of 1)
+};
+struct AxisPasses {
+  int n, npass, nl, ls, es;  // line length, passes, lines; line l, element m at l * ls + m * es
+  PassDesc d[kMaxPasses];
+};
+__device__ __forceinline__ int div_magic(int n, unsigned m) { return m ? (int)__umulhi((unsigned)n, m) : n; }
+
 // One radix-RAD Stockham pass over all lines, in place.  The butterflies of G complete
 // lines are one round (read all, barrier, write all, barrier): a line's outputs
 // overwrite positions other butterflies of the same line still read, so a line never
@@ -366,17 +380,10 @@ struct Div {
 // threads touch consecutive lines and at most the last deal of a round has idle threads.
 // G is the largest line count that T * MAXB butterflies cover, evened out over the rounds.
 template <typename R, int RAD, int MAXB>
-__device__ __forceinline__ void stockham_pass(cplx<R>* buf, int n, int Ns, LineSet L, const cplx<R>* tw) {
+__device__ __forceinline__ void stockham_pass(cplx<R>* buf, const AxisPasses& A, const PassDesc& d, const cplx<R>* tw) {
   const int T = blockDim.x;
-  const int nb = n / RAD;
-  const int stw = n / (Ns * RAD);
-  const int gmax = max(1, (T * MAXB) / nb);
-  const int rounds = (L.nl + gmax - 1) / gmax;
-  const int G = (L.nl + rounds - 1) / rounds;
-  const Div dg(G), dns(Ns);
-  const int items = G * nb;
   const int t = threadIdx.x;
-  for (int l0 = 0; l0 < L.nl; l0 += G) {
+  for (int l0 = 0; l0 < A.nl; l0 += d.G) {
     cplx<R> v[MAXB][RAD];
     int dst[MAXB];
     // (every value is defined on every path: left undefined for idle threads, the values of all
@@ -388,27 +395,27 @@ __device__ __forceinline__ void stockham_pass(cplx<R>* buf, int n, int Ns, LineS
 #pragma unroll
     for (int q = 0; q < MAXB; q++) {
       const int i = t + q * T;
-      const int j = (int)dg.q(i);
-      const int l = l0 + i - j * G;
+      const int j = div_magic(i, d.mG);
+      const int l = l0 + i - j * d.G;
       dst[q] = -1;
-      if (i < items && l < L.nl) {
-        const int jb = (int)dns.q(j);
-        const int k = j - jb * Ns;
-        const cplx<R>* src = buf + l * L.ls + j * L.es;
-        const int step = nb * L.es;
+      if (i < d.items && l < A.nl) {
+        const int jb = div_magic(j, d.mNs);
+        const int k = j - jb * d.ns;
+        const cplx<R>* src = buf + l * A.ls + j * A.es;
+        const int step = d.nb * A.es;
 #pragma unroll
         for (int u = 0; u < RAD; u++) v[q][u] = src[u * step];
         if (k > 0) {
-          const int kt = k * stw;
+          const int kt = k * d.stw;
 #pragma unroll
           for (int u = 1; u < RAD; u++) v[q][u] = cmul(v[q][u], tw[u * kt]);
         }
         Dft<R, RAD>::run(v[q], false);
-        dst[q] = l * L.ls + (jb * Ns * RAD + k) * L.es;
+        dst[q] = l * A.ls + (jb * d.ns * RAD + k) * A.es;
       }
     }
     __syncthreads();
-    const int ostep = Ns * L.es;
+    const int ostep = d.ns * A.es;
 #pragma unroll
     for (int q = 0; q < MAXB; q++) {
       if (dst[q] >= 0) {
@@ -614,15 +621,13 @@ constexpr int pass_maxb(int emax, int r) { return emax / r > 0 ? emax / r : 1; }
 // without them and the host picks by its axes (plan_level).  EMAX bounds the elements
 // a thread stages in registers per round.
 template <typename R, int EMAX, int RARE>
-__device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPlan& P, LineSet L, const cplx<R>* tw) {
-  const int n = P.n;
-  int Ns = 1;
+__device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPasses& A, const cplx<R>* tw) {
 #pragma unroll 1
-  for (int p = 0; p < P.npass; p++) {
-    const int r = P.radix[p];
-    switch (r) {
+  for (int p = 0; p < A.npass; p++) {
+    const PassDesc& d = A.d[p];
+    switch (d.radix) {
 #define FAME_PASS(r_) \
-  case r_: stockham_pass<R, r_, pass_maxb(EMAX, r_)>(buf, n, Ns, L, tw); break;
+  case r_: stockham_pass<R, r_, pass_maxb(EMAX, r_)>(buf, A, d, tw); break;
       FAME_PASS(2)
       FAME_PASS(3)
       FAME_PASS(4)
@@ -638,13 +643,42 @@ __device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPlan& P, LineS
 #undef FAME_PASS
       default:
         if constexpr (RARE >= 2) {
-          if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml>(buf, n, r, Ns, L, tw))
-            generic_pass<R, EMAX>(buf, n, r, Ns, L, tw);
+          const LineSet L{A.nl, A.ls, A.es};
+          if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml>(buf, A.n, d.radix, d.ns, L, tw))
+            generic_pass<R, EMAX>(buf, A.n, d.radix, d.ns, L, tw);
         }
         break;
     }
-    Ns *= r;
   }
+}
+
+// The passes of plan P over nl lines (line stride ls, element stride es) for T threads that
+// stage at most emax elements.
+inline AxisPasses axis_passes(const AxisPlan& P, int nl, int ls, int es, int T, int emax) {
+  AxisPasses A = {};
+  A.n = P.n;
+  A.npass = P.npass;
+  A.nl = nl;
+  A.ls = ls;
+  A.es = es;
+  auto magic = [](int d) { return d == 1 ? 0u : 0xffffffffu / (unsigned)d + 1u; };
+  int ns = 1;
+  for (int p = 0; p < P.npass; p++) {
+    PassDesc& d = A.d[p];
+    const int r = P.radix[p];
+    d.radix = r;
+    d.nb = P.n / r;
+    d.ns = ns;
+    d.stw = P.n / (ns * r);
+    const int gmax = T * pass_maxb(emax, r) / d.nb > 0 ? T * pass_maxb(emax, r) / d.nb : 1;
+    const int rounds = (nl + gmax - 1) / gmax;
+    d.G = (nl + rounds - 1) / rounds;
+    d.items = d.G * d.nb;
+    d.mG = magic(d.G);
+    d.mNs = magic(ns);
+    ns *= r;
+  }
+  return A;
 }
 
 // ---------------------------------------------------------------- compile-time plans

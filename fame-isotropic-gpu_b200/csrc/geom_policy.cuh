@@ -37,14 +37,12 @@ struct DynGeom {
   // reversed order (pencil stage), which takes the conjugations and sign choices of a runtime
   // direction out of every pass.
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const Geom& g, bool fast, const cplx<R>* tw) {
-    fft_lines<R, Emax<R>::v, RARE>(b, fast ? g.pf : g.pm, fast ? LineSet{g.Lm, g.S, 1} : LineSet{g.Lf, 1, g.S},
-                                   tw);
+  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const AxisPasses& A, bool, const cplx<R>* tw) {
+    fft_lines<R, Emax<R>::v, RARE>(b, A, tw);
   }
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom& g, const cplx<R>* tw) {
-    constexpr int TW = PencilTW<R>::v;
-    fft_lines<R, Emax<R>::v, RARE>(b, g.ps, LineSet{TW, 1, TW}, tw);
+  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const AxisPasses& A, const cplx<R>* tw) {
+    fft_lines<R, Emax<R>::v, RARE>(b, A, tw);
   }
 };
 
@@ -81,7 +79,7 @@ template <int LSL>
 struct DynGeomSlow : DynGeom {
   __device__ __forceinline__ static constexpr int pencil_threads() { return kPencilThreads; }
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom&, const cplx<R>* tw) {
+  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const AxisPasses&, const cplx<R>* tw) {
     constexpr int TW = PencilTW<R>::v;
     sfft<R, LSL, TW, kPencilThreads, SlowEmax<R>::v>(b, 1, TW, tw, false);
   }
@@ -99,7 +97,7 @@ struct DynGeomPlane : DynGeom {
   __device__ __forceinline__ static constexpr int plane_threads() { return T; }
   template <typename R, int RARE> static constexpr int plane_min_blocks() { return MB; }
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const Geom&, bool fast, const cplx<R>* tw) {
+  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const AxisPasses&, bool fast, const cplx<R>* tw) {
     if (fast)
       sfft<R, LF, LM, T, PlaneEmax<R>::v>(b, LF | 1, 1, tw, false);
     else
@@ -126,7 +124,7 @@ struct StatGeom {
   __device__ __forceinline__ static constexpr int P(const Geom&) { return LF * LM; }
   static_assert(LF == LM, "a static plane geometry has equal fast and mid lengths");
   template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const Geom&, const cplx<R>* tw) {
+  __device__ __forceinline__ static void fft_slow(cplx<R>* b, const AxisPasses&, const cplx<R>* tw) {
     fft_slow_c<R, false>(b, tw);
   }
   // Passes with the axis and the direction fixed at compile time: every

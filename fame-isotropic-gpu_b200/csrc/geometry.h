@@ -117,6 +117,7 @@ inline int layout_geom(const fame_lattice& L, Geom& g, long max_points, std::str
   g.Lm = g.Ny;
   g.Lf = g.general ? g.Nz : g.Nx;
   g.P = g.Lm * g.Lf;
+  g.mLf = g.Lf == 1 ? 0u : 0xffffffffu / (unsigned)g.Lf + 1u;
   g.S = g.Lf | 1;  // odd row pitch: bank-conflict-free passes along both plane axes
   if (!factor_axis(g.Lf, g.pf, radix_order) || !factor_axis(g.Lm, g.pm, radix_order) ||
       !factor_axis(g.Ls, g.ps, radix_order)) {
@@ -170,7 +171,7 @@ template <typename R> inline int plane_threads_min(const Geom& g) {
 // Threads of a runtime-plan CTA that works on `work` elements, for a launch of `ctas` CTAs with
 // `smem` bytes each, from `lo` up to `hi` in steps of 32; `sm_threads` is what the register
 // budget leaves resident per SM.  A CTA's time hardly falls with its threads (barriers and
-// global latency make up most of it: about 35 + 1.25 work / threads, in microseconds at 3,000
+// global latency make up most of it: about 35 + 1.6 work / threads, in microseconds at 3,000
 // elements), so what counts is how many run at once: the choice minimises waves times that
 // time, a partly filled last wave counted half beyond the first.  The clusters of three fill
 // about 0.94 of the CTA places.  Measured on launches of 4 to 6 k-points against about 12 elements per thread
@@ -180,6 +181,7 @@ inline int stage_threads(long work, long ctas, size_t smem, int sm_threads, int 
   constexpr int kSMs = 148;
   constexpr size_t kSmemSM = 228 * 1024, kSmemCta = 1024;
   lo = std::max(64, (lo + 31) / 32 * 32);
+  lo = (int)std::max<long>(lo, std::min<long>(std::min(192, hi), (work / 24 + 31) / 32 * 32));
   hi = (int)std::max<long>(lo, std::min<long>(hi, (work / 8 + 31) / 32 * 32));
   int best = lo;
   double best_cost = 1e300;
@@ -187,7 +189,7 @@ inline int stage_threads(long work, long ctas, size_t smem, int sm_threads, int 
     const int per_sm = std::min<int>({sm_threads / t, (int)(kSmemSM / (smem + kSmemCta)), 32});
     if (per_sm < 1) continue;
     const double w = ctas / (0.94 * kSMs * per_sm), up = ceil(w);
-    const double cost = (w <= 1.0 ? 1.0 : w + 0.5 * (up - w)) * (35.0 + 1.25 * work / t);
+    const double cost = (w <= 1.0 ? 1.0 : w + 0.5 * (up - w)) * (35.0 + 1.6 * work / t);
     if (cost < best_cost) {
       best_cost = cost;
       best = t;
@@ -215,6 +217,16 @@ inline int pencil_threads_rule(const Geom& g, int level, long vecs) {
   }
   return stage_threads((long)g.Ls * TW, 3 * vecs * ((g.P + TW - 1) / TW), pencil_smem_bytes<R>(g.Ls),
                        level < 2 ? 768 : 512, std::min(lo, kPencilThreads), kPencilThreads);
+}
+
+// The passes of the plane stage's two axes (a plane of pitch S) and of the pencil stage's, for
+// CTAs of `threads` threads.
+template <typename R> inline void plane_passes(const Geom& g, int threads, AxisPasses (&ax)[2]) {
+  ax[0] = axis_passes(g.pf, g.Lm, g.S, 1, threads, Emax<R>::v);
+  ax[1] = axis_passes(g.pm, g.Lf, 1, g.S, threads, Emax<R>::v);
+}
+template <typename R> inline AxisPasses pencil_passes(const Geom& g, int threads) {
+  return axis_passes(g.ps, PencilTW<R>::v, 1, PencilTW<R>::v, threads, Emax<R>::v);
 }
 
 // theta_x, theta_y(xy), theta_z(xyz) of wave vector k (FAME_Main/FAME_Matrix_Lambdas.cu:43-70)

@@ -121,12 +121,11 @@ template <typename R, class GP>
 __device__ __forceinline__ void plane_times_dkz(const Geom& g, const double2* tabs, const cplx<R>* dkz, cplx<R>* plane) {
   const PlanePos p = plane_pos();
   const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
-  const Div dlf(Lf);
   const cplx<R>* d = dkz ? dkz + (size_t)p.slot * g.N + (size_t)p.s * P : nullptr;
   const double2* tab = tabs + (size_t)p.slot * g.tab_stride;
 #pragma unroll 4
   for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
-    const int m = (int)dlf.q(e), q = e + m * (S - Lf);
+    const int m = div_magic(e, g.mLf), q = e + m * (S - Lf);
     plane[q] = cmulc(d ? d[e] : dkz_at<R>(g, tab, p.s, m, e - m * Lf), plane[q]);
   }
   __syncthreads();
@@ -150,7 +149,8 @@ template <bool SWAP, typename T> __device__ __forceinline__ T maybe_swap(T z) {
 // Unnormalised inverse 2-D transform of the CTA's plane: fast axis, (x D_kz), mid axis; x D_ky
 // follows in plane_store (General lattices, FAME_FFT_CUDA.cu:104-117).
 template <typename R, bool GEN, int RARE, class GP>
-__device__ __forceinline__ void plane_inverse(const Geom& g, const double2* tabs, const cplx<R>* dkz) {
+__device__ __forceinline__ void plane_inverse(const Geom& g, const AxisPasses* axes, const double2* tabs,
+                                              const cplx<R>* dkz) {
   const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
   if constexpr (GP::kStatic && !GEN) {
     GP::template fft_plane_c<R, true, true>(m.plane, m.twf);
@@ -159,7 +159,7 @@ __device__ __forceinline__ void plane_inverse(const Geom& g, const double2* tabs
     // one FFT call site per axis loop: the runtime plans' passes are long
 #pragma unroll 1
     for (int ax = 0; ax < 2; ax++) {
-      GP::template fft_plane<R, RARE>(m.plane, g, ax == 0, ax == 0 ? m.twf : m.twm);
+      GP::template fft_plane<R, RARE>(m.plane, axes[ax], ax == 0, ax == 0 ? m.twf : m.twm);
       if (GEN && ax == 0) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane);
     }
   }
@@ -168,7 +168,8 @@ __device__ __forceinline__ void plane_inverse(const Geom& g, const double2* tabs
 // Unnormalised forward 2-D transform.  General lattices (T*, FAME_FFT_CUDA.cu:128-150): x conj(D_ky)
 // (in plane_load), mid pass, x conj(D_kz), fast pass.  Simple lattices: fast then mid axis.
 template <typename R, bool GEN, int RARE, class GP>
-__device__ __forceinline__ void plane_forward(const Geom& g, const double2* tabs, const cplx<R>* dkz) {
+__device__ __forceinline__ void plane_forward(const Geom& g, const AxisPasses* axes, const double2* tabs,
+                                              const cplx<R>* dkz) {
   const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
   if constexpr (GP::kStatic && !GEN) {
     GP::template fft_plane_c<R, true, false>(m.plane, m.twf);
@@ -178,7 +179,7 @@ __device__ __forceinline__ void plane_forward(const Geom& g, const double2* tabs
     for (int ax = 0; ax < 2; ax++) {
       const bool fast = GEN ? ax == 1 : ax == 0;
       if (GEN && ax == 1) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane);
-      GP::template fft_plane<R, RARE>(m.plane, g, fast, fast ? m.twf : m.twm);
+      GP::template fft_plane<R, RARE>(m.plane, axes[fast ? 0 : 1], fast, fast ? m.twf : m.twm);
     }
   }
 }
@@ -194,10 +195,9 @@ __device__ __forceinline__ long plane_base(const Geom& g, const PlanePos& p, int
 template <typename R, bool GEN, class GP>
 __device__ __forceinline__ void plane_load(const Geom& g, const cplx<R>* T, const PlaneSmem<R>& m) {
   const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g), NT = GP::plane_threads();
-  const Div dlf(Lf);
   if constexpr (!GEN) {
     for (int e = threadIdx.x; e < P; e += NT) {
-      const int r = GP::kStatic ? e / Lf : (int)dlf.q(e);
+      const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf);
       cp_async_elem(m.plane + e + r * (S - Lf), T + e);
     }
   } else {
@@ -211,7 +211,7 @@ __device__ __forceinline__ void plane_load(const Geom& g, const cplx<R>* T, cons
       for (int u = 0; u < U; u++) {
         const int e = eb + u * NT;
         if (e < P) {
-          const int r = (int)dlf.q(e);
+          const int r = div_magic(e, g.mLf);
           m.plane[e + r * (S - Lf)] = cmulc(m.ly[r], v[u]);
         }
       }
@@ -224,10 +224,9 @@ template <typename R, bool GEN, class GP>
 __device__ __forceinline__ void plane_store(const Geom& g, cplx<R>* T) {
   const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
   const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
-  const Div dlf(Lf);
 #pragma unroll 4
   for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
-    const int r = GP::kStatic ? e / Lf : (int)dlf.q(e);
+    const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf);
     const cplx<R> v = maybe_swap<kSwapInv<GEN, GP>>(m.plane[e + r * (S - Lf)]);
     T[e] = GEN ? cmul(v, m.ly[r]) : v;
   }
@@ -278,6 +277,7 @@ template <typename R, bool GEN, int IN, bool PR, int RARE, class GP>
 __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
     k_plane_inv(PlaneInArgs<R> a) {
   FAME_COUNT_LAUNCH();
+  pdl_wait();
   const Geom& g = a.g;
   constexpr bool kAsyncMix = GP::kStatic;
   __shared__ __align__(8) unsigned long long xbar;
@@ -286,7 +286,6 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
   {
     const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
     const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
-    const Div dlf(Lf);  // row of plane element e: e / Lf (folds to a constant for static geometries)
     cg::cluster_group cl = cg::this_cluster();
     const PlanePos p = plane_pos();
     const Slot sl = a.slots[p.slot];
@@ -351,7 +350,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
         const int e = eb + k * NT;
         if (e >= e1) break;
         const int fi = p.s * P + e;
-        const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - r * Lf;
+        const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), f = e - r * Lf;
         cplx<R> v[3] = {mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0)};
         if (fi >= off) {
           const long i = fi - off;
@@ -385,7 +384,8 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     else
       cl.sync();
   }
-  plane_inverse<R, GEN, RARE, GP>(g, a.tabs, a.dkz);
+  plane_inverse<R, GEN, RARE, GP>(g, a.ax, a.tabs, a.dkz);
+  pdl_trigger();
   plane_store<R, GEN, GP>(g, a.T + plane_base<R, GP>(g, plane_pos(), a.vec_per_slot, a.fstride));
 }
 
@@ -408,7 +408,6 @@ template <typename R, bool GEN, int RARE, class GP>
 __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
     k_plane_cg(PlaneCgArgs<R> a) {
   FAME_COUNT_LAUNCH();
-  if ((threadIdx.x | blockIdx.x | blockIdx.y | blockIdx.z) == 0) set_cond(a.reset, 0);
   const Geom& g = a.g;
   constexpr bool kAsyncMix = GP::kStatic;
   __shared__ __align__(8) unsigned long long xbar;
@@ -418,6 +417,11 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
   {
     const PlanePos p = plane_pos();
     const Slot sl = a.slots[p.slot];
+    const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
+    // the tables are the solve's, older than the kernel before this one
+    if (sl.active) plane_tables<R, GEN, GP>(g, a.tw, a.tabs + (size_t)p.slot * g.tab_stride, p.s, m);
+    pdl_wait();
+    if ((threadIdx.x | blockIdx.x | blockIdx.y | blockIdx.z) == 0) set_cond(a.reset, 0);
     const CgState* st = a.cg + p.slot;
     if (!sl.active || !st->active) {  // uniform over the cluster
       if (blockIdx.x == 0 && threadIdx.x == 0) a.cg_copy[p.slot].active = 0;
@@ -433,14 +437,9 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       prefetch_l2(v + (long)p.slot * a.vstride + ((threadIdx.x & 1) ? sl.Nd : 0) + i0, (i1 - i0) * sizeof(cplx<R>));
     }
     if (kAsyncMix && threadIdx.x == 0) exchange_init(bar, &skip, a.fault);
-    const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
     const cplx<R>* T = a.T + plane_base<R, GP>(g, p, 1, a.fstride);
-    if constexpr (!GEN) plane_load<R, GEN, GP>(g, T, m);
-    plane_tables<R, GEN, GP>(g, a.tw, a.tabs + (size_t)p.slot * g.tab_stride, p.s, m);
-    if constexpr (GEN) {
-      __syncthreads();  // D_ky is in place
-      plane_load<R, GEN, GP>(g, T, m);
-    }
+    if constexpr (GEN) __syncthreads();  // D_ky is in place
+    plane_load<R, GEN, GP>(g, T, m);
     // gamma and rho from the pencil stage's partial sums of <r, A r>, summed in order by one warp
     // while the plane streams in
     if (threadIdx.x < 32) {
@@ -461,7 +460,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     if constexpr (!GEN) cp_async_wait_all();
     __syncthreads();
   }
-  plane_forward<R, GEN, RARE, GP>(g, a.tabs, a.dkz);
+  plane_forward<R, GEN, RARE, GP>(g, a.ax, a.tabs, a.dkz);
   double acc[1] = {0.0};
   {
     cg::cluster_group cl = cg::this_cluster();
@@ -475,7 +474,6 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     }
     const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
     const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
-    const Div dlf(Lf);
     const PlanePos p = plane_pos();
     const Slot sl = a.slots[p.slot];
     const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
@@ -515,7 +513,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
             Y1[k] = xo[i];
             Y2[k] = xo[Nd + i];
           }
-          const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), q = r * S + (e - r * Lf);
+          const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), q = r * S + (e - r * Lf);
 #pragma unroll
           for (int c = 0; c < 3; c++) t[k][c] = ex.dst[c][q];
         }
@@ -525,7 +523,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
         const int e = eb + k * NT;
         if (e >= e1) break;
         const int fi = p.s * P + e;
-        const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - r * Lf;
+        const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), f = e - r * Lf;
         cplx<R> v[3] = {mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0)};
         if (fi >= off) {
           const long i = fi - off;
@@ -556,7 +554,8 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     else
       cl.sync();
   }
-  plane_inverse<R, GEN, RARE, GP>(g, a.tabs, a.dkz);
+  plane_inverse<R, GEN, RARE, GP>(g, a.ax, a.tabs, a.dkz);
+  pdl_trigger();
   plane_store<R, GEN, GP>(g, a.T + plane_base<R, GP>(g, plane_pos(), 1, a.fstride));
   // this CTA's part of ||r'||^2; the pencil stage sums the slot's parts in order
   __shared__ double sred[32];
@@ -617,6 +616,7 @@ template <typename R, bool GEN, int MODE, int RARE, class GP>
 __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>())
     k_pencil(PencilArgs<R> a) {
   FAME_COUNT_LAUNCH();
+  if constexpr (MODE != PEN_QBQ_CG) pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Geom& g = a.g;
   constexpr int TW = PencilTW<R>::v;
@@ -630,16 +630,39 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
   // stage starts on fields that the other left in L2 (96^3, FP32 CG iteration: 66.8 -> 65.3 us
   // per k-point in a solve of 8).
   const int slot = MODE == PEN_QBQ_CG ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
-  if constexpr (MODE == PEN_QBQ_CG)
-    if (a.cg_in && blockIdx.x == 0 && blockIdx.y == 0 && slot == 0) cg_loop_decide(a, NT);
   const Slot sl = a.slots[slot];
-  if (!sl.active) return;
-  const CgState* st = MODE == PEN_QBQ_CG && a.cg_in ? a.cg_in + slot : a.cg + slot;
-  if (a.gate == 1 && !st->active) return;
-  if (a.gate == 2 && !st->outer_active) return;
   const int comp = blockIdx.y % 3, vec = blockIdx.y / 3;
   const int e0 = blockIdx.x * TW;
   const int tw_n = min(TW, P - e0);
+  const bool ib_field = !GEN || a.ib_field;  // 1/eps rows contiguous along the tile's positions
+  // twiddles and 1/eps rows: the CG's pencil stage copies them before it waits for the plane stage
+  for (int i = threadIdx.x; i < Ls; i += NT) tws[i] = a.tw[g.tws + i];
+  constexpr int CH = 16 / sizeof(cplx<R>);  // elements per 16-byte copy
+  constexpr int CHB = 16 / sizeof(R);       // 1/eps values per 16-byte copy
+  if (QBQ && ib_field && sl.active) {
+    const R* ib = a.invB + (long)comp * g.N + e0;
+    if (P % CHB == 0 && ((uintptr_t)a.invB & 15) == 0) {
+      for (int q = threadIdx.x; q < Ls * (TW / CHB); q += NT) {
+        const int s = q / (TW / CHB), c = (q - s * (TW / CHB)) * CHB;
+        if (c < tw_n) cp_async16(ibt + s * TW + c, ib + (long)s * P + c);
+      }
+    } else {
+      for (int q = threadIdx.x; q < Ls * TW; q += NT) {
+        const int s = q / TW, c = q - s * TW;
+        if (c < tw_n) cp_async_real(ibt + q, ib + (long)s * P + c);
+      }
+    }
+  }
+  if constexpr (MODE == PEN_QBQ_CG) {
+    pdl_wait();
+    if (a.cg_in && blockIdx.x == 0 && blockIdx.y == 0 && slot == 0) cg_loop_decide(a, NT);
+  }
+  if (!sl.active) return;
+  const CgState* st = MODE == PEN_QBQ_CG && a.cg_in ? a.cg_in + slot : a.cg + slot;
+  if ((a.gate == 1 && !st->active) || (a.gate == 2 && !st->outer_active)) {
+    cp_async_wait_all();
+    return;
+  }
   if constexpr (MODE == PEN_QBQ_CG) {
     // the field rows and 1/eps rows of the tile of the CTA one wave ahead
     int x2, y2, z2;
@@ -657,28 +680,23 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
     }
   }
   const double2* tab = a.tabs + (size_t)slot * g.tab_stride;
-  for (int i = threadIdx.x; i < Ls; i += NT) tws[i] = a.tw[g.tws + i];
   const long fb = (long)(slot * a.vec_per_slot + vec) * a.fstride + (long)comp * g.N;
-  const Div dlf(Lf);
   // spatial index of slow position s at plane position e (QR_OUT, QRS_IN, 1/eps in the
   // spatial layout)
   auto spatial = [&](int s, int e) -> long {
     if (!GEN) return (long)s * P + e;
-    const int m = (int)dlf.q(e);
+    const int m = div_magic(e, g.mLf);
     return ((long)(e - m * Lf) * g.Ny + m) * g.Nx + s;
   };
   auto dk_at = [&](int s, int e) -> double2 {  // D_k (Simple) or D_kx
     if (GEN) return tab[g.oDkx + s];
-    const int m = (int)dlf.q(e);
+    const int m = div_magic(e, g.mLf);
     return cmul(cmul(tab[g.oDz + s], tab[g.oDy + m]), tab[g.oDx + (e - m * Lf)]);
   };
-  // ---- load.  The QBQ streams the field rows (TW contiguous elements at stride P) and
-  // the 1/eps rows (1/eps in the field layout) straight into shared memory with
-  // cp.async: 16 bytes a copy when every row starts on a 16-byte boundary (P a
-  // multiple of the copy's elements, the base aligned), else one element.
-  constexpr int CH = 16 / sizeof(cplx<R>);    // elements per 16-byte copy
-  constexpr int CHB = 16 / sizeof(R);         // 1/eps values per 16-byte copy
-  const bool ib_field = !GEN || a.ib_field;  // 1/eps rows contiguous along the tile's positions
+  // ---- load.  The QBQ streams the field rows (TW contiguous elements at stride P), like the
+  // 1/eps rows above, straight into shared memory with cp.async: 16 bytes a copy when every row
+  // starts on a 16-byte boundary (P a multiple of the copy's elements, the base aligned), else
+  // one element.
   if constexpr (QBQ) {
     const cplx<R>* src = a.T + fb + e0;
     if (CH == 1 || P % CH == 0) {
@@ -690,20 +708,6 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
       for (int q = threadIdx.x; q < Ls * TW; q += NT) {
         const int s = q / TW, c = q - s * TW;
         if (c < tw_n) cp_async_elem(tile + q, src + (long)s * P + c);
-      }
-    }
-    if (ib_field) {
-      const R* ib = a.invB + (long)comp * g.N + e0;
-      if (P % CHB == 0 && ((uintptr_t)a.invB & 15) == 0) {
-        for (int q = threadIdx.x; q < Ls * (TW / CHB); q += NT) {
-          const int s = q / (TW / CHB), c = (q - s * (TW / CHB)) * CHB;
-          if (c < tw_n) cp_async16(ibt + s * TW + c, ib + (long)s * P + c);
-        }
-      } else {
-        for (int q = threadIdx.x; q < Ls * TW; q += NT) {
-          const int s = q / TW, c = q - s * TW;
-          if (c < tw_n) cp_async_real(ibt + q, ib + (long)s * P + c);
-        }
       }
     }
     if constexpr (MODE == PEN_QBQ_CG)
@@ -751,7 +755,7 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
     GP::template fft_slow_c<R, false>(tile, tws);
   }
   for (int dir = 0; !kStatQBQ && dir < ndir; dir++) {
-    GP::template fft_slow<R, RARE>(tile, g, tws);
+    GP::template fft_slow<R, RARE>(tile, a.ax, tws);
     if (MODE != PEN_QRS_IN && dir == 0) {
       const R invN = (R)(1.0 / g.N);
       for (int q = threadIdx.x; q < Ls * TW; q += NT) {
@@ -773,6 +777,7 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_min_blocks<R, RARE, GP>
       __syncthreads();
     }
   }
+  pdl_trigger();
   if constexpr (QBQ || MODE == PEN_QRS_IN) {
     for (int q = threadIdx.x; q < Ls * TW; q += NT) {
       const int row = q / TW, f = q - row * TW;
@@ -846,6 +851,7 @@ __device__ __forceinline__ void pencil_pipe_issue(const PencilArgs<R>& a, int t,
 template <typename R, bool DOT>
 __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_pencil_pipe(PencilArgs<R> a) {
   FAME_COUNT_LAUNCH();
+  pdl_wait();
   using GP = Stat96<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Geom& g = a.g;
@@ -896,7 +902,7 @@ __global__ void __launch_bounds__(kPencilThreads, sizeof(R) == 4 ? 3 : 2) k_penc
       // inverse, x B^{-1}/N, forward; one FFT call site for the register budget, both
       // transforms forward with the rows counted backwards in between (see k_pencil)
       for (int dir = 0; dir < 2; dir++) {
-        GP::template fft_slow<R, 0>(tile, g, tws);
+        GP::template fft_slow<R, 0>(tile, a.ax, tws);
         if (dir == 0) {
           const R invN = (R)(1.0 / g.N);
           const R* ibt = ibts + b * TILE;
@@ -944,6 +950,7 @@ template <typename R, bool GEN, int EPI, bool PR, int RARE, class GP>
 __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
     k_plane_fwd(PlaneOutArgs<R> a) {
   FAME_COUNT_LAUNCH();
+  pdl_wait();
   const Geom& g = a.g;
   {
     const PlanePos p = plane_pos();
@@ -965,13 +972,12 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     }
     __syncthreads();
   }
-  plane_forward<R, GEN, RARE, GP>(g, a.tabs, a.dkz);
+  plane_forward<R, GEN, RARE, GP>(g, a.ax, a.tabs, a.dkz);
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();  // all three component planes transformed
 
   const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
   const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
-  const Div dlf(Lf);
   const PlanePos p = plane_pos();
   const Slot sl = a.slots[p.slot];
   const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
@@ -997,7 +1003,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       va[k] = vb2[k] = t[k][0] = t[k][1] = t[k][2] = mk<R>(0, 0);
       if (e < e1 && fi >= off) {
         const long i = fi - off;
-        const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), q = r * S + (e - r * Lf);
+        const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), q = r * S + (e - r * Lf);
 #pragma unroll
         for (int c = 0; c < 3; c++) t[k][c] = src[c][q];
         if constexpr (EPI == EPI_RESID) {
@@ -1012,7 +1018,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       const int fi = p.s * P + e;
       if (e >= e1 || fi < off) continue;
       const long i = fi - off;
-      const int r = GP::kStatic ? e / Lf : (int)dlf.q(e), f = e - r * Lf;
+      const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), f = e - r * Lf;
       cplx<R> Lx, Ly, Lz;
       lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lz, p.s, r, f, Lx, Ly, Lz);
       cplx<R> Pc[6];

@@ -36,6 +36,7 @@ struct Geom {
   int general;
   int Ls, Lm, Lf, P;  // slow / mid / fast lengths, plane size
   int S;              // row pitch of a plane in shared memory: Lf rounded up to odd
+  unsigned mLf;       // ceil(2^32 / Lf) (0 if Lf is 1): row of plane element e, see div_magic
   double hx, hy, hz;
   double ihz;  // 1 / hz
   double tnz;  // 2 / Nz

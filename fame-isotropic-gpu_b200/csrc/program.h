@@ -52,25 +52,12 @@ class Program {
 
   template <typename... P, typename... A>
   void launch(void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
-    if (grid.x == 0 || grid.y == 0 || grid.z == 0) return;
-    if (!graph_) {
-      k<<<grid, block, smem, stream_>>>(args...);
-      FAME_CK(cudaGetLastError());
-      return;
-    }
-    auto vals = std::make_shared<std::tuple<P...>>(args...);
-    void* ptrs[sizeof...(P) + 1];
-    fill_ptrs(*vals, ptrs, std::index_sequence_for<P...>{});
-    cudaKernelNodeParams kp = {};
-    kp.func = reinterpret_cast<void*>(k);
-    kp.gridDim = grid;
-    kp.blockDim = block;
-    kp.sharedMemBytes = (unsigned)smem;
-    kp.kernelParams = ptrs;
-    cudaGraphNode_t node;
-    Frame& f = frames_.back();
-    FAME_CK(cudaGraphAddKernelNode(&node, f.g, f.last ? &f.last : nullptr, f.last ? 1 : 0, &kp));
-    f.last = node;
+    add(k, grid, block, smem, false, args...);
+  }
+  // A kernel that calls pdl_wait: it may start before the kernel in front of it has ended.
+  template <typename... P, typename... A>
+  void launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    add(k, grid, block, smem, true, args...);
   }
 
   // Condition object for one WHILE loop; pass it to the kernels that set it.
@@ -106,6 +93,7 @@ class Program {
     cudaGraphNode_t node;
     FAME_CK(cudaGraphAddNode(&node, f.g, f.last ? &f.last : nullptr, f.last ? 1 : 0, &np));
     f.last = node;
+    f.last_kernel = false;
     cudaGraph_t body_graph = np.conditional.phGraph_out[0];
     frames_.push_back({body_graph, nullptr});
     body();
@@ -126,7 +114,46 @@ class Program {
   struct Frame {
     cudaGraph_t g;
     cudaGraphNode_t last;
+    bool last_kernel = false;  // `last` is a kernel node (only those have a programmatic port)
   };
+  template <typename... P, typename... A>
+  void add(void (*k)(P...), dim3 grid, dim3 block, size_t smem, bool pdl, A... args) {
+    if (grid.x == 0 || grid.y == 0 || grid.z == 0) return;
+    if (!graph_) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = grid;
+      cfg.blockDim = block;
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = stream_;
+      cudaLaunchAttribute at = {};
+      at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at.val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = pdl ? 1 : 0;
+      FAME_CK(cudaLaunchKernelEx(&cfg, k, P(args)...));
+      return;
+    }
+    auto vals = std::make_shared<std::tuple<P...>>(args...);
+    void* ptrs[sizeof...(P) + 1];
+    fill_ptrs(*vals, ptrs, std::index_sequence_for<P...>{});
+    Frame& f = frames_.back();
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeKernel;
+    np.kernel.func = reinterpret_cast<void*>(k);
+    np.kernel.gridDim = grid;
+    np.kernel.blockDim = block;
+    np.kernel.sharedMemBytes = (unsigned)smem;
+    np.kernel.kernelParams = ptrs;
+    cudaGraphEdgeData edge = {};
+    if (pdl && f.last_kernel) {
+      edge.from_port = cudaGraphKernelNodePortProgrammatic;
+      edge.type = cudaGraphDependencyTypeProgrammatic;
+    }
+    cudaGraphNode_t node;
+    FAME_CK(cudaGraphAddNode_v2(&node, f.g, f.last ? &f.last : nullptr, f.last ? &edge : nullptr, f.last ? 1 : 0, &np));
+    f.last = node;
+    f.last_kernel = true;
+  }
   template <typename Tup, size_t... I>
   static void fill_ptrs(Tup& t, void** p, std::index_sequence<I...>) {
     ((p[I] = (void*)&std::get<I>(t)), ...);

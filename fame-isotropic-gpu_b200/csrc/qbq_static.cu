@@ -101,6 +101,7 @@ cudaError_t launch_qbq(const Geom& g, int threads, const Slot* slot, const doubl
   PlaneInArgs<double> ai;
   memset(&ai, 0, sizeof(ai));
   ai.g = g;
+  plane_passes<double>(g, threads, ai.ax);
   ai.slots = slot;
   ai.tabs = tabs;
   ai.tw = tw;
@@ -115,6 +116,8 @@ cudaError_t launch_qbq(const Geom& g, int threads, const Slot* slot, const doubl
   PencilArgs<double> ap;
   memset(&ap, 0, sizeof(ap));
   ap.g = g;
+  const int pen_threads = pencil_threads_rule<double>(g, pencil_level(g), 1);
+  ap.ax = pencil_passes<double>(g, pen_threads);
   ap.slots = slot;
   ap.tabs = tabs;
   ap.tw = tw;
@@ -125,12 +128,13 @@ cudaError_t launch_qbq(const Geom& g, int threads, const Slot* slot, const doubl
   ap.ib_field = 0;  // the caller's 1/eps is in the spatial layout
   ap.nslots = 1;
   ap.TW = TW;
-  kpen<<<dim3((g.P + TW - 1) / TW, 3, 1), dim3(pencil_threads_rule<double>(g, pencil_level(g), 1)), sm_pen, st>>>(ap);
+  kpen<<<dim3((g.P + TW - 1) / TW, 3, 1), dim3(pen_threads), sm_pen, st>>>(ap);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
 
   PlaneOutArgs<double> ao;
   memset(&ao, 0, sizeof(ao));
   ao.g = g;
+  plane_passes<double>(g, threads, ao.ax);
   ao.slots = slot;
   ao.tabs = tabs;
   ao.tw = tw;

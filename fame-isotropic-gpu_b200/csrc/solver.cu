@@ -235,13 +235,20 @@ struct Ops {
   int cg_fwd_parts() const { return 3 * g().Ls; }
 
   // per-slot tables, with D_kz in the precisions that are allocated (General lattices)
-  void tables(bool d64, bool d32) {
+  // (`one`: of that k-point alone, which becomes slot 0)
+  void tables(bool d64, bool d32, const Slot* one = nullptr) {
     const Geom& q = g();
     int n = std::max({q.Nx * q.Ny, q.Nx, q.Ny, q.Nz});
     if (q.general && (d64 || d32)) n = std::max(n, q.N);
+    double2* t64 = q.general && d64 ? c->dkz64.p : nullptr;
+    float2* t32 = q.general && d32 ? c->dkz32.p : nullptr;
+    if (one) {
+      P.launch(k_tables_of, dim3((n + 255) / 256), dim3(256), 0, q, *one, c->slots.p, c->tabs.p,
+               (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2], t64, t32);
+      return;
+    }
     P.launch(k_tables, dim3((n + 255) / 256, nslots), dim3(256), 0, q, (const Slot*)c->slots.p, c->tabs.p,
-             (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2],
-             q.general && d64 ? c->dkz64.p : (double2*)nullptr, q.general && d32 ? c->dkz32.p : (float2*)nullptr);
+             (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2], t64, t32);
   }
   template <typename R> const cplx<R>* dkz() const;
 
@@ -259,10 +266,11 @@ struct Ops {
     a.fstride = 3L * g().N;
     return a;
   }
-  template <typename R, typename A> void plane_launch(void (*k)(A), int nt, int nvec, const A& a, bool stat = false) {
+  template <typename R, typename A> void plane_launch(void (*k)(A), int nt, int nvec, A a, bool stat = false) {
+    plane_passes<R>(g(), nt, a.ax);
     const size_t sm = stat ? stat_plane_smem_bytes<R, Stat96<R>>() : plane_smem<R>(g());
     allow_smem(k, sm);
-    P.launch(k, dim3(3 * g().Ls, nvec, nslots), dim3(nt), sm, a);
+    P.launch_pdl(k, dim3(3 * g().Ls, nvec, nslots), dim3(nt), sm, a);
   }
 
   // plane inverse stage (the arguments of the input mode are set by the callers below)
@@ -354,6 +362,7 @@ struct Ops {
   void pencil(cplx<R>* T, int nvec, long fstride, const R* invB, int gate, cplx<R>* out = nullptr,
               const cplx<R>* in = nullptr, const Cond* cg_end = nullptr) {
     PencilArgs<R> a;
+    memset(&a, 0, sizeof(a));
     a.cg_in = cg_end ? c->cg_copy.p : nullptr;
     a.pen_parts = cg_pen_parts<R>();
     a.fwd_parts = cg_fwd_parts();
@@ -386,8 +395,9 @@ struct Ops {
       if (g().Ls == 64) k = k_pencil<R, true, MODE, 0, DynGeomSlow<64>>, nt = kPencilThreads;
       if (g().Ls == 128) k = k_pencil<R, true, MODE, 0, DynGeomSlow<128>>, nt = kPencilThreads;
       allow_smem(k, sm);
+      a.ax = pencil_passes<R>(g(), nt);
       if (MODE == PEN_QBQ_CG && c->prefetch) a.pf_dist = wave_ctas(c, k, nt, sm);
-      P.launch(k, grid, dim3(nt), sm, a);
+      P.launch_pdl(k, grid, dim3(nt), sm, a);
     } else {
       auto k = c->rare_pen == 2 ? k_pencil<R, false, MODE, 2, DynGeom> : k_pencil<R, false, MODE, 0, DynGeom>;
       if constexpr (kStatPen<R, MODE> && sizeof(R) == 4)
@@ -400,12 +410,13 @@ struct Ops {
           const size_t smp = pencil_pipe_smem_bytes<R>(g().Ls);
           allow_smem(kp, smp);
           const int total = (int)(grid.x * grid.y * grid.z);
-          P.launch(kp, dim3(std::min(total, c->pipe_ctas64)), dim3(kPencilThreads), smp, a);
+          P.launch_pdl(kp, dim3(std::min(total, c->pipe_ctas64)), dim3(kPencilThreads), smp, a);
           return;
         }
       allow_smem(k, sm);
+      a.ax = pencil_passes<R>(g(), nt);
       if (MODE == PEN_QBQ_CG && c->prefetch) a.pf_dist = wave_ctas(c, k, nt, sm);
-      P.launch(k, grid, dim3(nt), sm, a);
+      P.launch_pdl(k, grid, dim3(nt), sm, a);
     }
   }
 
@@ -1398,12 +1409,11 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
     if (precision == FAME_MIXED) ensure_workspace(c, 1, c->cap_nstep, c->cap_nwant, true, c->cap_vec);
     const Slot sl = make_slot(c->lat, k);
     if (Nd_out) *Nd_out = sl.Nd;
-    FAME_CK(cudaMemcpyAsync(c->slots.p, &sl, sizeof(Slot), cudaMemcpyHostToDevice, c->stream));
     Program P(c->stream, false, c->hflag, 100000);
     Ops o{c, P, 1};
     const Geom& g = c->g;
     const long M = 2L * g.N, F = 3L * g.N;
-    o.tables(precision == FAME_FP64, precision == FAME_MIXED);
+    o.tables(precision == FAME_FP64, precision == FAME_MIXED, &sl);
     if (precision == FAME_FP64) {
       const double2* x = (const double2*)in;
       double2* y = (double2*)out;
@@ -1448,19 +1458,25 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
           L.status = c->status.p;
           P.launch(k_lz_init, dim3(1, 1, 1), dim3(256), 0, o.va(Cond{}), L);
           FAME_CK(cudaMemcpyAsync(c->U.p, x, 2L * sl.Nd * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
-          SolveCfg s;
-          memset(&s, 0, sizeof(s));
-          s.nslots = 1;
-          s.ls_maxit = prm->ls_maxit;
-          s.ls_tol = prm->ls_tol;
-          s.mixed = 0;
-          const int nvb = vec_blocks(c, 1);
-          Cond cc = loop_cond(P, c->flags.p, kLoopCG, s.ls_maxit + 2);
-          P.launch(k_invar_pro<false>, dim3(nvb, 1, 1), dim3(256), 0, o.va(cc), L, 0, c->r64.p, c->x64.p,
-                   (double2*)nullptr, s.ls_tol * s.ls_tol, s.ls_maxit);
-          o.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
-          P.launch(k_invar_epi<false>, dim3(nvb, 1, 1), dim3(256), 0, o.va(Cond{}), L, 0,
-                   (const double2*)c->x64.p, (const double2*)c->x64b.p);
+          // the CG as a graph, kept like a solve's (the host's loop waited for the device every
+          // second iteration: hexagonal 36x30x26, 1404 -> 1079 us)
+          char key[96];
+          snprintf(key, sizeof key, "invar/%d/%.17g/%d/%d", prm->ls_maxit, prm->ls_tol, nstep, nwant);
+          auto it = c->progs.find(key);
+          if (it == c->progs.end()) {
+            auto prog = std::make_unique<Program>(c->stream, true, c->hflag, 0);
+            Ops og{c, *prog, 1};
+            const int nvb = vec_blocks(c, 1);
+            Cond cc = loop_cond(*prog, c->flags.p, kLoopCG, prm->ls_maxit + 2);
+            prog->launch(k_invar_pro<false>, dim3(nvb, 1, 1), dim3(256), 0, og.va(cc), L, 0, c->r64.p, c->x64.p,
+                         (double2*)nullptr, prm->ls_tol * prm->ls_tol, prm->ls_maxit);
+            og.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
+            prog->launch(k_invar_epi<false>, dim3(nvb, 1, 1), dim3(256), 0, og.va(Cond{}), L, 0,
+                         (const double2*)c->x64.p, (const double2*)c->x64b.p);
+            prog->instantiate();
+            it = c->progs.emplace(key, std::move(prog)).first;
+          }
+          it->second->run();
           FAME_CK(cudaMemcpyAsync(y, c->U.p + M, 2L * sl.Nd * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
           break;
         }

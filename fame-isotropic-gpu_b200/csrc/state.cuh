@@ -118,6 +118,7 @@ enum PencilMode { PEN_QBQ = 0, PEN_QR_OUT = 1, PEN_QRS_IN = 2, PEN_QBQ_CG = 3 };
 template <typename R>
 struct PlaneInArgs {
   Geom g;
+  AxisPasses ax[2];       // runtime plans: fast and mid axis
   const Slot* slots;
   const double2* tabs;
   const cplx<R>* dkz;     // General: D_kz of every slot (N values each), or NULL
@@ -137,6 +138,7 @@ struct PlaneInArgs {
 template <typename R>
 struct PlaneCgArgs {
   Geom g;
+  AxisPasses ax[2];
   const Slot* slots;
   const double2* tabs;
   const cplx<R>* dkz;
@@ -158,6 +160,7 @@ struct PlaneCgArgs {
 template <typename R>
 struct PencilArgs {
   Geom g;
+  AxisPasses ax;           // runtime plans: slow axis
   const Slot* slots;
   const double2* tabs;
   const cplx<R>* tw;
@@ -183,6 +186,7 @@ struct PencilArgs {
 template <typename R>
 struct PlaneOutArgs {
   Geom g;
+  AxisPasses ax[2];
   const Slot* slots;
   const double2* tabs;
   const cplx<R>* dkz;

@@ -243,12 +243,13 @@ int fame_bench_qbq(fame_ctx* ctx, const double* k, int precision, int reps, int 
                    double* stage_ms_out);
 
 /* CG-iteration benchmark: `reps` iterations of the mixed-precision solve's FP32 CG
- * (its three kernels: the plane stage, with the forward plane transforms, the 3 -> 2 unmix, the
- * vector updates, ||r||^2, the 2 -> 3 mix and the inverse plane transforms; the decision; the
- * slow-axis transforms with <r, A r>) on `nbatch` k-points (1..64, the k-point repeated), from
- * a fixed pseudo-random residual, each iteration preceded by an L2 flush outside the timed
- * span.  stage_ms_out[3] (optional) receives the mean time of the three kernels over the
- * batch, ms_out their sum.  The CG iteration of FAME_Main/CG.cu:36-77 on QBQ. */
+ * (its two kernels: the plane stage, with the forward plane transforms, the 3 -> 2 unmix, the
+ * vector updates, ||r||^2, the 2 -> 3 mix and the inverse plane transforms; the pencil stage, with
+ * the end of the iteration and the slow-axis transforms with <r, A r>) on `nbatch` k-points
+ * (1..64, the k-point repeated), from a fixed pseudo-random residual, each iteration preceded
+ * by an L2 flush outside the timed span.  stage_ms_out[3] (optional) receives the mean time
+ * of the two kernels over the batch (the third entry is the empty span after them), ms_out the
+ * sum.  The CG iteration of FAME_Main/CG.cu:36-77 on QBQ. */
 int fame_bench_cg(fame_ctx* ctx, const double* k, int reps, int nbatch, double* ms_out, double* stage_ms_out);
 
 /* Grid size N and maximum reduced size 2N of the context, for buffer sizing. */
