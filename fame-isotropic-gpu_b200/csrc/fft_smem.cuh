@@ -379,8 +379,11 @@ __device__ __forceinline__ int div_magic(int n, unsigned m) { return m ? (int)__
 // one, lines fastest (thread t takes t, t + T, ...; at most MAXB each), so consecutive
 // threads touch consecutive lines and at most the last deal of a round has idle threads.
 // G is the largest line count that T * MAXB butterflies cover, evened out over the rounds.
-template <typename R, int RAD, int MAXB>
-__device__ __forceinline__ void stockham_pass(cplx<R>* buf, const AxisPasses& A, const PassDesc& d, const cplx<R>* tw) {
+// MUL: the inputs are multiplied by conj(pre), the outputs by conj(post), tables in global memory
+// with element m of line l at m * nl + l (either may be null).
+template <typename R, int RAD, int MAXB, bool MUL>
+__device__ __forceinline__ void stockham_pass(cplx<R>* buf, const AxisPasses& A, const PassDesc& d, const cplx<R>* tw,
+                                              const cplx<R>* pre, const cplx<R>* post) {
   const int T = blockDim.x;
   const int t = threadIdx.x;
   for (int l0 = 0; l0 < A.nl; l0 += d.G) {
@@ -405,13 +408,26 @@ __device__ __forceinline__ void stockham_pass(cplx<R>* buf, const AxisPasses& A,
         const int step = d.nb * A.es;
 #pragma unroll
         for (int u = 0; u < RAD; u++) v[q][u] = src[u * step];
+        if (MUL && pre) {
+          const cplx<R>* m = pre + j * A.nl + l;
+          const int ms = d.nb * A.nl;
+#pragma unroll
+          for (int u = 0; u < RAD; u++) v[q][u] = cmulc(m[u * ms], v[q][u]);
+        }
         if (k > 0) {
           const int kt = k * d.stw;
 #pragma unroll
           for (int u = 1; u < RAD; u++) v[q][u] = cmul(v[q][u], tw[u * kt]);
         }
         Dft<R, RAD>::run(v[q], false);
-        dst[q] = l * A.ls + (jb * d.ns * RAD + k) * A.es;
+        const int o = jb * d.ns * RAD + k;
+        if (MUL && post) {
+          const cplx<R>* m = post + o * A.nl + l;
+          const int ms = d.ns * A.nl;
+#pragma unroll
+          for (int u = 0; u < RAD; u++) v[q][u] = cmulc(m[u * ms], v[q][u]);
+        }
+        dst[q] = l * A.ls + o * A.es;
       }
     }
     __syncthreads();
@@ -620,14 +636,19 @@ constexpr int pass_maxb(int emax, int r) { return emax / r > 0 ? emax / r : 1; }
 // factors >= 17 in; they are register hungry, so each stage kernel exists with and
 // without them and the host picks by its axes (plan_level).  EMAX bounds the elements
 // a thread stages in registers per round.
-template <typename R, int EMAX, int RARE>
-__device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPasses& A, const cplx<R>* tw) {
+// MUL: conj(pre) on the inputs and conj(post) on the outputs of the transform (stockham_pass); the
+// first or last pass must not be a prime one then.
+template <typename R, int EMAX, int RARE, bool MUL = false>
+__device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPasses& A, const cplx<R>* tw,
+                                          const cplx<R>* pre = nullptr, const cplx<R>* post = nullptr) {
 #pragma unroll 1
   for (int p = 0; p < A.npass; p++) {
     const PassDesc& d = A.d[p];
     switch (d.radix) {
 #define FAME_PASS(r_) \
-  case r_: stockham_pass<R, r_, pass_maxb(EMAX, r_)>(buf, A, d, tw); break;
+  case r_: stockham_pass<R, r_, pass_maxb(EMAX, r_), MUL>(buf, A, d, tw, p == 0 ? pre : nullptr,                  \
+                                                         p == A.npass - 1 ? post : nullptr);                      \
+           break;
       FAME_PASS(2)
       FAME_PASS(3)
       FAME_PASS(4)
@@ -722,8 +743,10 @@ constexpr int splan_radix(int n, int p) {
 // One radix-RAD pass with the line length N, line count NL and thread count T
 // compile-time: line stride ls, element stride es (constants fold when the caller
 // passes literals).  Same round structure as stockham_pass.
+// pre, post: as in stockham_pass.
 template <typename R, int N, int NL, int T, int NS, int RAD, int MAXB>
-__device__ __forceinline__ void spass(cplx<R>* buf, int ls, int es, const cplx<R>* tw, bool inv) {
+__device__ __forceinline__ void spass(cplx<R>* buf, int ls, int es, const cplx<R>* tw, bool inv,
+                                      const cplx<R>* pre = nullptr, const cplx<R>* post = nullptr) {
   constexpr int nb = N / RAD;
   constexpr int stw = N / (NS * RAD);
   constexpr int per_line = (nb + MAXB - 1) / MAXB;
@@ -758,6 +781,7 @@ __device__ __forceinline__ void spass(cplx<R>* buf, int ls, int es, const cplx<R
 #pragma unroll
         for (int u = 0; u < RAD; u++) {
           cplx<R> a = base[(j + u * nb) * es];
+          if (pre) a = cmulc(pre[(j + u * nb) * NL + l], a);
           if (NS > 1 && u > 0) {
             cplx<R> w = tw[u * k * stw];
             if (inv) w.y = -w.y;
@@ -766,6 +790,10 @@ __device__ __forceinline__ void spass(cplx<R>* buf, int ls, int es, const cplx<R
           v[q][u] = a;
         }
         Dft<R, RAD>::run(v[q], inv);
+        if (post) {
+#pragma unroll
+          for (int u = 0; u < RAD; u++) v[q][u] = cmulc(post[(jbk[q] + u * NS) * NL + l], v[q][u]);
+        }
       }
     }
     __syncthreads();
@@ -791,7 +819,8 @@ constexpr int smaxb(int N, int NL, int T, int EMAX, int RAD) {
 }
 
 template <typename R, int N, int NL, int T, int EMAX, int P = 0, int NS = 1>
-__device__ __forceinline__ void sfft(cplx<R>* buf, int ls, int es, const cplx<R>* tw, bool inv) {
+__device__ __forceinline__ void sfft(cplx<R>* buf, int ls, int es, const cplx<R>* tw, bool inv,
+                                     const cplx<R>* pre = nullptr, const cplx<R>* post = nullptr) {
   static_assert(N == 1 || splan_count(N) > 0, "line length without a static plan");
   if constexpr (P < splan_count(N)) {
     constexpr int RAD = splan_radix(N, P);
@@ -803,9 +832,10 @@ __device__ __forceinline__ void sfft(cplx<R>* buf, int ls, int es, const cplx<R>
         generic_pass<R, EMAX>(buf, N, RAD, NS, L, tw);
     } else {
       constexpr int MB = smaxb(N, NL, T, EMAX, RAD);
-      spass<R, N, NL, T, NS, RAD, MB>(buf, ls, es, tw, inv);
+      spass<R, N, NL, T, NS, RAD, MB>(buf, ls, es, tw, inv, P == 0 ? pre : nullptr,
+                                      P == splan_count(N) - 1 ? post : nullptr);
     }
-    sfft<R, N, NL, T, EMAX, P + 1, NS * RAD>(buf, ls, es, tw, inv);
+    sfft<R, N, NL, T, EMAX, P + 1, NS * RAD>(buf, ls, es, tw, inv, pre, post);
   }
 }
 

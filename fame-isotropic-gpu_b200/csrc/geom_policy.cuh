@@ -36,9 +36,15 @@ struct DynGeom {
   // only: the inverse ones run on values with swapped parts (plane stages) or come out in
   // reversed order (pencil stage), which takes the conjugations and sign choices of a runtime
   // direction out of every pass.
-  template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const AxisPasses& A, bool, const cplx<R>* tw) {
-    fft_lines<R, Emax<R>::v, RARE>(b, A, tw);
+  // MUL (General lattices): conj(pre) on the inputs, conj(post) on the outputs of the mid axis
+  template <typename R, int RARE, bool MUL>
+  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const AxisPasses& A, bool, const cplx<R>* tw,
+                                                   const cplx<R>* pre, const cplx<R>* post) {
+    fft_lines<R, Emax<R>::v, RARE, MUL>(b, A, tw, pre, post);
+  }
+  // whether the mid axis can take pre and post (its first and last pass are butterflies)
+  __device__ __forceinline__ static bool mul_ok(const AxisPasses& A) {
+    return A.d[0].radix <= 13 && A.d[A.npass - 1].radix <= 13;
   }
   template <typename R, int RARE>
   __device__ __forceinline__ static void fft_slow(cplx<R>* b, const AxisPasses& A, const cplx<R>* tw) {
@@ -96,12 +102,16 @@ struct DynGeomPlane : DynGeom {
   template <typename R, int RARE> static constexpr int max_plane_threads() { return T; }
   __device__ __forceinline__ static constexpr int plane_threads() { return T; }
   template <typename R, int RARE> static constexpr int plane_min_blocks() { return MB; }
-  template <typename R, int RARE>
-  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const AxisPasses&, bool fast, const cplx<R>* tw) {
+  template <typename R, int RARE, bool MUL>
+  __device__ __forceinline__ static void fft_plane(cplx<R>* b, const AxisPasses&, bool fast, const cplx<R>* tw,
+                                                   const cplx<R>* pre, const cplx<R>* post) {
     if (fast)
       sfft<R, LF, LM, T, PlaneEmax<R>::v>(b, LF | 1, 1, tw, false);
     else
-      sfft<R, LM, LF, T, PlaneEmax<R>::v>(b, 1, LF | 1, tw, false);
+      sfft<R, LM, LF, T, PlaneEmax<R>::v>(b, 1, LF | 1, tw, false, pre, post);
+  }
+  __device__ __forceinline__ static constexpr bool mul_ok(const AxisPasses&) {
+    return splan_radix(LM, 0) <= 13 && splan_radix(LM, splan_count(LM) - 1) <= 13;
   }
 };
 

@@ -9,22 +9,26 @@
 namespace fame {
 
 // Lambda_x, Lambda_y, Lambda_z at plane element (m, f) of plane s, in precision R.
-// Simple lattices read the per-CTA shared tables lx[f], ly[m] and the plane's lz.
+// Simple lattices read the per-CTA shared tables lx[f], ly[m]; `lp` is what is constant on the
+// plane: Lambda_z (Simple) or Lambda_x (General).  (A table of Lambda_z in FP32, 8 bytes a point, was
+// slower than the two loads and the FP64 product: FCC 64 CG plane stage 14.8 against 14.4 us per
+// k-point.)
 template <typename R, bool GEN>
 __device__ __forceinline__ void lam_elem(const Geom& g, const double2* tab, const cplx<R>* lx, const cplx<R>* ly, int lys,
-                                         cplx<R> lz, int s, int m, int f, cplx<R>& Lx, cplx<R>& Ly,
-                                         cplx<R>& Lz) {
+                                         cplx<R> lp, int s, int m, int f, cplx<R>& Lx, cplx<R>& Ly, cplx<R>& Lz) {
   if constexpr (!GEN) {
     Lx = lx[f];
     Ly = ly[m * lys];
-    Lz = lz;
+    Lz = lp;
   } else {
-    double2 a, b, c;
-    lambdas_at(g, tab, s, m, f, a, b, c);
-    Lx = cvt<R>(a);
-    Ly = cvt<R>(b);
-    Lz = cvt<R>(c);
+    Lx = lp;
+    Ly = cvt<R>(tab[g.oLy + s * g.Ny + m]);
+    const double2 e = cmul(tab[g.oExy + s * g.Ny + m], tab[g.oWz + f]);
+    Lz = cvt<R>(make_double2((e.x - 1.0) * g.ihz, e.y * g.ihz));
   }
+}
+template <typename R, bool GEN> __device__ __forceinline__ cplx<R> lam_plane(const Geom& g, const double2* tab, int s) {
+  return cvt<R>(tab[(GEN ? g.oLx : g.oLz) + s]);
 }
 
 // ------------------------------------------------------------------ L2 prefetch
@@ -131,6 +135,14 @@ __device__ __forceinline__ void plane_times_dkz(const Geom& g, const double2* ta
   __syncthreads();
 }
 
+// The plane's part of the D_kz table where the mid axis' passes can multiply by it, else null.
+template <typename R, class GP>
+__device__ __forceinline__ const cplx<R>* plane_dkz(const Geom& g, const AxisPasses& mid, const cplx<R>* dkz) {
+  if (!dkz || !GP::mul_ok(mid)) return nullptr;
+  const PlanePos p = plane_pos();
+  return dkz + (size_t)p.slot * g.N + (size_t)p.s * GP::P(g);
+}
+
 // Whether the inverse transforms of a plane run as forward ones on values with swapped real and
 // imaginary parts, swap(z) = i conj(z): swap(IDFT z) = DFT swap(z).  The mix writes them so and
 // plane_store swaps them back.  (Static Simple geometries have the direction at compile time.)
@@ -147,7 +159,9 @@ template <bool SWAP, typename T> __device__ __forceinline__ T maybe_swap(T z) {
 }
 
 // Unnormalised inverse 2-D transform of the CTA's plane: fast axis, (x D_kz), mid axis; x D_ky
-// follows in plane_store (General lattices, FAME_FFT_CUDA.cu:104-117).
+// follows in plane_store (General lattices, FAME_FFT_CUDA.cu:104-117).  D_kz multiplies the mid axis'
+// inputs (forward: its outputs) in the pass that reads (writes) them, coalesced there; a pass of its own
+// (a prime mid axis, or no table) is another round trip of the plane through shared memory.
 template <typename R, bool GEN, int RARE, class GP>
 __device__ __forceinline__ void plane_inverse(const Geom& g, const AxisPasses* axes, const double2* tabs,
                                               const cplx<R>* dkz) {
@@ -159,8 +173,9 @@ __device__ __forceinline__ void plane_inverse(const Geom& g, const AxisPasses* a
     // one FFT call site per axis loop: the runtime plans' passes are long
 #pragma unroll 1
     for (int ax = 0; ax < 2; ax++) {
-      GP::template fft_plane<R, RARE>(m.plane, axes[ax], ax == 0, ax == 0 ? m.twf : m.twm);
-      if (GEN && ax == 0) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane);
+      const cplx<R>* pre = GEN && ax == 1 ? plane_dkz<R, GP>(g, axes[1], dkz) : nullptr;
+      if (GEN && ax == 1 && !pre) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane);
+      GP::template fft_plane<R, RARE, GEN>(m.plane, axes[ax], ax == 0, ax == 0 ? m.twf : m.twm, pre, nullptr);
     }
   }
 }
@@ -178,8 +193,9 @@ __device__ __forceinline__ void plane_forward(const Geom& g, const AxisPasses* a
 #pragma unroll 1
     for (int ax = 0; ax < 2; ax++) {
       const bool fast = GEN ? ax == 1 : ax == 0;
-      if (GEN && ax == 1) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane);
-      GP::template fft_plane<R, RARE>(m.plane, axes[fast ? 0 : 1], fast, fast ? m.twf : m.twm);
+      const cplx<R>* post = GEN && !fast ? plane_dkz<R, GP>(g, axes[1], dkz) : nullptr;
+      GP::template fft_plane<R, RARE, GEN>(m.plane, axes[fast ? 0 : 1], fast, fast ? m.twf : m.twm, nullptr, post);
+      if (GEN && !fast && !post) plane_times_dkz<R, GP>(g, tabs, dkz, m.plane);
     }
   }
 }
@@ -298,7 +314,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     if (kAsyncMix && threadIdx.x == 0) exchange_init(bar, &skip, a.fault);
     const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
     plane_tables<R, GEN, GP>(g, a.tw, tab, p.s, m);
-    const cplx<R> lz = GEN ? mk<R>(0, 0) : cvt<R>(tab[g.oLz + p.s]);
+    const cplx<R> lp = lam_plane<R, GEN>(g, tab, p.s);
     cl.sync();  // every CTA of the cluster is running (and the tables and barriers are in place)
     if constexpr (kAsyncMix) {
       if (*cl.map_shared_rank(&skip, 0)) {
@@ -355,7 +371,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
         if (fi >= off) {
           const long i = fi - off;
           cplx<R> Lx, Ly, Lz;
-          lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lz, p.s, r, f, Lx, Ly, Lz);
+          lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lp, p.s, r, f, Lx, Ly, Lz);
           cplx<R> x1 = A1[k], x2 = A2[k];
           if constexpr (IN == IN_VEC) {
             if (a.sigma) {
@@ -477,7 +493,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     const PlanePos p = plane_pos();
     const Slot sl = a.slots[p.slot];
     const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
-    const cplx<R> lz = GEN ? mk<R>(0, 0) : cvt<R>(tab[g.oLz + p.s]);
+    const cplx<R> lp = lam_plane<R, GEN>(g, tab, p.s);
     const PlaneExchange<R, kAsyncMix, kSwapInv<GEN, GP>> ex(m.plane, bar);
     const int iter = a.cg[p.slot].iter, cur = iter & 1;
     const bool have_r = iter > 1, have_x = iter > 2;  // r_old = 0 at k = 1; x = 0 at k = 1, x_old = 0 at k = 2
@@ -528,7 +544,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
         if (fi >= off) {
           const long i = fi - off;
           cplx<R> Lx, Ly, Lz;
-          lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lz, p.s, r, f, Lx, Ly, Lz);
+          lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lp, p.s, r, f, Lx, Ly, Lz);
           cplx<R> Pc[6];
           pi_from<R>(GEN, false, Lx, Ly, Lz, Pc);
           const cplx<R> w1 = cadd(cadd(cmulc(Pc[0], t[k][0]), cmulc(Pc[1], t[k][1])), cmulc(Pc[2], t[k][2]));
@@ -981,7 +997,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
   const PlanePos p = plane_pos();
   const Slot sl = a.slots[p.slot];
   const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
-  const cplx<R> lz = GEN ? mk<R>(0, 0) : cvt<R>(tab[g.oLz + p.s]);
+  const cplx<R> lp = lam_plane<R, GEN>(g, tab, p.s);
   const cplx<R>* src[3] = {cl.map_shared_rank(m.plane, 0), cl.map_shared_rank(m.plane, 1),
                            cl.map_shared_rank(m.plane, 2)};
   const int per = (P + 2) / 3;
@@ -1020,7 +1036,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       const long i = fi - off;
       const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), f = e - r * Lf;
       cplx<R> Lx, Ly, Lz;
-      lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lz, p.s, r, f, Lx, Ly, Lz);
+      lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lp, p.s, r, f, Lx, Ly, Lz);
       cplx<R> Pc[6];
       pi_from<R>(GEN, PR, Lx, Ly, Lz, Pc);
       const cplx<R> t0 = t[k][0], t1 = t[k][1], t2 = t[k][2];
