@@ -444,14 +444,6 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       return;
     }
     const int cur = st->iter & 1;
-    // this CTA's own part of r, r_old, x and x_old: it streams into L2 during the transforms
-    long i0, i1;
-    if (a.self_pf && threadIdx.x < (st->iter == 1 ? 2 : st->iter == 2 ? 6 : 8) &&
-        plane_vec_range(GP::P(g), p.s, p.comp, sl, i0, i1)) {
-      const int which = threadIdx.x >> 1;
-      const cplx<R>* v = which == 0 ? a.r[cur] : which == 1 ? a.r[cur ^ 1] : which == 2 ? a.x[cur] : a.x[cur ^ 1];
-      prefetch_l2(v + (long)p.slot * a.vstride + ((threadIdx.x & 1) ? sl.Nd : 0) + i0, (i1 - i0) * sizeof(cplx<R>));
-    }
     if (kAsyncMix && threadIdx.x == 0) exchange_init(bar, &skip, a.fault);
     const cplx<R>* T = a.T + plane_base<R, GP>(g, p, 1, a.fstride);
     if constexpr (GEN) __syncthreads();  // D_ky is in place
@@ -475,6 +467,17 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     }
     if constexpr (!GEN) cp_async_wait_all();
     __syncthreads();
+    // This CTA's own part of r, r_old, x and x_old: it streams into L2 during the forward
+    // transforms.  Asked for before the plane had arrived it only delayed the plane, and the
+    // vectors pass through as streams (evicted first), which leaves the L2 to the field that the
+    // pencil stage reads next: together 38.7 -> 34.8 us per k-point at 96^3 (20 per launch).
+    long i0, i1;
+    if (a.self_pf && threadIdx.x < (st->iter == 1 ? 2 : st->iter == 2 ? 6 : 8) &&
+        plane_vec_range(GP::P(g), p.s, p.comp, sl, i0, i1)) {
+      const int which = threadIdx.x >> 1;
+      const cplx<R>* v = which == 0 ? a.r[cur] : which == 1 ? a.r[cur ^ 1] : which == 2 ? a.x[cur] : a.x[cur ^ 1];
+      prefetch_l2(v + (long)p.slot * a.vstride + ((threadIdx.x & 1) ? sl.Nd : 0) + i0, (i1 - i0) * sizeof(cplx<R>));
+    }
   }
   plane_forward<R, GEN, RARE, GP>(g, a.ax, a.tabs, a.dkz);
   double acc[1] = {0.0};
@@ -517,17 +520,17 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
         t[k][0] = t[k][1] = t[k][2] = mk<R>(0, 0);
         if (e < e1 && fi >= off) {
           const long i = fi - off;
-          R1[k] = rc[i];
-          R2[k] = rc[Nd + i];
+          R1[k] = __ldcs(&rc[i]);
+          R2[k] = __ldcs(&rc[Nd + i]);
           if (have_r) {
-            O1[k] = ro[i];
-            O2[k] = ro[Nd + i];
-            X1[k] = xc[i];
-            X2[k] = xc[Nd + i];
+            O1[k] = __ldcs(&ro[i]);
+            O2[k] = __ldcs(&ro[Nd + i]);
+            X1[k] = __ldcs(&xc[i]);
+            X2[k] = __ldcs(&xc[Nd + i]);
           }
           if (have_x) {
-            Y1[k] = xo[i];
-            Y2[k] = xo[Nd + i];
+            Y1[k] = __ldcs(&xo[i]);
+            Y2[k] = __ldcs(&xo[Nd + i]);
           }
           const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), q = r * S + (e - r * Lf);
 #pragma unroll
@@ -552,10 +555,10 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
           // x' = x + rho gamma r + (rho - 1)(x - x_old), r' the same with -w: the corrections added to x and r
           const cplx<R> n1 = cfma_r(csub(R1[k], O1[k]), rm, cfma_r(w1, -rg, R1[k]));
           const cplx<R> n2 = cfma_r(csub(R2[k], O2[k]), rm, cfma_r(w2, -rg, R2[k]));
-          ro[i] = n1;
-          ro[Nd + i] = n2;
-          xo[i] = cfma_r(csub(X1[k], Y1[k]), rm, cfma_r(R1[k], rg, X1[k]));
-          xo[Nd + i] = cfma_r(csub(X2[k], Y2[k]), rm, cfma_r(R2[k], rg, X2[k]));
+          __stcs(&ro[i], n1);
+          __stcs(&ro[Nd + i], n2);
+          __stcs(&xo[i], cfma_r(csub(X1[k], Y1[k]), rm, cfma_r(R1[k], rg, X1[k])));
+          __stcs(&xo[Nd + i], cfma_r(csub(X2[k], Y2[k]), rm, cfma_r(R2[k], rg, X2[k])));
           acc[0] += (double)(cabs2(n1) + cabs2(n2));
 #pragma unroll
           for (int c = 0; c < 3; c++) v[c] = cadd(cmul(Pc[c], n1), cmul(Pc[3 + c], n2));
