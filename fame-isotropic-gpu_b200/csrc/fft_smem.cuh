@@ -624,10 +624,18 @@ __device__ __forceinline__ bool prime_pass(cplx<R>* buf, int n, int r, int Ns, L
   return true;
 }
 
-// outputs x lines a thread accumulates in the prime pass
-template <typename R> struct PrimeBlock;
-template <> struct PrimeBlock<float> { static constexpr int mu = 4, ml = 3; };
-template <> struct PrimeBlock<double> { static constexpr int mu = 2, ml = 2; };
+// Outputs x lines a thread accumulates in the prime pass.  Per s it loads 2 ML values P_s, Q_s (two
+// shared-memory cycles each per warp in FP32, four in FP64) and MU cosines and sines (one or
+// two) for MU * ML * 2 complex multiply-adds, so shared memory bounds the pass until the
+// block is as large as the registers allow.
+// FP64 takes 4 x 2 in the pencil stage (92 = 4 x 23 points: 47.4 -> 36.2 us per k-point) and in the
+// static plans (hexagonal 128 operator 397 -> 363), not in the runtime plane stages, where it
+// spills (51x43x37 operator 34.3 -> 37.1).  FP32: 5 x 4 on the 107-point axis is one round instead
+// of two, but slower where the launch leaves SMs with one CTA (plane stage, one k-point: 186 ->
+// 201 us; four: 150 -> 148).
+template <typename R, bool LARGE> struct PrimeBlock { static constexpr int mu = 4, ml = 3; };
+template <> struct PrimeBlock<double, false> { static constexpr int mu = 2, ml = 2; };
+template <> struct PrimeBlock<double, true> { static constexpr int mu = 4, ml = 2; };
 
 // Butterflies of radix r a thread stages per round when it holds at most emax elements.
 constexpr int pass_maxb(int emax, int r) { return emax / r > 0 ? emax / r : 1; }
@@ -638,7 +646,7 @@ constexpr int pass_maxb(int emax, int r) { return emax / r > 0 ? emax / r : 1; }
 // a thread stages in registers per round.
 // MUL: conj(pre) on the inputs and conj(post) on the outputs of the transform (stockham_pass); the
 // first or last pass must not be a prime one then.
-template <typename R, int EMAX, int RARE, bool MUL = false>
+template <typename R, int EMAX, int RARE, bool LARGE, bool MUL = false>
 __device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPasses& A, const cplx<R>* tw,
                                           const cplx<R>* pre = nullptr, const cplx<R>* post = nullptr) {
 #pragma unroll 1
@@ -665,7 +673,8 @@ __device__ __forceinline__ void fft_lines(cplx<R>* buf, const AxisPasses& A, con
       default:
         if constexpr (RARE >= 2) {
           const LineSet L{A.nl, A.ls, A.es};
-          if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml>(buf, A.n, d.radix, d.ns, L, tw))
+          using B = PrimeBlock<R, LARGE>;
+          if (!prime_pass<R, B::mu, B::ml>(buf, A.n, d.radix, d.ns, L, tw))
             generic_pass<R, EMAX>(buf, A.n, d.radix, d.ns, L, tw);
         }
         break;
@@ -828,7 +837,8 @@ __device__ __forceinline__ void sfft(cplx<R>* buf, int ls, int es, const cplx<R>
       // a prime factor >= 17: the symmetric-pair pass, its sizes compile-time constants
       const LineSet L{NL, ls, es};
       // (forward only, as all plans with primes run)
-      if (!prime_pass<R, PrimeBlock<R>::mu, PrimeBlock<R>::ml, T>(buf, N, RAD, NS, L, tw))
+      using B = PrimeBlock<R, true>;
+      if (!prime_pass<R, B::mu, B::ml, T>(buf, N, RAD, NS, L, tw))
         generic_pass<R, EMAX>(buf, N, RAD, NS, L, tw);
     } else {
       constexpr int MB = smaxb(N, NL, T, EMAX, RAD);

@@ -40,7 +40,7 @@ struct DynGeom {
   template <typename R, int RARE, bool MUL>
   __device__ __forceinline__ static void fft_plane(cplx<R>* b, const AxisPasses& A, bool, const cplx<R>* tw,
                                                    const cplx<R>* pre, const cplx<R>* post) {
-    fft_lines<R, Emax<R>::v, RARE, MUL>(b, A, tw, pre, post);
+    fft_lines<R, Emax<R>::v, RARE, false, MUL>(b, A, tw, pre, post);
   }
   // whether the mid axis can take pre and post (its first and last pass are butterflies)
   __device__ __forceinline__ static bool mul_ok(const AxisPasses& A) {
@@ -48,7 +48,7 @@ struct DynGeom {
   }
   template <typename R, int RARE>
   __device__ __forceinline__ static void fft_slow(cplx<R>* b, const AxisPasses& A, const cplx<R>* tw) {
-    fft_lines<R, Emax<R>::v, RARE>(b, A, tw);
+    fft_lines<R, Emax<R>::v, RARE, true>(b, A, tw);
   }
 };
 

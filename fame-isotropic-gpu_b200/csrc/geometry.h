@@ -209,7 +209,7 @@ inline int plane_threads_rule(const Geom& g, int level, long planes) {
 // (92 = 4 x 23 in FP64: 51.7 us per k-point with 256 threads, 81.6 with 64).
 template <typename R>
 inline int pencil_threads_rule(const Geom& g, int level, long vecs) {
-  constexpr int TW = PencilTW<R>::v, mu = PrimeBlock<R>::mu, ml = PrimeBlock<R>::ml;
+  constexpr int TW = PencilTW<R>::v, mu = PrimeBlock<R, true>::mu, ml = PrimeBlock<R, true>::ml;
   int lo = plan_threads(g.ps, Emax<R>::v);
   for (int p = 0; p < g.ps.npass; p++) {
     const int r = g.ps.radix[p];
