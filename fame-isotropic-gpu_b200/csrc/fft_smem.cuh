@@ -752,12 +752,12 @@ constexpr int splan_radix(int n, int p) {
 // One radix-RAD pass with the line length N, line count NL and thread count T
 // compile-time: line stride ls, element stride es (constants fold when the caller
 // passes literals).  Same round structure as stockham_pass.
-// pre, post: as in stockham_pass.
-template <typename R, int N, int NL, int T, int NS, int RAD, int MAXB>
+// pre, post: as in stockham_pass.  tw is the table of length TS * N.
+template <typename R, int N, int NL, int T, int NS, int RAD, int MAXB, int TS = 1>
 __device__ __forceinline__ void spass(cplx<R>* buf, int ls, int es, const cplx<R>* tw, bool inv,
                                       const cplx<R>* pre = nullptr, const cplx<R>* post = nullptr) {
   constexpr int nb = N / RAD;
-  constexpr int stw = N / (NS * RAD);
+  constexpr int stw = TS * N / (NS * RAD);
   constexpr int per_line = (nb + MAXB - 1) / MAXB;
   constexpr int G0 = T / per_line;
   constexpr int G = G0 < 1 ? 1 : (G0 > NL ? NL : G0);
@@ -827,13 +827,14 @@ constexpr int smaxb(int N, int NL, int T, int EMAX, int RAD) {
   return want < cap ? want : cap;
 }
 
-template <typename R, int N, int NL, int T, int EMAX, int P = 0, int NS = 1>
+template <typename R, int N, int NL, int T, int EMAX, int TS = 1, int P = 0, int NS = 1>
 __device__ __forceinline__ void sfft(cplx<R>* buf, int ls, int es, const cplx<R>* tw, bool inv,
                                      const cplx<R>* pre = nullptr, const cplx<R>* post = nullptr) {
   static_assert(N == 1 || splan_count(N) > 0, "line length without a static plan");
   if constexpr (P < splan_count(N)) {
     constexpr int RAD = splan_radix(N, P);
     if constexpr (RAD >= 17) {
+      static_assert(TS == 1, "prime passes take a table of the line's own length");
       // a prime factor >= 17: the symmetric-pair pass, its sizes compile-time constants
       const LineSet L{NL, ls, es};
       // (forward only, as all plans with primes run)
@@ -842,10 +843,10 @@ __device__ __forceinline__ void sfft(cplx<R>* buf, int ls, int es, const cplx<R>
         generic_pass<R, EMAX>(buf, N, RAD, NS, L, tw);
     } else {
       constexpr int MB = smaxb(N, NL, T, EMAX, RAD);
-      spass<R, N, NL, T, NS, RAD, MB>(buf, ls, es, tw, inv, P == 0 ? pre : nullptr,
+      spass<R, N, NL, T, NS, RAD, MB, TS>(buf, ls, es, tw, inv, P == 0 ? pre : nullptr,
                                       P == splan_count(N) - 1 ? post : nullptr);
     }
-    sfft<R, N, NL, T, EMAX, P + 1, NS * RAD>(buf, ls, es, tw, inv, pre, post);
+    sfft<R, N, NL, T, EMAX, TS, P + 1, NS * RAD>(buf, ls, es, tw, inv, pre, post);
   }
 }
 

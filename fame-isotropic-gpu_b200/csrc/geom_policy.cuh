@@ -30,6 +30,8 @@ struct DynGeom {
   __device__ __forceinline__ static int Ls(const Geom& g) { return g.Ls; }
   __device__ __forceinline__ static int S(const Geom& g) { return g.S; }
   __device__ __forceinline__ static int P(const Geom& g) { return g.P; }
+  static constexpr int kHalves = 1;  // CTAs that share a component's plane (StatGeom)
+  __device__ __forceinline__ static int PL(const Geom& g) { return g.P; }  // points of a CTA's share
   // lines of a plane (pitch S) along its fast axis (fast = true) or mid axis, and
   // the TW lines of a pencil tile.  One FFT call site per kernel keeps the kernel
   // within its register budget, so the plane axis is a runtime argument.  Forward transforms
@@ -115,23 +117,26 @@ struct DynGeomPlane : DynGeom {
   }
 };
 
-template <int LF, int LM, int LSL, int T, int MB>
+// H = 2: two CTAs share a component's plane, split by the first radix-2 step of the mid axis
+// (decimation in frequency): half h holds the frequencies 2 r + h as row r, so that a
+// transform of LM / 2 points on each CTA's own rows is all that is left of that axis.  The forward
+// stage takes its step as it loads the plane (rows m and m + LM / 2 are read by both halves, the
+// second time from L2), the inverse one as it stores it (through distributed shared memory).
+template <int LF, int LM, int LSL, int T, int MB, int H = 1>
 struct StatGeom {
   static constexpr bool kStatic = true;
-  static constexpr int kS = LF | 1, kLf = LF, kLm = LM, kThreads = T;
-  // 384 = 4 threads per line of a 96 x 96 plane: every pass of the 8 x 12 plan
-  // is one round with all threads busy
+  static constexpr int kHalves = H;
+  static constexpr int kS = LF | 1, kLf = LF, kLm = LM / H, kThreads = T;
   template <typename R, int RARE> static constexpr int max_plane_threads() { return T; }
-  // two FP32 plane CTAs per SM (80 registers), one FP64 plane CTA; three FP32 and
-  // two FP64 pencil CTAs
   __device__ __forceinline__ static constexpr int plane_threads() { return T; }
   __device__ __forceinline__ static constexpr int pencil_threads() { return kPencilThreads; }
   template <typename R, int RARE> static constexpr int plane_min_blocks() { return MB; }
   __device__ __forceinline__ static constexpr int Lf(const Geom&) { return LF; }
-  __device__ __forceinline__ static constexpr int Lm(const Geom&) { return LM; }
+  __device__ __forceinline__ static constexpr int Lm(const Geom&) { return kLm; }  // rows of a CTA's share
   __device__ __forceinline__ static constexpr int Ls(const Geom&) { return LSL; }
   __device__ __forceinline__ static constexpr int S(const Geom&) { return kS; }
   __device__ __forceinline__ static constexpr int P(const Geom&) { return LF * LM; }
+  __device__ __forceinline__ static constexpr int PL(const Geom&) { return LF * kLm; }
   static_assert(LF == LM, "a static plane geometry has equal fast and mid lengths");
   template <typename R, int RARE>
   __device__ __forceinline__ static void fft_slow(cplx<R>* b, const AxisPasses&, const cplx<R>* tw) {
@@ -141,7 +146,10 @@ struct StatGeom {
   // stride, twiddle sign and rotation folds to a constant (one call site each).
   template <typename R, bool FAST, bool INV>
   __device__ __forceinline__ static void fft_plane_c(cplx<R>* b, const cplx<R>* tw) {
-    sfft<R, LF, LM, T, SEmax<R>::v>(b, FAST ? kS : 1, FAST ? 1 : kS, tw, INV);
+    if constexpr (FAST)
+      sfft<R, LF, kLm, T, SEmax<R>::v>(b, kS, 1, tw, INV);
+    else
+      sfft<R, kLm, LF, T, SEmax<R>::v, H>(b, 1, kS, tw, INV);
   }
   template <typename R, bool INV>
   __device__ __forceinline__ static void fft_slow_c(cplx<R>* b, const cplx<R>* tw) {
@@ -150,7 +158,16 @@ struct StatGeom {
   }
 };
 
-template <typename R> using Stat96 = StatGeom<96, 96, 96, sizeof(R) == 4 ? 192 : 384, sizeof(R) == 4 ? 3 : 1>;
+// 96^3.  FP32: three plane CTAs of 192 threads per SM.  An FP64 plane is 149 KB, one CTA per SM, and one
+// k-point is then three rounds of clusters (45 of 96 at a time); with halves (75 KB) it is
+// again three CTAs of 192 threads per SM: FP64 operator 151.9 -> 132.9 us (one k-point), 105.2 -> 93.6
+// (ten).  256 threads, at two or three CTAs per SM, 149.5 and 142.5; 128 threads 142.0.
+template <typename R> using Stat96 = StatGeom<96, 96, 96, 192, 3, sizeof(R) == 4 ? 1 : 2>;
+// The CG plane stage keeps whole planes in FP64: at the 96 registers of three CTAs a thread has one point of the
+// recurrences in flight, and what the halves gain in the transforms is lost (plain FP64 solve of
+// one k-point: 324 ms whole, 343 halves, 326 halves of 128 threads).
+template <typename R>
+using Stat96Cg = StatGeom<96, 96, 96, sizeof(R) == 4 ? 192 : 384, sizeof(R) == 4 ? 3 : 1>;
 // static plane plans of the general-lattice benchmark grids (fast, mid, threads, CTAs per SM)
 template <typename R> using PlaneFcc64 = DynGeomPlane<52, 55, 128, sizeof(R) == 4 ? 5 : 4>;
 template <typename R> using PlaneBcc48 = DynGeomPlane<39, 45, 128, sizeof(R) == 4 ? 5 : 4>;

@@ -63,20 +63,24 @@ __device__ __forceinline__ bool plane_vec_range(int P, int s, int comp, const Sl
 }
 
 // ------------------------------------------------------------------ plane stages
-// One cluster = 3 CTAs = the 3 components of plane s.  grid = (3*Ls, vec_per_slot, nslots)
+// One cluster = 3 CTAs = the 3 components of plane s, or 6 where two CTAs share a component
+// (GP::kHalves).  grid = (3*kHalves*Ls, vec_per_slot, nslots)
 struct PlanePos {
-  int s, comp, vec, slot;
+  int s, comp, half, vec, slot;
 };
 // Read afresh from the special registers at every call (the empty asm hides the value from
 // the compiler): a kernel asks again after its transforms, so that nothing but the plane
 // lives across them.  Kept in registers instead, the two dozen values of the mixing
 // phase were spilled and reloaded around every one of the runtime plans' passes.
-__device__ __forceinline__ PlanePos plane_pos() {
+template <class GP> __device__ __forceinline__ PlanePos plane_pos() {
   unsigned x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
   asm volatile("" : "+r"(x), "+r"(y), "+r"(z));
   PlanePos p;
-  p.s = (int)(x / 3);
-  p.comp = (int)x - 3 * p.s;
+  constexpr int C = 3 * GP::kHalves;
+  p.s = (int)(x / C);
+  const int rank = (int)x - C * p.s;
+  p.half = GP::kHalves == 1 ? 0 : rank / 3;
+  p.comp = rank - 3 * p.half;
   p.vec = (int)y;
   p.slot = (int)z;
   return p;
@@ -96,24 +100,37 @@ template <typename R, class GP> __device__ __forceinline__ PlaneSmem<R> plane_sm
   m.plane = reinterpret_cast<cplx<R>*>(smem_raw);
   m.twf = m.plane + GP::Lm(g) * GP::S(g);
   m.twm = GP::kStatic ? m.twf : m.twf + GP::Lf(g);
-  m.lx = m.twm + GP::Lm(g);
+  m.lx = GP::kStatic ? m.twf + GP::Lf(g) : m.twm + GP::Lm(g);
   m.ly = GP::kStatic ? m.plane + GP::Lf(g) : m.lx + GP::Lf(g);
   m.lys = GP::kStatic ? GP::S(g) : 1;
   return m;
 }
 
+// Lambda_x of the plane's axis: in shared memory, or (half planes, FP64) the k-point's table itself.
+template <typename R, class GP>
+__device__ __forceinline__ const cplx<R>* plane_lx(const Geom& g, const double2* tab, const PlaneSmem<R>& m) {
+  if constexpr (GP::kHalves == 1)
+    return m.lx;
+  else
+    return tab + g.oLx;
+}
+// Where element e (row r) of the CTA's share lies in the plane.
+template <class GP> __device__ __forceinline__ int plane_elem(const Geom& g, int half, int e, int r) {
+  return GP::kHalves == 1 ? e : e + (r + half) * GP::Lf(g);
+}
+
 // Twiddle and Lambda (or D_ky) tables into shared memory; a barrier must follow.
 template <typename R, bool GEN, class GP>
 __device__ __forceinline__ void plane_tables(const Geom& g, const cplx<R>* tw, const double2* tab, int s,
-                                             const PlaneSmem<R>& m) {
+                                             int half, const PlaneSmem<R>& m) {
   const int Lf = GP::Lf(g), Lm = GP::Lm(g);
   for (int i = threadIdx.x; i < Lf; i += GP::plane_threads()) {
     m.twf[i] = tw[g.twf + i];
-    if constexpr (!GEN) m.lx[i] = cvt<R>(tab[g.oLx + i]);
+    if constexpr (!GEN && GP::kHalves == 1) m.lx[i] = cvt<R>(tab[g.oLx + i]);
   }
   for (int i = threadIdx.x; i < Lm; i += GP::plane_threads()) {
     if constexpr (!GP::kStatic) m.twm[i] = tw[g.twm + i];
-    m.ly[i * m.lys] = cvt<R>(GEN ? tab[g.oDky + s * g.Ny + i] : tab[g.oLy + i]);
+    m.ly[i * m.lys] = cvt<R>(GEN ? tab[g.oDky + s * g.Ny + i] : tab[g.oLy + GP::kHalves * i + half]);
   }
 }
 
@@ -123,7 +140,7 @@ __device__ __forceinline__ void plane_tables(const Geom& g, const cplx<R>* tw, c
 // and multiplying by the conjugate is what multiplies the value by D_kz.
 template <typename R, class GP>
 __device__ __forceinline__ void plane_times_dkz(const Geom& g, const double2* tabs, const cplx<R>* dkz, cplx<R>* plane) {
-  const PlanePos p = plane_pos();
+  const PlanePos p = plane_pos<GP>();
   const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
   const cplx<R>* d = dkz ? dkz + (size_t)p.slot * g.N + (size_t)p.s * P : nullptr;
   const double2* tab = tabs + (size_t)p.slot * g.tab_stride;
@@ -139,7 +156,7 @@ __device__ __forceinline__ void plane_times_dkz(const Geom& g, const double2* ta
 template <typename R, class GP>
 __device__ __forceinline__ const cplx<R>* plane_dkz(const Geom& g, const AxisPasses& mid, const cplx<R>* dkz) {
   if (!dkz || !GP::mul_ok(mid)) return nullptr;
-  const PlanePos p = plane_pos();
+  const PlanePos p = plane_pos<GP>();
   return dkz + (size_t)p.slot * g.N + (size_t)p.s * GP::P(g);
 }
 
@@ -207,11 +224,29 @@ __device__ __forceinline__ long plane_base(const Geom& g, const PlanePos& p, int
 }
 
 // The plane into shared memory (x conj(D_ky), General): the tables must be in place for
-// General lattices; Simple ones leave cp.async copies in flight (cp_async_wait_all).
+// General lattices; Simple ones leave cp.async copies in flight (cp_async_wait_all).  A half of a plane
+// takes the mid axis' first step here: x_m + x_{m + Lm} or (x_m - x_{m + Lm}) w^m.
 template <typename R, bool GEN, class GP>
-__device__ __forceinline__ void plane_load(const Geom& g, const cplx<R>* T, const PlaneSmem<R>& m) {
-  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g), NT = GP::plane_threads();
-  if constexpr (!GEN) {
+__device__ __forceinline__ void plane_load(const Geom& g, const cplx<R>* T, const cplx<R>* tw, int half,
+                                           const PlaneSmem<R>& m) {
+  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::PL(g), NT = GP::plane_threads();
+  if constexpr (GP::kHalves == 2) {
+    constexpr int U = 6;  // pairs in flight per thread
+    static_assert(GP::kLm * GP::kLf % (U * GP::kThreads) == 0, "whole batches");
+    for (int eb = threadIdx.x; eb < P; eb += U * NT) {
+      cplx<R> v[U], u[U];
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        v[k] = T[eb + k * NT];
+        u[k] = T[P + eb + k * NT];
+      }
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        const int e = eb + k * NT, r = e / Lf;
+        m.plane[e + r * (S - Lf)] = half ? cmul(tw[g.twm + r], csub(v[k], u[k])) : cadd(v[k], u[k]);
+      }
+    }
+  } else if constexpr (!GEN) {
     for (int e = threadIdx.x; e < P; e += NT) {
       const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf);
       cp_async_elem(m.plane + e + r * (S - Lf), T + e);
@@ -235,17 +270,49 @@ __device__ __forceinline__ void plane_load(const Geom& g, const cplx<R>* T, cons
   }
 }
 
-// The plane out to global memory (x D_ky, General).
+// The plane out to global memory (x D_ky, General).  Halves: each combines rows of both, x_m = E_m + conj(w^m) O_m,
+// x_{m + Lm} = E_m - conj(w^m) O_m; plane_store_end must follow before the CTA exits.
 template <typename R, bool GEN, class GP>
 __device__ __forceinline__ void plane_store(const Geom& g, cplx<R>* T) {
   const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
-  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
+  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::PL(g);
+  if constexpr (GP::kHalves == 2) {
+    cg::cluster_group cl = cg::this_cluster();
+    const PlanePos p = plane_pos<GP>();
+    const cplx<R>* peer = cl.map_shared_rank(m.plane, p.comp + 3 * (1 - p.half));
+    constexpr int U = 6;  // remote reads in flight per thread
+    const int NT = GP::plane_threads();
+    for (int eb = threadIdx.x; eb < P; eb += U * NT) {
+      cplx<R> v[U];
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        const int e = eb + k * NT;
+        v[k] = peer[e + e / Lf * (S - Lf)];
+      }
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        const int e = eb + k * NT, r = e / Lf;
+        const cplx<R> own = m.plane[e + r * (S - Lf)], w = m.twf[r];
+        T[p.half * P + e] = p.half ? csub(v[k], cmulc(w, own)) : cadd(own, cmulc(w, v[k]));
+      }
+    }
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+  } else {
 #pragma unroll 4
-  for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
-    const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf);
-    const cplx<R> v = maybe_swap<kSwapInv<GEN, GP>>(m.plane[e + r * (S - Lf)]);
-    T[e] = GEN ? cmul(v, m.ly[r]) : v;
+    for (int e = threadIdx.x; e < P; e += GP::plane_threads()) {
+      const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf);
+      const cplx<R> v = maybe_swap<kSwapInv<GEN, GP>>(m.plane[e + r * (S - Lf)]);
+      T[e] = GEN ? cmul(v, m.ly[r]) : v;
+    }
   }
+}
+
+// Before it: both halves are transformed.  After it: both have been read.
+template <class GP> __device__ __forceinline__ void plane_store_begin() {
+  if constexpr (GP::kHalves == 2) cg::this_cluster().sync();
+}
+template <class GP> __device__ __forceinline__ void plane_store_end() {
+  if constexpr (GP::kHalves == 2) asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
 }
 
 // Exchange of mixed components between the three CTAs.  Static geometries send them with
@@ -255,13 +322,13 @@ __device__ __forceinline__ void plane_store(const Geom& g, cplx<R>* T) {
 template <typename R, bool ASYNC, bool SWAP> struct PlaneExchange {
   cplx<R>* dst[3];
   unsigned rplane[3], rbar[3];
-  __device__ __forceinline__ PlaneExchange(cplx<R>* plane, unsigned bar) {
+  __device__ __forceinline__ PlaneExchange(cplx<R>* plane, unsigned bar, int rank0) {
     cg::cluster_group cl = cg::this_cluster();
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      dst[c] = cl.map_shared_rank(plane, c);
-      rplane[c] = ASYNC ? mapa_u32(smem_u32(plane), c) : 0u;
-      rbar[c] = ASYNC ? mapa_u32(bar, c) : 0u;
+      dst[c] = cl.map_shared_rank(plane, rank0 + c);
+      rplane[c] = ASYNC ? mapa_u32(smem_u32(plane), rank0 + c) : 0u;
+      rbar[c] = ASYNC ? mapa_u32(bar, rank0 + c) : 0u;
     }
   }
   __device__ __forceinline__ void put(int q, const cplx<R>* v) const {
@@ -290,7 +357,7 @@ __device__ __forceinline__ void exchange_wait(unsigned bar, int* fault) {
 }
 
 template <typename R, bool GEN, int IN, bool PR, int RARE, class GP>
-__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
+__global__ void __cluster_dims__(3 * GP::kHalves, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
     k_plane_inv(PlaneInArgs<R> a) {
   FAME_COUNT_LAUNCH();
   pdl_wait();
@@ -301,9 +368,9 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
   const unsigned bar = smem_u32(&xbar);
   {
     const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
-    const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
+    const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g), PL = GP::PL(g);
     cg::cluster_group cl = cg::this_cluster();
-    const PlanePos p = plane_pos();
+    const PlanePos p = plane_pos<GP>();
     const Slot sl = a.slots[p.slot];
     if (!sl.active) return;  // uniform over the cluster
     const CgState* st = nullptr;
@@ -313,7 +380,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     }
     if (kAsyncMix && threadIdx.x == 0) exchange_init(bar, &skip, a.fault);
     const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
-    plane_tables<R, GEN, GP>(g, a.tw, tab, p.s, m);
+    plane_tables<R, GEN, GP>(g, a.tw, tab, p.s, p.half, m);
     const cplx<R> lp = lam_plane<R, GEN>(g, tab, p.s);
     cl.sync();  // every CTA of the cluster is running (and the tables and barriers are in place)
     if constexpr (kAsyncMix) {
@@ -321,13 +388,13 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
         cl.sync();  // rank 0's marker stays readable until all three have read it
         return;
       }
-      if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, (unsigned)(P * sizeof(cplx<R>)));
+      if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, (unsigned)(PL * sizeof(cplx<R>)));
     }
-    const PlaneExchange<R, kAsyncMix, kSwapInv<GEN, GP>> ex(m.plane, bar);
+    const PlaneExchange<R, kAsyncMix, kSwapInv<GEN, GP>> ex(m.plane, bar, 3 * p.half);
     const long vb = (long)(p.slot * a.vec_per_slot + p.vec) * a.vstride;
     const int Nd = sl.Nd, off = sl.off;
-    const int per = (P + 2) / 3;
-    const int e0 = p.comp * per, e1 = min(P, e0 + per);
+    const int per = (PL + 2) / 3;
+    const int e0 = p.comp * per, e1 = min(PL, e0 + per);
     R rscale = 0;
     const float2* x32 = nullptr;
     if constexpr (IN == IN_REFINE) {
@@ -338,7 +405,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     // Input stage and the 2 -> 3 mix.  IN_CG: the start residual r.  IN_REFINE: y += x32 / scale.
     // The operands of KB points per thread are loaded up front, so one global-load latency
     // covers KB points.
-    constexpr int KB = !GP::kStatic ? 2 : IN == IN_REFINE ? 2 : 8;
+    constexpr int KB = !GP::kStatic || IN == IN_REFINE ? 2 : 8 / GP::kHalves;
     const int NT = GP::plane_threads();
     for (int eb = e0 + threadIdx.x; eb < e1; eb += KB * NT) {
       cplx<R> A1[KB], A2[KB];
@@ -348,8 +415,10 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
         const int e = eb + k * NT;
         A1[k] = A2[k] = mk<R>(0, 0);
         F1[k] = F2[k] = make_float2(0.f, 0.f);
-        if (e < e1 && p.s * P + e >= off) {
-          const long i = p.s * P + e - off;
+        const int r = GP::kHalves == 1 ? 0 : e / Lf;
+        const int fi = p.s * P + plane_elem<GP>(g, p.half, e, r);
+        if (e < e1 && fi >= off) {
+          const long i = fi - off;
           if constexpr (IN == IN_REFINE) {
             A1[k] = a.y64[vb + i];
             A2[k] = a.y64[vb + Nd + i];
@@ -365,13 +434,13 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       for (int k = 0; k < KB; k++) {
         const int e = eb + k * NT;
         if (e >= e1) break;
-        const int fi = p.s * P + e;
         const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), f = e - r * Lf;
+        const int fi = p.s * P + plane_elem<GP>(g, p.half, e, r);
         cplx<R> v[3] = {mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0)};
         if (fi >= off) {
           const long i = fi - off;
           cplx<R> Lx, Ly, Lz;
-          lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lp, p.s, r, f, Lx, Ly, Lz);
+          lam_elem<R, GEN>(g, tab, plane_lx<R, GP>(g, tab, m), m.ly, m.lys, lp, p.s, r, f, Lx, Ly, Lz);
           cplx<R> x1 = A1[k], x2 = A2[k];
           if constexpr (IN == IN_VEC) {
             if (a.sigma) {
@@ -401,8 +470,10 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
       cl.sync();
   }
   plane_inverse<R, GEN, RARE, GP>(g, a.ax, a.tabs, a.dkz);
+  plane_store_begin<GP>();
   pdl_trigger();
-  plane_store<R, GEN, GP>(g, a.T + plane_base<R, GP>(g, plane_pos(), a.vec_per_slot, a.fstride));
+  plane_store<R, GEN, GP>(g, a.T + plane_base<R, GP>(g, plane_pos<GP>(), a.vec_per_slot, a.fstride));
+  plane_store_end<GP>();
 }
 
 // ------------------------------------------------------------------ CG plane stage
@@ -423,6 +494,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
 template <typename R, bool GEN, int RARE, class GP>
 __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
     k_plane_cg(PlaneCgArgs<R> a) {
+  static_assert(GP::kHalves == 1, "whole planes");
   FAME_COUNT_LAUNCH();
   const Geom& g = a.g;
   constexpr bool kAsyncMix = GP::kStatic;
@@ -431,11 +503,11 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
   __shared__ double s_coef[2];
   const unsigned bar = smem_u32(&xbar);
   {
-    const PlanePos p = plane_pos();
+    const PlanePos p = plane_pos<GP>();
     const Slot sl = a.slots[p.slot];
     const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
     // the tables are the solve's, older than the kernel before this one
-    if (sl.active) plane_tables<R, GEN, GP>(g, a.tw, a.tabs + (size_t)p.slot * g.tab_stride, p.s, m);
+    if (sl.active) plane_tables<R, GEN, GP>(g, a.tw, a.tabs + (size_t)p.slot * g.tab_stride, p.s, 0, m);
     pdl_wait();
     if ((threadIdx.x | blockIdx.x | blockIdx.y | blockIdx.z) == 0) set_cond(a.reset, 0);
     const CgState* st = a.cg + p.slot;
@@ -447,7 +519,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     if (kAsyncMix && threadIdx.x == 0) exchange_init(bar, &skip, a.fault);
     const cplx<R>* T = a.T + plane_base<R, GP>(g, p, 1, a.fstride);
     if constexpr (GEN) __syncthreads();  // D_ky is in place
-    plane_load<R, GEN, GP>(g, T, m);
+    plane_load<R, GEN, GP>(g, T, a.tw, 0, m);
     // gamma and rho from the pencil stage's partial sums of <r, A r>, summed in order by one warp
     // while the plane streams in
     if (threadIdx.x < 32) {
@@ -493,11 +565,11 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     }
     const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
     const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
-    const PlanePos p = plane_pos();
+    const PlanePos p = plane_pos<GP>();
     const Slot sl = a.slots[p.slot];
     const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
     const cplx<R> lp = lam_plane<R, GEN>(g, tab, p.s);
-    const PlaneExchange<R, kAsyncMix, kSwapInv<GEN, GP>> ex(m.plane, bar);
+    const PlaneExchange<R, kAsyncMix, kSwapInv<GEN, GP>> ex(m.plane, bar, 0);
     const int iter = a.cg[p.slot].iter, cur = iter & 1;
     const bool have_r = iter > 1, have_x = iter > 2;  // r_old = 0 at k = 1; x = 0 at k = 1, x_old = 0 at k = 2
     const long vb = (long)p.slot * a.vstride;
@@ -575,7 +647,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
   }
   plane_inverse<R, GEN, RARE, GP>(g, a.ax, a.tabs, a.dkz);
   pdl_trigger();
-  plane_store<R, GEN, GP>(g, a.T + plane_base<R, GP>(g, plane_pos(), 1, a.fstride));
+  plane_store<R, GEN, GP>(g, a.T + plane_base<R, GP>(g, plane_pos<GP>(), 1, a.fstride));
   // this CTA's part of ||r'||^2; the pencil stage sums the slot's parts in order
   __shared__ double sred[32];
   block_reduce<1>(acc, sred);
@@ -966,13 +1038,13 @@ template <typename R> __device__ __forceinline__ void plane_fwd_decide(const Pla
 }
 
 template <typename R, bool GEN, int EPI, bool PR, int RARE, class GP>
-__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
+__global__ void __cluster_dims__(3 * GP::kHalves, 1, 1) __launch_bounds__(GP::template max_plane_threads<R, RARE>(), GP::template plane_min_blocks<R, RARE>())
     k_plane_fwd(PlaneOutArgs<R> a) {
   FAME_COUNT_LAUNCH();
   pdl_wait();
   const Geom& g = a.g;
   {
-    const PlanePos p = plane_pos();
+    const PlanePos p = plane_pos<GP>();
     bool live = a.slots[p.slot].active;
     if constexpr (EPI == EPI_RESID) live = live && a.cg[p.slot].outer_active;
     if (!live) {
@@ -981,11 +1053,11 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     }
     const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
     const cplx<R>* T = a.T + plane_base<R, GP>(g, p, a.vec_per_slot, a.fstride);
-    if constexpr (!GEN) plane_load<R, GEN, GP>(g, T, m);
-    plane_tables<R, GEN, GP>(g, a.tw, a.tabs + (size_t)p.slot * g.tab_stride, p.s, m);
+    if constexpr (!GEN) plane_load<R, GEN, GP>(g, T, a.tw, p.half, m);
+    plane_tables<R, GEN, GP>(g, a.tw, a.tabs + (size_t)p.slot * g.tab_stride, p.s, p.half, m);
     if constexpr (GEN) {
       __syncthreads();  // D_ky is in place
-      plane_load<R, GEN, GP>(g, T, m);
+      plane_load<R, GEN, GP>(g, T, a.tw, p.half, m);
     } else {
       cp_async_wait_all();
     }
@@ -996,33 +1068,35 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
   cl.sync();  // all three component planes transformed
 
   const PlaneSmem<R> m = plane_smem_of<R, GP>(g);
-  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g);
-  const PlanePos p = plane_pos();
+  const int Lf = GP::Lf(g), S = GP::S(g), P = GP::P(g), PL = GP::PL(g);
+  const PlanePos p = plane_pos<GP>();
   const Slot sl = a.slots[p.slot];
   const double2* tab = a.tabs + (size_t)p.slot * g.tab_stride;
   const cplx<R> lp = lam_plane<R, GEN>(g, tab, p.s);
-  const cplx<R>* src[3] = {cl.map_shared_rank(m.plane, 0), cl.map_shared_rank(m.plane, 1),
-                           cl.map_shared_rank(m.plane, 2)};
-  const int per = (P + 2) / 3;
-  const int e0 = p.comp * per, e1 = min(P, e0 + per);
+  const int rank0 = 3 * p.half;
+  const cplx<R>* src[3] = {cl.map_shared_rank(m.plane, rank0), cl.map_shared_rank(m.plane, rank0 + 1),
+                           cl.map_shared_rank(m.plane, rank0 + 2)};
+  const int per = (PL + 2) / 3;
+  const int e0 = p.comp * per, e1 = min(PL, e0 + per);
   const int Nd = sl.Nd, off = sl.off;
   const long vb = (long)(p.slot * a.vec_per_slot + p.vec) * a.vstride;
   double acc[1] = {0.0};
   // 3 -> 2 unmix and the epilogue.  The three components (remote shared memory) and
   // the vector operand of KB points per thread are read up front, so one latency of
   // each kind covers KB points.
-  constexpr int KB = GP::kStatic ? 4 : 2;
+  constexpr int KB = GP::kStatic ? 4 / GP::kHalves : 2;
   const int NT = GP::plane_threads();
   for (int eb = e0 + threadIdx.x; eb < e1; eb += KB * NT) {
     cplx<R> t[KB][3], va[KB], vb2[KB];
 #pragma unroll
     for (int k = 0; k < KB; k++) {
       const int e = eb + k * NT;
-      const int fi = p.s * P + e;
+      const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf);
+      const int fi = p.s * P + plane_elem<GP>(g, p.half, e, r);
       va[k] = vb2[k] = t[k][0] = t[k][1] = t[k][2] = mk<R>(0, 0);
       if (e < e1 && fi >= off) {
         const long i = fi - off;
-        const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), q = r * S + (e - r * Lf);
+        const int q = r * S + (e - r * Lf);
 #pragma unroll
         for (int c = 0; c < 3; c++) t[k][c] = src[c][q];
         if constexpr (EPI == EPI_RESID) {
@@ -1034,12 +1108,12 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
 #pragma unroll
     for (int k = 0; k < KB; k++) {
       const int e = eb + k * NT;
-      const int fi = p.s * P + e;
+      const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), f = e - r * Lf;
+      const int fi = p.s * P + plane_elem<GP>(g, p.half, e, r);
       if (e >= e1 || fi < off) continue;
       const long i = fi - off;
-      const int r = GP::kStatic ? e / Lf : div_magic(e, g.mLf), f = e - r * Lf;
       cplx<R> Lx, Ly, Lz;
-      lam_elem<R, GEN>(g, tab, m.lx, m.ly, m.lys, lp, p.s, r, f, Lx, Ly, Lz);
+      lam_elem<R, GEN>(g, tab, plane_lx<R, GP>(g, tab, m), m.ly, m.lys, lp, p.s, r, f, Lx, Ly, Lz);
       cplx<R> Pc[6];
       pi_from<R>(GEN, PR, Lx, Ly, Lz, Pc);
       const cplx<R> t0 = t[k][0], t1 = t[k][1], t2 = t[k][2];

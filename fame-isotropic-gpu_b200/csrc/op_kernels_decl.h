@@ -10,9 +10,10 @@ __host__ __device__ inline size_t plane_smem_bytes(int Lf, int Lm, int S) {
   return sizeof(cplx<R>) * ((size_t)Lm * S + 2 * (size_t)Lf + 2 * (size_t)Lm);
 }
 
-// ... of a static geometry: plane | tw [LF] | lx [LF] (ly in the padding column)
+// ... of a static geometry: plane | tw [LF] | lx [LF] (ly in the padding column).  Half planes read
+// lx from global memory: with it three CTAs would not fit on an SM.
 template <typename R, class GP> constexpr size_t stat_plane_smem_bytes() {
-  return sizeof(cplx<R>) * ((size_t)GP::kLm * GP::kS + 2 * GP::kLf);
+  return sizeof(cplx<R>) * ((size_t)GP::kLm * GP::kS + (GP::kHalves == 1 ? 2 : 1) * GP::kLf);
 }
 
 // shared memory of a pencil CTA: tile [Ls x TW] | 1/eps tile [Ls x TW] | twiddles [Ls]

@@ -6,7 +6,7 @@ namespace fame {
 template __global__ void k_plane_inv<double, false, IN_CG, false, 0, Stat96<double>>(PlaneInArgs<double>);
 template __global__ void k_plane_inv<double, false, IN_VEC, false, 0, Stat96<double>>(PlaneInArgs<double>);
 template __global__ void k_plane_inv<double, false, IN_REFINE, false, 0, Stat96<double>>(PlaneInArgs<double>);
-template __global__ void k_plane_cg<double, false, 0, Stat96<double>>(PlaneCgArgs<double>);
+template __global__ void k_plane_cg<double, false, 0, Stat96Cg<double>>(PlaneCgArgs<double>);
 template __global__ void k_plane_fwd<double, false, EPI_OUT, false, 0, Stat96<double>>(PlaneOutArgs<double>);
 template __global__ void k_plane_fwd<double, false, EPI_RESID, false, 0, Stat96<double>>(PlaneOutArgs<double>);
 template __global__ void k_pencil_pipe<double, false>(PencilArgs<double>);

@@ -266,11 +266,16 @@ struct Ops {
     a.fstride = 3L * g().N;
     return a;
   }
-  template <typename R, typename A> void plane_launch(void (*k)(A), int nt, int nvec, A a, bool stat = false) {
+  template <typename R, typename A> void plane_launch(void (*k)(A), int nt, int nvec, A a) {
     plane_passes<R>(g(), nt, a.ax);
-    const size_t sm = stat ? stat_plane_smem_bytes<R, Stat96<R>>() : plane_smem<R>(g());
+    allow_smem(k, plane_smem<R>(g()));
+    P.launch_pdl(k, dim3(3 * g().Ls, nvec, nslots), dim3(nt), plane_smem<R>(g()), a);
+  }
+  // ... of a static geometry
+  template <typename R, class GP, typename A> void stat_launch(void (*k)(A), int nvec, A a) {
+    constexpr size_t sm = stat_plane_smem_bytes<R, GP>();
     allow_smem(k, sm);
-    P.launch_pdl(k, dim3(3 * g().Ls, nvec, nslots), dim3(nt), sm, a);
+    P.launch_pdl(k, dim3(3 * GP::kHalves * g().Ls, nvec, nslots), dim3(GP::kThreads), sm, a);
   }
 
   // plane inverse stage (the arguments of the input mode are set by the callers below)
@@ -292,7 +297,7 @@ struct Ops {
     } else {
       auto k = c->rare == 2 ? k_plane_inv<R, false, IN, PR, 2, DynGeom> : k_plane_inv<R, false, IN, PR, 0, DynGeom>;
       if constexpr (kStatInv<R, IN, PR>)
-        if (c->stat96) return plane_launch<R>(k_plane_inv<R, false, IN, PR, 0, Stat96<R>>, Stat96<R>::kThreads, nvec, a, true);
+        if (c->stat96) return stat_launch<R, Stat96<R>>(k_plane_inv<R, false, IN, PR, 0, Stat96<R>>, nvec, a);
       plane_launch<R>(k, nt, nvec, a);
     }
   }
@@ -336,7 +341,7 @@ struct Ops {
       plane_launch<R>(k, nt, 1, a);
     } else {
       auto k = c->rare == 2 ? k_plane_cg<R, false, 2, DynGeom> : k_plane_cg<R, false, 0, DynGeom>;
-      if (c->stat96) return plane_launch<R>(k_plane_cg<R, false, 0, Stat96<R>>, Stat96<R>::kThreads, 1, a, true);
+      if (c->stat96) return stat_launch<R, Stat96Cg<R>>(k_plane_cg<R, false, 0, Stat96Cg<R>>, 1, a);
       plane_launch<R>(k, nt, 1, a);
     }
   }
@@ -447,7 +452,7 @@ struct Ops {
     } else {
       auto k = c->rare == 2 ? k_plane_fwd<R, false, EPI, PR, 2, DynGeom> : k_plane_fwd<R, false, EPI, PR, 0, DynGeom>;
       if constexpr (kStatFwd<R, EPI, PR>)
-        if (c->stat96) return plane_launch<R>(k_plane_fwd<R, false, EPI, PR, 0, Stat96<R>>, Stat96<R>::kThreads, nvec, a, true);
+        if (c->stat96) return stat_launch<R, Stat96<R>>(k_plane_fwd<R, false, EPI, PR, 0, Stat96<R>>, nvec, a);
       plane_launch<R>(k, nt, nvec, a);
     }
   }

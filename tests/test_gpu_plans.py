@@ -66,3 +66,23 @@ def test_operators_and_cg_at_plan_edges(grid, general, gamma):
         assert f64["rc"] == fb.OK and f32["rc"] == fb.OK
         assert np.max(np.abs(f64["freq"] - f32["freq"])) < 1e-6 * np.max(f64["freq"])
     ctx.close()
+
+
+@pytest.mark.parametrize("gamma", [False, True])
+def test_fp64_half_planes(gamma):
+    """The 96^3 FP64 plane stages share a component's plane between two CTAs."""
+    par = _par((96, 96, 96), False)
+    N = par["N"]
+    k = np.zeros(3) if gamma else np.array([0.21, -0.13, 0.37])
+    rng = np.random.default_rng(N)
+    B = rng.uniform(1.0, 13.0, 3 * N)
+    ctx = fb.Context.from_par(par)
+    ctx.set_eps(B)
+    L = fo.lambdas(k, par)
+    x = rng.standard_normal(2 * L.Nd) + 1j * rng.standard_normal(2 * L.Nd)
+    v = rng.standard_normal(3 * N) + 1j * rng.standard_normal(3 * N)
+    for op, inp, ref in ((fb.OP_QR, x, fo.Qr(x, L)), (fb.OP_QRS, v, fo.Qrs(v, L)), (fb.OP_QBQ, x, fo.QBQ(x, L, 1.0 / B))):
+        y = torch.zeros(ref.size, dtype=torch.complex128, device="cuda")
+        ctx.apply(op, k, torch.from_numpy(inp).to("cuda"), y, fb.FP64)
+        assert _rel(y, ref) < 1e-12, op
+    ctx.close()
