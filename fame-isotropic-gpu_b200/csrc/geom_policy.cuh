@@ -54,19 +54,19 @@ struct DynGeom {
   }
 };
 
-// elements a thread stages per round in the static passes: plane passes (FP32 at
-// most 80 registers, two CTAs per SM) and pencil passes
+// elements a thread stages per round in the static passes: plane passes (96 registers at three
+// CTAs per SM) and pencil passes
 template <typename R> struct SEmax;
 template <> struct SEmax<float> { static constexpr int v = 24; };
 template <> struct SEmax<double> { static constexpr int v = 12; };
 template <typename R> struct SPenEmax;
 template <> struct SPenEmax<float> { static constexpr int v = 24; };
 template <> struct SPenEmax<double> { static constexpr int v = 12; };
-// static plane passes of the runtime-geometry grids (128 registers at two 256-thread
-// CTAs per SM, the general-lattice Pi mixing in the same kernel): half the 96^3
-// staging in FP32, a third in FP64, which keeps the radix-11 and radix-13 passes of
-// the FCC and BCC planes in registers (FCC 64x55x52: FP32 CG iteration 37.5 -> 33.9
-// us per k-point; BCC 48x45x39: FP64 plane stages 23.5 -> 20.7 us)
+// static plane passes of the runtime-geometry grids (96 to 128 registers, the general-lattice
+// Pi mixing in the same kernel): half the 96^3 staging in FP32, a third in FP64, which
+// keeps the radix-11 and radix-13 passes of the FCC and BCC planes in registers (measured with two
+// 256-thread CTAs per SM; FCC 64x55x52: FP32 CG iteration 37.5 -> 33.9 us per k-point; BCC
+// 48x45x39: FP64 plane stages 23.5 -> 20.7 us)
 template <typename R> struct PlaneEmax;
 template <> struct PlaneEmax<float> { static constexpr int v = 12; };
 template <> struct PlaneEmax<double> { static constexpr int v = 4; };

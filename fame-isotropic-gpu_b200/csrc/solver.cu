@@ -1469,6 +1469,9 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
           snprintf(key, sizeof key, "invar/%d/%.17g/%d/%d", prm->ls_maxit, prm->ls_tol, nstep, nwant);
           auto it = c->progs.find(key);
           if (it == c->progs.end()) {
+            // one such graph at a time: a caller may change the tolerance from call to call
+            for (auto q = c->progs.lower_bound("invar/"); q != c->progs.end() && q->first.compare(0, 6, "invar/") == 0;)
+              q = c->progs.erase(q);
             auto prog = std::make_unique<Program>(c->stream, true, c->hflag, 0);
             Ops og{c, *prog, 1};
             const int nvb = vec_blocks(c, 1);

@@ -6,7 +6,7 @@
 // one) has free parameters: the radix order of the axis plans, the threads of a plane
 // CTA in FP32 and FP64, and the L2 prefetch of the mixed-precision CG kernels.  The
 // tuner times candidates with CUDA events on the context's stream (fame_bench_cg for
-// FAME_MIXED: one FP32 CG iteration, its three kernels; fame_bench_qbq for FAME_FP64:
+// FAME_MIXED: one FP32 CG iteration, its two kernels; fame_bench_qbq for FAME_FP64:
 // one Q_r^* B^-1 Q_r apply), each on `batch` copies of the k-point with the L2 flushed
 // before every repetition, and keeps the fastest by coordinate descent: radix order,
 // then CTA size, then prefetch, from the context's current options.  The winner is applied to the context and appended to

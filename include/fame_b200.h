@@ -200,8 +200,8 @@ int fame_set_loop_cap(fame_ctx* ctx, int max_trips);
  *                      FP32 / FP64 kernels, a multiple of 32 in 64..512, or 0 for the
  *                      built-in rule (which goes by the launch's size; fame_get_option then gives
  *                      its choice for one k-point).
- *   "self_prefetch"    1 (default): the CG plane stage prefetches its own vectors into L2
- *                      at the CTA's start; 0: off.
+ *   "self_prefetch"    1 (default): each CTA of the CG plane stage prefetches its own vectors into L2
+ *                      once its plane has arrived; 0: off.
  *   "static_planes"    1 (default): the plane stages of the FCC 64x55x52, BCC 48x45x39 and
  *                      hexagonal 128x107x92 grids run compile-time FFT plans (fixed CTA
  *                      sizes; the plane-thread options do not apply to them); 0: runtime plans.
