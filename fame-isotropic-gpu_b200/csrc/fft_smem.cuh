@@ -862,14 +862,25 @@ inline int plan_level(const AxisPlan& P) {
   return lv;
 }
 
-// Threads a CTA needs so that every pass of the plan can stage one whole line.
-inline int plan_threads(const AxisPlan& P, int emax) {
+// Threads a CTA needs so that every pass of the plan covers one whole line: a butterfly pass
+// stages it in one round; a prime pass holds its u-groups of MU outputs (`mu`: PrimeBlock), one per
+// thread, or, where those are more than any CTA has (kMaxPassThreads), the output-stationary
+// pass that replaces it stages emax outputs a thread.  A pass with fewer threads would leave part
+// of the line as it was.
+constexpr int kMaxPassThreads = 512;  // the prime kernels' launch bound
+inline int plan_threads(const AxisPlan& P, int emax, int mu) {
   int t = 1;
   for (int p = 0; p < P.npass; p++) {
-    const int r = P.radix[p];
-    if (r > 13) continue;
-    const int nb = P.n / r, mb = pass_maxb(emax, r);
-    t = t > (nb + mb - 1) / mb ? t : (nb + mb - 1) / mb;
+    const int r = P.radix[p], nb = P.n / r;
+    int need;
+    if (r > 13) {
+      const int cells = nb * (((r - 1) / 2 + mu) / mu);
+      need = cells <= kMaxPassThreads ? cells : (P.n + emax - 1) / emax;
+    } else {
+      const int mb = pass_maxb(emax, r);
+      need = (nb + mb - 1) / mb;
+    }
+    t = t > need ? t : need;
   }
   return t;
 }

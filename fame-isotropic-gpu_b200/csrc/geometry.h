@@ -163,10 +163,13 @@ inline int geom_level(const Geom& g) {
 inline int plane_level(const Geom& g) { return std::max(plan_level(g.pf), plan_level(g.pm)); }
 inline int pencil_level(const Geom& g) { return plan_level(g.ps); }
 
-// Threads a plane CTA of precision R must have: every pass stages whole lines.
+// Threads a plane CTA of precision R must have (every pass covers whole lines), and may have (the
+// kernels' launch bounds, DynGeom::max_plane_threads).
 template <typename R> inline int plane_threads_min(const Geom& g) {
-  return (std::max(plan_threads(g.pf, Emax<R>::v), plan_threads(g.pm, Emax<R>::v)) + 31) / 32 * 32;
+  constexpr int mu = PrimeBlock<R, false>::mu;
+  return (std::max(plan_threads(g.pf, Emax<R>::v, mu), plan_threads(g.pm, Emax<R>::v, mu)) + 31) / 32 * 32;
 }
+template <typename R> constexpr int plane_threads_most(int level) { return sizeof(R) == 4 && level < 2 ? 768 : kMaxPassThreads; }
 
 // Threads of a runtime-plan CTA that works on `work` elements, for a launch of `ctas` CTAs with
 // `smem` bytes each, from `lo` up to `hi` in steps of 32; `sm_threads` is what the register
@@ -201,16 +204,15 @@ inline int stage_threads(long work, long ctas, size_t smem, int sm_threads, int 
 // ... of a plane stage: `planes` planes (3 CTAs each) of precision R.
 template <typename R>
 inline int plane_threads_rule(const Geom& g, int level, long planes) {
-  // the kernels' launch bounds (DynGeom::max_plane_threads)
-  const int most = sizeof(R) == 4 && level < 2 ? 768 : 512;
-  return stage_threads(g.P, 3 * planes, plane_smem_bytes<R>(g.Lf, g.Lm, g.S), most, plane_threads_min<R>(g), 512);
+  return stage_threads(g.P, 3 * planes, plane_smem_bytes<R>(g.Lf, g.Lm, g.S), plane_threads_most<R>(level),
+                       plane_threads_min<R>(g), 512);
 }
 // ... and of a pencil stage over `vecs` vectors: with a prime pass, enough that it is one round
 // (92 = 4 x 23 in FP64: 51.7 us per k-point with 256 threads, 81.6 with 64).
 template <typename R>
 inline int pencil_threads_rule(const Geom& g, int level, long vecs) {
   constexpr int TW = PencilTW<R>::v, mu = PrimeBlock<R, true>::mu, ml = PrimeBlock<R, true>::ml;
-  int lo = plan_threads(g.ps, Emax<R>::v);
+  int lo = plan_threads(g.ps, Emax<R>::v, mu);
   for (int p = 0; p < g.ps.npass; p++) {
     const int r = g.ps.radix[p];
     if (r > 13) lo = std::max(lo, g.ps.n / r * (((r - 1) / 2 + mu) / mu) * ((TW + ml - 1) / ml));

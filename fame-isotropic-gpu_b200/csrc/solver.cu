@@ -252,8 +252,7 @@ struct Ops {
   }
   template <typename R> const cplx<R>* dkz() const;
 
-  // What the plane kernels share: geometry, tables, twiddles; then the launch of kernel k
-  // (static plane plans: `pick` swaps in the kernel and its thread count).
+  // What the plane kernels share: geometry, tables, twiddles; then the launch of kernel k.
   template <typename R, typename A> A plane_args() const {
     A a;
     memset(&a, 0, sizeof(a));
@@ -267,6 +266,9 @@ struct Ops {
     return a;
   }
   template <typename R, typename A> void plane_launch(void (*k)(A), int nt, int nvec, A a) {
+    if (nt > plane_threads_most<R>(c->rare))
+      throw CudaError(cudaErrorInvalidConfiguration, "an axis of this grid needs " + std::to_string(nt) +
+                                                         " threads in a plane CTA, more than its kernels take");
     plane_passes<R>(g(), nt, a.ax);
     allow_smem(k, plane_smem<R>(g()));
     P.launch_pdl(k, dim3(3 * g().Ls, nvec, nslots), dim3(nt), plane_smem<R>(g()), a);
