@@ -286,7 +286,8 @@ __global__ void __launch_bounds__(256) k_invar_epi(VecArgs va, LzArgs L, int j, 
       L.prof[slot * 3 + 0] += MIXED ? st->total : st->iter;
       L.prof[slot * 3 + 1] += 1;
       if (MIXED) L.prof[slot * 3 + 2] += st->outer_total;
-      if (MIXED ? st->rr > st->otol2 : st->r1 > st->tol2) L.status[slot] |= kStatusCG;
+      // (a NaN ends the loops and is no convergence either)
+      if (!(MIXED ? st->rr <= st->otol2 : st->r1 <= st->tol2)) L.status[slot] |= kStatusCG;
     }
   }
 }

@@ -29,10 +29,18 @@ struct CgState {
 };
 
 // gamma = ||r||^2 / <r, A r> and rho of the three-term CG recurrences (k_plane_cg) from the state
-// before the iteration and <r, A r>.  <r, A r> <= 0 (a residual of zero): no step.
-__device__ __forceinline__ void cg_coefficients(const CgState& st, double rAr, double& gm, double& rho) {
+// before the iteration and <r, A r>.  <r, A r> <= 0 (a residual of zero, or an FP32 sum that
+// underflowed): no step, gamma = 0.  rho = 1 starts the recurrences afresh from the current r and x: in
+// the first iteration, after one without a step, and where rounding leaves nothing of the
+// denominator (1 / rho is a product of step ratios of CG, far above 1e-12 in exact arithmetic).
+__host__ __device__ __forceinline__ void cg_coefficients(const CgState& st, double rAr, double& gm, double& rho) {
   gm = rAr > 0 ? st.r1 / rAr : 0.0;
-  rho = st.iter == 1 ? 1.0 : 1.0 / (1.0 - (gm / st.gm) * (st.r1 / st.r1p) / st.rho);
+  if (!(gm <= 1e300)) gm = 0.0;
+  rho = 1.0;
+  if (st.iter > 1 && gm > 0 && st.gm > 0) {
+    const double den = 1.0 - (gm / st.gm) * (st.r1 / st.r1p) / st.rho;
+    if (den > 1e-12) rho = 1.0 / den;
+  }
 }
 
 struct LzState {
