@@ -68,6 +68,16 @@ template <typename T> struct DBuf {
   }
 };
 
+// What the first pass over device permittivities finds: entries that are not finite and positive
+// (count, first edge), and the range of the others (bit patterns, which order like the values).
+struct EpsScan {
+  int bad, first;
+  unsigned long long lo, hi;
+};
+static int contrast_log2_of(double lo, double hi) {
+  return (int)std::min(40.0, std::max(4.0, ceil(log2(hi / lo))));
+}
+
 }  // namespace fame
 
 using namespace fame;
@@ -139,7 +149,9 @@ struct fame_ctx {
   DBuf<double> adj;  // fame_adjoint_vjp: [nwant] w, [nwant] grad_w, [nwant] denominators
   DBuf<double> bpart;     // per-band partial sums of the solve's split reductions (kBandSplit per band)
   DBuf<double> adj_part;  // the same for the adjoint entry points (never read by a recorded solve)
-  DBuf<int> eps_bad;  // fame_set_eps_device: [0] bad count, [1] first bad edge
+  DBuf<EpsScan> eps_scan;  // fame_set_eps_device
+  // ceil(log2(largest / smallest permittivity)), at least 4 (contrast 16) and at most 40
+  int contrast_log2 = 4;
   // recorded programs keyed by configuration
   std::map<std::string, std::unique_ptr<Program>> progs;
 };
@@ -514,6 +526,15 @@ static int keep_vectors(int nstep, int nwant, bool mixed) {
   return mixed ? nwant + (nstep - nwant) * 3 / 5 : nwant;
 }
 
+// Relative tolerance of an FP32 inner solve.  2e-6 up to a contrast of 16: two FP64 refinement
+// steps reach 1e-12.  Beyond it the true residual of the three-term recurrences (k_plane_cg) stays
+// behind the recursive one by about 0.02 contrast^2 roundings (2^-24), and the products spent below that are lost:
+// a tolerance that grows with the contrast ends the inner solve before, and the refinement goes on from the true
+// residual.  FP32 products of one A_r^-1 to 1e-10 on a 14^3 grid, a sphere of the given contrast / the same
+// inverted, with 2e-6, with this rule, and in the form with search directions (2e-6): 1,000: 75 / 85, 53 / 60,
+// 53 / 62; 10,000: 98 / 140, 72 / 70, 63 / 86; 100,000: 154 / 231, 97 / 95, 104 / 104.
+static double default_inner_tol(int contrast_log2) { return std::min(1e-2, ldexp(2e-6, contrast_log2 - 4)); }
+
 static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool mixed, bool vec) {
   if (nslots <= c->cap_slots && nstep <= c->cap_nstep && nwant <= c->cap_nwant &&
       (!mixed || c->cap_mixed) && (!vec || c->cap_vec))
@@ -729,21 +750,37 @@ __global__ void __launch_bounds__(256) k_adj_vjp(const double2* E, const double*
 }
 
 // Edge permittivities from device memory: count and locate entries that are not
-// finite and positive (pass 0), then write B, 1/B in FP64 and FP32 and, for General
-// lattices, 1/B in the field layout (x, y, z; z fastest) of the pencil stage (pass 1).
-__global__ void __launch_bounds__(256) k_eps_device(Geom g, const double* B, int pass, int* bad, double* B64,
+// finite and positive and find the range of the values (pass 0), then write B, 1/B in FP64 and FP32
+// and, for General lattices, 1/B in the field layout (x, y, z; z fastest) of the pencil stage (pass 1).
+__global__ void __launch_bounds__(256) k_eps_device(Geom g, const double* B, int pass, EpsScan* scan, double* B64,
                                                     double* ib64, float* ib32, double* ib64q, float* ib32q) {
   FAME_COUNT_LAUNCH();
   const long n3 = 3L * g.N;
+  if (pass == 0) {
+    unsigned long long lo = 0x7ff0000000000000ull, hi = 0;  // +inf, 0
+    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n3; e += (long)gridDim.x * blockDim.x) {
+      const double b = B[e];
+      if (!(b > 0.0) || !isfinite(b)) {
+        atomicAdd(&scan->bad, 1);
+        atomicMin(&scan->first, (int)e);
+        continue;
+      }
+      const unsigned long long u = (unsigned long long)__double_as_longlong(b);
+      lo = min(lo, u);
+      hi = max(hi, u);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicMin(&scan->lo, lo);
+      atomicMax(&scan->hi, hi);
+    }
+    return;
+  }
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n3; e += (long)gridDim.x * blockDim.x) {
     const double b = B[e];
-    if (pass == 0) {
-      if (!(b > 0.0) || !isfinite(b)) {
-        atomicAdd(bad, 1);
-        atomicMin(bad + 1, (int)e);
-      }
-      continue;
-    }
     const double ib = 1.0 / b;
     B64[e] = b;
     ib64[e] = ib;
@@ -999,7 +1036,7 @@ void fame_ctx_destroy(fame_ctx* c) {
   for (auto* b : {&c->invB64, &c->invB64q, &c->B64, &c->partials, &c->T0, &c->T1, &c->hcoef, &c->theta, &c->Z, &c->G,
                   &c->stats, &c->adj, &c->bpart, &c->adj_part})
     b->release();
-  c->eps_bad.release();
+  c->eps_scan.release();
   c->invB32.release();
   c->invB32q.release();
   c->slots.release();
@@ -1031,6 +1068,7 @@ int fame_set_eps(fame_ctx* c, const double* B) {
   const long n3 = 3L * c->g.N;
   std::vector<double> ib(n3);
   std::vector<float> ib32(n3);
+  double lo = B[0], hi = B[0];
   for (long i = 0; i < n3; i++) {
     if (!(B[i] > 0.0) || !isfinite(B[i])) {
       set_err("permittivity must be finite and positive (edge " + std::to_string(i) + ")");
@@ -1038,6 +1076,8 @@ int fame_set_eps(fame_ctx* c, const double* B) {
     }
     ib[i] = 1.0 / B[i];
     ib32[i] = (float)ib[i];
+    lo = std::min(lo, B[i]);
+    hi = std::max(hi, B[i]);
   }
   try {
     FAME_CK(cudaSetDevice(c->device));
@@ -1067,6 +1107,7 @@ int fame_set_eps(fame_ctx* c, const double* B) {
     set_err(e.what());
     return FAME_ERR_CUDA;
   }
+  c->contrast_log2 = contrast_log2_of(lo, hi);
   c->have_eps = true;
   c->eps_ver++;
   return FAME_OK;
@@ -1141,7 +1182,7 @@ static int solve_batched(fame_ctx* c, const double* k_xyz, int nk, const fame_so
     s.enorm = resabs_out ? 1 : 0;
     s.es_tol = p.es_tol;
     s.ls_tol = p.ls_tol;
-    s.inner_tol = p.inner_tol > 0 ? p.inner_tol : 2e-6;  // two FP64 refinement steps reach 1e-12
+    s.inner_tol = p.inner_tol > 0 ? p.inner_tol : default_inner_tol(c->contrast_log2);
     s.inner_maxit = p.inner_maxit > 0 ? p.inner_maxit : 200;
     s.loop_cap = c->loop_cap;
     const bool graph = p.use_graph != 0;
@@ -1804,24 +1845,23 @@ int fame_set_eps_device(fame_ctx* c, const double* B) {
     set_err("null argument");
     return FAME_ERR_BAD_INPUT;
   }
+  EpsScan scan = {0, 0x7fffffff, 0x7ff0000000000000ull, 0};
   try {
     FAME_CK(cudaSetDevice(c->device));
-    c->eps_bad.ensure(2);
-    const int init[2] = {0, 0x7fffffff};
-    FAME_CK(cudaMemcpyAsync(c->eps_bad.p, init, sizeof(init), cudaMemcpyHostToDevice, c->stream));
+    c->eps_scan.ensure(1);
+    FAME_CK(cudaMemcpyAsync(c->eps_scan.p, &scan, sizeof(scan), cudaMemcpyHostToDevice, c->stream));
     const Geom& g = c->g;
     const int blocks = (int)std::min<long>(4096, (3L * g.N + 255) / 256);
-    k_eps_device<<<blocks, 256, 0, c->stream>>>(g, B, 0, c->eps_bad.p, nullptr, nullptr, nullptr, nullptr, nullptr);
+    k_eps_device<<<blocks, 256, 0, c->stream>>>(g, B, 0, c->eps_scan.p, nullptr, nullptr, nullptr, nullptr, nullptr);
     FAME_CK(cudaGetLastError());
-    int bad[2];
-    FAME_CK(cudaMemcpyAsync(bad, c->eps_bad.p, sizeof(bad), cudaMemcpyDeviceToHost, c->stream));
+    FAME_CK(cudaMemcpyAsync(&scan, c->eps_scan.p, sizeof(scan), cudaMemcpyDeviceToHost, c->stream));
     FAME_CK(cudaStreamSynchronize(c->stream));
-    if (bad[0]) {
-      set_err("permittivity must be finite and positive (" + std::to_string(bad[0]) + " edges, first " +
-              std::to_string(bad[1]) + ")");
+    if (scan.bad) {
+      set_err("permittivity must be finite and positive (" + std::to_string(scan.bad) + " edges, first " +
+              std::to_string(scan.first) + ")");
       return FAME_ERR_BAD_INPUT;
     }
-    k_eps_device<<<blocks, 256, 0, c->stream>>>(g, B, 1, c->eps_bad.p, c->B64.p, c->invB64.p, c->invB32.p,
+    k_eps_device<<<blocks, 256, 0, c->stream>>>(g, B, 1, c->eps_scan.p, c->B64.p, c->invB64.p, c->invB32.p,
                                                   c->invB64q.p, c->invB32q.p);
     FAME_CK(cudaGetLastError());
     FAME_CK(cudaStreamSynchronize(c->stream));
@@ -1829,6 +1869,10 @@ int fame_set_eps_device(fame_ctx* c, const double* B) {
     set_err(e.what());
     return FAME_ERR_CUDA;
   }
+  double lo, hi;
+  memcpy(&lo, &scan.lo, sizeof lo);
+  memcpy(&hi, &scan.hi, sizeof hi);
+  c->contrast_log2 = contrast_log2_of(lo, hi);
   c->have_eps = true;
   c->eps_ver++;
   return FAME_OK;

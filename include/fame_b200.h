@@ -72,7 +72,8 @@ typedef struct {
   int precision;    /* FAME_FP64 or FAME_MIXED */
   int batch;        /* k-points per launch (0 = automatic: what 60% of free device memory holds, <= 64) */
   int use_graph;    /* 1 = run each batch as one CUDA graph (default), 0 = host-driven loop */
-  double inner_tol; /* FAME_MIXED: relative tolerance of each FP32 inner solve (0 = 2e-6) */
+  double inner_tol; /* FAME_MIXED: relative tolerance of each FP32 inner solve (0 = 2e-6 up to a permittivity
+                       contrast of 16, and in proportion to the contrast up to 1e-2 beyond it) */
   int inner_maxit;  /* FAME_MIXED: products per FP32 inner solve (0 = 200) */
   int want_vectors; /* 1 = compute and return the eigenvectors E */
 } fame_solver_params;
