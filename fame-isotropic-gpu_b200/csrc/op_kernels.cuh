@@ -350,9 +350,13 @@ __device__ __forceinline__ void exchange_init(unsigned bar, int* skip, int* faul
   *skip = fault ? *(volatile int*)fault : 0;
 }
 // End of it: the CTA's plane is complete once all P values have arrived.  A wait that runs out
-// (about 0.1 s; it cannot unless the exchange is broken) records the fault and goes on.
-__device__ __forceinline__ void exchange_wait(unsigned bar, int* fault) {
-  if (!mbar_wait(bar, 0, 200000000LL) && fault) atomicExch(fault, 1);
+// (about 0.1 s; it cannot unless the exchange is broken) records the fault, on the device for later
+// launches and in the host's memory for the caller, and goes on.
+__device__ __forceinline__ void exchange_wait(unsigned bar, int* fault, int* fault_host) {
+  if (!mbar_wait(bar, 0, 200000000LL) && fault) {
+    atomicExch(fault, 1);
+    *(volatile int*)fault_host = 1;
+  }
   __syncthreads();
 }
 
@@ -465,7 +469,7 @@ __global__ void __cluster_dims__(3 * GP::kHalves, 1, 1) __launch_bounds__(GP::te
       }
     }
     if constexpr (kAsyncMix)
-      exchange_wait(bar, a.fault);
+      exchange_wait(bar, a.fault, a.fault_host);
     else
       cl.sync();
   }
@@ -641,7 +645,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(GP::template max_pla
     // All P values have arrived: every CTA has read its elements of this plane too, since an
     // owner sends an element after reading it.
     if constexpr (kAsyncMix)
-      exchange_wait(bar, a.fault);
+      exchange_wait(bar, a.fault, a.fault_host);
     else
       cl.sync();
   }

@@ -141,7 +141,7 @@ struct fame_ctx {
   DBuf<float2> r32, x32, r32b, x32b, T32;
   DBuf<double2> dkz64;  // General lattices: D_kz of every slot
   DBuf<float2> dkz32;
-  int* hflag = nullptr;  // pinned
+  int* hflag = nullptr;  // pinned: [0] a host-driven loop's condition, [1] the fault marker's copy for the caller
   // eigenvectors kept on the device by the last solve (evec_out NULL): its k-points,
   // whether each is the Gamma point (Gamma keeps nwant - 2 restored bands), nwant
   int dev_vec_nk = 0, dev_vec_nwant = 0;
@@ -205,6 +205,7 @@ template <typename K> static int resident_ctas(K* k, size_t smem) {
 // (a bounded wait that ran out) at flags[kFaultFlag].
 // CTAs per band of the split per-band reductions (band statistics, norms, adjoint)
 constexpr int kBandSplit = 64;
+constexpr const char* kExchangeFault = "a bounded device wait ran out (shared-memory exchange of a plane cluster)";
 constexpr int kLoopCG = 0, kLoopOuter = 1, kLoopInner = 2, kLoopRestart = 4, kFaultFlag = 30, kTrips = 32;
 
 struct Ops {
@@ -256,7 +257,7 @@ struct Ops {
     float2* t32 = q.general && d32 ? c->dkz32.p : nullptr;
     if (one) {
       P.launch(k_tables_of, dim3((n + 255) / 256), dim3(256), 0, q, *one, c->slots.p, c->tabs.p,
-               (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2], t64, t32);
+               (double)c->lat.m[0], (double)c->lat.m[1], (double)c->lat.m[2], t64, t32, c->flags.p + kFaultFlag);
       return;
     }
     P.launch(k_tables, dim3((n + 255) / 256, nslots), dim3(256), 0, q, (const Slot*)c->slots.p, c->tabs.p,
@@ -297,7 +298,8 @@ struct Ops {
     a.vec_per_slot = nvec;
     a.cg = c->cg.p;
     a.T = T;
-    a.fault = c->flags.p ? c->flags.p + kFaultFlag : nullptr;
+    a.fault = c->flags.p + kFaultFlag;
+    a.fault_host = c->hflag + 1;
     int nt = c->template plane_nt<R>((long)g().Ls * nvec * nslots);
     if (g().general) {
       auto k = c->rare == 2 ? k_plane_inv<R, true, IN, PR, 2, DynGeom> : k_plane_inv<R, true, IN, PR, 0, DynGeom>;
@@ -344,7 +346,8 @@ struct Ops {
     a.pen_parts = cg_pen_parts<R>();
     a.reset = reset;
     a.self_pf = c->self_prefetch;
-    a.fault = c->flags.p ? c->flags.p + kFaultFlag : nullptr;
+    a.fault = c->flags.p + kFaultFlag;
+    a.fault_host = c->hflag + 1;
     int nt = c->template plane_nt<R>((long)g().Ls * nslots);
     if (g().general) {
       auto k = c->rare == 2 ? k_plane_cg<R, true, 2, DynGeom> : k_plane_cg<R, true, 0, DynGeom>;
@@ -558,9 +561,9 @@ static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool
   c->partials.ensure((size_t)nslots * part);
   c->part_stride = (long)part;
   c->counters.ensure(nslots + 1);
-  FAME_CK(cudaMemset(c->counters.p, 0, (nslots + 1) * sizeof(unsigned)));
+  FAME_CK(cudaMemsetAsync(c->counters.p, 0, (nslots + 1) * sizeof(unsigned), c->stream));
   c->tri_ctr.ensure(1);
-  FAME_CK(cudaMemset(c->tri_ctr.p, 0, sizeof(unsigned)));
+  FAME_CK(cudaMemsetAsync(c->tri_ctr.p, 0, sizeof(unsigned), c->stream));
   c->T0.ensure((size_t)nslots * nstep);
   c->T1.ensure((size_t)nslots * nstep);
   c->hcoef.ensure((size_t)nslots * 2 * (nstep + 2));
@@ -572,6 +575,7 @@ static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool
   c->prof.ensure((size_t)nslots * 3);
   c->status.ensure(nslots);
   c->flags.ensure(64);
+  FAME_CK(cudaMemsetAsync(c->flags.p, 0, 64 * sizeof(int), c->stream));
   const int nphys = nstep + 1 + keep_vectors(nstep, nwant, mixed) + 1;
   c->U.ensure((size_t)nslots * nphys * M);
   c->r64.ensure((size_t)nslots * M);
@@ -1005,7 +1009,8 @@ int fame_ctx_create(int device, const fame_lattice* lat, fame_ctx** out) {
       return rc;
     }
     FAME_CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-    FAME_CK(cudaMallocHost(&c->hflag, sizeof(int)));
+    FAME_CK(cudaMallocHost(&c->hflag, 2 * sizeof(int)));
+    c->hflag[0] = c->hflag[1] = 0;
     c->invB64.ensure(3L * c->g.N);
     c->B64.ensure(3L * c->g.N);
     c->invB32.ensure(3L * c->g.N);
@@ -1245,7 +1250,7 @@ static int solve_batched(fame_ctx* c, const double* k_xyz, int nk, const fame_so
           return FAME_ERR_WATCHDOG;
         }
       if (hflags[kFaultFlag]) {
-        set_err("a bounded device wait ran out (shared-memory exchange of a plane cluster)");
+        set_err(kExchangeFault);
         return FAME_ERR_WATCHDOG;
       }
       for (int q = 0; q < nb; q++) {
@@ -1457,6 +1462,7 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
     if (precision == FAME_MIXED) ensure_workspace(c, 1, c->cap_nstep, c->cap_nwant, true, c->cap_vec);
     const Slot sl = make_slot(c->lat, k);
     if (Nd_out) *Nd_out = sl.Nd;
+    c->hflag[1] = 0;
     Program P(c->stream, false, c->hflag, 100000);
     Ops o{c, P, 1};
     const Geom& g = c->g;
@@ -1560,6 +1566,10 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
       }
     }
     FAME_CK(cudaStreamSynchronize(c->stream));
+    if (c->hflag[1]) {
+      set_err(kExchangeFault);
+      return FAME_ERR_WATCHDOG;
+    }
   } catch (const CudaError& e) {
     set_err(e.what());
     return FAME_ERR_CUDA;
@@ -1707,6 +1717,7 @@ int fame_bench_qbq(fame_ctx* c, const double* k, int precision, int reps, int nb
     FAME_CK(cudaSetDevice(c->device));
     ensure_workspace(c, nbatch, std::max(2, c->cap_nstep), std::max(1, c->cap_nwant), precision == FAME_MIXED,
                      c->cap_vec);
+    FAME_CK(cudaMemsetAsync(c->flags.p, 0, 64 * sizeof(int), c->stream));
     const Slot sl = make_slot(c->lat, k);
     std::vector<Slot> hs(nbatch, sl);  // the same k-point in every slot of the batch
     FAME_CK(cudaMemcpyAsync(c->slots.p, hs.data(), nbatch * sizeof(Slot), cudaMemcpyHostToDevice, c->stream));
@@ -1775,6 +1786,7 @@ int fame_bench_cg(fame_ctx* c, const double* k, int reps, int nbatch, double* ms
   try {
     FAME_CK(cudaSetDevice(c->device));
     ensure_workspace(c, nbatch, std::max(2, c->cap_nstep), std::max(1, c->cap_nwant), true, c->cap_vec);
+    FAME_CK(cudaMemsetAsync(c->flags.p, 0, 64 * sizeof(int), c->stream));
     const Slot sl = make_slot(c->lat, k);
     std::vector<Slot> hs(nbatch, sl);
     FAME_CK(cudaMemcpyAsync(c->slots.p, hs.data(), nbatch * sizeof(Slot), cudaMemcpyHostToDevice, c->stream));

@@ -11,7 +11,8 @@ namespace fame {
 // values per slot), which the plane stages read instead of evaluating it six times per CG
 // iteration.
 // k_tables_of: the one k-point of an operator apply comes as an argument and is stored as
-// slot 0 too (a copy of 48 bytes from the host in front of the kernels cost more than they do).
+// slot 0 too (a copy of 48 bytes from the host in front of the kernels cost more than they do).  It also
+// clears the fault marker, which an earlier call may have left set.
 __device__ __forceinline__ void tables_of(const Geom& g, const Slot& sl, int slot, double2* tabs, double m1, double m2,
                                           double m3, double2* dkz64, float2* dkz32) {
   double2* t = tabs + (size_t)slot * g.tab_stride;
@@ -73,9 +74,12 @@ __global__ void k_tables(Geom g, const Slot* slots, double2* tabs, double m1, do
   tables_of(g, slots[blockIdx.y], blockIdx.y, tabs, m1, m2, m3, dkz64, dkz32);
 }
 __global__ void k_tables_of(Geom g, Slot sl, Slot* slots, double2* tabs, double m1, double m2, double m3, double2* dkz64,
-                            float2* dkz32) {
+                            float2* dkz32, int* fault) {
   FAME_COUNT_LAUNCH();
-  if (blockIdx.x == 0 && threadIdx.x == 0) slots[0] = sl;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    slots[0] = sl;
+    *fault = 0;
+  }
   tables_of(g, sl, 0, tabs, m1, m2, m3, dkz64, dkz32);
 }
 

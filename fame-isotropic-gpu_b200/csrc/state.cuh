@@ -141,6 +141,7 @@ struct PlaneInArgs {
   int sigma;              // IN_VEC: multiply the input by sqrt(Lambda_q) first (Sigma, …_Isotropic.cu:109)
   cplx<R>* T;             // output field (3 components)
   int* fault;             // set to 1 if a bounded wait of the component exchange ran out (or NULL)
+  int* fault_host;        // the same in pinned host memory
 };
 
 template <typename R>
@@ -161,8 +162,8 @@ struct PlaneCgArgs {
   long pstride;           // per-slot stride of `partials`
   int pen_parts;
   Cond reset;             // loop condition cleared by this kernel, the first of the loop body
-  int self_pf;            // L2 prefetch of this CTA's own vectors at its start
-  int* fault;
+  int self_pf;            // L2 prefetch of this CTA's own vectors, once its plane has arrived
+  int *fault, *fault_host;
 };
 
 template <typename R>
