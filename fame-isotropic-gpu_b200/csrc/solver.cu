@@ -538,6 +538,14 @@ static int keep_vectors(int nstep, int nwant, bool mixed) {
 // 53 / 62; 10,000: 98 / 140, 72 / 70, 63 / 86; 100,000: 154 / 231, 97 / 95, 104 / 104.
 static double default_inner_tol(int contrast_log2) { return std::min(1e-2, ldexp(2e-6, contrast_log2 - 4)); }
 
+// The same for plain FP64, in its roundings (2^-53 for 2^-24), beyond a contrast of 32; 0 below, where
+// both forms of the recurrences are equally far off (7.1e-15 and 8.1e-15 at a contrast of 30 and ls_tol 1e-14) and one
+// CG solve is all.  True residuals at ls_tol 1e-12 without the restarts, with them, and of the form with search
+// directions: contrast 10,000: 2.0e-10, 9.7e-13, 1.2e-12 (60, 49 + 3 and 48 products); 100,000: 2.1e-8, 6.6e-12, 1.1e-11.
+static double refine64_tol(int contrast_log2) {
+  return contrast_log2 <= 5 ? 0.0 : std::min(1e-2, ldexp(2e-6, contrast_log2 - 4 - 29));
+}
+
 static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool mixed, bool vec) {
   if (nslots <= c->cap_slots && nstep <= c->cap_nstep && nwant <= c->cap_nwant &&
       (!mixed || c->cap_mixed) && (!vec || c->cap_vec))
@@ -805,13 +813,15 @@ struct SolveCfg {
   int enorm;     // restore E (norms only) for the reference-scaled residual
   int loop_cap;  // bound on every device loop's trips (0: the defaults)
   double es_tol, ls_tol, inner_tol;
+  double refine_tol;  // plain FP64: refine64_tol
+  int contrast_log2;
 };
 
 static std::string cfg_key(const SolveCfg& s, bool graph) {
   char b[256];
-  snprintf(b, sizeof b, "%d/%d/%d/%d/%d/%d/%d/%d/%d/%.17g/%.17g/%.17g/%d/%d", s.nslots, s.nstep, s.nwant,
+  snprintf(b, sizeof b, "%d/%d/%d/%d/%d/%d/%d/%d/%d/%.17g/%.17g/%.17g/%.17g/%d/%d/%d", s.nslots, s.nstep, s.nwant,
            s.es_maxit, s.ls_maxit, s.mixed, s.vec, s.enorm, s.inner_maxit, s.es_tol, s.ls_tol, s.inner_tol,
-           (int)graph, s.loop_cap);
+           s.refine_tol, s.refine_tol > 0 ? s.contrast_log2 : 0, (int)graph, s.loop_cap);
   return b;
 }
 
@@ -819,6 +829,39 @@ static std::string cfg_key(const SolveCfg& s, bool graph) {
 // Lanczos vector u_j of every live slot, leaving w in U[:, j+1]; then one Lanczos step.
 static Cond loop_cond(Program& P, int* flags, int id, int cap, int loop_cap = 0) {
   return P.make_cond(flags + id, flags + kTrips + 2 * id, loop_cap > 0 ? std::min(cap, loop_cap) : cap);
+}
+
+// The A_r^-1 product of Lanczos step j in FP64.  With refine_tol (refine64_tol) the CG is restarted from the true
+// residual; its sum y and the right-hand side take the buffers of the Ritz vectors and their images, which are
+// only filled after the last Lanczos step.
+static void emit_invar64(Ops& o, LzArgs L, int j, double ls_tol, int ls_maxit, double refine_tol, int contrast_log2,
+                         int* flag_base, int loop_cap) {
+  fame_ctx* c = o.c;
+  Program& P = o.P;
+  const long F = 3L * c->g.N;
+  const dim3 vgrid(vec_blocks(c, o.nslots), 1, o.nslots), vblk(256);
+  const double tol2 = ls_tol * ls_tol;
+  Cond cc = loop_cond(P, flag_base, kLoopCG, ls_maxit + 2, loop_cap);
+  if (!(refine_tol > 0)) {
+    P.launch(k_invar_pro<false>, vgrid, vblk, 0, o.va(cc), L, j, c->r64.p, c->x64.p, (double2*)nullptr, tol2, ls_maxit);
+    o.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
+    P.launch(k_invar_epi<INV_PLAIN>, vgrid, vblk, 0, o.va(Cond{}), L, j, (const double2*)c->x64.p,
+             (const double2*)c->x64b.p);
+    return;
+  }
+  double2 *y = c->EV.p, *b = c->AV.p;
+  const double round = ldexp(1.0, contrast_log2 - 50);  // 8 contrast 2^-53
+  Cond outer = loop_cond(P, flag_base, kLoopOuter, 42, loop_cap);
+  P.launch(k_invar_pro<true>, vgrid, vblk, 0, o.va(outer), L, j, c->r64.p, y, b, tol2, ls_maxit);
+  P.while_loop(outer, [&] {
+    P.launch(k_cg64_init, dim3(1), dim3(32), 0, o.va(cc), refine_tol * refine_tol, round * round, ls_maxit, outer);
+    o.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
+    P.launch(k_cg64_add, vgrid, vblk, 0, o.va(Cond{}), y, (const double2*)c->x64.p, (const double2*)c->x64b.p);
+    o.plane_inv_vec<double, false>(y, c->T64.p, 1, 0);
+    o.pencil<double, PEN_QBQ>(c->T64.p, 1, F, c->ibq64(), 2);
+    o.plane_fwd<double, EPI_RESID, false>(c->T64.p, c->r64.p, 1, b, outer, tol2);
+  });
+  P.launch(k_invar_epi<INV_REFINE64>, vgrid, vblk, 0, o.va(Cond{}), L, j, (const double2*)y, (const double2*)nullptr);
 }
 
 static void emit_step(Ops& o, const SolveCfg& s, LzArgs L, int j, int* flag_base) {
@@ -830,12 +873,7 @@ static void emit_step(Ops& o, const SolveCfg& s, LzArgs L, int j, int* flag_base
   const long F = 3L * g.N;
   const double tol2 = s.ls_tol * s.ls_tol;
   if (!s.mixed) {
-    Cond cc = loop_cond(P, flag_base, kLoopCG, s.ls_maxit + 2, s.loop_cap);
-    P.launch(k_invar_pro<false>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(cc), L, j, c->r64.p, c->x64.p,
-             (double2*)nullptr, tol2, s.ls_maxit);
-    o.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
-    P.launch(k_invar_epi<false>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L, j,
-             (const double2*)c->x64.p, (const double2*)c->x64b.p);
+    emit_invar64(o, L, j, s.ls_tol, s.ls_maxit, s.refine_tol, s.contrast_log2, flag_base, s.loop_cap);
   } else {
     Cond outer = loop_cond(P, flag_base, kLoopOuter, 42, s.loop_cap);
     Cond inner = loop_cond(P, flag_base, kLoopInner, s.inner_maxit + 2, s.loop_cap);
@@ -853,7 +891,7 @@ static void emit_step(Ops& o, const SolveCfg& s, LzArgs L, int j, int* flag_base
       o.pencil<double, PEN_QBQ>(c->T64.p, 1, F, c->ibq64(), 2);
       o.plane_fwd<double, EPI_RESID, false>(c->T64.p, c->r64.p, 1, c->b64.p, outer, tol2);
     });
-    P.launch(k_invar_epi<true>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L, j,
+    P.launch(k_invar_epi<INV_MIXED>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L, j,
              (const double2*)c->x64.p, (const double2*)nullptr);
   }
   const int ndots = (int)((M + kLzRows - 1) / kLzRows);
@@ -1188,6 +1226,8 @@ static int solve_batched(fame_ctx* c, const double* k_xyz, int nk, const fame_so
     s.es_tol = p.es_tol;
     s.ls_tol = p.ls_tol;
     s.inner_tol = p.inner_tol > 0 ? p.inner_tol : default_inner_tol(c->contrast_log2);
+    s.refine_tol = s.mixed ? 0.0 : refine64_tol(c->contrast_log2);
+    s.contrast_log2 = c->contrast_log2;
     s.inner_maxit = p.inner_maxit > 0 ? p.inner_maxit : 200;
     s.loop_cap = c->loop_cap;
     const bool graph = p.use_graph != 0;
@@ -1514,8 +1554,10 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
           FAME_CK(cudaMemcpyAsync(c->U.p, x, 2L * sl.Nd * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
           // the CG as a graph, kept like a solve's (the host's loop waited for the device every
           // second iteration: hexagonal 36x30x26, 1404 -> 1079 us)
+          const double refine_tol = refine64_tol(c->contrast_log2);
           char key[96];
-          snprintf(key, sizeof key, "invar/%d/%.17g/%d/%d", prm->ls_maxit, prm->ls_tol, nstep, nwant);
+          snprintf(key, sizeof key, "invar/%d/%.17g/%d/%d/%d", prm->ls_maxit, prm->ls_tol, nstep, nwant,
+                   refine_tol > 0 ? c->contrast_log2 : 0);
           auto it = c->progs.find(key);
           if (it == c->progs.end()) {
             // one such graph at a time: a caller may change the tolerance from call to call
@@ -1523,13 +1565,7 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
               q = c->progs.erase(q);
             auto prog = std::make_unique<Program>(c->stream, true, c->hflag, 0);
             Ops og{c, *prog, 1};
-            const int nvb = vec_blocks(c, 1);
-            Cond cc = loop_cond(*prog, c->flags.p, kLoopCG, prm->ls_maxit + 2);
-            prog->launch(k_invar_pro<false>, dim3(nvb, 1, 1), dim3(256), 0, og.va(cc), L, 0, c->r64.p, c->x64.p,
-                         (double2*)nullptr, prm->ls_tol * prm->ls_tol, prm->ls_maxit);
-            og.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
-            prog->launch(k_invar_epi<false>, dim3(nvb, 1, 1), dim3(256), 0, og.va(Cond{}), L, 0,
-                         (const double2*)c->x64.p, (const double2*)c->x64b.p);
+            emit_invar64(og, L, 0, prm->ls_tol, prm->ls_maxit, refine_tol, c->contrast_log2, c->flags.p, 0);
             prog->instantiate();
             it = c->progs.emplace(key, std::move(prog)).first;
           }

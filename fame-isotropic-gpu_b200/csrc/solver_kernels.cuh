@@ -102,8 +102,8 @@ struct VecArgs {
 // ---------------------------------------------------------------- invAr prologue
 // rhs = u / sqrt(Lambda_q) (…invAr.cu:26), CG start x = 0, r = rhs (CG.cu:30-33).
 // Plain FP64 (MIXED = false): r64 is the CG's residual (k_plane_cg takes x = 0 at k = 1 as
-// read).  Mixed: b = rhs, y = x64 = 0, r64 = b, and the outer refinement loop state is
-// initialised.
+// read).  Mixed, and FP64 with refinement: b = rhs, y = x64 = 0, r64 = b, and the outer refinement
+// loop state is initialised (REFINE).
 struct LzArgs {
   double2* U;              // [nslots][nphys][ustride]
   long ustride;            // column stride (elements)
@@ -135,7 +135,7 @@ __device__ __forceinline__ double2* ucol(const LzArgs& L, int slot, int logical)
   return L.U + ((size_t)slot * L.nphys + ph) * L.ustride;
 }
 
-template <bool MIXED>
+template <bool REFINE>
 __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, double2* r64,
                                                    double2* x64, double2* b64, double tol2, int maxit) {
   FAME_COUNT_LAUNCH();
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, 
       const double s = lq_sqrt_at(va.g, tab, full_index(i, Nd, sl.off));
       const double2 v = make_double2(u[i].x / s, u[i].y / s);
       r64[b + i] = v;
-      if (MIXED) {
+      if (REFINE) {
         x64[b + i] = make_double2(0.0, 0.0);
         b64[b + i] = v;
       }
@@ -165,9 +165,8 @@ __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, 
     if (slot_reduce<1>(acc, va.partials + (size_t)slot * gridDim.x, va.counters + slot, blockIdx.x,
                        gridDim.x, tot)) {
       if (threadIdx.x == 0) {
-        if (!MIXED) {
+        if (!REFINE) {
           st->r1 = tot[0];
-          st->r1_0 = tot[0];
           st->tol2 = tol2;
           st->iter = 1;
           st->maxit = maxit;
@@ -178,6 +177,7 @@ __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, 
           st->scale = 1.0 / sqrt(tot[0] > 0 ? tot[0] : 1.0);
           st->outer = 0;
           st->outer_max = 40;  // refinement steps per solve; each gains ~5 digits
+          st->rounded = 0;
           st->total = 0;
           st->outer_total = 0;
           st->outer_active = tot[0] > tol2;
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, 
     if (threadIdx.x == 0) {
       int any = 0;
       for (int q = 0; q < va.nslots; q++)
-        any |= va.slots[q].active && (MIXED ? va.cg[q].outer_active : va.cg[q].active);
+        any |= va.slots[q].active && (REFINE ? va.cg[q].outer_active : va.cg[q].active);
       start_cond(va.cond, any);
     }
   }
@@ -231,7 +231,6 @@ __global__ void __launch_bounds__(256) k_cg32_init(VecArgs va, const double2* r6
       if (threadIdx.x == 0) {
         const double need = st->rr > 0 ? 0.25 * outer_tol2 / st->rr : 0.0;
         st->r1 = tot[0];
-        st->r1_0 = tot[0];
         st->tol2 = (need > tau2 ? need : tau2) * tot[0];
         st->iter = 1;
         st->maxit = maxit;
@@ -251,10 +250,58 @@ __global__ void __launch_bounds__(256) k_cg32_init(VecArgs va, const double2* r6
   }
 }
 
+// FP64 CG with restarts from the true residual, for a permittivity contrast beyond 32
+// (refine64_tol): the start of one CG solve, from r64 = b - A y (r64 is the CG's start residual as it
+// stands).  It ends at ls_tol or after a reduction by `floor2` (squared), where the three-term recurrences stop
+// being worth more; maxit bounds the products over all restarts.  A restart that has not halved the true
+// residual has reached what rounding leaves: that counts as solved where it is within the
+// rounding of the form with search directions, `rounding2` ||b||^2, which could not tell either.
+__global__ void __launch_bounds__(32) k_cg64_init(VecArgs va, double floor2, double rounding2, int maxit, Cond outer_reset) {
+  FAME_COUNT_LAUNCH();
+  if (threadIdx.x == 0) set_cond(outer_reset, 0);
+  int any = 0;
+  for (int q = threadIdx.x; q < va.nslots; q += 32) {
+    CgState* st = va.cg + q;
+    st->active = 0;
+    if (!va.slots[q].active || !st->outer_active) continue;
+    const double rr = st->rr;
+    if (st->outer == 0) st->bb = rr;
+    const bool halved = st->outer == 0 || rr <= 0.25 * st->rr_old;
+    if (!halved || st->total >= maxit) {
+      st->rounded = !halved && rr <= rounding2 * st->bb;
+      st->outer_active = 0;
+      continue;
+    }
+    st->rr_old = rr;
+    st->r1 = rr;
+    st->tol2 = fmax(st->otol2, floor2 * rr);
+    st->iter = 1;
+    st->maxit = maxit - st->total;
+    st->active = 1;
+    any = 1;
+  }
+  any = __any_sync(0xffffffffu, any);
+  if (threadIdx.x == 0) start_cond(va.cond, any);
+}
+
+// The end of it: y += x, the CG's solution in the buffer of its last iteration's parity.
+__global__ void __launch_bounds__(256) k_cg64_add(VecArgs va, double2* y, const double2* x64, const double2* x64b) {
+  FAME_COUNT_LAUNCH();
+  const int slot = blockIdx.z;
+  const Slot sl = va.slots[slot];
+  const CgState* st = va.cg + slot;
+  if (!sl.active || !st->outer_active || st->iter == 1) return;
+  const long b = (long)slot * va.vstride;
+  const double2* xs = (st->iter & 1) ? x64 : x64b;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * sl.Nd; i += gridDim.x * blockDim.x)
+    y[b + i] = cadd(y[b + i], xs[b + i]);
+}
+
 // invAr epilogue: w = x / sqrt(Lambda_q) into U[:, j+1] (…invAr.cu:45) and
 // alpha_j = Re<w, u_j> (Lanczos_decomp_gpu.cu:64-66); profile counters
-// (…invAr.cu:41-43: ls_iter += k, es_iter++).
-template <bool MIXED>
+// (…invAr.cu:41-43: ls_iter += k, es_iter++).  MODE: plain FP64 CG, FP64 with refinement, mixed.
+enum InvMode { INV_PLAIN = 0, INV_REFINE64 = 1, INV_MIXED = 2 };
+template <int MODE>
 __global__ void __launch_bounds__(256) k_invar_epi(VecArgs va, LzArgs L, int j, const double2* x64,
                                                    const double2* x64b) {
   FAME_COUNT_LAUNCH();
@@ -267,10 +314,11 @@ __global__ void __launch_bounds__(256) k_invar_epi(VecArgs va, LzArgs L, int j, 
   double2* w = ucol(L, slot, j + 1);
   const int Nd = sl.Nd, n = 2 * Nd;
   // plain FP64: the solution is in the buffer of the last iteration's parity (x64 odd, x64b
-  // even), and zero if the CG did no product; mixed: the refinement's sum, in x64
+  // even), and zero if the CG did no product; else the refinement's sum, in x64
+  constexpr bool kSum = MODE != INV_PLAIN;
   const int iter = va.cg[slot].iter;
-  const double2* xs = MIXED || (iter & 1) ? x64 : x64b;
-  const bool none = !MIXED && iter == 1;
+  const double2* xs = kSum || (iter & 1) ? x64 : x64b;
+  const bool none = !kSum && iter == 1;
   double acc[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double s = lq_sqrt_at(va.g, tab, full_index(i, Nd, sl.off));
@@ -287,11 +335,12 @@ __global__ void __launch_bounds__(256) k_invar_epi(VecArgs va, LzArgs L, int j, 
     if (threadIdx.x == 0) {
       L.T0[slot * L.nstep + j] = tot[0];
       const CgState* st = va.cg + slot;
-      L.prof[slot * 3 + 0] += MIXED ? st->total : st->iter;
+      L.prof[slot * 3 + 0] += MODE == INV_MIXED ? st->total : MODE == INV_REFINE64 ? st->total + 1 : st->iter;
       L.prof[slot * 3 + 1] += 1;
-      if (MIXED) L.prof[slot * 3 + 2] += st->outer_total;
+      if (kSum) L.prof[slot * 3 + 2] += st->outer_total;
       // (a NaN ends the loops and is no convergence either)
-      if (!(MIXED ? st->rr <= st->otol2 : st->r1 <= st->tol2)) L.status[slot] |= kStatusCG;
+      const bool solved = kSum ? st->rr <= st->otol2 || (MODE == INV_REFINE64 && st->rounded) : st->r1 <= st->tol2;
+      if (!solved) L.status[slot] |= kStatusCG;
     }
   }
 }

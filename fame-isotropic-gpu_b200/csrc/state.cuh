@@ -17,15 +17,17 @@ template <typename R> struct PencilTW { static constexpr int v = 256 / (int)size
 struct CgState {
   double r1, r1p;            // ||r||^2 now / one iteration before
   double gm, rho;            // the last iteration's gamma and rho (cg_coefficients)
-  double r1_0, tol2;         // initial ||r||^2, stop threshold on ||r||^2
+  double tol2;               // stop threshold on ||r||^2
   int iter;                  // the reference's counter k (starts at 1, CG.cu:36)
   int active;
   int maxit;
   int total;                 // CG products accumulated for the profile counter
-  // outer iterative refinement (mixed precision)
+  // outer iterative refinement (mixed precision; FP64 at a high contrast)
   double rr, scale;          // ||b - A y||^2, 1/||b - A y|| used to scale the FP32 rhs
   double otol2;              // stop threshold of the refinement on ||b - A y||^2 (ls_tol^2)
   int outer, outer_active, outer_max, outer_total;
+  double bb, rr_old;         // FP64: ||b||^2, and rr one restart before
+  int rounded;               // FP64: the residual has reached what FP64 can hold
 };
 
 // gamma = ||r||^2 / <r, A r> and rho of the three-term CG recurrences (k_plane_cg) from the state

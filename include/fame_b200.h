@@ -68,7 +68,8 @@ typedef struct {
   int es_maxit;     /* ES.maxit: maximum Lanczos restarts */
   double es_tol;    /* ES.tol: |beta_m z_m,i| < tol */
   int ls_maxit;     /* LS.maxit */
-  double ls_tol;    /* LS.tol: absolute ||r|| of the inner solve */
+  double ls_tol;    /* LS.tol: absolute ||r|| of the inner solve (FP64 beyond a permittivity contrast of 32, and
+                       FAME_MIXED: the true residual's, or what rounding leaves of it) */
   int precision;    /* FAME_FP64 or FAME_MIXED */
   int batch;        /* k-points per launch (0 = automatic: what 60% of free device memory holds, <= 64) */
   int use_graph;    /* 1 = run each batch as one CUDA graph (default), 0 = host-driven loop */
@@ -86,7 +87,8 @@ typedef struct {
   int restarts;     /* Lanczos restarts */
   int status;       /* FAME_OK / FAME_ERR_NO_CONVERGENCE for this k */
   int Nd;           /* N or N-1 (Gamma point) */
-  int refine;       /* FAME_MIXED: FP64 refinement steps (each one FP64 Q_r^* B^-1 Q_r); else 0 */
+  int refine;       /* FAME_MIXED, and FP64 beyond a permittivity contrast of 32: true residuals taken (each one
+                       FP64 Q_r^* B^-1 Q_r); else 0 */
   int detail;       /* why status is FAME_ERR_NO_CONVERGENCE, FAME_KSTATUS_* bits (0 when FAME_OK) */
 } fame_kcounters;
 

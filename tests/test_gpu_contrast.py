@@ -1,9 +1,11 @@
 """High permittivity contrast: accuracy and cost of the CG in A_r^-1.
 
 The three-term recurrences of the CG kernels lose accuracy with the square of the contrast, the
-textbook form (the oracle's) with the contrast itself, so the library restarts them from the
-true residual earlier.
+textbook form (the oracle's) with the contrast itself, so beyond a contrast of 32 the library restarts them
+from the true residual.
 
+  - FP64 A_r^-1: the true residual ||b - A x|| is at most ls_tol, or the oracle CG's where rounding does not
+    let it reach ls_tol either (10% for the residual's own evaluation);
   - mixed precision: as many products per A_r^-1 as the form with search directions needs, 1.3 to 1.7 times those
     of an FP64 CG to 1e-10 at these contrasts (restated on the CPU in FP32 on these crystals; the
     three-term form with the default inner tolerance takes 1.9 to 3.4 times)."""
@@ -35,6 +37,31 @@ def _ctx(n, B):
     ctx = fb.Context.from_par(_par(n))
     ctx.set_eps(B)
     return ctx
+
+
+@pytest.mark.parametrize("inverted", [False, True])
+@pytest.mark.parametrize("contrast", [20, 100, 1e3, 1e4, 1e5])
+@pytest.mark.parametrize("k", [GEN, NEAR], ids=["general", "near"])
+def test_fp64_inverse_reaches_the_plain_form_s_residual(k, contrast, inverted):
+    n = 14
+    B = _eps(n, contrast, inverted)
+    k = np.array(k)
+    L = fo.lambdas(k, _par(n))
+    s = np.concatenate([L.Lq_sqrt, L.Lq_sqrt])
+    rng = np.random.default_rng(5)
+    b = rng.standard_normal(2 * L.Nd) + 1j * rng.standard_normal(2 * L.Nd)
+    b /= np.linalg.norm(b)
+    ctx = _ctx(n, B)
+    for tol in (1e-10, 1e-12, 1e-14):
+        ref, _ = fo.cg(lambda p: fo.QBQ(p, L, 1.0 / B), b, tol, 2000)
+        plain = np.linalg.norm(b - fo.QBQ(ref, L, 1.0 / B))
+        y = torch.zeros(2 * L.Nd, dtype=torch.complex128, device="cuda")
+        ctx.apply(fb.OP_INVAR, k, torch.from_numpy(b * s).to("cuda"), y, fb.FP64, fb.solver_params(ls_tol=tol, ls_maxit=2000))
+        z = torch.from_numpy(y.cpu().numpy() * s).to("cuda")
+        ctx.apply(fb.OP_QBQ, k, z, y, fb.FP64)  # each form's residual by its own operator: they differ by as much
+        true = np.linalg.norm(b - y.cpu().numpy())
+        assert true <= 1.1 * max(tol, plain), (tol, true, plain)
+    ctx.close()
 
 
 @pytest.mark.parametrize("inverted", [False, True])
@@ -72,3 +99,15 @@ def test_permittivity_on_the_device_takes_the_same_path():
         assert oa["counters"] == oc["counters"] and np.array_equal(oa["freq"], oc["freq"])
     for q in (a, b, c):
         q.close()
+
+
+def test_fp64_solve_at_high_contrast_reports_a_cap():
+    """ls_maxit bounds the products of an A_r^-1 solve, restarts included."""
+    n = 14
+    ctx = _ctx(n, _eps(n, 1e4, False))
+    k = np.array([GEN])
+    out = ctx.solve(k, nwant=4, nstep=20, es_maxit=1, es_tol=1e-10, ls_tol=1e-12, ls_maxit=20, precision=fb.FP64)
+    c = out["counters"][0]
+    assert out["rc"] == fb.ERR_NO_CONVERGENCE and c["detail"] & fb.KSTATUS_CG
+    assert c["ls_iter"] <= 21 * c["es_iter"]  # the counter starts at 1 per solve
+    ctx.close()
