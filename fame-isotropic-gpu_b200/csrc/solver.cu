@@ -529,6 +529,16 @@ static int keep_vectors(int nstep, int nwant, bool mixed) {
   return mixed ? nwant + (nstep - nwant) * 3 / 5 : nwant;
 }
 
+// Restarts that es_maxit allows.  It counts restarts that keep nwant vectors and run nstep - nwant steps;
+// the thick restarts of mixed precision run fewer, so the cap is the number of them (after the first) that takes
+// the same steps, rounded up.
+static int restart_cap(int es_maxit, int nstep, int nwant, bool mixed) {
+  if (es_maxit <= 1) return es_maxit;
+  const long step = nstep - keep_vectors(nstep, nwant, mixed);
+  const long cap = 1 + ((long)(es_maxit - 1) * (nstep - nwant) + step - 1) / step;
+  return (int)std::min<long>(cap, 1L << 30);
+}
+
 // Relative tolerance of an FP32 inner solve.  2e-6 up to a contrast of 16: two FP64 refinement
 // steps reach 1e-12.  Beyond it the true residual of the three-term recurrences (k_plane_cg) stays
 // behind the recursive one by about 0.02 contrast^2 roundings (2^-24), and the products spent below that are lost:
@@ -906,6 +916,7 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   const long F = 3L * g.N;
   const int nvb = vec_blocks(c, s.nslots);
   const int nkeep = keep_vectors(s.nstep, s.nwant, s.mixed);
+  const int max_restarts = restart_cap(s.es_maxit, s.nstep, s.nwant, s.mixed);
   const int nphys = s.nstep + 1 + nkeep + 1;
   LzArgs L;
   L.U = c->U.p;
@@ -925,7 +936,7 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   o.tables(true, s.mixed);
   P.launch(k_lz_init, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L);
   for (int j = 0; j < s.nstep; j++) emit_step(o, s, L, j, flags);
-  Cond restart = loop_cond(P, flags, kLoopRestart, s.es_maxit + 2, s.loop_cap);
+  Cond restart = loop_cond(P, flags, kLoopRestart, max_restarts + 2, s.loop_cap);
   TriArgs ta;
   ta.L = L;
   ta.slots = c->slots.p;
@@ -933,7 +944,7 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   ta.Z = c->Z.p;
   ta.G = c->G.p;
   ta.tol = s.es_tol;
-  ta.maxit = s.es_maxit;
+  ta.maxit = max_restarts;
   ta.cond = restart;
   ta.nslots = s.nslots;
   ta.status = c->status.p;

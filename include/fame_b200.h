@@ -65,7 +65,8 @@ typedef struct {
 typedef struct {
   int nwant;        /* ES.nwant */
   int nstep;        /* ES.nstep (<= 64) */
-  int es_maxit;     /* ES.maxit: maximum Lanczos restarts */
+  int es_maxit;     /* ES.maxit: maximum Lanczos restarts, of nstep - nwant steps each.  FAME_MIXED's restarts after the
+                       first keep more than nwant vectors and run fewer steps: as many more are allowed */
   double es_tol;    /* ES.tol: |beta_m z_m,i| < tol */
   int ls_maxit;     /* LS.maxit */
   double ls_tol;    /* LS.tol: absolute ||r|| of the inner solve (FP64 beyond a permittivity contrast of 32, and
@@ -95,7 +96,7 @@ typedef struct {
 /* fame_kcounters.detail bits.  The reference only prints these cases
  * (FAME_Main/CG.cu:81-84, FAME_Main/Lanczos_Isotropic.cu:84-85). */
 #define FAME_KSTATUS_QL 1      /* the tridiagonal eigensolve did not converge */
-#define FAME_KSTATUS_LANCZOS 2 /* Lanczos stopped at es_maxit restarts unconverged */
+#define FAME_KSTATUS_LANCZOS 2 /* Lanczos stopped at es_maxit unconverged */
 #define FAME_KSTATUS_CG 4      /* an A_r^-1 solve stopped above ls_tol: ls_maxit products (FP64) or
                                   the refinement cap (FAME_MIXED) */
 
@@ -188,7 +189,7 @@ int fame_launch_count(fame_ctx* ctx, unsigned long long* count_out);
 /* Bound on the trips of every device loop of later solves on this context: the CG,
  * refinement, inner FP32 and Lanczos restart loops each stop after at most
  * `max_trips` trips (0 restores the defaults: ls_maxit + 2, 42, inner_maxit + 2 and
- * es_maxit + 2, which only a fault reaches).  A loop that reaches its bound ends the
+ * the restarts es_maxit allows + 2, which only a fault reaches).  A loop that reaches its bound ends the
  * solve with FAME_ERR_WATCHDOG instead of running on.  No counterpart in the
  * reference, whose loops are host-driven. */
 int fame_set_loop_cap(fame_ctx* ctx, int max_trips);
