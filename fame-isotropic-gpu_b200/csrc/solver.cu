@@ -135,7 +135,7 @@ struct fame_ctx {
   DBuf<LzState> lz;
   DBuf<double> partials, T0, T1, hcoef, theta, Z, G, stats;
   DBuf<unsigned> counters, tri_ctr;
-  DBuf<int> map, prof, status, flags;
+  DBuf<int> prof, status, flags;
   // CG vectors r and x come in pairs, the buffer of odd iterations first (r64, r64b ...)
   DBuf<double2> U, r64, x64, b64, r64b, x64b, T64, EV, AV, Tb, E;
   DBuf<float2> r32, x32, r32b, x32b, T32;
@@ -589,13 +589,11 @@ static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool
   c->Z.ensure((size_t)nslots * nstep * nstep);
   c->G.ensure((size_t)nslots * (nstep + 1) * (keep_vectors(nstep, nwant, mixed) + 1));
   c->stats.ensure((size_t)nslots * nwant * 8);
-  c->map.ensure((size_t)nslots * (nstep + 1) + (size_t)nslots * (keep_vectors(nstep, nwant, mixed) + 1));
   c->prof.ensure((size_t)nslots * 3);
   c->status.ensure(nslots);
   c->flags.ensure(64);
   FAME_CK(cudaMemsetAsync(c->flags.p, 0, 64 * sizeof(int), c->stream));
-  const int nphys = nstep + 1 + keep_vectors(nstep, nwant, mixed) + 1;
-  c->U.ensure((size_t)nslots * nphys * M);
+  c->U.ensure((size_t)nslots * (nstep + 1) * M);
   c->r64.ensure((size_t)nslots * M);
   c->x64.ensure((size_t)nslots * M);
   c->T64.ensure((size_t)nslots * 3 * N);
@@ -917,12 +915,9 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   const int nvb = vec_blocks(c, s.nslots);
   const int nkeep = keep_vectors(s.nstep, s.nwant, s.mixed);
   const int max_restarts = restart_cap(s.es_maxit, s.nstep, s.nwant, s.mixed);
-  const int nphys = s.nstep + 1 + nkeep + 1;
   LzArgs L;
   L.U = c->U.p;
   L.ustride = M;
-  L.nphys = nphys;
-  L.map = c->map.p;
   L.nstep = s.nstep;
   L.nwant = s.nwant;
   L.nkeep = nkeep;
@@ -954,18 +949,17 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   allow_smem(k_tridiag, tsm);
   P.launch(k_tridiag, dim3(s.nslots), dim3(32), tsm, ta);
   ta.first = 0;
+  const size_t rsm = restart_smem(s.nstep, nkeep);
+  allow_smem(k_restart, rsm);
   P.while_loop(restart, [&] {
-    for (int c0 = 0; c0 <= nkeep; c0 += 8)
-      P.launch(k_ugemm<8>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(restart), L, (const double*)c->G.p,
-               s.nstep + 1, s.nstep + 1, nkeep + 1, 0, (double2*)nullptr, c0);
-    P.launch(k_remap, dim3(s.nslots), dim3(32), 0, L, (const Slot*)c->slots.p, s.nslots);
+    P.launch(k_restart, dim3(nvb, 1, s.nslots), dim3(256), rsm, o.va(restart), L, (const double*)c->G.p);
     for (int j = s.nwant; j < s.nstep; j++) emit_step(o, s, L, j, flags);
     P.launch(k_tridiag, dim3(s.nslots), dim3(32), tsm, ta);
   });
   // Ritz vectors ev = U(:, 0:nstep) z(:, 0:nwant)   (Lanczos_Isotropic.cu:93)
   for (int c0 = 0; c0 < s.nwant; c0 += 8)
     P.launch(k_ugemm<8>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L, (const double*)c->Z.p,
-             s.nstep, s.nstep, s.nwant, 1, c->EV.p, c0);
+             c->EV.p, c0);
   // FP64 residual and Rayleigh quotient per band: v = QBQ(Sigma y)
   o.plane_inv_vec<double, false>(c->EV.p, c->Tb.p, s.nwant, 1);
   o.pencil<double, PEN_QBQ>(c->Tb.p, s.nwant, F, c->ibq64(), 0);
@@ -990,7 +984,7 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
 // Device bytes of one slot's workspace (the per-slot buffers of ensure_workspace).
 static double slot_bytes(const fame_ctx* c, int nstep, int nwant, bool mixed, bool vec) {
   const double N = c->g.N, M = 2.0 * N, z = 16.0;
-  double b = (nstep + 1 + keep_vectors(nstep, nwant, mixed) + 1) * M * z   // Lanczos basis U
+  double b = (nstep + 1) * M * z               // Lanczos basis U
              + 2 * M * z + 3 * N * z           // r64, x64, T64
              + 2 * nwant * M * z + nwant * 3 * N * z  // EV, AV, Tb
              + 2 * M * z;                      // r64b, x64b
@@ -1099,7 +1093,6 @@ void fame_ctx_destroy(fame_ctx* c) {
   c->lz.release();
   c->counters.release();
   c->tri_ctr.release();
-  c->map.release();
   c->prof.release();
   c->status.release();
   c->flags.release();
@@ -1551,8 +1544,6 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
           LzArgs L;
           L.U = c->U.p;
           L.ustride = M;
-          L.nphys = nstep + 1 + nwant + 1;
-          L.map = c->map.p;
           L.nstep = nstep;
           L.nwant = L.nkeep = nwant;
           L.T0 = c->T0.p;

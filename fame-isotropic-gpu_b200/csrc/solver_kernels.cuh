@@ -105,10 +105,8 @@ struct VecArgs {
 // read).  Mixed, and FP64 with refinement: b = rhs, y = x64 = 0, r64 = b, and the outer refinement
 // loop state is initialised (REFINE).
 struct LzArgs {
-  double2* U;              // [nslots][nphys][ustride]
+  double2* U;              // [nslots][nstep + 1][ustride]
   long ustride;            // column stride (elements)
-  int nphys;
-  int* map;                // [nslots][nstep+1] logical -> physical column
   int nstep, nwant;
   int nkeep;               // Lanczos vectors a restart after the first keeps (keep_vectors, >= nwant)
   double* T0;              // [nslots][nstep]
@@ -130,9 +128,8 @@ __device__ __forceinline__ bool lz_live(const LzArgs& L, int slot, int j) {
   return !L.lz[slot].converged && j >= L.lz[slot].keep;
 }
 
-__device__ __forceinline__ double2* ucol(const LzArgs& L, int slot, int logical) {
-  const int ph = L.map[slot * (L.nstep + 1) + logical];
-  return L.U + ((size_t)slot * L.nphys + ph) * L.ustride;
+__device__ __forceinline__ double2* ucol(const LzArgs& L, int slot, int c) {
+  return L.U + ((size_t)slot * (L.nstep + 1) + c) * L.ustride;
 }
 
 template <bool REFINE>
@@ -479,7 +476,7 @@ __device__ __forceinline__ double hash_unit(unsigned long long z) {
 }
 
 // Start vector e_M (Lanczos_decomp_gpu.cu:93-107) plus a fixed pseudo-random
-// perturbation of total norm 1e-12, and map/pool initialisation.  When a lattice
+// perturbation of total norm 1e-12, and the Lanczos state.  When a lattice
 // symmetry makes A_r block diagonal (a permittivity independent of z decouples the
 // z frequencies), e_M lies in one block and exact Krylov spaces never leave it; the
 // reference escapes through cuFFT rounding noise, which the perturbation stands in
@@ -488,9 +485,6 @@ __global__ void k_lz_init(VecArgs va, LzArgs L) {
   FAME_COUNT_LAUNCH();
   const int slot = blockIdx.z;
   const Slot sl = va.slots[slot];
-  if (blockIdx.x == 0 && threadIdx.x <= L.nstep) L.map[slot * (L.nstep + 1) + threadIdx.x] = threadIdx.x;
-  if (blockIdx.x == 0 && threadIdx.x <= L.nkeep)
-    L.map[va.nslots * (L.nstep + 1) + slot * (L.nkeep + 1) + threadIdx.x] = L.nstep + 1 + threadIdx.x;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     L.lz[slot].converged = 0;
     L.lz[slot].restarts = 0;
@@ -501,7 +495,7 @@ __global__ void k_lz_init(VecArgs va, LzArgs L) {
     L.prof[slot * 3 + 2] = 0;
   }
   if (!sl.active) return;
-  double2* u = L.U + (size_t)slot * L.nphys * L.ustride;  // physical column 0 == logical 0
+  double2* u = ucol(L, slot, 0);
   const int n = 2 * sl.Nd;
   const double eta = 1e-12 / sqrt((double)n);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -517,7 +511,7 @@ __global__ void k_lz_init(VecArgs va, LzArgs L) {
 // (3) If not converged: the lock/purge restart of Lanczos_LockPurge_gpu.cu:7-48
 // (exact shifts = unwanted Ritz values, GVqrrq_g steps, :95-190), applied to an
 // identity matrix G of order nstep+1 instead of to U, so that U is updated later by
-// one product U*G[:, 0..nkeep].
+// one product U*G[:, 0..keep] (k_restart).
 constexpr int kMaxStep = 64;
 
 struct TriArgs {
@@ -803,83 +797,88 @@ __global__ void __launch_bounds__(32) k_tridiag(TriArgs a) {
 }
 
 // ---------------------------------------------------------------- U * G products
-// out[:, c] = sum_r U[:, map[r]] * G[r, c] for c < ncols (G real, column-major,
-// leading dimension ldg).  Used for the restart (lock/purge) and for the Ritz
-// vectors ev = U(:, 0:nstep) z(:, 0:nwant) (Lanczos_Isotropic.cu:93).
-// mode 0: restart (writes into the free physical columns, then remaps)
-// mode 1: Ritz vectors into `out` ([slot][ncols][ustride])
-template <int CH>
-__global__ void __launch_bounds__(256) k_ugemm(VecArgs va, LzArgs L, const double* G, int ldg, int nrows,
-                                               int ncols, int mode, double2* out, int c0) {
+// The restart: U[:, c] = sum_r U[:, r] * G[r, c] for c <= keep, in place (G real, column-major, order
+// nstep + 1).  A CTA holds kRestartRows rows of all nstep + 1 columns in shared memory, so U is read once
+// and needs no second copy: with the products out of place, a slot's basis took nkeep + 1 columns more (of 70 at nwant 10
+// of 40, 28 MB each at 96^3) and U was read once per 8 new columns.  Eight warps share the
+// new columns, a lane to a row, four columns at a time.
+constexpr int kRestartRows = 32;
+inline size_t restart_smem(int nstep, int nkeep) {
+  return sizeof(double2) * kRestartRows * (nstep + 1) + sizeof(double) * (nstep + 1) * (nkeep + 1);
+}
+__global__ void __launch_bounds__(256) k_restart(VecArgs va, LzArgs L, const double* G) {
   FAME_COUNT_LAUNCH();
-  if (mode == 0 && c0 == 0 && (threadIdx.x | blockIdx.x | blockIdx.y | blockIdx.z) == 0) set_cond(va.cond, 0);
+  extern __shared__ __align__(16) unsigned char rsm[];
+  if ((threadIdx.x | blockIdx.x | blockIdx.y | blockIdx.z) == 0) set_cond(va.cond, 0);
+  const int slot = blockIdx.z;
+  const Slot sl = va.slots[slot];
+  if (!sl.active || L.lz[slot].converged) return;
+  const int n1 = L.nstep + 1, nc = L.lz[slot].keep + 1;
+  double2* us = reinterpret_cast<double2*>(rsm);                    // [n1][kRestartRows]
+  double* Gs = reinterpret_cast<double*>(us + kRestartRows * n1);  // [nc][n1]
+  const double* Gg = G + (size_t)slot * n1 * (L.nkeep + 1);
+  for (int q = threadIdx.x; q < n1 * nc; q += blockDim.x) Gs[q] = Gg[q];
+  const int n = 2 * sl.Nd, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double2* U = ucol(L, slot, 0);
+  for (int i0 = blockIdx.x * kRestartRows; i0 < n; i0 += gridDim.x * kRestartRows) {
+    const bool in = i0 + lane < n;
+    __syncthreads();  // the last rows are done with
+    for (int r = warp; r < n1; r += 8)
+      us[r * kRestartRows + lane] = in ? U[(size_t)r * L.ustride + i0 + lane] : make_double2(0.0, 0.0);
+    __syncthreads();
+    for (int c0 = 4 * warp; c0 < nc; c0 += 32) {
+      double2 acc[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) acc[c] = make_double2(0.0, 0.0);
+      for (int r = 0; r < n1; r++) {
+        const double2 u = us[r * kRestartRows + lane];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          const double gv = Gs[min(c0 + c, nc - 1) * n1 + r];
+          acc[c].x += gv * u.x;
+          acc[c].y += gv * u.y;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+        if (in && c0 + c < nc) U[(size_t)(c0 + c) * L.ustride + i0 + lane] = acc[c];
+    }
+  }
+}
+
+// Ritz vectors: out[:, c] = sum_r U[:, r] * Z[r, c] for c < nwant (Z real, column-major, leading dimension
+// nstep), ev = U(:, 0:nstep) z(:, 0:nwant) (Lanczos_Isotropic.cu:93), CH columns from c0 on.
+template <int CH>
+__global__ void __launch_bounds__(256) k_ugemm(VecArgs va, LzArgs L, const double* Z, double2* out, int c0) {
+  FAME_COUNT_LAUNCH();
   const int slot = blockIdx.z;
   const Slot sl = va.slots[slot];
   if (!sl.active) return;
-  if (mode == 0) {
-    if (L.lz[slot].converged) return;
-    ncols = L.lz[slot].keep + 1;
-    if (c0 >= ncols) return;
-  }
-  __shared__ double Gs[(kMaxStep + 1) * CH];
-  __shared__ int cols[kMaxStep + 1];
-  const double* Gg = G + (size_t)slot * ldg * (mode == 0 ? (L.nkeep + 1) : L.nstep);
-  const int nc = min(CH, ncols - c0);
-  for (int q = threadIdx.x; q < nrows * nc; q += blockDim.x) {
-    const int r = q % nrows, c = q / nrows;
-    Gs[r + c * nrows] = Gg[r + (c0 + c) * ldg];
-  }
-  for (int r = threadIdx.x; r < nrows; r += blockDim.x) cols[r] = L.map[slot * (L.nstep + 1) + r];
+  __shared__ double Zs[kMaxStep * CH];
+  const int nrows = L.nstep;
+  const double* Zg = Z + (size_t)slot * nrows * nrows;
+  const int nc = min(CH, L.nwant - c0);
+  for (int q = threadIdx.x; q < nrows * nc; q += blockDim.x) Zs[q] = Zg[q + c0 * nrows];
   __syncthreads();
   const int n = 2 * sl.Nd;
-  const double2* U = L.U + (size_t)slot * L.nphys * L.ustride;
+  const double2* U = ucol(L, slot, 0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double2 acc[CH];
 #pragma unroll
     for (int c = 0; c < CH; c++) acc[c] = make_double2(0.0, 0.0);
     for (int r = 0; r < nrows; r++) {
-      const double2 u = U[(size_t)cols[r] * L.ustride + i];
+      const double2 u = U[(size_t)r * L.ustride + i];
 #pragma unroll
       for (int c = 0; c < CH; c++) {
-        const double gv = Gs[r + c * nrows];
+        const double gv = Zs[r + c * nrows];
         acc[c].x += gv * u.x;
         acc[c].y += gv * u.y;
       }
     }
 #pragma unroll
-    for (int c = 0; c < CH; c++) {
-      if (c < nc) {
-        double2* dst;
-        if (mode == 0) {
-          // free physical column: the pool entries after the logical map
-          const int ph = L.map[va.nslots * (L.nstep + 1) + slot * (L.nkeep + 1) + c0 + c];
-          dst = L.U + ((size_t)slot * L.nphys + ph) * L.ustride;
-        } else {
-          dst = out + ((size_t)slot * ncols + c0 + c) * L.ustride;
-        }
-        dst[i] = acc[c];
-      }
-    }
+    for (int c = 0; c < CH; c++)
+      if (c < nc) out[((size_t)slot * L.nwant + c0 + c) * L.ustride + i] = acc[c];
   }
-}
-
-// After the restart product: logical 0..keep -> the first free columns; the first
-// nstep - keep old columns become logical keep+1..nstep, the others take the freed places
-// of the pool (nkeep + 1 columns).
-__global__ void k_remap(LzArgs L, const Slot* slots, int nslots) {
-  FAME_COUNT_LAUNCH();
-  const int slot = blockIdx.x;
-  if (threadIdx.x != 0 || !slots[slot].active || L.lz[slot].converged) return;
-  int* mp = L.map + slot * (L.nstep + 1);
-  const int keep = L.lz[slot].keep;
-  int* pool = L.map + nslots * (L.nstep + 1) + slot * (L.nkeep + 1);
-  int old[kMaxStep + 1], fr[kMaxStep + 1];
-  for (int c = 0; c <= L.nstep; c++) old[c] = mp[c];
-  for (int c = 0; c <= keep; c++) fr[c] = pool[c];
-  for (int c = 0; c <= keep; c++) mp[c] = fr[c];
-  const int rest = L.nstep - keep;
-  for (int c = 0; c < rest; c++) mp[keep + 1 + c] = old[c];
-  for (int c = 0; c <= keep; c++) pool[c] = old[rest + c];
 }
 
 }  // namespace fame

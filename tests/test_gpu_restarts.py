@@ -1,5 +1,5 @@
 """Lanczos restarts: thick restarts in mixed precision (from a solve's second restart on), slots that restart
-differently often in one batch, and es_maxit as a budget of products."""
+differently often in one batch, the restart product, es_maxit as a budget of products, and the memory a k-point takes."""
 import numpy as np
 import pytest
 
@@ -40,6 +40,25 @@ def test_mixed_restarts_agree_with_fp64(nwant, nstep):
     ctx.close()
 
 
+@pytest.mark.parametrize("nwant,nstep", [(1, 2), (3, 5), (30, 64), (48, 64)])
+def test_restart_product_at_its_edges(nwant, nstep):
+    """Row counts that leave every kind of remainder against the 32-row tiles (2 N = 1386 and, at Gamma, 1384), the
+    smallest and the largest bases; random permittivities, so no bands coincide."""
+    grid = (7, 9, 11)
+    N = int(np.prod(grid))
+    ctx = fb.Context(grid, np.full(3, 1.0 / 7), np.diag([n / 7 for n in grid]).reshape(-1), True)
+    ctx.set_eps(np.random.default_rng(2).uniform(1.0, 13.0, 3 * N))
+    k = np.array([[0.11, -0.23, 0.31], [0.0, 0.0, 0.0]])
+    kw = dict(nwant=nwant, nstep=nstep, es_tol=1e-9, ls_tol=1e-11, es_maxit=1000)
+    f64 = ctx.solve(k, precision=fb.FP64, **kw)
+    mix = ctx.solve(k, precision=fb.MIXED, **kw)
+    assert f64["rc"] == fb.OK and mix["rc"] == fb.OK
+    assert min(c["restarts"] for c in f64["counters"] + mix["counters"]) >= 1
+    assert np.max(np.abs(mix["freq"] - f64["freq"])) < 1e-7 * np.max(f64["freq"])
+    assert max(np.max(f64["relres"]), np.max(mix["relres"])) < 1e-4
+    ctx.close()
+
+
 @pytest.mark.parametrize("nwant,nstep", [(8, 12), (5, 7)])
 def test_es_maxit_allows_what_equal_restarts_would_take(nwant, nstep):
     """A mixed solve gets by with the es_maxit that the FP64 solve, whose restarts all keep nwant vectors, needs."""
@@ -51,3 +70,37 @@ def test_es_maxit_allows_what_equal_restarts_would_take(nwant, nstep):
     # and no more products than the cap stood for
     assert max(c["es_iter"] for c in out["counters"]) <= nstep + need * (nstep - nwant)
     ctx.close()
+
+
+@pytest.mark.parametrize("general", [False, True])
+def test_a_k_point_takes_no_more_memory_than_equal_restarts(general):
+    """A slot's vectors fit what U with nstep + nwant + 2 columns and four FP64 and three FP32 CG vectors took."""
+    n = 64
+    if general:
+        a = np.array([[1.0, 0, 0], [0, 1.0, 0], [0, -0.5, np.sqrt(0.75)]])
+        grid = (n, n, n)
+        h = np.diag(a) / n
+        lat = dict(grid=grid, mesh_len=h, lattice_vec_a=a.reshape(-1), simple=False, m=(0, 0, int(0.5 / h[1] + 0.49), 0),
+                   t1=(0.0, 1.0, 0.0))
+    else:
+        grid = (n, n, n)
+        lat = dict(grid=grid, mesh_len=np.full(3, 1.0 / n), lattice_vec_a=np.eye(3).reshape(-1), simple=True)
+    N, nwant, nstep, nb = n ** 3, 10, 40, 3
+    M = 2 * N
+    old = ((nstep + 1 + nwant + 1) * M + 4 * M + 3 * N + 2 * nwant * M + nwant * 3 * N + M) * 16 + 3 * M * 8 + 3 * N * 8
+    B = np.random.default_rng(1).uniform(1.0, 13.0, 3 * N)
+    k = np.array([[0.1, 0.2, 0.3], [0.11, 0.2, 0.3], [0.12, 0.2, 0.3]])
+    kw = dict(nwant=nwant, nstep=nstep, es_tol=1e-2, ls_tol=1e-2, batch=nb)
+
+    def run():
+        ctx = fb.Context(**lat)
+        ctx.set_eps(B)
+        torch.cuda.synchronize()
+        free0 = torch.cuda.mem_get_info()[0]
+        ctx.solve(k, precision=fb.MIXED, **kw)
+        used = free0 - torch.cuda.mem_get_info()[0]
+        ctx.close()
+        return used
+
+    run()  # code, graphs and the driver's own pools are loaded
+    assert run() <= nb * old + (64 << 20), (nb * old) >> 20
