@@ -450,13 +450,18 @@ __global__ void __launch_bounds__(256) k_lz_update(VecArgs va, LzArgs L, int j) 
   double2* w = ucol(L, slot, j + 1);
   const double2* uj = ucol(L, slot, j);
   const double2* ujm = j > 0 ? ucol(L, slot, j - 1) : uj;
+  const double2* u0 = ucol(L, slot, 0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double2 v = w[i];
     v.x -= al * uj[i].x + be * ujm[i].x;
     v.y -= al * uj[i].y + be * ujm[i].y;
     if (j > 0) {
+      const double2* uc = u0 + i;
+      // (one column at a time: with 4 or 8 loads of a thread in flight the 40 steps of a 96^3 k-point take
+      // 4.82 and 5.09 ms, with 1 or 2 4.57; the resident warps keep DRAM busy)
+#pragma unroll 1
       for (int c = 0; c <= j; c++) {
-        const double2 u = ucol(L, slot, c)[i];
+        const double2 u = uc[c * L.ustride];
         const double2 hc = hs[c];
         v.x -= hc.x * u.x - hc.y * u.y;
         v.y -= hc.x * u.y + hc.y * u.x;
@@ -800,8 +805,9 @@ __global__ void __launch_bounds__(32) k_tridiag(TriArgs a) {
 // The restart: U[:, c] = sum_r U[:, r] * G[r, c] for c <= keep, in place (G real, column-major, order
 // nstep + 1).  A CTA holds kRestartRows rows of all nstep + 1 columns in shared memory, so U is read once
 // and needs no second copy: with the products out of place, a slot's basis took nkeep + 1 columns more (of 70 at nwant 10
-// of 40, 28 MB each at 96^3) and U was read once per 8 new columns.  Eight warps share the
-// new columns, a lane to a row, four columns at a time.
+// of 40, 28 MB each at 96^3) and U was read once per 8 new columns (two restarts of a 96^3 k-point, to 11 and
+// 29 columns: 1.71 ms out of place, 1.38 so).  Eight warps share the new columns, a lane to a row, four
+// columns at a time.
 constexpr int kRestartRows = 32;
 inline size_t restart_smem(int nstep, int nkeep) {
   return sizeof(double2) * kRestartRows * (nstep + 1) + sizeof(double) * (nstep + 1) * (nkeep + 1);
