@@ -1150,7 +1150,7 @@ __global__ void __cluster_dims__(3 * GP::kHalves, 1, 1) __launch_bounds__(GP::te
         st->rr = tot[0];
         st->outer++;
         st->outer_total++;
-        st->outer_active = (tot[0] > a.tol2) && (st->outer < st->outer_max);
+        st->outer_active = (tot[0] > st->otol2) && (st->outer < st->outer_max);
         st->scale = 1.0 / sqrt(tot[0] > 0 ? tot[0] : 1.0);
         __threadfence();
       }

@@ -132,6 +132,7 @@ struct fame_ctx {
   DBuf<Slot> slots;
   DBuf<double2> tabs;
   DBuf<CgState> cg, cg_copy;
+  DBuf<LsParams> ls_prm;  // bounds of an operator apply's A_r^-1
   DBuf<LzState> lz;
   DBuf<double> partials, T0, T1, hcoef, theta, Z, G, stats;
   DBuf<unsigned> counters, tri_ctr;
@@ -154,6 +155,7 @@ struct fame_ctx {
   int contrast_log2 = 4;
   // recorded programs keyed by configuration
   std::map<std::string, std::unique_ptr<Program>> progs;
+  int graphs_recorded = 0;
 };
 
 namespace fame {
@@ -443,8 +445,7 @@ struct Ops {
   }
 
   template <typename R, int EPI, bool PR>
-  void plane_fwd(const cplx<R>* T, cplx<R>* out, int nvec, const cplx<R>* b = nullptr, Cond cond = Cond{},
-                 double tol2 = 0) {
+  void plane_fwd(const cplx<R>* T, cplx<R>* out, int nvec, const cplx<R>* b = nullptr, Cond cond = Cond{}) {
     auto a = plane_args<R, PlaneOutArgs<R>>();
     a.vec_per_slot = nvec;
     a.T = T;
@@ -455,7 +456,6 @@ struct Ops {
     a.counters = c->counters.p;
     a.cond = cond;
     a.nslots = nslots;
-    a.tol2 = tol2;
     int nt = c->template plane_nt<R>((long)g().Ls * nvec * nslots);
     if (g().general) {
       auto k = c->rare == 2 ? k_plane_fwd<R, true, EPI, PR, 2, DynGeom> : k_plane_fwd<R, true, EPI, PR, 0, DynGeom>;
@@ -572,6 +572,7 @@ static void ensure_workspace(fame_ctx* c, int nslots, int nstep, int nwant, bool
   c->tabs.ensure((size_t)nslots * g.tab_stride);
   c->cg.ensure(nslots);
   c->cg_copy.ensure(nslots);
+  c->ls_prm.ensure(1);
   c->lz.ensure(nslots);
   const size_t lzblk = (M + kLzRows - 1) / kLzRows;
   const size_t part = std::max({lzblk * (2 * 64 + 1), (size_t)3 * g.Ls * 2 * 16, (size_t)1184 * 4,
@@ -821,15 +822,14 @@ struct SolveCfg {
   int enorm;     // restore E (norms only) for the reference-scaled residual
   int loop_cap;  // bound on every device loop's trips (0: the defaults)
   double es_tol, ls_tol, inner_tol;
-  double refine_tol;  // plain FP64: refine64_tol
-  int contrast_log2;
+  int contrast_log2;  // plain FP64 with restarts from the true residual (refine64_tol); else 0
 };
 
 static std::string cfg_key(const SolveCfg& s, bool graph) {
   char b[256];
-  snprintf(b, sizeof b, "%d/%d/%d/%d/%d/%d/%d/%d/%d/%.17g/%.17g/%.17g/%.17g/%d/%d/%d", s.nslots, s.nstep, s.nwant,
+  snprintf(b, sizeof b, "%d/%d/%d/%d/%d/%d/%d/%d/%d/%.17g/%.17g/%.17g/%d/%d/%d", s.nslots, s.nstep, s.nwant,
            s.es_maxit, s.ls_maxit, s.mixed, s.vec, s.enorm, s.inner_maxit, s.es_tol, s.ls_tol, s.inner_tol,
-           s.refine_tol, s.refine_tol > 0 ? s.contrast_log2 : 0, (int)graph, s.loop_cap);
+           s.contrast_log2, (int)graph, s.loop_cap);
   return b;
 }
 
@@ -839,35 +839,38 @@ static Cond loop_cond(Program& P, int* flags, int id, int cap, int loop_cap = 0)
   return P.make_cond(flags + id, flags + kTrips + 2 * id, loop_cap > 0 ? std::min(cap, loop_cap) : cap);
 }
 
-// The A_r^-1 product of Lanczos step j in FP64.  With refine_tol (refine64_tol) the CG is restarted from the true
-// residual; its sum y and the right-hand side take the buffers of the Ritz vectors and their images, which are
-// only filled after the last Lanczos step.
-static void emit_invar64(Ops& o, LzArgs L, int j, double ls_tol, int ls_maxit, double refine_tol, int contrast_log2,
+static LsParams ls_params(double ls_tol, int ls_maxit, int contrast_log2) {
+  const double floor = refine64_tol(contrast_log2), round = ldexp(1.0, contrast_log2 - 50);  // 8 contrast 2^-53
+  return {ls_tol * ls_tol, floor * floor, round * round, ls_maxit};
+}
+
+// The A_r^-1 product of Lanczos step j in FP64, bounded by ls, or by *lsp on the device.  `refine`: the CG is
+// restarted from the true residual (refine64_tol); its sum y and the right-hand side take the buffers of
+// the Ritz vectors and their images, which are only filled after the last Lanczos step.
+static void emit_invar64(Ops& o, LzArgs L, int j, const LsParams& ls, const LsParams* lsp, bool refine, int cg_cap,
                          int* flag_base, int loop_cap) {
   fame_ctx* c = o.c;
   Program& P = o.P;
   const long F = 3L * c->g.N;
   const dim3 vgrid(vec_blocks(c, o.nslots), 1, o.nslots), vblk(256);
-  const double tol2 = ls_tol * ls_tol;
-  Cond cc = loop_cond(P, flag_base, kLoopCG, ls_maxit + 2, loop_cap);
-  if (!(refine_tol > 0)) {
-    P.launch(k_invar_pro<false>, vgrid, vblk, 0, o.va(cc), L, j, c->r64.p, c->x64.p, (double2*)nullptr, tol2, ls_maxit);
+  Cond cc = loop_cond(P, flag_base, kLoopCG, cg_cap, loop_cap);
+  if (!refine) {
+    P.launch(k_invar_pro<false>, vgrid, vblk, 0, o.va(cc), L, j, c->r64.p, c->x64.p, (double2*)nullptr, ls, lsp);
     o.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
     P.launch(k_invar_epi<INV_PLAIN>, vgrid, vblk, 0, o.va(Cond{}), L, j, (const double2*)c->x64.p,
              (const double2*)c->x64b.p);
     return;
   }
   double2 *y = c->EV.p, *b = c->AV.p;
-  const double round = ldexp(1.0, contrast_log2 - 50);  // 8 contrast 2^-53
   Cond outer = loop_cond(P, flag_base, kLoopOuter, 42, loop_cap);
-  P.launch(k_invar_pro<true>, vgrid, vblk, 0, o.va(outer), L, j, c->r64.p, y, b, tol2, ls_maxit);
+  P.launch(k_invar_pro<true>, vgrid, vblk, 0, o.va(outer), L, j, c->r64.p, y, b, ls, lsp);
   P.while_loop(outer, [&] {
-    P.launch(k_cg64_init, dim3(1), dim3(32), 0, o.va(cc), refine_tol * refine_tol, round * round, ls_maxit, outer);
+    P.launch(k_cg64_init, dim3(1), dim3(32), 0, o.va(cc), ls, lsp, outer);
     o.cg_solve<double>({c->r64b.p, c->r64.p}, {c->x64b.p, c->x64.p}, c->T64.p, c->ibq64(), cc);
     P.launch(k_cg64_add, vgrid, vblk, 0, o.va(Cond{}), y, (const double2*)c->x64.p, (const double2*)c->x64b.p);
     o.plane_inv_vec<double, false>(y, c->T64.p, 1, 0);
     o.pencil<double, PEN_QBQ>(c->T64.p, 1, F, c->ibq64(), 2);
-    o.plane_fwd<double, EPI_RESID, false>(c->T64.p, c->r64.p, 1, b, outer, tol2);
+    o.plane_fwd<double, EPI_RESID, false>(c->T64.p, c->r64.p, 1, b, outer);
   });
   P.launch(k_invar_epi<INV_REFINE64>, vgrid, vblk, 0, o.va(Cond{}), L, j, (const double2*)y, (const double2*)nullptr);
 }
@@ -879,17 +882,17 @@ static void emit_step(Ops& o, const SolveCfg& s, LzArgs L, int j, int* flag_base
   const int nvb = vec_blocks(c, s.nslots);
   const long M = 2L * g.N;
   const long F = 3L * g.N;
-  const double tol2 = s.ls_tol * s.ls_tol;
+  const LsParams ls = ls_params(s.ls_tol, s.ls_maxit, s.contrast_log2);
   if (!s.mixed) {
-    emit_invar64(o, L, j, s.ls_tol, s.ls_maxit, s.refine_tol, s.contrast_log2, flag_base, s.loop_cap);
+    emit_invar64(o, L, j, ls, nullptr, s.contrast_log2 > 0, s.ls_maxit + 2, flag_base, s.loop_cap);
   } else {
     Cond outer = loop_cond(P, flag_base, kLoopOuter, 42, s.loop_cap);
     Cond inner = loop_cond(P, flag_base, kLoopInner, s.inner_maxit + 2, s.loop_cap);
     P.launch(k_invar_pro<true>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(outer), L, j, c->r64.p, c->x64.p,
-             c->b64.p, tol2, s.ls_maxit);
+             c->b64.p, ls, (const LsParams*)nullptr);
     P.while_loop(outer, [&] {
       P.launch(k_cg32_init, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(inner), (const double2*)c->r64.p,
-               c->r32.p, s.inner_tol * s.inner_tol, s.inner_maxit, tol2, outer);
+               c->r32.p, s.inner_tol * s.inner_tol, s.inner_maxit, ls.tol2, outer);
       o.cg_solve<float>({c->r32b.p, c->r32.p}, {c->x32b.p, c->x32.p}, c->T32.p, c->ibq32(), inner);
       auto a = o.plane_args<double, PlaneInArgs<double>>();
       a.y64 = c->x64.p;
@@ -897,7 +900,7 @@ static void emit_step(Ops& o, const SolveCfg& s, LzArgs L, int j, int* flag_base
       a.x32[1] = c->x32.p;
       o.plane_inv<double, IN_REFINE, false>(a, c->T64.p, 1);
       o.pencil<double, PEN_QBQ>(c->T64.p, 1, F, c->ibq64(), 2);
-      o.plane_fwd<double, EPI_RESID, false>(c->T64.p, c->r64.p, 1, c->b64.p, outer, tol2);
+      o.plane_fwd<double, EPI_RESID, false>(c->T64.p, c->r64.p, 1, c->b64.p, outer);
     });
     P.launch(k_invar_epi<INV_MIXED>, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L, j,
              (const double2*)c->x64.p, (const double2*)nullptr);
@@ -929,7 +932,7 @@ static void record_solve(fame_ctx* c, Program& P, const SolveCfg& s) {
   L.status = c->status.p;
   int* flags = c->flags.p;
   o.tables(true, s.mixed);
-  P.launch(k_lz_init, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L);
+  P.launch(k_lz_init, dim3(nvb, 1, s.nslots), dim3(256), 0, o.va(Cond{}), L, (LsParams*)nullptr, LsParams{});
   for (int j = 0; j < s.nstep; j++) emit_step(o, s, L, j, flags);
   Cond restart = loop_cond(P, flags, kLoopRestart, max_restarts + 2, s.loop_cap);
   TriArgs ta;
@@ -1090,6 +1093,7 @@ void fame_ctx_destroy(fame_ctx* c) {
   c->slots.release();
   c->cg.release();
   c->cg_copy.release();
+  c->ls_prm.release();
   c->lz.release();
   c->counters.release();
   c->tri_ctr.release();
@@ -1230,8 +1234,7 @@ static int solve_batched(fame_ctx* c, const double* k_xyz, int nk, const fame_so
     s.es_tol = p.es_tol;
     s.ls_tol = p.ls_tol;
     s.inner_tol = p.inner_tol > 0 ? p.inner_tol : default_inner_tol(c->contrast_log2);
-    s.refine_tol = s.mixed ? 0.0 : refine64_tol(c->contrast_log2);
-    s.contrast_log2 = c->contrast_log2;
+    s.contrast_log2 = !s.mixed && refine64_tol(c->contrast_log2) > 0 ? c->contrast_log2 : 0;
     s.inner_maxit = p.inner_maxit > 0 ? p.inner_maxit : 200;
     s.loop_cap = c->loop_cap;
     const bool graph = p.use_graph != 0;
@@ -1244,6 +1247,7 @@ static int solve_batched(fame_ctx* c, const double* k_xyz, int nk, const fame_so
         auto prog = std::make_unique<Program>(c->stream, true, c->hflag, 0);
         record_solve(c, *prog, s);
         prog->instantiate();
+        c->graphs_recorded++;
         P = prog.get();
         c->progs[key] = std::move(prog);
       } else {
@@ -1552,23 +1556,21 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
           L.lz = c->lz.p;
           L.prof = c->prof.p;
           L.status = c->status.p;
-          P.launch(k_lz_init, dim3(1, 1, 1), dim3(256), 0, o.va(Cond{}), L);
+          P.launch(k_lz_init, dim3(1, 1, 1), dim3(256), 0, o.va(Cond{}), L, c->ls_prm.p,
+                   ls_params(prm->ls_tol, prm->ls_maxit, c->contrast_log2));
           FAME_CK(cudaMemcpyAsync(c->U.p, x, 2L * sl.Nd * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
           // the CG as a graph, kept like a solve's (the host's loop waited for the device every
-          // second iteration: hexagonal 36x30x26, 1404 -> 1079 us)
-          const double refine_tol = refine64_tol(c->contrast_log2);
-          char key[96];
-          snprintf(key, sizeof key, "invar/%d/%.17g/%d/%d/%d", prm->ls_maxit, prm->ls_tol, nstep, nwant,
-                   refine_tol > 0 ? c->contrast_log2 : 0);
+          // second iteration: hexagonal 36x30x26, 1404 -> 1079 us); its bounds are read on the device (and end
+          // its loop: the trip cap is no limit here), so that one graph serves every call
+          const bool refine = refine64_tol(c->contrast_log2) > 0;
+          const char* key = refine ? "invar/refine" : "invar";
           auto it = c->progs.find(key);
           if (it == c->progs.end()) {
-            // one such graph at a time: a caller may change the tolerance from call to call
-            for (auto q = c->progs.lower_bound("invar/"); q != c->progs.end() && q->first.compare(0, 6, "invar/") == 0;)
-              q = c->progs.erase(q);
             auto prog = std::make_unique<Program>(c->stream, true, c->hflag, 0);
             Ops og{c, *prog, 1};
-            emit_invar64(og, L, 0, prm->ls_tol, prm->ls_maxit, refine_tol, c->contrast_log2, c->flags.p, 0);
+            emit_invar64(og, L, 0, LsParams{}, c->ls_prm.p, refine, 1 << 30, c->flags.p, 0);
             prog->instantiate();
+            c->graphs_recorded++;
             it = c->progs.emplace(key, std::move(prog)).first;
           }
           it->second->run();
@@ -1689,6 +1691,8 @@ int fame_get_option(fame_ctx* c, const char* name, int* value) {
     *value = c->plane_nt<double>(c->g.Ls);
   } else if (n == "plane_threads32_set" || n == "plane_threads64_set") {
     *value = n == "plane_threads32_set" ? c->threads32_opt : c->threads64_opt;  // 0: by the rule
+  } else if (n == "graphs_recorded") {
+    *value = c->graphs_recorded;
   } else if (n == "static96") {
     *value = c->stat96 ? 1 : 0;
   } else if (n == "general") {

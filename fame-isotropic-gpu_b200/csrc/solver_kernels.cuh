@@ -134,8 +134,11 @@ __device__ __forceinline__ double2* ucol(const LzArgs& L, int slot, int c) {
 
 template <bool REFINE>
 __global__ void __launch_bounds__(256) k_invar_pro(VecArgs va, LzArgs L, int j, double2* r64,
-                                                   double2* x64, double2* b64, double tol2, int maxit) {
+                                                   double2* x64, double2* b64, LsParams ls, const LsParams* lsp) {
   FAME_COUNT_LAUNCH();
+  if (lsp) ls = *lsp;
+  const double tol2 = ls.tol2;
+  const int maxit = ls.maxit;
   const int slot = blockIdx.z;
   const Slot sl = va.slots[slot];
   CgState* st = va.cg + slot;
@@ -249,12 +252,13 @@ __global__ void __launch_bounds__(256) k_cg32_init(VecArgs va, const double2* r6
 
 // FP64 CG with restarts from the true residual, for a permittivity contrast beyond 32
 // (refine64_tol): the start of one CG solve, from r64 = b - A y (r64 is the CG's start residual as it
-// stands).  It ends at ls_tol or after a reduction by `floor2` (squared), where the three-term recurrences stop
-// being worth more; maxit bounds the products over all restarts.  A restart that has not halved the true
+// stands).  It ends at ls_tol or after a reduction by ls.floor2 (squared), where the three-term recurrences stop
+// being worth more; ls.maxit bounds the products over all restarts.  A restart that has not halved the true
 // residual has reached what rounding leaves: that counts as solved where it is within the
-// rounding of the form with search directions, `rounding2` ||b||^2, which could not tell either.
-__global__ void __launch_bounds__(32) k_cg64_init(VecArgs va, double floor2, double rounding2, int maxit, Cond outer_reset) {
+// rounding of the form with search directions, ls.rounding2 ||b||^2, which could not tell either.
+__global__ void __launch_bounds__(32) k_cg64_init(VecArgs va, LsParams ls, const LsParams* lsp, Cond outer_reset) {
   FAME_COUNT_LAUNCH();
+  if (lsp) ls = *lsp;
   if (threadIdx.x == 0) set_cond(outer_reset, 0);
   int any = 0;
   for (int q = threadIdx.x; q < va.nslots; q += 32) {
@@ -264,16 +268,16 @@ __global__ void __launch_bounds__(32) k_cg64_init(VecArgs va, double floor2, dou
     const double rr = st->rr;
     if (st->outer == 0) st->bb = rr;
     const bool halved = st->outer == 0 || rr <= 0.25 * st->rr_old;
-    if (!halved || st->total >= maxit) {
-      st->rounded = !halved && rr <= rounding2 * st->bb;
+    if (!halved || st->total >= ls.maxit) {
+      st->rounded = !halved && rr <= ls.rounding2 * st->bb;
       st->outer_active = 0;
       continue;
     }
     st->rr_old = rr;
     st->r1 = rr;
-    st->tol2 = fmax(st->otol2, floor2 * rr);
+    st->tol2 = fmax(st->otol2, ls.floor2 * rr);
     st->iter = 1;
-    st->maxit = maxit - st->total;
+    st->maxit = ls.maxit - st->total;
     st->active = 1;
     any = 1;
   }
@@ -486,9 +490,11 @@ __device__ __forceinline__ double hash_unit(unsigned long long z) {
 // z frequencies), e_M lies in one block and exact Krylov spaces never leave it; the
 // reference escapes through cuFFT rounding noise, which the perturbation stands in
 // for, so the same lowest bands are found.
-__global__ void k_lz_init(VecArgs va, LzArgs L) {
+// ls_out (an operator apply): where the solve's bounds go, for its graph.
+__global__ void k_lz_init(VecArgs va, LzArgs L, LsParams* ls_out, LsParams ls) {
   FAME_COUNT_LAUNCH();
   const int slot = blockIdx.z;
+  if (ls_out && (threadIdx.x | blockIdx.x | blockIdx.z) == 0) *ls_out = ls;
   const Slot sl = va.slots[slot];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     L.lz[slot].converged = 0;

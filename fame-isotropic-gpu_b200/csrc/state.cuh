@@ -45,6 +45,14 @@ __host__ __device__ __forceinline__ void cg_coefficients(const CgState& st, doub
   }
 }
 
+// What bounds an A_r^-1 solve: by value in a solve's graph, from device memory in the graph of the
+// operator apply, which serves every tolerance and product cap.
+struct LsParams {
+  double tol2;               // ls_tol^2
+  double floor2, rounding2;  // FP64 with restarts: k_cg64_init
+  int maxit;
+};
+
 struct LzState {
   int converged;
   int restarts;
@@ -212,7 +220,6 @@ struct PlaneOutArgs {
   unsigned* counters;      // [nslots] ticket counters, plus [nslots] = grid counter
   Cond cond;               // EPI_RESID: outer WHILE condition
   int nslots;
-  double tol2;             // EPI_RESID: absolute tolerance^2 on ||b - A y||
 };
 
 // Ordered sum of p[0], p[stride], ..., p[(n - 1) stride] by one warp (lane-strided,

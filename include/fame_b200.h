@@ -218,8 +218,9 @@ int fame_set_loop_cap(fame_ctx* ctx, int max_trips);
  *                      it no longer needs; a call whose lane contexts cannot be created
  *                      runs as one batch.
  * Read-only (fame_get_option): "static96", "general", "grid_x", "grid_y", "grid_z",
- * "level" (the FFT pass level the grid needs), "plane_threads32_set", "plane_threads64_set"
- * (the options above, 0 when the rule decides).  fame_tune picks the first four by timing.
+ * "level" (the FFT pass level the grid needs), "graphs_recorded" (CUDA graphs this context has
+ * recorded so far), "plane_threads32_set", "plane_threads64_set" (the options above, 0 when the
+ * rule decides).  fame_tune picks the first four by timing.
  * Unknown names or values are FAME_ERR_BAD_INPUT.  No counterpart in the reference. */
 int fame_set_option(fame_ctx* ctx, const char* name, int value);
 int fame_get_option(fame_ctx* ctx, const char* name, int* value);
