@@ -11,7 +11,7 @@
 // before every repetition, and keeps the fastest by coordinate descent: radix order,
 // then CTA size, then prefetch, from the context's current options.  The winner is applied to the context and appended to
 // a plain-text cache file under a key of grid, lattice family, precision and batch, so
-// a later run with the same key applies it without timing.
+// a later run with the same key and plan version applies it without timing.
 //
 // Built only on the public C ABI (include/fame_b200.h).
 #include <stdio.h>
@@ -34,16 +34,22 @@ struct Plan {
   int radix_order = 0, threads32 = 0, threads64 = 0, prefetch = 1;
 };
 
+// What the numbers of a plan stand for: to be raised when radix orders, thread options or the kernels
+// they were timed on change.  Lines without it (the first version) or with another are passed over.
+constexpr int kPlanVersion = 2;
+
 std::string plan_text(const Plan& p) {
   char b[160];
-  snprintf(b, sizeof b, "radix_order=%d plane_threads32=%d plane_threads64=%d prefetch=%d", p.radix_order,
-           p.threads32, p.threads64, p.prefetch);
+  snprintf(b, sizeof b, "radix_order=%d plane_threads32=%d plane_threads64=%d prefetch=%d plans=%d", p.radix_order,
+           p.threads32, p.threads64, p.prefetch, kPlanVersion);
   return b;
 }
 
 bool parse_plan(const std::string& s, Plan& p) {
-  return sscanf(s.c_str(), "radix_order=%d plane_threads32=%d plane_threads64=%d prefetch=%d", &p.radix_order,
-                &p.threads32, &p.threads64, &p.prefetch) == 4;
+  int version = 0;
+  return sscanf(s.c_str(), "radix_order=%d plane_threads32=%d plane_threads64=%d prefetch=%d plans=%d", &p.radix_order,
+                &p.threads32, &p.threads64, &p.prefetch, &version) == 5 &&
+         version == kPlanVersion;
 }
 
 int apply(fame_ctx* c, const Plan& p) {

@@ -231,7 +231,8 @@ int fame_get_option(fame_ctx* ctx, const char* name, int* value);
  * repetition): one FP32 CG iteration for FAME_MIXED, one FP64 Q_r^* B^-1 Q_r apply for
  * FAME_FP64.  The winner is applied to the context.  cache_file (or NULL): a text
  * file of "key | plan" lines, key = grid, lattice family, precision and batch; a
- * cached plan is applied without timing, a new one is appended.  plan_out (or NULL)
+ * cached plan is applied without timing, a new one is appended (lines of another version of the
+ * plans are passed over).  plan_out (or NULL)
  * receives the plan as text.  Replaces the fixed cuFFT plans of the reference
  * (FAME_Main/FAME_Create_cublas.cu:16-25). */
 int fame_tune(fame_ctx* ctx, const double* k, int precision, int batch, const char* cache_file, char* plan_out,
