@@ -166,6 +166,16 @@ def _check_device_tensor(t, name, dtype, numel, device):
         raise ValueError(f"{name} must have {numel} elements (got {t.numel()})")
 
 
+def _wait_for_caller(device):
+    """Waits for the work queued on the caller's current torch stream: the context runs on a
+    stream of its own, which is not ordered after it, and reads or overwrites the caller's
+    tensors.  (An idle stream, the usual case, only costs the query.)"""
+    import torch
+    s = torch.cuda.current_stream(device)
+    if not s.query():
+        s.synchronize()
+
+
 def make_lattice(grid, mesh_len, lattice_vec_a, simple, m=(0, 0, 0, 0), t1=(0.0, 0.0, 0.0)):
     L = Lattice()
     L.grid[:] = [int(v) for v in grid]
@@ -223,6 +233,7 @@ class Context:
         context's device (stays on the GPU)."""
         import torch
         _check_device_tensor(B, "B", torch.float64, 3 * self.N, self.device)
+        _wait_for_caller(self.device)
         _check(load().fame_set_eps_device(self._h, C.c_void_p(B.data_ptr())))
 
     def set_material(self, binout, material_num, eps_in, eps_out):
@@ -269,8 +280,9 @@ class Context:
     def apply(self, op, k, x, y, precision=FP64, params=None):
         """Applies operator `op` at wave vector k to device buffers x -> y (contiguous
         torch CUDA tensors on the context's device, complex128 for FP64 / complex64 for
-        MIXED; reduced vectors have 2*Nd elements, fields 3N).  Returns Nd.  Raises
-        ValueError on a tensor of the wrong device, type, layout or size."""
+        MIXED; reduced vectors have 2*Nd elements, fields 3N), after the work queued on the
+        current torch stream.  Returns Nd.  Raises ValueError on a tensor of the wrong device,
+        type, layout or size."""
         import torch
         kk = np.ascontiguousarray(np.asarray(k, dtype=np.float64))
         Nd = reduced_size(self._lat, kk)
@@ -281,6 +293,7 @@ class Context:
         _check_device_tensor(y, "y", dt, n_out, self.device)
         nd = C.c_int()
         p = params or solver_params()
+        _wait_for_caller(self.device)
         _check(load().fame_apply(self._h, int(op), _dptr(kk), C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr()),
                                  int(precision), C.byref(p), C.byref(nd)))
         return nd.value
@@ -348,6 +361,7 @@ class Context:
         if out is None:
             out = torch.empty(self.N, dtype=torch.float64, device=f"cuda:{self.device}")
         _check_device_tensor(out, "out", torch.float64, self.N, self.device)
+        _wait_for_caller(self.device)
         _check(load().fame_adjoint_vjp(self._h, int(kidx), _dptr(f), _dptr(g), f.size, float(rel_gap),
                                        C.c_void_p(out.data_ptr())))
         return out

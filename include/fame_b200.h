@@ -147,6 +147,9 @@ int fame_solve_kpoints(fame_ctx* ctx, const double* k_xyz, int nk, const fame_so
  * in/out are device pointers of length given in the FAME_OP_* comments.
  * precision: FAME_FP64 (complex128 buffers) or FAME_MIXED (complex64 buffers, not
  * for FAME_OP_INVAR).  For FAME_OP_INVAR ls_tol / ls_maxit come from `params`.
+ * The work runs on the context's own stream, which does not wait for other streams, and has ended
+ * when the call returns: `in` must be complete, and nothing may still use `out`, when it is made (so
+ * for the device buffers of fame_set_eps_device and fame_adjoint_vjp).
  * Returns Nd through *Nd_out when not NULL. */
 int fame_apply(fame_ctx* ctx, int op, const double* k_xyz, const void* in, void* out, int precision,
                const fame_solver_params* params, int* Nd_out);
