@@ -1485,8 +1485,8 @@ int fame_solve_kpoints(fame_ctx* c, const double* k_xyz, int nk, const fame_solv
   return out;
 }
 
-int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, int precision,
-               const fame_solver_params* prm, int* Nd_out) {
+static int apply_op(fame_ctx* c, int op, const double* k, const void* in, void* out, int precision,
+                    const fame_solver_params* prm, int* Nd_out, const cudaStream_t* after) {
   if (!c || !k || !in || !out) {
     set_err("null argument");
     return FAME_ERR_BAD_INPUT;
@@ -1516,6 +1516,15 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
     const Geom& g = c->g;
     const long M = 2L * g.N, F = 3L * g.N;
     o.tables(precision == FAME_FP64, precision == FAME_MIXED, &sl);
+    if (after) {  // behind the table kernel, which does not touch the caller's buffers
+      const cudaError_t q = cudaStreamQuery(*after);
+      if (q == cudaErrorNotReady) {
+        cudaGetLastError();
+        FAME_CK(cudaStreamSynchronize(*after));
+      } else {
+        FAME_CK(q);
+      }
+    }
     if (precision == FAME_FP64) {
       const double2* x = (const double2*)in;
       double2* y = (double2*)out;
@@ -1618,6 +1627,17 @@ int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, 
     return FAME_ERR_WATCHDOG;
   }
   return FAME_OK;
+}
+
+int fame_apply(fame_ctx* c, int op, const double* k, const void* in, void* out, int precision,
+               const fame_solver_params* prm, int* Nd_out) {
+  return apply_op(c, op, k, in, out, precision, prm, Nd_out, nullptr);
+}
+
+int fame_apply_after(fame_ctx* c, int op, const double* k, const void* in, void* out, int precision,
+                     const fame_solver_params* prm, int* Nd_out, void* stream) {
+  const cudaStream_t st = (cudaStream_t)stream;
+  return apply_op(c, op, k, in, out, precision, prm, Nd_out, &st);
 }
 
 void* fame_ctx_stream(fame_ctx* c) { return c ? (void*)c->stream : nullptr; }

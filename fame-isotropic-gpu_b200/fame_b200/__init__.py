@@ -28,8 +28,8 @@ OP_QR, OP_QRS, OP_QBQ, OP_PR, OP_PRS, OP_INVAR = range(6)
 
 # every symbol declared in include/fame_b200.h
 EXPORTS = ("fame_ctx_create", "fame_ctx_destroy", "fame_set_eps", "fame_set_material", "fame_solve_kpoints",
-           "fame_apply", "fame_adjoint", "fame_ctx_sizes", "fame_last_error", "fame_version", "fame_ctx_stream",
-           "fame_launch_count", "fame_bench_qbq", "fame_qbq_static", "fame_material_locate",
+           "fame_apply", "fame_apply_after", "fame_adjoint", "fame_ctx_sizes", "fame_last_error", "fame_version",
+           "fame_ctx_stream", "fame_launch_count", "fame_bench_qbq", "fame_qbq_static", "fame_material_locate",
            "fame_write_eigenvectors", "fame_writer_start", "fame_writer_finish", "fame_set_loop_cap",
            "fame_bench_cg", "fame_set_eps_device", "fame_adjoint_vjp", "fame_set_option", "fame_get_option",
            "fame_tune")
@@ -93,6 +93,7 @@ def load():
     lib.fame_set_material.argtypes = [P, C.POINTER(C.c_int), C.c_int, D, C.c_double]
     lib.fame_solve_kpoints.argtypes = [P, D, C.c_int, C.POINTER(SolverParams), D, D, D, D, D, C.POINTER(KCounters)]
     lib.fame_apply.argtypes = [P, C.c_int, D, P, P, C.c_int, C.POINTER(SolverParams), C.POINTER(C.c_int)]
+    lib.fame_apply_after.argtypes = [*lib.fame_apply.argtypes, P]
     lib.fame_adjoint.argtypes = [P, D, D, C.c_int, C.c_int, D]
     lib.fame_ctx_sizes.argtypes = [P, C.POINTER(C.c_longlong)]
     lib.fame_ctx_stream.argtypes = [P]
@@ -115,7 +116,8 @@ def load():
     lib.fame_last_error.restype = C.c_char_p
     lib.fame_version.restype = C.c_char_p
     for fn in ("fame_ctx_create", "fame_set_eps", "fame_set_material", "fame_solve_kpoints", "fame_apply",
-               "fame_adjoint", "fame_ctx_sizes", "fame_launch_count", "fame_bench_qbq", "fame_qbq_static",
+               "fame_apply_after", "fame_adjoint", "fame_ctx_sizes", "fame_launch_count", "fame_bench_qbq",
+               "fame_qbq_static",
                "fame_material_locate", "fame_write_eigenvectors", "fame_writer_start", "fame_writer_finish",
                "fame_set_loop_cap", "fame_bench_cg", "fame_set_eps_device", "fame_adjoint_vjp",
                "fame_set_option", "fame_get_option", "fame_tune"):
@@ -293,9 +295,9 @@ class Context:
         _check_device_tensor(y, "y", dt, n_out, self.device)
         nd = C.c_int()
         p = params or solver_params()
-        _wait_for_caller(self.device)
-        _check(load().fame_apply(self._h, int(op), _dptr(kk), C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr()),
-                                 int(precision), C.byref(p), C.byref(nd)))
+        _check(load().fame_apply_after(self._h, int(op), _dptr(kk), C.c_void_p(x.data_ptr()),
+                                       C.c_void_p(y.data_ptr()), int(precision), C.byref(p), C.byref(nd),
+                                       C.c_void_p(torch._C._cuda_getCurrentRawStream(self.device))))
         return nd.value
 
     def set_loop_cap(self, max_trips):

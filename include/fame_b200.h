@@ -154,6 +154,11 @@ int fame_solve_kpoints(fame_ctx* ctx, const double* k_xyz, int nk, const fame_so
 int fame_apply(fame_ctx* ctx, int op, const double* k_xyz, const void* in, void* out, int precision,
                const fame_solver_params* params, int* Nd_out);
 
+/* The same, after the work queued so far on `stream` (a cudaStream_t of the context's device, NULL: the
+ * legacy default stream), which may still write `in` or use `out`. */
+int fame_apply_after(fame_ctx* ctx, int op, const double* k_xyz, const void* in, void* out, int precision,
+                     const fame_solver_params* params, int* Nd_out, void* stream);
+
 /* Hellmann-Feynman adjoint for the isotropic problem C^H C E = w^2 B E:
  * dw_i/dB_e = -(w_i/2) |E_i,e|^2 / (E_i^H B E_i) for every edge e, summed over the
  * three edges of each voxel (B_x = B_y = B_z = eps per voxel).  evec is the
