@@ -206,15 +206,26 @@ def cpu_baseline(W, counters):
 
 def solve_bytes(counters, N, nwant, nstep, mixed):
     """Algorithmic HBM bytes of a band solve, summed from its per-k counters: every
-    FP32 (mixed) or FP64 CG iteration moves B_QBQ + 7M.s (operator: x in, the field out
-    of Q_r and into Q_r^*, y out, 1/eps; CG vectors: read r, p, x, Ap, write x, r, p),
+    FP32 (mixed) or FP64 CG iteration counts as the textbook form with search directions,
+    B_QBQ + 7M.s with B_QBQ = (2M + 6N).s + 3N.r (operator: x in, the field out
+    of Q_r and into Q_r^*, y out, 1/eps; CG vectors: read r, p, x, Ap, write x, r, p; the form that
+    runs needs less, cg_iter_bytes),
     every FP64 refinement step B_QBQ(FP64) + 3M.16, Lanczos step j 4M.16 + 2(j+1)M.16
-    (the CGS pass reads U twice), every restart (nstep + 1 + nwant + 1)M.16 (U times the
+    (the CGS pass reads U twice), every restart (nstep + 1 + kept + 1)M.16 (U times the
     rotation), and the restoration nwant(M + 6N).16, with M = 2N complex values per
     reduced vector, s = 8 (FP32) or 16 bytes per complex value.  Lanczos step t of a k
-    has j = t for t < nstep and j = nwant + (t - nstep) mod (nstep - nwant) after a
-    restart."""
+    has j = t for t < nstep; each restart then continues at j = kept: nwant vectors at
+    the first, and in mixed precision nwant + 3 (nstep - nwant) // 5 at the others."""
     M = 2 * N
+    nkeep = nwant + (nstep - nwant) * 3 // 5 if mixed else nwant
+
+    def lz_step(t):
+        if t < nstep:
+            return t
+        t -= nstep
+        if t < nstep - nwant:
+            return nwant + t
+        return nkeep + (t - (nstep - nwant)) % (nstep - nkeep)
 
     def qbq(s, r):
         return (2 * M + 6 * N) * s + 3 * N * r
@@ -225,9 +236,10 @@ def solve_bytes(counters, N, nwant, nstep, mixed):
         b = c["ls_iter"] * (qbq(s, r) + 7 * M * s)
         if mixed:
             b += c.get("refine", 0) * (qbq(16, 8) + 3 * M * 16)
-        js = sum(1 + (t if t < nstep else nwant + (t - nstep) % (nstep - nwant)) for t in range(c["es_iter"]))
+        js = sum(1 + lz_step(t) for t in range(c["es_iter"]))
         b += c["es_iter"] * 4 * M * 16 + 2 * js * M * 16
-        b += c.get("restarts", 0) * (nstep + 1 + nwant + 1) * M * 16
+        rs = c.get("restarts", 0)
+        b += (min(rs, 1) * (nstep + 1 + nwant + 1) + max(rs - 1, 0) * (nstep + 1 + nkeep + 1)) * M * 16
         b += nwant * (M + 6 * N) * 16
         total += b
     return total
@@ -346,7 +358,7 @@ def run_ours(args):
             "stage_ms": [round(x, 5) for x in stages],
             "stage_GBps": [round(b / (t * 1e-3) / 1e9, 1) for b, t in zip(stage_bytes, stages)],
             "l2": "flushed (256 MiB write) before every launch"}
-    # ---- the dominant work of the mixed solve: one FP32 CG iteration (3 fused kernels)
+    # ---- the dominant work of the mixed solve: one FP32 CG iteration (2 fused kernels)
     # on a batch of nb k-points; the line's `roofline` is this one, the QBQ apply beside it
     if prec == fb.MIXED:
         roof_qbq = roof
@@ -403,7 +415,8 @@ def run_ours(args):
         solve_roof = {"bound": "hbm", "algorithmic_bytes_per_step": int(sb), "seconds_per_step": round(t_step, 4),
                       "achieved": round(sb / t_step / 1e9, 1), "peak": hbm, "unit": "GB/s",
                       "frac": round(sb / t_step / 1e9 / hbm, 4),
-                      "counts": "CG iterations, FP64 refinements, Lanczos steps, restarts, restoration (bench.solve_bytes)"}
+                      "counts": "CG iterations (textbook form with search directions), FP64 refinements, Lanczos steps, "
+                                "restarts, restoration (bench.solve_bytes)"}
     except (KeyError, TypeError, ValueError, ZeroDivisionError):
         solve_roof = None
     cpu = None
@@ -437,14 +450,13 @@ def run_ours(args):
 
 
 def cg_iter_bytes(N):
-    """Algorithmic bytes of one FP32 CG iteration per k-point, B_QBQ + 7M.s with
-    B_QBQ = (2M + 6N).s + 3N.r: the operator's vector in and out, the field out of Q_r
-    and into Q_r^* (one read and one write of the 3-component field per 3-D transform),
-    1/eps, and the CG vectors (read r, p, x, Ap; write x, r, p), s = 8, r = 4.  The
-    kernels move a different set (cg_stage_bytes): r, r_old, x, x_old for r, p, x, Ap, two of
-    them written instead of three, and one more round trip of the field between the stages."""
+    """Algorithmic bytes of one FP32 CG iteration per k-point in the three-term form that runs:
+    the field out of Q_r and into Q_r^* (6N.s, one read and one write of the 3-component field
+    between the two), 1/eps (3N.r), and the vectors (6M.s: read r, r_old, x, x_old, write r, x; the
+    operator's input is r, its output stays in registers), s = 8, r = 4.  The kernels move one more
+    round trip of the field between the stages (cg_stage_bytes)."""
     M = 2 * N
-    return (2 * M + 6 * N) * 8 + 3 * N * 4 + 7 * M * 8
+    return 6 * N * 8 + 3 * N * 4 + 6 * M * 8
 
 
 def cg_stage_bytes(N):

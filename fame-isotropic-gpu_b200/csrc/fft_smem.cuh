@@ -629,8 +629,10 @@ __device__ __forceinline__ bool prime_pass(cplx<R>* buf, int n, int r, int Ns, L
 // two) for MU * ML * 2 complex multiply-adds, so shared memory bounds the pass until the
 // block is as large as the registers allow.
 // FP64 takes 4 x 2 in the pencil stage (92 = 4 x 23 points: 47.4 -> 36.2 us per k-point) and in the
-// static plans (hexagonal 128 operator 397 -> 363), not in the runtime plane stages, where it
-// spills (51x43x37 operator 34.3 -> 37.1).  FP32: 5 x 4 on the 107-point axis is one round instead
+// static plans (hexagonal 128 operator 397 -> 363), not in the runtime plane stages (51x43x37 operator
+// 34.3 -> 37.1).  The line is what was measured: at 128 registers 4 x 2 spills in all of them (32 to
+// 200 bytes a thread in the pencils, 8 to 20 in the static hexagonal planes), and where the halved
+// shared-memory reads outweigh that it stays.  FP32: 5 x 4 on the 107-point axis is one round instead
 // of two, but slower where the launch leaves SMs with one CTA (plane stage, one k-point: 186 ->
 // 201 us; four: 150 -> 148).
 template <typename R, bool LARGE> struct PrimeBlock { static constexpr int mu = 4, ml = 3; };

@@ -160,7 +160,7 @@ struct StatGeom {
 
 // 96^3.  FP32: three plane CTAs of 192 threads per SM.  An FP64 plane is 149 KB, one CTA per SM, and one
 // k-point is then three rounds of clusters (45 of 96 at a time); with halves (75 KB) it is
-// again three CTAs of 192 threads per SM: FP64 operator 151.9 -> 132.9 us (one k-point), 105.2 -> 93.6
+// again three CTAs of 192 threads per SM: FP64 operator 151.9 -> 133.9 us (one k-point), 105.9 -> 94.1
 // (ten).  256 threads, at two or three CTAs per SM, 149.5 and 142.5; 128 threads 142.0.
 template <typename R> using Stat96 = StatGeom<96, 96, 96, 192, 3, sizeof(R) == 4 ? 1 : 2>;
 // The CG plane stage keeps whole planes in FP64: at the 96 registers of three CTAs a thread has one point of the

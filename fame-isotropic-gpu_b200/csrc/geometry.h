@@ -184,6 +184,9 @@ inline int stage_threads(long work, long ctas, size_t smem, int sm_threads, int 
   constexpr int kSMs = 148;
   constexpr size_t kSmemSM = 228 * 1024, kSmemCta = 1024;
   lo = std::max(64, (lo + 31) / 32 * 32);
+  // At most 24 elements a thread up to 192 threads.  It cuts both ways (us per k-point with and without, FP32
+  // CG iteration at 12 k-points): 45x66x50 14.8 and 15.8, 92x80x75 at four 74.5 and 75.8, but 50x63x45 15.2
+  // and 13.6, 64^3 21.3 and 19.8: the model has no term for the passes' rounds, which decide here.
   lo = (int)std::max<long>(lo, std::min<long>(std::min(192, hi), (work / 24 + 31) / 32 * 32));
   hi = (int)std::max<long>(lo, std::min<long>(hi, (work / 8 + 31) / 32 * 32));
   int best = lo;

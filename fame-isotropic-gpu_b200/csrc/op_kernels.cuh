@@ -33,8 +33,8 @@ template <typename R, bool GEN> __device__ __forceinline__ cplx<R> lam_plane(con
 
 // ------------------------------------------------------------------ L2 prefetch
 // The CTAs of a stage kernel run in waves in launch order, and each one spends most of
-// its time on shared-memory transforms.  A CTA therefore issues, at its start, bulk L2
-// prefetches of the global operands of the CTA pf_dist places later (about one wave
+// its time on shared-memory transforms.  With the option "prefetch" a CTA of the CG's pencil stage
+// issues bulk L2 prefetches of the global operands of the CTA pf_dist places later (about one wave
 // ahead), so that CTA finds them in L2 instead of waiting on DRAM.  The prefetches only
 // cover bytes that CTA will read.
 

@@ -88,9 +88,9 @@ struct fame_ctx {
   Geom g;
   cudaStream_t stream = nullptr;
   int pipe_ctas64 = 0;  // resident k_pencil_pipe<double> CTAs on the device
-  int prefetch = 0;     // L2 prefetch one wave ahead in the CG stage kernels (fame_set_option; measured slower)
-  int self_prefetch = 1;  // CG plane stages: L2 prefetch of the CTA's own operands at its start
-  int radix_order = 0;  // kRadixOrders index of the runtime-geometry axis plans
+  int prefetch = 0;     // L2 prefetch one wave ahead in the CG's pencil stage (fame_set_option; measured slower)
+  int self_prefetch = 1;  // CG plane stage: L2 prefetch of the CTA's own vectors, once its plane has arrived
+  int radix_order = 0;  // of the runtime-geometry axis plans (factor_axis)
   int threads32_opt = 0, threads64_opt = 0;  // plane CTA sizes set by fame_set_option (0: rule)
   // threads of a runtime-geometry plane CTA in a launch of `planes` planes (an option below what
   // the axis plans need is raised to it)

@@ -343,8 +343,8 @@ class Context:
         return ms.value, st
 
     def bench_cg(self, k, reps=20, nbatch=1):
-        """Mean device ms of one FP32 CG iteration (its three kernels, L2 flushed
-        before each) on a batch of nbatch k-points, and of each kernel."""
+        """Mean device ms of one FP32 CG iteration (its two kernels, L2 flushed before
+        it) on a batch of nbatch k-points, and of each kernel (the third entry is empty)."""
         kk = np.ascontiguousarray(np.asarray(k, dtype=np.float64))
         ms = C.c_double()
         st = np.zeros(3)
